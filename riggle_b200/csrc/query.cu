@@ -721,8 +721,22 @@ struct SweepParams {
     const uint2* tab2;       // rank tables, bin b = (#starts, #ends) below b << shift
     uint64_t item_cap;
     uint32_t rows, D, chunk;
+    uint32_t spread;         // work items wanted at least (0: items of exactly `chunk` positions)
     int smem_tally;          // 1: one row, shared-memory histograms
 };
+
+// Positions per work item of a work space of `total` positions: `chunk`, or fewer where that would
+// leave fewer than `spread` items, in whole pair-sweep steps of 128 and at least one.  A run's totals
+// are known only on the device, so every kernel that walks the items computes this for itself.
+// Without it a small work space runs on a few warps, one step after the other: the 272 thousand
+// candidates of 37 rows (102 thousand intervals) against 3.2e6 database intervals were 5 block items
+// of 8,192 positions a warp, and the call took 1,306 us; sized so, 534 us.  Work spaces of at least
+// `spread` full items are cut as before (2.1e8 candidates: 1,374 and 1,382 us a call, within noise).
+__host__ __device__ __forceinline__ uint32_t item_size(uint64_t total, uint32_t chunk, uint32_t spread) {
+    if (!spread) return chunk;
+    const uint64_t even = ((total + spread - 1) / spread + 127) & ~127ull;
+    return even < 128 ? (chunk < 128u ? chunk : 128u) : even < chunk ? (uint32_t)even : chunk;
+}
 
 // Galloping (exponential) search from a lower bound: first index in [lo, hi) with a[i] >= x
 // (UPPER = false) or a[i] > x (UPPER = true).  Cost ~2 log2(answer - lo), so a rank found from
@@ -780,7 +794,7 @@ __device__ __forceinline__ uint32_t range_advance(const uint64_t* __restrict__ r
 template <bool PDL>
 __global__ void k_item_ranges(uint32_t* __restrict__ small, const uint32_t* __restrict__ Rp,
                               const uint64_t* __restrict__ rpos, const uint32_t* __restrict__ Lp,
-                              const uint64_t* __restrict__ ppos, uint32_t chunk, uint64_t item_cap,
+                              const uint64_t* __restrict__ ppos, uint32_t chunk, uint32_t spread, uint64_t item_cap,
                               uint32_t* __restrict__ item_r0, uint32_t* __restrict__ item_t0) {
     if constexpr (PDL) {
         pdl_wait();
@@ -794,13 +808,14 @@ __global__ void k_item_ranges(uint32_t* __restrict__ small, const uint32_t* __re
         s64[5] = rtot;
         s64[6] = ptot;
     }
-    const uint64_t ri = min((rtot + chunk - 1) / chunk, item_cap);
-    const uint64_t pi = min((ptot + chunk - 1) / chunk, item_cap);
+    const uint32_t rc = item_size(rtot, chunk, spread), pc = item_size(ptot, chunk, spread);
+    const uint64_t ri = min((rtot + rc - 1) / rc, item_cap);
+    const uint64_t pi = min((ptot + pc - 1) / pc, item_cap);
     for (uint64_t g = g0; g < ri + pi; g += (uint64_t)gridDim.x * blockDim.x) {
         const bool rank = g < ri;
         const uint64_t* a = rank ? rpos : ppos;
         const uint64_t i = rank ? g : g - ri;
-        const uint64_t p = i * chunk;
+        const uint64_t p = i * (rank ? rc : pc);
         uint64_t lo = 0, hi = rank ? R : L;
         while (lo < hi) {
             uint64_t m = (lo + hi + 1) >> 1;
@@ -1043,6 +1058,7 @@ __global__ void __launch_bounds__(256, 5) k_sweep(SweepParams P) {
 
     const uint32_t rcap = *P.rcount;
     const uint64_t total = P.rpos[rcap];
+    P.chunk = item_size(total, P.chunk, P.spread);
     if (P.smem_tally) {
         for (uint32_t k = threadIdx.x; k < P.D; k += blockDim.x) {
             s_cnt[k] = 0;
@@ -1253,6 +1269,7 @@ __global__ void __launch_bounds__(256, MULTI ? 6 : 8) k_pairs(SweepParams P) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t rcap = *P.pcount;
     const uint64_t total = P.ppos[rcap];
+    P.chunk = item_size(total, P.chunk, P.spread);
     if (SMEM)
         for (uint32_t k = threadIdx.x; k < P.D; k += blockDim.x) {
             s_cnt[k] = 0;
@@ -1409,6 +1426,7 @@ struct rgl_context {
     uint64_t last_tot = 0;
     uint32_t last_launches = 0;
     uint32_t last_n = 0;
+    uint32_t last_chunk = 1024, last_spread = 0;  // its work-item size (see item_size)
 };
 
 namespace {
@@ -1554,10 +1572,11 @@ inline unsigned grid_for(uint64_t n, unsigned block) { return (unsigned)((n + bl
 
 struct Launch {
     uint32_t chunk, ctas_per_sm, block, pair_ratio;
+    uint32_t spread;  // see item_size; set per run unless the caller chose the work-item size
 };
 
 Launch pick_launch(const rgl_query_opts* o) {
-    Launch l{1024, 8, 256, 4};
+    Launch l{1024, 8, 256, 4, 0};
     if (o) {
         if (o->chunk) l.chunk = o->chunk;
         if (o->ctas_per_sm) l.ctas_per_sm = o->ctas_per_sm;
@@ -1608,7 +1627,9 @@ int finish(rgl_context* c, const Launch& L, rgl_query_stats* stats) {
         }
         stats->rank_positions = TR;
         stats->pair_candidates = TP;
-        stats->work_items = (TR + L.chunk - 1) / L.chunk + (TP + L.chunk - 1) / L.chunk;
+        const uint32_t rc = item_size(TR, c->last_chunk, c->last_spread);
+        const uint32_t pc = item_size(TP, c->last_chunk, c->last_spread);
+        stats->work_items = (TR + rc - 1) / rc + (TP + pc - 1) / pc;
         stats->sweep_ms = c->last_n ? t_sweep : 0.f;
         stats->device_ms = c->last_n ? t_all : 0.f;
         stats->chunk = L.chunk;
@@ -1792,6 +1813,8 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     // several rows: the block items flush their row histogram, so larger work items pay (measured
     // on the 2e9-interval database: 1024 -> 8192 positions, sweeps 3.45 -> 2.46 s per 4,096 files)
     if (rows > 1 && !(opts && opts->chunk)) L.chunk = kMultiRowChunk;
+    // four work items for every warp of the sweeps' grid, unless the caller set the items' size
+    if (!(opts && opts->chunk)) L.spread = (uint32_t)c->num_sms * L.ctas_per_sm * kCtaItems * 4;
     const bool with_bp = d_bp != nullptr && !(opts && (opts->flags & RGL_QF_NO_OVERLAP));
     const bool ev = mode.events && stats;
     const bool pdl = in.n <= kPdlMaxIntervals;
@@ -1999,7 +2022,7 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
         return RGL_OK;
     }
     (void)launch_chain(pdl, k_item_ranges<true>, k_item_ranges<false>, (unsigned)(c->num_sms * 8), 256, 0, st,
-                     d_small, Rp, c->rpos.as<uint64_t>(), Lp, c->ppos.as<uint64_t>(), L.chunk, kItemCap,
+                     d_small, Rp, c->rpos.as<uint64_t>(), Lp, c->ppos.as<uint64_t>(), L.chunk, L.spread, kItemCap,
                      c->item_r0.as<uint32_t>(), c->item_t0.as<uint32_t>());
     launches++;
     SweepParams P;
@@ -2027,6 +2050,9 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     P.rows = rows;
     P.D = D;
     P.chunk = L.chunk;
+    P.spread = L.spread;
+    c->last_chunk = L.chunk;
+    c->last_spread = L.spread;
     size_t smem = (size_t)D * (with_bp ? 12 : 4);
     // tally: one row in a block-wide histogram for the whole kernel (1); several rows in a histogram
     // of each block item's row (2); else (or with RGL_QF_GLOBAL_TALLY) atomics on the outputs (0)
