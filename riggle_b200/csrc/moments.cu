@@ -56,9 +56,6 @@ __device__ __forceinline__ DD dd_mul_d(DD a, double b) {
     e = fma(a.lo, b, e);
     return dd_two_sum(p, e);
 }
-struct DDAdd {
-    __device__ __forceinline__ DD operator()(const DD& a, const DD& b) const { return dd_add(a, b); }
-};
 
 // ---- K4: impulses ---------------------------------------------------------------------------------
 // Two records per interval end: (bin, impulse), or (n_bins, 0) where there is none.  The start records
@@ -219,28 +216,6 @@ __global__ void k_apply_carry(uint64_t full, const int* __restrict__ count, cons
     }
 }
 
-// ---- K5 ---------------------------------------------------------------------------------------------
-__global__ void k_to_dd(uint64_t n, const float* __restrict__ g, DD* __restrict__ out) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < n) out[i] = DD{(double)g[i], 0.0};
-}
-
-// u = g - gbar into the zero-padded complex FFT input and a DD array (u[N] = 0) for the U scan.
-__global__ void k_center(uint64_t n, uint64_t M, const float* __restrict__ g, const DD* __restrict__ gsum,
-                         double2* __restrict__ x, DD* __restrict__ udd) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= M) return;
-    const double gbar = gsum->hi / (double)n + gsum->lo / (double)n;
-    const double u = i < n ? (double)g[i] - gbar : 0.0;
-    x[i] = make_double2(u, 0.0);
-    if (i <= n) udd[i] = DD{i < n ? u : 0.0, 0.0};
-}
-
-__global__ void k_dd_to_double(uint64_t n, const DD* __restrict__ in, double* __restrict__ out) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < n) out[i] = in[i].hi + in[i].lo;
-}
-
 // ---- K6: Stockham FFT (FP64) ----------------------------------------------------------------------
 // One pass of the out-of-place Stockham formulation (Govindaraju et al., "High performance discrete
 // Fourier transforms on graphics processors", SC 2008): thread j loads R elements at stride M/R,
@@ -313,43 +288,6 @@ __global__ void k_power(uint64_t M, double2* __restrict__ x) {
     }
 }
 
-// ---- K7 -----------------------------------------------------------------------------------------
-enum Term : int { T_A = 0, T_MA = 1, T_U2 = 2, T_V2 = 3, T_U = 4 };
-
-// Scan inputs for the prefix sums: element t of term T (t = 0..len-1).
-__global__ void k_term(uint64_t len, int term, const double2* __restrict__ y, double inv_m,
-                       const double* __restrict__ U, uint64_t n, DD* __restrict__ out) {
-    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (t >= len) return;
-    double v = 0.0;
-    switch (term) {
-        case T_A: v = (t >= 1 && t < n) ? y[t].x * inv_m : 0.0; break;                  // A[t], t >= 1
-        case T_MA: v = (t >= 1 && t < n) ? (double)t * (y[t].x * inv_m) : 0.0; break;  // t A[t]
-        case T_U2: v = (t >= 1 && t <= n) ? U[t] * U[t] : 0.0; break;                    // U[t]^2, t >= 1
-        case T_V2: {                                                                   // (U[N]-U[N-t])^2
-            if (t >= 1 && t < n) {
-                const double d = U[n] - U[n - t];
-                v = d * d;
-            }
-            break;
-        }
-        default: v = (t <= n) ? U[t] : 0.0;  // U[t]
-    }
-    out[t] = DD{v, 0.0};
-}
-
-// Gathers inclusive prefix values at the requested indices (pre[i] = sum of terms 0..i).
-__global__ void k_gather(uint32_t k, const uint64_t* __restrict__ at, const DD* __restrict__ pre, DD* __restrict__ out) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < k) out[i] = pre[at[i]];
-}
-
-// Windows with few positions (nw = N - L + 1 small, L close to N): the window sums F_L(j) then differ
-// from one another by a small part of their size, and any formula that forms the second moment and
-// subtracts the squared mean cancels (the reference's own f64 formula loses all digits there).
-// These L are reduced directly: d_j = F_L(j) - F_L(0) = (U[j+L] - U[j]) - U[L] from the prefix sums
-// U of the centred signal (U[0] = 0), summed with d_j^2 in double-double over the nw windows, and
-// var = sum d^2 / nw - (sum d / nw)^2.  One block per such L; out[i] = var.
 __device__ __forceinline__ DD dd_mul(DD a, DD b) {
     const double p = a.hi * b.hi;
     double e = fma(a.hi, b.hi, -p);
@@ -366,65 +304,11 @@ template <typename UT>
 __device__ __forceinline__ DD u_at(const UT* U, uint64_t i);
 template <>
 __device__ __forceinline__ DD u_at<double>(const double* U, uint64_t i) { return DD{U[i], 0.0}; }
-template <typename UT>
-__global__ void __launch_bounds__(256) k_direct_var(const uint32_t* __restrict__ which, const uint64_t* __restrict__ ls,
-                                                    uint64_t n, const UT* __restrict__ U, double uscale,
-                                                    double* __restrict__ out) {
-    const uint32_t i = which[blockIdx.x];
-    const uint64_t L = ls[i], nw = n - L + 1;
-    const DD uL = u_at<UT>(U, L);
-    DD s1{0.0, 0.0}, s2{0.0, 0.0};
-    for (uint64_t j = threadIdx.x; j < nw; j += blockDim.x) {
-        const DD d = dd_add(dd_add(u_at<UT>(U, j + L), dd_neg(u_at<UT>(U, j))), dd_neg(uL));
-        s1 = dd_add(s1, d);
-        s2 = dd_add(s2, dd_mul(d, d));
-    }
-    __shared__ DD r1[256], r2[256];
-    r1[threadIdx.x] = s1;
-    r2[threadIdx.x] = s2;
-    __syncthreads();
-    for (uint32_t k = blockDim.x / 2; k > 0; k >>= 1) {
-        if (threadIdx.x < k) {
-            r1[threadIdx.x] = dd_add(r1[threadIdx.x], r1[threadIdx.x + k]);
-            r2[threadIdx.x] = dd_add(r2[threadIdx.x], r2[threadIdx.x + k]);
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        const DD m1 = dd_div_d(r1[0], (double)nw), m2 = dd_div_d(r2[0], (double)nw);
-        const DD v = dd_add(m2, dd_neg(dd_mul(m1, m1)));
-        const double var = (v.hi + v.lo) * uscale * uscale;
-        out[i] = var > 0.0 ? var : 0.0;
-    }
-}
 
-__global__ void k_window_moments(uint32_t G, const uint64_t* __restrict__ ls, uint64_t n,
-                                 const DD* __restrict__ gsum, double a0, const DD* __restrict__ P0,
-                                 const DD* __restrict__ P1, const DD* __restrict__ Q, const DD* __restrict__ V,
-                                 const DD* __restrict__ UU_L, const DD* __restrict__ UU_R, DD uu_total,
-                                 float2* __restrict__ out, double* __restrict__ mean_out, double* __restrict__ var_out,
-                                 const double* __restrict__ direct_var) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= G) return;
-    const uint64_t L = ls[i];
-    const double nw = (double)(n - L + 1);
-    const double gbar = gsum->hi / (double)n + gsum->lo / (double)n;
-    // sum_j F_L(j) = (UU(N+1) - UU(L)) - UU(N-L+1)
-    const DD sf = dd_add(dd_add(uu_total, dd_neg(UU_L[i])), dd_neg(UU_R[i]));
-    const double fbar = (sf.hi + sf.lo) / nw;
-    // sum_j F_L(j)^2 = L A[0] + 2 (L P0 - P1) - Q - V
-    DD s2 = DD{(double)L * a0, fma((double)L, a0, -(double)L * a0)};
-    const DD inner = dd_add(dd_mul_d(P0[i], (double)L), dd_neg(P1[i]));
-    s2 = dd_add(s2, dd_mul_d(inner, 2.0));
-    s2 = dd_add(s2, dd_neg(Q[i]));
-    s2 = dd_add(s2, dd_neg(V[i]));
-    const double mean = (double)L * gbar + fbar;
-    double var = (s2.hi + s2.lo) / nw - fbar * fbar;
-    if (!(var > 0.0)) var = 0.0;
-    if (direct_var && direct_var[i] >= 0.0) var = direct_var[i];  // few windows: reduced directly
-    out[i] = make_float2((float)mean, (float)var);
-    if (mean_out) mean_out[i] = mean;
-    if (var_out) var_out[i] = var;
+// A[t] = Re y[t] / M, t < n.
+__global__ void k_autocorr(uint64_t n, const double2* __restrict__ y, double inv_m, double* __restrict__ A) {
+    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (t < n) A[t] = y[t].x * inv_m;
 }
 
 // ---- the compensated-FP32 path (K5-K7 with float-float arithmetic) ------------------------------
@@ -479,9 +363,6 @@ __device__ __forceinline__ CFF cff_sub(CFF a, CFF b) { return CFF{ff_sub(a.re, b
 __device__ __forceinline__ CFF cff_mul(CFF a, CFF b) {
     return CFF{ff_sub(ff_mul(a.re, b.re), ff_mul(a.im, b.im)), ff_add(ff_mul(a.re, b.im), ff_mul(a.im, b.re))};
 }
-struct FFAdd {
-    __device__ __forceinline__ FF operator()(const FF& a, const FF& b) const { return ff_add(a, b); }
-};
 template <>
 __device__ __forceinline__ DD u_at<FF>(const FF* U, uint64_t i) {
     return dd_two_sum((double)U[i].hi, (double)U[i].lo);
@@ -546,31 +427,6 @@ __global__ void __launch_bounds__(128) k_ff_fft_pass(const CFF* __restrict__ in,
     for (int r = 0; r < R; r++) out[base + r * Ns] = v[r];
 }
 
-// u = (g - gbar) 2^-e into the zero-padded complex input (u[N] = 0 for the U scan).
-__global__ void k_ff_center(uint64_t n, uint64_t M, const float* __restrict__ g, const FF* __restrict__ gsum,
-                            float scale, CFF* __restrict__ x, FF* __restrict__ u_out) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= M) return;
-    FF u = FF{0.f, 0.f};
-    if (i < n) {
-        // gbar = gsum / n in float-float: one Newton step on the float quotient
-        const FF S = *gsum;
-        const float q = __fdiv_rn(S.hi, (float)n);
-        const FF qn = ff_mul(FF{q, 0.f}, ff_from_double_exact(n));
-        const FF r = ff_sub(S, qn);
-        const FF gbar = ff_quick(q, __fdiv_rn(r.hi, (float)n));
-        u = ff_sub(FF{g[i], 0.f}, gbar);
-        u = FF{u.hi * scale, u.lo * scale};  // exact: scale is a power of two
-    }
-    x[i] = CFF{u, FF{0.f, 0.f}};
-    if (i <= n) u_out[i] = u;
-}
-
-__global__ void k_ff_from_float(uint64_t n, const float* __restrict__ g, FF* __restrict__ out) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < n) out[i] = FF{g[i], 0.f};
-}
-
 __global__ void k_ff_power(uint64_t M, CFF* __restrict__ x) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i < M) {
@@ -579,49 +435,418 @@ __global__ void k_ff_power(uint64_t M, CFF* __restrict__ x) {
     }
 }
 
-// Scan inputs of the compensated path, as k_term (A[t] = Re Y[t] / M, an exact power-of-two scale).
-__global__ void k_ff_term(uint64_t len, int term, const CFF* __restrict__ y, float inv_m, const FF* __restrict__ U,
-                          uint64_t n, FF* __restrict__ out) {
+__global__ void k_ff_autocorr(uint64_t n, const CFF* __restrict__ y, float inv_m, FF* __restrict__ A) {
     const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (t >= len) return;
-    FF v = FF{0.f, 0.f};
-    switch (term) {
-        case T_A:
-            if (t >= 1 && t < n) v = FF{y[t].re.hi * inv_m, y[t].re.lo * inv_m};
-            break;
-        case T_MA:
-            if (t >= 1 && t < n) v = ff_mul(ff_from_double_exact(t), FF{y[t].re.hi * inv_m, y[t].re.lo * inv_m});
-            break;
-        case T_U2:
-            if (t >= 1 && t <= n) v = ff_mul(U[t], U[t]);
-            break;
-        case T_V2:
-            if (t >= 1 && t < n) {
-                const FF d = ff_sub(U[n], U[n - t]);
-                v = ff_mul(d, d);
-            }
-            break;
-        default:
-            if (t <= n) v = U[t];
-    }
-    out[t] = v;
+    if (t < n) A[t] = FF{y[t].re.hi * inv_m, y[t].re.lo * inv_m};  // exact: inv_m is a power of two
 }
 
-// Inclusive prefix values at the requested indices, widened to double-double and scaled back by
-// the exact power of two 2^sc (the FP64 final reduction starts here).
-__global__ void k_ff_gather(uint32_t k, const uint64_t* __restrict__ at, const FF* __restrict__ pre, int sc,
-                            DD* __restrict__ out) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < k) {
-        const FF v = pre[at[i]];
-        out[i] = DD{ldexp((double)v.hi, sc), ldexp((double)v.lo, sc)};
+// ---- K5, K7: prefix sums at the grid's points ------------------------------------------------------
+// The window moments need prefix sums of five terms (A[t], t A[t], U[t]^2, (U[N] - U[N-t])^2, U[t]) at
+// the grid's ~1,000 points only, so no prefix is written out: one pass sums tiles of the terms, one
+// block per term scans the tile sums, and one block per grid point adds the part of its last tile.
+// Bound: one read of A and U (16 to 24 bytes a bin), from L2 at these sizes.  Five device-wide scans of
+// 16-byte pairs, each over an array of terms written first, took 580 us at 2.5e6 bins (FP64); the
+// three kernels take 86.
+//
+// Both arithmetics run the same kernels: P64 sums doubles in double-double, PFF sums float-float
+// values in float-float.
+struct P64 {
+    using S = double;  // a value of the signal
+    using T = DD;      // a sum
+    static __device__ __forceinline__ T zero() { return DD{0.0, 0.0}; }
+    static __device__ __forceinline__ T add(T a, T b) { return dd_add(a, b); }
+    static __device__ __forceinline__ T add_s(T a, S v) {
+        const DD s = dd_two_sum(a.hi, v);
+        return dd_two_sum(s.hi, s.lo + a.lo);
+    }
+    static __device__ __forceinline__ S sub(S a, S b) { return a - b; }
+    static __device__ __forceinline__ S mul(S a, S b) { return a * b; }
+    static __device__ __forceinline__ S of_index(uint64_t t) { return (double)t; }
+    static __device__ __forceinline__ S none() { return 0.0; }
+    static __device__ __forceinline__ DD sum_dd(T a, int) { return a; }
+    static __device__ __forceinline__ double value(S a, int) { return a; }
+};
+struct PFF {
+    using S = FF;
+    using T = FF;
+    static __device__ __forceinline__ T zero() { return FF{0.f, 0.f}; }
+    static __device__ __forceinline__ T add(T a, T b) { return ff_add(a, b); }
+    static __device__ __forceinline__ T add_s(T a, S v) { return ff_add(a, v); }
+    static __device__ __forceinline__ S sub(S a, S b) { return ff_sub(a, b); }
+    static __device__ __forceinline__ S mul(S a, S b) { return ff_mul(a, b); }
+    static __device__ __forceinline__ S of_index(uint64_t t) { return ff_from_double_exact(t); }
+    static __device__ __forceinline__ S none() { return FF{0.f, 0.f}; }
+    // a sum in double-double, scaled back by the exact power of two 2^sc
+    static __device__ __forceinline__ DD sum_dd(T a, int sc) {
+        return DD{ldexp((double)a.hi, sc), ldexp((double)a.lo, sc)};
+    }
+    static __device__ __forceinline__ double value(S a, int sc) { return ldexp((double)a.hi + (double)a.lo, sc); }
+};
+template <class P>
+struct SumOp {
+    __device__ __forceinline__ typename P::T operator()(const typename P::T& a, const typename P::T& b) const {
+        return P::add(a, b);
+    }
+};
+
+template <class P>
+__device__ __forceinline__ typename P::T warp_sum(typename P::T v) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        typename P::T w;
+        w.hi = __shfl_down_sync(0xffffffffu, v.hi, o);
+        w.lo = __shfl_down_sync(0xffffffffu, v.lo, o);
+        v = P::add(v, w);
+    }
+    return v;  // lane 0's
+}
+
+// What the passes over one signal share, on the device.
+struct MomentState {
+    DD gsum;       // sum of g
+    double gbar;   // its mean as the centring uses it (P64)
+    FF gbar_ff;    // and in float-float (PFF)
+    float scale;   // 2^-e (PFF): u is scaled to O(1)
+    int e;
+};
+
+constexpr int kSigThreads = 256, kSigItems = 8, kSigTile = kSigThreads * kSigItems;
+
+// Tile sums of g (and the tile's largest value, for PFF's scale).
+template <class P>
+__global__ void __launch_bounds__(kSigThreads) k_g_tiles(uint64_t n, const float* __restrict__ g,
+                                                         typename P::T* __restrict__ tsum, float* __restrict__ tmax) {
+    __shared__ typename P::T part[kSigThreads / 32];
+    __shared__ float top[kSigThreads / 32];
+    const uint64_t base = blockIdx.x * (uint64_t)kSigTile + threadIdx.x;
+    typename P::T s = P::zero();
+    float m = 0.f;
+#pragma unroll
+    for (int k = 0; k < kSigItems; k++) {
+        const uint64_t i = base + (uint64_t)k * kSigThreads;
+        const float v = i < n ? g[i] : 0.f;
+        if constexpr (std::is_same<P, P64>::value) s = P::add_s(s, (double)v);
+        else s = P::add_s(s, FF{v, 0.f});
+        m = fmaxf(m, v);
+    }
+    s = warp_sum<P>(s);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) {
+        part[threadIdx.x >> 5] = s;
+        top[threadIdx.x >> 5] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kSigThreads / 32; w++) {
+            s = P::add(s, part[w]);
+            m = fmaxf(m, top[w]);
+        }
+        tsum[blockIdx.x] = s;
+        tmax[blockIdx.x] = m;
     }
 }
 
-// U[0] = 0, U[s] = inclusive scan of u at s - 1.
-__global__ void k_ff_shift(uint64_t n, const FF* __restrict__ incl, FF* __restrict__ U) {
-    const uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (s <= n) U[s] = s ? incl[s - 1] : FF{0.f, 0.f};
+// One block: sums[0..nt) becomes its exclusive prefix sums, *total the whole.
+template <class P>
+__device__ __forceinline__ void scan_tiles(uint64_t nt, typename P::T* __restrict__ sums, typename P::T* total) {
+    using T = typename P::T;
+    using BS = cub::BlockScan<T, 1024>;
+    __shared__ typename BS::TempStorage tmp;
+    T run = P::zero();
+    for (uint64_t b0 = 0; b0 < nt; b0 += 1024) {
+        const uint64_t b = b0 + threadIdx.x;
+        const T v = b < nt ? sums[b] : P::zero();
+        T ex, agg;
+        BS(tmp).ExclusiveScan(v, ex, P::zero(), SumOp<P>(), agg);
+        if (b < nt) sums[b] = P::add(run, ex);
+        run = P::add(run, agg);
+        __syncthreads();
+    }
+    *total = run;
+}
+
+// The sum and mean of g and, for PFF, the scale: 2^e >= max(g) >= |u| (coverage is non-negative).
+template <class P>
+__global__ void __launch_bounds__(1024) k_g_tops(uint64_t n, uint64_t nt, typename P::T* __restrict__ tsum,
+                                                 const float* __restrict__ tmax, MomentState* __restrict__ ms) {
+    typename P::T total;
+    scan_tiles<P>(nt, tsum, &total);
+    __shared__ float top[1024];
+    float m = 0.f;
+    for (uint64_t b = threadIdx.x; b < nt; b += 1024) m = fmaxf(m, tmax[b]);
+    top[threadIdx.x] = m;
+    __syncthreads();
+    for (int k = 512; k; k >>= 1) {
+        if (threadIdx.x < k) top[threadIdx.x] = fmaxf(top[threadIdx.x], top[threadIdx.x + k]);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        if constexpr (std::is_same<P, P64>::value) {
+            ms->gsum = total;
+            ms->gbar = total.hi / (double)n + total.lo / (double)n;
+            ms->e = 0;
+        } else {
+            // the double-double copy of the sum for the final reduction (exact: hi + lo of a float-float)
+            ms->gsum = DD{(double)total.hi + (double)total.lo, 0.0};
+            // gbar = gsum / n in float-float: one Newton step on the float quotient
+            const float q = __fdiv_rn(total.hi, (float)n);
+            const FF r = ff_sub(total, ff_mul(FF{q, 0.f}, ff_from_double_exact(n)));
+            ms->gbar_ff = ff_quick(q, __fdiv_rn(r.hi, (float)n));
+            int e = 0;
+            if (top[0] > 0.f) (void)frexpf(top[0], &e);
+            ms->e = e;
+            ms->scale = ldexpf(1.0f, -e);
+        }
+    }
+}
+
+// u = g - gbar (PFF: times 2^-e, exact).
+template <class P>
+__device__ __forceinline__ typename P::S centred(float g, const MomentState& ms) {
+    if constexpr (std::is_same<P, P64>::value) return (double)g - ms.gbar;
+    else {
+        const FF u = ff_sub(FF{g, 0.f}, ms.gbar_ff);
+        return FF{u.hi * ms.scale, u.lo * ms.scale};
+    }
+}
+
+// PFF: tile sums of u.  (P64 takes them from those of g: sum of g less count x gbar, in double-double.)
+__global__ void __launch_bounds__(kSigThreads) k_u_tiles(uint64_t n, const float* __restrict__ g,
+                                                         const MomentState* __restrict__ ms, FF* __restrict__ tsum) {
+    __shared__ FF part[kSigThreads / 32];
+    const MomentState st = *ms;
+    const uint64_t base = blockIdx.x * (uint64_t)kSigTile + threadIdx.x;
+    FF s = FF{0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < kSigItems; k++) {
+        const uint64_t i = base + (uint64_t)k * kSigThreads;
+        if (i < n) s = ff_add(s, centred<PFF>(g[i], st));
+    }
+    s = warp_sum<PFF>(s);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kSigThreads / 32; w++) s = ff_add(s, part[w]);
+        tsum[blockIdx.x] = s;
+    }
+}
+__global__ void __launch_bounds__(1024) k_u_tops(uint64_t nt, FF* __restrict__ tsum) {
+    FF total;
+    scan_tiles<PFF>(nt, tsum, &total);
+}
+
+// u into x (the transform's input, as a real signal) and U[s] = sum of u before s, s = 0 .. n.
+template <class P>
+__global__ void __launch_bounds__(kSigThreads) k_center(uint64_t n, const float* __restrict__ g,
+                                                        const MomentState* __restrict__ msp,
+                                                        const typename P::T* __restrict__ tpre,
+                                                        typename P::S* __restrict__ x, typename P::S* __restrict__ U) {
+    using T = typename P::T;
+    using S = typename P::S;
+    using BS = cub::BlockScan<T, kSigThreads>;
+    __shared__ typename BS::TempStorage tmp;
+    const MomentState ms = *msp;
+    const uint64_t tile = blockIdx.x * (uint64_t)kSigTile, base = tile + (uint64_t)threadIdx.x * kSigItems;
+    S u[kSigItems];
+    T s = P::zero();
+#pragma unroll
+    for (int k = 0; k < kSigItems; k++) {
+        u[k] = base + k < n ? centred<P>(g[base + k], ms) : P::none();
+        s = P::add_s(s, u[k]);
+    }
+    T ex;
+    BS(tmp).ExclusiveScan(s, ex, P::zero(), SumOp<P>());
+    T run = tpre[blockIdx.x];
+    if constexpr (std::is_same<P, P64>::value) run = dd_add(run, dd_neg(dd_mul_d(DD{ms.gbar, 0.0}, (double)tile)));
+    run = P::add(run, ex);
+    if (blockIdx.x == 0 && threadIdx.x == 0) U[0] = P::none();
+#pragma unroll
+    for (int k = 0; k < kSigItems; k++) {
+        if (base + k >= n) break;
+        run = P::add_s(run, u[k]);
+        x[2 * (base + k)] = u[k];  // the real parts of a complex signal
+        if constexpr (std::is_same<P, P64>::value) U[base + k + 1] = run.hi + run.lo;
+        else U[base + k + 1] = run;
+    }
+}
+
+enum Term : int { T_A = 0, T_MA = 1, T_U2 = 2, T_V2 = 3, T_U = 4, kTerms = 5 };
+
+// Adds the five terms of element t (0 .. n) to s.  uN = U[n].
+template <class P>
+__device__ __forceinline__ void add_terms(uint64_t t, uint64_t n, const typename P::S* __restrict__ A,
+                                          const typename P::S* __restrict__ U, typename P::S uN,
+                                          typename P::T* s) {
+    using S = typename P::S;
+    if (t > n) return;
+    const S u = U[t];
+    s[T_U] = P::add_s(s[T_U], u);
+    if (t == 0) return;
+    s[T_U2] = P::add_s(s[T_U2], P::mul(u, u));  // U[t]^2, t >= 1
+    if (t >= n) return;
+    const S a = A[t], d = P::sub(uN, U[n - t]);
+    s[T_A] = P::add_s(s[T_A], a);                              // A[t], 1 <= t < n
+    s[T_MA] = P::add_s(s[T_MA], P::mul(P::of_index(t), a));    // t A[t]
+    s[T_V2] = P::add_s(s[T_V2], P::mul(d, d));                 // (U[n] - U[n - t])^2
+}
+
+constexpr int kTermThreads = 256, kTermTile = 1024;
+
+// tsum[q * nt + tile] = sum of term q over the tile.
+template <class P>
+__global__ void __launch_bounds__(kTermThreads) k_term_tiles(uint64_t n, uint64_t nt,
+                                                             const typename P::S* __restrict__ A,
+                                                             const typename P::S* __restrict__ U,
+                                                             typename P::T* __restrict__ tsum) {
+    using T = typename P::T;
+    __shared__ T part[kTerms][kTermThreads / 32];
+    const typename P::S uN = U[n];
+    T s[kTerms];
+#pragma unroll
+    for (int q = 0; q < kTerms; q++) s[q] = P::zero();
+#pragma unroll
+    for (int k = 0; k < kTermTile / kTermThreads; k++)
+        add_terms<P>(blockIdx.x * (uint64_t)kTermTile + k * kTermThreads + threadIdx.x, n, A, U, uN, s);
+#pragma unroll
+    for (int q = 0; q < kTerms; q++) {
+        const T v = warp_sum<P>(s[q]);
+        if ((threadIdx.x & 31) == 0) part[q][threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < kTerms) {
+        T v = part[threadIdx.x][0];
+        for (int w = 1; w < kTermThreads / 32; w++) v = P::add(v, part[threadIdx.x][w]);
+        tsum[threadIdx.x * nt + blockIdx.x] = v;
+    }
+}
+
+// Block q: term q's tile sums into exclusive prefix sums; total[q] = the whole.
+template <class P>
+__global__ void __launch_bounds__(1024) k_term_tops(uint64_t nt, typename P::T* __restrict__ tsum,
+                                                    typename P::T* __restrict__ total) {
+    typename P::T t;
+    scan_tiles<P>(nt, tsum + blockIdx.x * nt, &t);
+    if (threadIdx.x == 0) total[blockIdx.x] = t;
+}
+
+// Windows with few positions (nw = N - L + 1 small, L close to N): the window sums F_L(j) then differ
+// from one another by a small part of their size, and any formula that forms the second moment and
+// subtracts the squared mean cancels (the reference's own f64 formula loses all digits there).
+// These L, the last of the grid, are reduced directly: d_j = F_L(j) - F_L(0) = (U[j+L] - U[j]) - U[L]
+// from the prefix sums U of the centred signal (U[0] = 0), summed with d_j^2 in double-double over the
+// nw windows, and var = sum d^2 / nw - (sum d / nw)^2.  Block (p, y): part p of the windows of the
+// y-th such L (one block for all the windows of an L: 116 us for 15 L of up to 65,536 windows).
+template <typename UT>
+__global__ void __launch_bounds__(256) k_direct_part(const uint64_t* __restrict__ grid, uint32_t first, uint64_t n,
+                                                     const UT* __restrict__ U, uint64_t per_part,
+                                                     DD* __restrict__ out) {
+    __shared__ DD r1[8], r2[8];
+    const uint64_t L = grid[first + blockIdx.y], nw = n - L + 1;
+    const uint64_t a = blockIdx.x * per_part, b = min(a + per_part, nw);
+    const DD uL = dd_neg(u_at<UT>(U, L));
+    DD s1{0.0, 0.0}, s2{0.0, 0.0};
+    for (uint64_t j = a + threadIdx.x; j < b; j += blockDim.x) {
+        const DD d = dd_add(dd_add(u_at<UT>(U, j + L), dd_neg(u_at<UT>(U, j))), uL);
+        s1 = dd_add(s1, d);
+        s2 = dd_add(s2, dd_mul(d, d));
+    }
+    s1 = warp_sum<P64>(s1);
+    s2 = warp_sum<P64>(s2);
+    if ((threadIdx.x & 31) == 0) {
+        r1[threadIdx.x >> 5] = s1;
+        r2[threadIdx.x >> 5] = s2;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) {
+            s1 = dd_add(s1, r1[w]);
+            s2 = dd_add(s2, r2[w]);
+        }
+        DD* o = out + 2 * ((uint64_t)blockIdx.y * gridDim.x + blockIdx.x);
+        o[0] = s1;
+        o[1] = s2;
+    }
+}
+
+// One block per grid point: its prefix sums (the tiles before plus the part of its own tile), then the
+// final reduction and the variance subtraction in FP64.  parts > 0: grid points from `first` on take
+// their variance from k_direct_part's sums.
+constexpr int kPointThreads = 128;
+template <class P>
+__global__ void __launch_bounds__(kPointThreads) k_window_moments(
+    const uint64_t* __restrict__ grid, uint64_t n, uint64_t nt, const typename P::S* __restrict__ A,
+    const typename P::S* __restrict__ U, const typename P::T* __restrict__ tpre,
+    const typename P::T* __restrict__ total, const MomentState* __restrict__ msp, uint32_t first, uint32_t parts,
+    const DD* __restrict__ direct, float2* __restrict__ out, double* __restrict__ mean_out,
+    double* __restrict__ var_out) {
+    using T = typename P::T;
+    __shared__ T part[kTerms + 1][kPointThreads / 32];
+    const uint32_t i = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t L = grid[i];
+    // inclusive prefix up to t = L - 1 (the t = 0 terms of A and t A are zero); UU(N-L+1) = sum of U[0 .. N-L]
+    const uint64_t at_l = L - 1, at_r = n - L;
+    const uint64_t tl = at_l / kTermTile, tr = at_r / kTermTile;
+    const typename P::S uN = U[n];
+    T s[kTerms + 1];
+#pragma unroll
+    for (int q = 0; q <= kTerms; q++) s[q] = P::zero();
+    for (uint64_t t = tl * kTermTile + threadIdx.x; t <= at_l; t += kPointThreads) add_terms<P>(t, n, A, U, uN, s);
+    for (uint64_t t = tr * kTermTile + threadIdx.x; t <= at_r; t += kPointThreads)
+        s[kTerms] = P::add_s(s[kTerms], U[t]);
+#pragma unroll
+    for (int q = 0; q <= kTerms; q++) {
+        const T v = warp_sum<P>(s[q]);
+        if (lane == 0) part[q][warp] = v;
+    }
+    DD d1{0.0, 0.0}, d2{0.0, 0.0};
+    const bool few = parts && i >= first;
+    if (few && warp == 0) {
+        const DD* d = direct + 2 * (uint64_t)(i - first) * parts;
+        for (uint32_t p = lane; p < parts; p += 32) {
+            d1 = dd_add(d1, d[2 * p]);
+            d2 = dd_add(d2, d[2 * p + 1]);
+        }
+        d1 = warp_sum<P64>(d1);
+        d2 = warp_sum<P64>(d2);
+    }
+    __syncthreads();
+    if (threadIdx.x) return;
+    const MomentState ms = *msp;
+    const int e = ms.e;
+    DD p[kTerms + 1];
+#pragma unroll
+    for (int q = 0; q <= kTerms; q++) {
+        const int term = q < kTerms ? q : T_U;
+        T v = tpre[term * nt + (q < kTerms ? tl : tr)];
+        for (int w = 0; w < kPointThreads / 32; w++) v = P::add(v, part[q][w]);
+        p[q] = P::sum_dd(v, term == T_U ? e : 2 * e);
+    }
+    const double nw = (double)(n - L + 1);
+    const double gbar = ms.gsum.hi / (double)n + ms.gsum.lo / (double)n;
+    const double a0 = P::value(A[0], 2 * e);
+    // sum_j F_L(j) = (UU(N+1) - UU(L)) - UU(N-L+1)
+    const DD sf = dd_add(dd_add(P::sum_dd(total[T_U], e), dd_neg(p[T_U])), dd_neg(p[kTerms]));
+    const double fbar = (sf.hi + sf.lo) / nw;
+    // sum_j F_L(j)^2 = L A[0] + 2 (L P0 - P1) - Q - V
+    DD s2 = DD{(double)L * a0, fma((double)L, a0, -(double)L * a0)};
+    const DD inner = dd_add(dd_mul_d(p[T_A], (double)L), dd_neg(p[T_MA]));
+    s2 = dd_add(s2, dd_mul_d(inner, 2.0));
+    s2 = dd_add(s2, dd_neg(p[T_U2]));
+    s2 = dd_add(s2, dd_neg(p[T_V2]));
+    const double mean = (double)L * gbar + fbar;
+    double var = (s2.hi + s2.lo) / nw - fbar * fbar;
+    if (!(var > 0.0)) var = 0.0;
+    if (few) {  // few windows: reduced directly
+        const DD m1 = dd_div_d(d1, nw), m2 = dd_div_d(d2, nw);
+        const DD v = dd_add(m2, dd_neg(dd_mul(m1, m1)));
+        const double scale = ldexp(1.0, e);
+        var = (v.hi + v.lo) * scale * scale;
+        if (!(var > 0.0)) var = 0.0;
+    }
+    out[i] = make_float2((float)mean, (float)var);
+    if (mean_out) mean_out[i] = mean;
+    if (var_out) var_out[i] = var;
 }
 
 }  // namespace rgl
@@ -631,8 +856,8 @@ using namespace rgl;
 // Per-build device workspace (grown on demand) and the host twiddle table.
 namespace {
 struct MomentWs {
-    DevBuf iv, key_a, key_b, val_a, val_b, g, totals, nz, idx, cum, cnt, fa, fb, U, dd_in, dd_out, at, gl, outs, tmp,
-        gsum, grid, mv, dv;
+    DevBuf iv, key_a, key_b, val_a, val_b, g, totals, nz, idx, cum, cnt, fa, fb, U, A, sums, state, direct, gl, tmp,
+        tw, mv;
 };
 std::mutex g_ws_mu;
 MomentWs g_ws[16];  // one workspace per device ordinal
@@ -728,31 +953,9 @@ int fft_forward(MomentWs& w, uint64_t M, cudaStream_t st, double2** result) {
     return RGL_OK;
 }
 
-int dd_scan(MomentWs& w, uint64_t len, cudaStream_t st) {
-    // inclusive double-double scan of w.dd_in into w.dd_out
-    size_t tb = 0;
-    cub::DeviceScan::InclusiveScan(nullptr, tb, w.dd_in.as<DD>(), w.dd_out.as<DD>(), DDAdd(), (int)len, st);
-    RGL_TRY(w.tmp.ensure(tb + 256));
-    tb = w.tmp.cap;
-    RGL_CUDA(cub::DeviceScan::InclusiveScan(w.tmp.p, tb, w.dd_in.as<DD>(), w.dd_out.as<DD>(), DDAdd(), (int)len, st));
-    return RGL_OK;
-}
-
 }  // namespace
 
 namespace {
-int ff_scan(MomentWs& w, uint64_t len, cudaStream_t st) {
-    // inclusive float-float scan of w.dd_in (as FF) into w.dd_out
-    FF* in = reinterpret_cast<FF*>(w.dd_in.p);
-    FF* out = reinterpret_cast<FF*>(w.dd_out.p);
-    size_t tb = 0;
-    cub::DeviceScan::InclusiveScan(nullptr, tb, in, out, FFAdd(), (int)len, st);
-    RGL_TRY(w.tmp.ensure(tb + 256));
-    tb = w.tmp.cap;
-    RGL_CUDA(cub::DeviceScan::InclusiveScan(w.tmp.p, tb, in, out, FFAdd(), (int)len, st));
-    return RGL_OK;
-}
-
 // Float-float value of a long double: hi = nearest float, lo = nearest float of the remainder.
 inline void ff_of(long double v, float* hi, float* lo) {
     *hi = (float)v;
@@ -791,8 +994,8 @@ int ff_twiddles(MomentWs& w, uint64_t M, int device, int* tb_out) {
         ff_of(cosl(a), &q[0], &q[1]);
         ff_of(sinl(a), &q[2], &q[3]);
     }
-    RGL_TRY(w.grid.ensure(h.size() * 4));
-    RGL_CUDA(cudaMemcpy(w.grid.p, h.data(), h.size() * 4, cudaMemcpyHostToDevice));
+    RGL_TRY(w.tw.ensure(h.size() * 4));
+    RGL_CUDA(cudaMemcpy(w.tw.p, h.data(), h.size() * 4, cudaMemcpyHostToDevice));
     *tb_out = tb;
     return RGL_OK;
 }
@@ -800,7 +1003,7 @@ int ff_twiddles(MomentWs& w, uint64_t M, int device, int* tb_out) {
 int ff_fft_forward(MomentWs& w, uint64_t M, int tb, cudaStream_t st, CFF** result) {
     CFF* src = reinterpret_cast<CFF*>(w.fa.p);
     CFF* dst = reinterpret_cast<CFF*>(w.fb.p);
-    const CFF* wf = reinterpret_cast<const CFF*>(w.grid.p);
+    const CFF* wf = reinterpret_cast<const CFF*>(w.tw.p);
     const CFF* wc = wf + (1ull << tb);
     uint64_t Ns = 1;
     int logm = 0;
@@ -825,74 +1028,74 @@ int ff_fft_forward(MomentWs& w, uint64_t M, int tb, cudaStream_t st, CFF** resul
     return RGL_OK;
 }
 
-struct GMax {
-    __device__ __forceinline__ float operator()(float a, float b) const { return fmaxf(a, b); }
-};
-
-// K5-K7 of the compensated-FP32 path for the depth signal in w.g (N bins): fills outs (P0, P1, Q,
-// V, UU_L, UU_R as double-double, scaled back), *uu_total, *a0 and w.gsum (as DD) for
-// k_window_moments.
-int moments_ff(MomentWs& w, uint64_t N, uint64_t M, int device, uint32_t G, const uint64_t* d_at, DD* outs,
-               DD* uu_total, double* a0, int* scale_exp, cudaStream_t st) {
+// K5-K7 for the depth signal in w.g (N bins): the moments of the L grid (G points, on the device at
+// w.gl) into `table` and, where given, d_mean / d_var.
+template <class P>
+int moments_dev(MomentWs& w, uint64_t N, uint64_t M, int device, const std::vector<uint64_t>& grid, float2* table,
+                double* d_mean, double* d_var, cudaStream_t st) {
+    using S = typename P::S;
+    using T = typename P::T;
+    constexpr bool kFF = std::is_same<P, PFF>::value;
+    const uint32_t G = (uint32_t)grid.size();
+    const uint64_t nt = (N + kSigTile - 1) / kSigTile, mt = N / kTermTile + 1;  // tiles of g and of the terms (0 .. N)
+    RGL_TRY(w.fa.ensure(M * 16));
+    RGL_TRY(w.fb.ensure(M * 16));
+    RGL_TRY(w.U.ensure((N + 2) * sizeof(S)));
+    RGL_TRY(w.A.ensure((N + 2) * sizeof(S)));
+    RGL_TRY(w.sums.ensure((2 * nt + kTerms * (mt + 1) + 4) * sizeof(T)));
+    RGL_TRY(w.state.ensure(sizeof(MomentState) + nt * 4 + 64));
+    // windows with few positions: reduced directly, in parts of at least 2,048 windows
+    const uint64_t few = std::max<uint64_t>(65536, N / 32);
+    uint32_t first = G;
+    while (first > 0 && N - grid[first - 1] + 1 <= few) first--;
+    const uint64_t most = first < G ? N - grid[first] + 1 : 0;
+    const uint32_t parts = (uint32_t)std::min<uint64_t>(64, (most + 2047) / 2048);
+    RGL_TRY(w.direct.ensure(std::max<uint64_t>(1, (uint64_t)(G - first) * parts) * 2 * sizeof(DD)));
     int tb = 0;
-    RGL_TRY(ff_twiddles(w, M, device, &tb));
-    FF* ffin = reinterpret_cast<FF*>(w.dd_in.p);
-    FF* ffout = reinterpret_cast<FF*>(w.dd_out.p);
-    FF* U = reinterpret_cast<FF*>(w.U.p);
-    // gsum in float-float, max(g) for the per-chromosome scale
-    k_ff_from_float<<<blocks_for(N), 256, 0, st>>>(N, w.g.as<float>(), ffin);
-    FF* d_gsum = reinterpret_cast<FF*>(w.gsum.p) + 4;  // beside the DD copy at w.gsum[0]
-    float* d_gmax = reinterpret_cast<float*>(w.gsum.p) + 12;
-    {
-        size_t t1 = 0, t2 = 0;
-        cub::DeviceReduce::Reduce(nullptr, t1, ffin, d_gsum, (int)N, FFAdd(), FF{0.f, 0.f}, st);
-        cub::DeviceReduce::Reduce(nullptr, t2, w.g.as<float>(), d_gmax, (int)N, GMax(), 0.0f, st);
-        RGL_TRY(w.tmp.ensure(std::max(t1, t2) + 256));
-        t1 = w.tmp.cap;
-        RGL_CUDA(cub::DeviceReduce::Reduce(w.tmp.p, t1, ffin, d_gsum, (int)N, FFAdd(), FF{0.f, 0.f}, st));
-        t2 = w.tmp.cap;
-        RGL_CUDA(cub::DeviceReduce::Reduce(w.tmp.p, t2, w.g.as<float>(), d_gmax, (int)N, GMax(), 0.0f, st));
+    if constexpr (kFF) RGL_TRY(ff_twiddles(w, M, device, &tb));
+    const float* g = w.g.as<float>();
+    const uint64_t* d_grid = w.gl.as<uint64_t>();
+    MomentState* ms = w.state.as<MomentState>();
+    float* tmax = reinterpret_cast<float*>(ms + 1);
+    T* tsum = w.sums.as<T>();
+    T* usum = kFF ? tsum + nt : tsum;
+    T* terms = tsum + 2 * nt;
+    T* totals = terms + kTerms * mt;
+    S* U = w.U.as<S>();
+    S* A = w.A.as<S>();
+    k_g_tiles<P><<<(unsigned)nt, kSigThreads, 0, st>>>(N, g, tsum, tmax);
+    k_g_tops<P><<<1, 1024, 0, st>>>(N, nt, tsum, tmax, ms);
+    if constexpr (kFF) {
+        k_u_tiles<<<(unsigned)nt, kSigThreads, 0, st>>>(N, g, ms, usum);
+        k_u_tops<<<1, 1024, 0, st>>>(nt, usum);
     }
-    FF gs;
-    float gmax = 0.f;
-    RGL_CUDA(cudaMemcpyAsync(&gs, d_gsum, sizeof(FF), cudaMemcpyDeviceToHost, st));
-    RGL_CUDA(cudaMemcpyAsync(&gmax, d_gmax, 4, cudaMemcpyDeviceToHost, st));
-    RGL_CUDA(cudaStreamSynchronize(st));
-    // the DD copy of the sum for the final reduction (exact: hi + lo of a float-float)
-    const DD gsum_dd{(double)gs.hi + (double)gs.lo, 0.0};
-    RGL_CUDA(cudaMemcpyAsync(w.gsum.p, &gsum_dd, sizeof(DD), cudaMemcpyHostToDevice, st));
-    // |u| <= max(g) (coverage is non-negative): scale u by 2^-e with 2^e >= max(g)
-    int e = 0;
-    if (gmax > 0.f) (void)std::frexp((double)gmax, &e);
-    const float scale = std::ldexp(1.0f, -e);
-    *scale_exp = e;
-    k_ff_center<<<blocks_for(M), 256, 0, st>>>(N, M, w.g.as<float>(), d_gsum, scale, reinterpret_cast<CFF*>(w.fa.p),
-                                                ffin);
-    RGL_TRY(ff_scan(w, N + 1, st));
-    k_ff_shift<<<blocks_for(N + 1), 256, 0, st>>>(N, ffout, U);
-    CFF* X = nullptr;
-    RGL_TRY(ff_fft_forward(w, M, tb, st, &X));
-    k_ff_power<<<blocks_for(M), 256, 0, st>>>(M, X);
-    if (X != reinterpret_cast<CFF*>(w.fa.p)) RGL_CUDA(cudaMemcpyAsync(w.fa.p, X, M * 16, cudaMemcpyDeviceToDevice, st));
-    CFF* Y = nullptr;
-    RGL_TRY(ff_fft_forward(w, M, tb, st, &Y));
-    const float inv_m = std::ldexp(1.0f, -(int)std::lround(std::log2((double)M)));
-    const int terms[4] = {T_A, T_MA, T_U2, T_V2};
-    for (int q = 0; q < 4; q++) {
-        k_ff_term<<<blocks_for(N + 1), 256, 0, st>>>(N + 1, terms[q], Y, inv_m, U, N, ffin);
-        RGL_TRY(ff_scan(w, N + 1, st));
-        k_ff_gather<<<blocks_for(G), 256, 0, st>>>(G, d_at, ffout, 2 * e, outs + (uint64_t)q * G);
+    RGL_CUDA(cudaMemsetAsync(w.fa.p, 0, M * 16, st));
+    k_center<P><<<(unsigned)nt, kSigThreads, 0, st>>>(N, g, ms, usum, w.fa.as<S>(), U);
+    // K6: A[m] = Re(FFT(|FFT(u)|^2))[m] / M
+    const double inv_m = 1.0 / (double)M;
+    if constexpr (kFF) {
+        CFF *X = nullptr, *Y = nullptr;
+        RGL_TRY(ff_fft_forward(w, M, tb, st, &X));
+        k_ff_power<<<blocks_for(M), 256, 0, st>>>(M, X);
+        if (X != w.fa.as<CFF>()) RGL_CUDA(cudaMemcpyAsync(w.fa.p, X, M * 16, cudaMemcpyDeviceToDevice, st));
+        RGL_TRY(ff_fft_forward(w, M, tb, st, &Y));
+        k_ff_autocorr<<<blocks_for(N), 256, 0, st>>>(N, Y, (float)inv_m, A);
+    } else {
+        double2 *X = nullptr, *Y = nullptr;
+        RGL_TRY(fft_forward(w, M, st, &X));
+        k_power<<<blocks_for(M), 256, 0, st>>>(M, X);
+        if (X != w.fa.as<double2>()) RGL_CUDA(cudaMemcpyAsync(w.fa.p, X, M * 16, cudaMemcpyDeviceToDevice, st));
+        RGL_TRY(fft_forward(w, M, st, &Y));
+        k_autocorr<<<blocks_for(N), 256, 0, st>>>(N, Y, inv_m, A);
     }
-    k_ff_term<<<blocks_for(N + 1), 256, 0, st>>>(N + 1, T_U, Y, inv_m, U, N, ffin);
-    RGL_TRY(ff_scan(w, N + 1, st));
-    k_ff_gather<<<blocks_for(G), 256, 0, st>>>(G, d_at, ffout, e, outs + 4ull * G);
-    k_ff_gather<<<blocks_for(G), 256, 0, st>>>(G, d_at + G, ffout, e, outs + 5ull * G);
-    FF tot, y0;
-    RGL_CUDA(cudaMemcpyAsync(&tot, ffout + N, sizeof(FF), cudaMemcpyDeviceToHost, st));
-    RGL_CUDA(cudaMemcpyAsync(&y0, &Y[0].re, sizeof(FF), cudaMemcpyDeviceToHost, st));
-    RGL_CUDA(cudaStreamSynchronize(st));
-    *uu_total = DD{std::ldexp((double)tot.hi, e), std::ldexp((double)tot.lo, e)};
-    *a0 = std::ldexp(((double)y0.hi + (double)y0.lo) * (double)inv_m, 2 * e);
+    // K7
+    k_term_tiles<P><<<(unsigned)mt, kTermThreads, 0, st>>>(N, mt, A, U, terms);
+    k_term_tops<P><<<kTerms, 1024, 0, st>>>(mt, terms, totals);
+    if (parts)
+        k_direct_part<S><<<dim3(parts, G - first), 256, 0, st>>>(d_grid, first, N, U, (most + parts - 1) / parts,
+                                                                 w.direct.as<DD>());
+    k_window_moments<P><<<G, kPointThreads, 0, st>>>(d_grid, N, mt, A, U, terms, totals, ms, first, parts,
+                                                     w.direct.as<DD>(), table, d_mean, d_var);
     RGL_CUDA(cudaGetLastError());
     return RGL_OK;
 }
@@ -947,104 +1150,17 @@ int rgl_moments_build_ex(rgl_moments* m, uint32_t sid, uint32_t chrom, const rgl
     RGL_TRY(depth_signal_dev(w, intervals, n, N, bin_size, st));
     uint64_t M = 1;
     while (M < 2 * N) M <<= 1;
-    RGL_TRY(w.fa.ensure(M * 16));
-    RGL_TRY(w.fb.ensure(M * 16));
-    RGL_TRY(w.dd_in.ensure((N + 2) * 16));
-    RGL_TRY(w.dd_out.ensure((N + 2) * 16));
-    RGL_TRY(w.U.ensure((N + 2) * 8));
-    RGL_TRY(w.gsum.ensure(64));
-    // K7 gather points: the L grid of the store
+    // K7 points: the L grid of the store
     const std::vector<uint64_t> grid = moment_grid(N);
     const uint32_t G = (uint32_t)grid.size();
     if (G != slots) return fail(RGL_ERR_INVALID_ARGUMENT, "moment table size does not match the L grid");
-    std::vector<uint64_t> at_l(G), at_r(G);
-    for (uint32_t i = 0; i < G; i++) {
-        at_l[i] = grid[i] - 1;  // inclusive prefix over t < L (the t = 0 term of P0 / P1 is zero)
-        at_r[i] = N - grid[i];  // UU(N-L+1) = sum_{s<=N-L} U[s]
-    }
-    RGL_TRY(w.at.ensure(G * 8 * 3ull + 64));
     RGL_TRY(w.gl.ensure(G * 8ull + 64));
-    RGL_TRY(w.outs.ensure(G * 16 * 7ull + 64));
-    uint64_t* d_at = w.at.as<uint64_t>();
-    RGL_CUDA(cudaMemcpyAsync(d_at, at_l.data(), G * 8, cudaMemcpyHostToDevice, st));
-    RGL_CUDA(cudaMemcpyAsync(d_at + G, at_r.data(), G * 8, cudaMemcpyHostToDevice, st));
     RGL_CUDA(cudaMemcpyAsync(w.gl.p, grid.data(), G * 8, cudaMemcpyHostToDevice, st));
-    DD* outs = w.outs.as<DD>();  // P0, P1, Q, V, UU_L, UU_R (G each)
-    DD uu_total{0.0, 0.0};
-    double a0 = 0.0;
-    int ff_exp = 0;
-    if (precision == RGL_MOM_FP32C) {
-        RGL_TRY(moments_ff(w, N, M, device, G, d_at, outs, &uu_total, &a0, &ff_exp, st));
-    } else {
-        // K5: mean of g (double-double sum), centred signal, U = prefix of u
-        k_to_dd<<<blocks_for(N), 256, 0, st>>>(N, w.g.as<float>(), w.dd_in.as<DD>());
-        {
-            size_t tb = 0;
-            cub::DeviceReduce::Reduce(nullptr, tb, w.dd_in.as<DD>(), w.gsum.as<DD>(), (int)N, DDAdd(), DD{0.0, 0.0}, st);
-            RGL_TRY(w.tmp.ensure(tb + 256));
-            tb = w.tmp.cap;
-            RGL_CUDA(cub::DeviceReduce::Reduce(w.tmp.p, tb, w.dd_in.as<DD>(), w.gsum.as<DD>(), (int)N, DDAdd(),
-                                               DD{0.0, 0.0}, st));
-        }
-        k_center<<<blocks_for(M), 256, 0, st>>>(N, M, w.g.as<float>(), w.gsum.as<DD>(), w.fa.as<double2>(),
-                                                 w.dd_in.as<DD>());
-        // exclusive prefix: U[s] = sum_{k<s} u[k] for s = 0..N -> inclusive scan of u shifted by one
-        RGL_TRY(dd_scan(w, N + 1, st));  // dd_out[s] = sum_{k<=s} u[k]
-        RGL_CUDA(cudaMemsetAsync(w.U.p, 0, 8, st));
-        k_dd_to_double<<<blocks_for(N), 256, 0, st>>>(N, w.dd_out.as<DD>(), w.U.as<double>() + 1);
-        // K6: A[m] = Re(FFT(|FFT(u)|^2))[m] / M
-        double2* X = nullptr;
-        RGL_TRY(fft_forward(w, M, st, &X));
-        k_power<<<blocks_for(M), 256, 0, st>>>(M, X);
-        if (X != w.fa.as<double2>()) RGL_CUDA(cudaMemcpyAsync(w.fa.p, X, M * 16, cudaMemcpyDeviceToDevice, st));
-        double2* Y = nullptr;
-        RGL_TRY(fft_forward(w, M, st, &Y));
-        // K7: prefix sums at the grid points
-        const double inv_m = 1.0 / (double)M;
-        const int terms[4] = {T_A, T_MA, T_U2, T_V2};
-        for (int q = 0; q < 4; q++) {
-            k_term<<<blocks_for(N + 1), 256, 0, st>>>(N + 1, terms[q], Y, inv_m, w.U.as<double>(), N, w.dd_in.as<DD>());
-            RGL_TRY(dd_scan(w, N + 1, st));
-            k_gather<<<blocks_for(G), 256, 0, st>>>(G, d_at, w.dd_out.as<DD>(), outs + (uint64_t)q * G);
-        }
-        k_term<<<blocks_for(N + 1), 256, 0, st>>>(N + 1, T_U, Y, inv_m, w.U.as<double>(), N, w.dd_in.as<DD>());
-        RGL_TRY(dd_scan(w, N + 1, st));
-        // UU(L) = sum_{s<L} U[s] = inclusive[L-1]; UU(N-L+1) = inclusive[N-L]; UU(N+1) = inclusive[N]
-        k_gather<<<blocks_for(G), 256, 0, st>>>(G, d_at, w.dd_out.as<DD>(), outs + 4ull * G);
-        k_gather<<<blocks_for(G), 256, 0, st>>>(G, d_at + G, w.dd_out.as<DD>(), outs + 5ull * G);
-        double2 a0c;
-        RGL_CUDA(cudaMemcpyAsync(&uu_total, w.dd_out.as<DD>() + N, sizeof(DD), cudaMemcpyDeviceToHost, st));
-        RGL_CUDA(cudaMemcpyAsync(&a0c, Y, sizeof(double2), cudaMemcpyDeviceToHost, st));
-        RGL_CUDA(cudaStreamSynchronize(st));
-        a0 = a0c.x * inv_m;
-    }
-    // the final reduction and the variance subtraction, FP64 (both paths)
-    DevBuf& dm = w.mv;
-    RGL_TRY(dm.ensure(G * 16ull + 64));
-    double* d_mean = mean_out ? dm.as<double>() : nullptr;
-    double* d_var = var_out ? dm.as<double>() + G : nullptr;
-    // windows with few positions: the variance reduced directly from the prefix sums (k_direct_var)
-    const uint64_t few = std::max<uint64_t>(65536, N / 32);
-    std::vector<uint32_t> direct;
-    for (uint32_t i = 0; i < G; i++)
-        if (N - grid[i] + 1 <= few) direct.push_back(i);
-    RGL_TRY(w.dv.ensure(G * 8ull + 64));
-    RGL_CUDA(cudaMemsetAsync(w.dv.p, 0xFF, G * 8ull, st));  // NaN: not reduced directly
-    if (!direct.empty()) {
-        uint32_t* d_which = reinterpret_cast<uint32_t*>(d_at + 2ull * G);
-        RGL_CUDA(cudaMemcpyAsync(d_which, direct.data(), direct.size() * 4, cudaMemcpyHostToDevice, st));
-        if (precision == RGL_MOM_FP32C)
-            k_direct_var<FF><<<(unsigned)direct.size(), 256, 0, st>>>(
-                d_which, w.gl.as<uint64_t>(), N, reinterpret_cast<const FF*>(w.U.p), std::ldexp(1.0, ff_exp),
-                w.dv.as<double>());
-        else
-            k_direct_var<double><<<(unsigned)direct.size(), 256, 0, st>>>(d_which, w.gl.as<uint64_t>(), N,
-                                                                           w.U.as<double>(), 1.0, w.dv.as<double>());
-    }
-    k_window_moments<<<blocks_for(G), 256, 0, st>>>(G, w.gl.as<uint64_t>(), N, w.gsum.as<DD>(), a0, outs, outs + G,
-                                                    outs + 2ull * G, outs + 3ull * G, outs + 4ull * G, outs + 5ull * G,
-                                                    uu_total, table, d_mean, d_var, w.dv.as<double>());
-    RGL_CUDA(cudaGetLastError());
+    RGL_TRY(w.mv.ensure(G * 16ull + 64));
+    double* d_mean = mean_out ? w.mv.as<double>() : nullptr;
+    double* d_var = var_out ? w.mv.as<double>() + G : nullptr;
+    if (precision == RGL_MOM_FP32C) RGL_TRY(moments_dev<PFF>(w, N, M, device, grid, table, d_mean, d_var, st));
+    else RGL_TRY(moments_dev<P64>(w, N, M, device, grid, table, d_mean, d_var, st));
     if (mean_out) RGL_CUDA(cudaMemcpyAsync(mean_out, d_mean, G * 8, cudaMemcpyDeviceToHost, st));
     if (var_out) RGL_CUDA(cudaMemcpyAsync(var_out, d_var, G * 8, cudaMemcpyDeviceToHost, st));
     RGL_CUDA(cudaStreamSynchronize(st));
