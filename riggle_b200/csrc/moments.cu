@@ -216,78 +216,6 @@ __global__ void k_apply_carry(uint64_t full, const int* __restrict__ count, cons
     }
 }
 
-// ---- K6: Stockham FFT (FP64) ----------------------------------------------------------------------
-// One pass of the out-of-place Stockham formulation (Govindaraju et al., "High performance discrete
-// Fourier transforms on graphics processors", SC 2008): thread j loads R elements at stride M/R,
-// twiddles them by exp(-2 pi i (j mod Ns) r / (Ns R)), applies a radix-R DFT in registers and
-// stores them at (j / Ns) Ns R + (j mod Ns) + r Ns.  log_R passes with Ns = 1, R, R^2, ... leave the
-// transform in natural order.
-__constant__ double2 c_tw16[16];  // exp(-2 pi i k / 16), k < 16 (host-computed)
-
-template <int R>
-__device__ __forceinline__ void dft_regs(double2* v) {
-    // in-register radix-2 DIT on R = 2^r points (bit-reversed input order, natural output)
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-        int j = 0;
-#pragma unroll
-        for (int b = 1; b < R; b <<= 1) j = (j << 1) | ((i / b) & 1);
-        if (i < j) {
-            const double2 t = v[i];
-            v[i] = v[j];
-            v[j] = t;
-        }
-    }
-#pragma unroll
-    for (int len = 2; len <= R; len <<= 1) {
-#pragma unroll
-        for (int i = 0; i < R; i += len) {
-#pragma unroll
-            for (int k = 0; k < len / 2; k++) {
-                const double2 w = c_tw16[k * (16 / len)];
-                const double2 a = v[i + k], b = v[i + k + len / 2];
-                const double2 t = make_double2(b.x * w.x - b.y * w.y, b.x * w.y + b.y * w.x);
-                v[i + k] = make_double2(a.x + t.x, a.y + t.y);
-                v[i + k + len / 2] = make_double2(a.x - t.x, a.y - t.y);
-            }
-        }
-    }
-}
-
-template <int R>
-__global__ void __launch_bounds__(256) k_fft_pass(const double2* __restrict__ in, double2* __restrict__ out,
-                                                  uint64_t M, uint64_t Ns) {
-    const uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    const uint64_t stride = M / R;
-    if (j >= stride) return;
-    double2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) v[r] = in[j + r * stride];
-    const uint64_t k = j % Ns;
-    if (Ns > 1) {
-#pragma unroll
-        for (int r = 1; r < R; r++) {
-            // angle -2 pi k r / (Ns R), as sincospi of the exact rational -2 k r / (Ns R)
-            double s, c;
-            sincospi(-2.0 * (double)(k * r) / (double)(Ns * R), &s, &c);
-            const double2 a = v[r];
-            v[r] = make_double2(a.x * c - a.y * s, a.x * s + a.y * c);
-        }
-    }
-    dft_regs<R>(v);
-    const uint64_t base = (j / Ns) * Ns * R + k;
-#pragma unroll
-    for (int r = 0; r < R; r++) out[base + r * Ns] = v[r];
-}
-
-__global__ void k_power(uint64_t M, double2* __restrict__ x) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < M) {
-        const double2 a = x[i];
-        x[i] = make_double2(a.x * a.x + a.y * a.y, 0.0);
-    }
-}
-
 __device__ __forceinline__ DD dd_mul(DD a, DD b) {
     const double p = a.hi * b.hi;
     double e = fma(a.hi, b.hi, -p);
@@ -305,12 +233,6 @@ __device__ __forceinline__ DD u_at(const UT* U, uint64_t i);
 template <>
 __device__ __forceinline__ DD u_at<double>(const double* U, uint64_t i) { return DD{U[i], 0.0}; }
 
-// A[t] = Re y[t] / M, t < n.
-__global__ void k_autocorr(uint64_t n, const double2* __restrict__ y, double inv_m, double* __restrict__ A) {
-    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (t < n) A[t] = y[t].x * inv_m;
-}
-
 // ---- the compensated-FP32 path (K5-K7 with float-float arithmetic) ------------------------------
 // Every value is an unevaluated sum hi + lo of two floats (|lo| <= ulp(hi) / 2), about 48 bits of
 // significand, kept by the error-free transformations two-sum (Knuth) and two-product (one FMA)
@@ -321,10 +243,10 @@ __global__ void k_autocorr(uint64_t n, const double2* __restrict__ y, double inv
 // parts), the FFT, the power spectrum and the prefix sums run in float-float, and FP64 appears only
 // when the per-L results are combined (k_window_moments: the final reduction and the variance
 // subtraction).
-struct FF {
+struct __align__(8) FF {
     float hi, lo;
 };
-struct CFF {
+struct __align__(16) CFF {
     FF re, im;
 };
 __device__ __forceinline__ FF ff_two_sum(float a, float b) {
@@ -368,78 +290,6 @@ __device__ __forceinline__ DD u_at<FF>(const FF* U, uint64_t i) {
     return dd_two_sum((double)U[i].hi, (double)U[i].lo);
 }
 
-__constant__ CFF c_tw16f[16];  // exp(-2 pi i k / 16) as float-float (host-computed)
-
-template <int R>
-__device__ __forceinline__ void dft_regs_ff(CFF* v) {
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-        int j = 0;
-#pragma unroll
-        for (int b = 1; b < R; b <<= 1) j = (j << 1) | ((i / b) & 1);
-        if (i < j) {
-            const CFF t = v[i];
-            v[i] = v[j];
-            v[j] = t;
-        }
-    }
-#pragma unroll
-    for (int len = 2; len <= R; len <<= 1) {
-#pragma unroll
-        for (int i = 0; i < R; i += len) {
-#pragma unroll
-            for (int k = 0; k < len / 2; k++) {
-                const CFF a = v[i + k];
-                const CFF t = k == 0 ? v[i + k + len / 2] : cff_mul(v[i + k + len / 2], c_tw16f[k * (16 / len)]);
-                v[i + k] = cff_add(a, t);
-                v[i + k + len / 2] = cff_sub(a, t);
-            }
-        }
-    }
-}
-
-// One Stockham pass as k_fft_pass, in float-float.  The twiddle exp(-2 pi i t / M), t = k r M / (Ns R),
-// is the product of two table entries: wc[t >> tb] (coarse) and wf[t & (2^tb - 1)] (fine).
-template <int R>
-__global__ void __launch_bounds__(128) k_ff_fft_pass(const CFF* __restrict__ in, CFF* __restrict__ out, uint64_t M,
-                                                     uint64_t Ns, const CFF* __restrict__ wc,
-                                                     const CFF* __restrict__ wf, int tb) {
-    const uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    const uint64_t stride = M / R;
-    if (j >= stride) return;
-    CFF v[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) v[r] = in[j + r * stride];
-    const uint64_t k = j % Ns;
-    if (Ns > 1) {
-        const uint64_t step = M / (Ns * R);  // t = k r step < M
-        const uint64_t mask = (1ull << tb) - 1;
-#pragma unroll
-        for (int r = 1; r < R; r++) {
-            const uint64_t t = k * (uint64_t)r * step;
-            const CFF w = cff_mul(wc[t >> tb], wf[t & mask]);
-            v[r] = cff_mul(v[r], w);
-        }
-    }
-    dft_regs_ff<R>(v);
-    const uint64_t base = (j / Ns) * Ns * R + k;
-#pragma unroll
-    for (int r = 0; r < R; r++) out[base + r * Ns] = v[r];
-}
-
-__global__ void k_ff_power(uint64_t M, CFF* __restrict__ x) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < M) {
-        const CFF a = x[i];
-        x[i] = CFF{ff_add(ff_mul(a.re, a.re), ff_mul(a.im, a.im)), FF{0.f, 0.f}};
-    }
-}
-
-__global__ void k_ff_autocorr(uint64_t n, const CFF* __restrict__ y, float inv_m, FF* __restrict__ A) {
-    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (t < n) A[t] = FF{y[t].re.hi * inv_m, y[t].re.lo * inv_m};  // exact: inv_m is a power of two
-}
-
 // ---- K5, K7: prefix sums at the grid's points ------------------------------------------------------
 // The window moments need prefix sums of five terms (A[t], t A[t], U[t]^2, (U[N] - U[N-t])^2, U[t]) at
 // the grid's ~1,000 points only, so no prefix is written out: one pass sums tiles of the terms, one
@@ -451,8 +301,17 @@ __global__ void k_ff_autocorr(uint64_t n, const CFF* __restrict__ y, float inv_m
 // Both arithmetics run the same kernels: P64 sums doubles in double-double, PFF sums float-float
 // values in float-float.
 struct P64 {
-    using S = double;  // a value of the signal
-    using T = DD;      // a sum
+    using S = double;   // a value of the signal
+    using C = double2;  // a complex value
+    using T = DD;       // a sum
+    static __device__ __forceinline__ S re(C a) { return a.x; }
+    static __device__ __forceinline__ S im(C a) { return a.y; }
+    static __device__ __forceinline__ C pack(S re, S im) { return make_double2(re, im); }
+    static __device__ __forceinline__ C conj(C a) { return make_double2(a.x, -a.y); }
+    static __device__ __forceinline__ C half(C a) { return make_double2(0.5 * a.x, 0.5 * a.y); }
+    static __device__ __forceinline__ S norm(C a) { return a.x * a.x + a.y * a.y; }
+    static __device__ __forceinline__ S addv(S a, S b) { return a + b; }
+    static __device__ __forceinline__ S scaled(S a, uint64_t m) { return a * (1.0 / (double)m); }  // m a power of two
     static __device__ __forceinline__ T zero() { return DD{0.0, 0.0}; }
     static __device__ __forceinline__ T add(T a, T b) { return dd_add(a, b); }
     static __device__ __forceinline__ T add_s(T a, S v) {
@@ -468,7 +327,21 @@ struct P64 {
 };
 struct PFF {
     using S = FF;
+    using C = CFF;
     using T = FF;
+    static __device__ __forceinline__ S re(C a) { return a.re; }
+    static __device__ __forceinline__ S im(C a) { return a.im; }
+    static __device__ __forceinline__ C pack(S re, S im) { return CFF{re, im}; }
+    static __device__ __forceinline__ C conj(C a) { return CFF{a.re, ff_neg(a.im)}; }
+    static __device__ __forceinline__ C half(C a) {
+        return CFF{FF{0.5f * a.re.hi, 0.5f * a.re.lo}, FF{0.5f * a.im.hi, 0.5f * a.im.lo}};
+    }
+    static __device__ __forceinline__ S norm(C a) { return ff_add(ff_mul(a.re, a.re), ff_mul(a.im, a.im)); }
+    static __device__ __forceinline__ S addv(S a, S b) { return ff_add(a, b); }
+    static __device__ __forceinline__ S scaled(S a, uint64_t m) {
+        const float r = 1.0f / (float)m;  // exact
+        return FF{a.hi * r, a.lo * r};
+    }
     static __device__ __forceinline__ T zero() { return FF{0.f, 0.f}; }
     static __device__ __forceinline__ T add(T a, T b) { return ff_add(a, b); }
     static __device__ __forceinline__ T add_s(T a, S v) { return ff_add(a, v); }
@@ -499,6 +372,263 @@ __device__ __forceinline__ typename P::T warp_sum(typename P::T v) {
         v = P::add(v, w);
     }
     return v;  // lane 0's
+}
+
+// ---- K6: the autocorrelation by two real transforms -------------------------------------------------
+// The signal is real and its power spectrum real and even, so both transforms of length M run as complex
+// transforms of H = M / 2 points over packed pairs (even elements real parts, odd elements imaginary),
+// untangled afterwards: X[k] = E + W^k O, X[H-k] = conj(E - W^k O), E = (Z[k] + conj Z[H-k]) / 2,
+// O = (Z[k] - conj Z[H-k]) / 2i, W = exp(-2 pi i / M).
+//
+// One pass is a step of the out-of-place Stockham formulation (Govindaraju et al., "High performance
+// discrete Fourier transforms on graphics processors", SC 2008) with radix R = 16 R2 <= 256: column j
+// gathers R elements at stride H/R, twiddles them by exp(-2 pi i (j mod Ns) r / (Ns R)), transforms them
+// and scatters to (j / Ns) Ns R + (j mod Ns) + k Ns.  A block takes 256 / R2 neighbouring columns: each
+// thread does a 16-point transform in registers, the block exchanges through shared memory, and the
+// R2-point transforms finish the column, so that reads and writes of neighbouring columns coalesce and
+// 2^22 points take three passes over memory instead of six (one 16-point transform a pass) and half the
+// points.  Bound: FP64 by HBM / L2 traffic (32 bytes a point a pass), float-float by FP32 issue.
+// Both transforms with the spectrum and the autocorrelation: FP64 at 2.5e6 bins (M = 2^23) 720 -> 250 us,
+// float-float at 2.1e6 bins (M = 2^22) 1,150 -> 375 us.
+__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double2 cmul(double2 a, double2 w) {
+    return make_double2(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
+}
+__device__ __forceinline__ double2 crot(double2 a) { return make_double2(a.y, -a.x); }  // times -i
+__device__ __forceinline__ CFF cadd(CFF a, CFF b) { return cff_add(a, b); }
+__device__ __forceinline__ CFF csub(CFF a, CFF b) { return cff_sub(a, b); }
+__device__ __forceinline__ CFF cmul(CFF a, CFF w) { return cff_mul(a, w); }
+__device__ __forceinline__ CFF crot(CFF a) { return CFF{a.im, ff_neg(a.re)}; }
+// times exp(-i pi / 4) and exp(-3 i pi / 4)
+constexpr double kHalfRoot = 0.70710678118654752440;
+__device__ __forceinline__ double2 crot45(double2 a) {
+    return make_double2(kHalfRoot * (a.x + a.y), kHalfRoot * (a.y - a.x));
+}
+__device__ __forceinline__ double2 crot135(double2 a) {
+    return make_double2(kHalfRoot * (a.y - a.x), -kHalfRoot * (a.x + a.y));
+}
+__device__ __forceinline__ FF ff_const(double v) { return FF{(float)v, (float)(v - (double)(float)v)}; }
+__device__ __forceinline__ CFF crot45(CFF a) {
+    const FF h = ff_const(kHalfRoot);
+    return CFF{ff_mul(h, ff_add(a.re, a.im)), ff_mul(h, ff_sub(a.im, a.re))};
+}
+__device__ __forceinline__ CFF crot135(CFF a) {
+    const FF h = ff_const(kHalfRoot);
+    return CFF{ff_mul(h, ff_sub(a.im, a.re)), ff_neg(ff_mul(h, ff_add(a.re, a.im)))};
+}
+__device__ __forceinline__ void cset(double2& w, double c, double s) { w = make_double2(c, s); }
+__device__ __forceinline__ void cset(CFF& w, double c, double s) { w = CFF{ff_const(c), ff_const(s)}; }
+
+// b times exp(-2 pi i K / 16), K < 8.
+template <int K, class C>
+__device__ __forceinline__ C ctw16(C b) {
+    constexpr double c1 = 0.92387953251128675613, s1 = 0.38268343236508977173;  // cos, sin of pi / 8
+    if constexpr (K == 0) return b;
+    else if constexpr (K == 4) return crot(b);
+    else if constexpr (K == 2) return crot45(b);
+    else if constexpr (K == 6) return crot135(b);
+    else {
+        C w;
+        cset(w, K == 1 ? c1 : K == 3 ? s1 : K == 5 ? -s1 : -c1, (K == 1 || K == 7) ? -s1 : -c1);
+        return cmul(b, w);
+    }
+}
+template <int LEN, int K, int R, class C>
+__device__ __forceinline__ void dft_level(C* v) {
+    if constexpr (K < LEN / 2) {
+#pragma unroll
+        for (int i = 0; i < R; i += LEN) {
+            const C a = v[i + K], t = ctw16<K*(16 / LEN)>(v[i + K + LEN / 2]);
+            v[i + K] = cadd(a, t);
+            v[i + K + LEN / 2] = csub(a, t);
+        }
+        dft_level<LEN, K + 1, R>(v);
+    }
+}
+template <int LEN, int R, class C>
+__device__ __forceinline__ void dft_levels(C* v) {
+    if constexpr (LEN <= R) {
+        dft_level<LEN, 0, R>(v);
+        dft_levels<2 * LEN, R>(v);
+    }
+}
+// In-register transform of R <= 16 points (radix-2 decimation in time), natural order in and out.
+template <int R, class C>
+__device__ __forceinline__ void dft_regs(C* v) {
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        int j = 0;
+#pragma unroll
+        for (int b = 1; b < R; b <<= 1) j = (j << 1) | ((i / b) & 1);
+        if (i < j) {
+            const C t = v[i];
+            v[i] = v[j];
+            v[j] = t;
+        }
+    }
+    dft_levels<2, R>(v);
+}
+
+// exp(-2 pi i k / 256), host-computed.
+__constant__ double2 c_tw256[256];
+__constant__ CFF c_tw256f[256];
+
+// exp(-2 pi i t / M), by sincospi of the exact quotient.  The float-float path splits it in two floats
+// each (2^-49): the FP64 units stand idle there, and products of coarse and fine float-float table
+// entries cost two gathers and a complex float-float product more (114 us a pass of 2^21 points).
+template <class P>
+__device__ __forceinline__ typename P::C twiddle(uint64_t t, uint64_t M) {
+    double s, c;
+    sincospi(-2.0 * (double)t / (double)M, &s, &c);
+    if constexpr (std::is_same<P, P64>::value) return make_double2(c, s);
+    else return CFF{ff_const(c), ff_const(s)};
+}
+template <class P, int N>
+__device__ __forceinline__ typename P::C tw_inner(int k) {  // exp(-2 pi i k / N), N <= 256
+    if constexpr (std::is_same<P, P64>::value) return c_tw256[k * (256 / N)];
+    else return c_tw256f[k * (256 / N)];
+}
+
+// Element idx of the packed input: 0 a complex array, 1 a real signal of n elements (zero past them), 2
+// the power spectrum P[0 .. H], mirrored (P[M - k] = P[k]).
+template <class P, int SRC>
+__device__ __forceinline__ typename P::C fft_input(const void* __restrict__ in, uint64_t idx, uint64_t H, uint64_t n) {
+    using C = typename P::C;
+    using S = typename P::S;
+    if constexpr (SRC == 0) return reinterpret_cast<const C*>(in)[idx];
+    else {
+        const S* x = reinterpret_cast<const S*>(in);
+        const uint64_t i = 2 * idx;
+        if constexpr (SRC == 1) {
+            if (i + 1 < n) return *reinterpret_cast<const C*>(x + i);
+            return P::pack(i < n ? x[i] : P::none(), P::none());
+        } else {
+            if (i < H) return *reinterpret_cast<const C*>(x + i);  // H is even: i + 1 < H
+            return P::pack(x[2 * H - i], x[2 * H - i - 1]);
+        }
+    }
+}
+
+template <class P, int R2, int SRC>
+__global__ void __launch_bounds__(256) k_fft_pass(const void* __restrict__ in, typename P::C* __restrict__ out,
+                                                  uint64_t H, uint64_t Ns, uint64_t n) {
+    using C = typename P::C;
+    constexpr int R = 16 * R2, kCols = 256 / R2;
+    extern __shared__ __align__(16) unsigned char fft_smem[];
+    C* sm = reinterpret_cast<C*>(fft_smem);
+    const uint64_t stride = H / R, j0 = blockIdx.x * (uint64_t)kCols;
+    {
+        const int c = threadIdx.x % kCols, b = threadIdx.x / kCols;
+        const uint64_t j = j0 + c;
+        C v[16];
+        if (j < stride) {
+#pragma unroll
+            for (int a = 0; a < 16; a++) v[a] = fft_input<P, SRC>(in, j + (uint64_t)(b + R2 * a) * stride, H, n);
+            if constexpr (SRC == 0) {
+                const uint64_t k = j & (Ns - 1);
+#pragma unroll
+                for (int a = 0; a < 16; a++)
+                    v[a] = cmul(v[a], twiddle<P>(k * (uint64_t)(b + R2 * a), Ns * R));
+            }
+        } else {
+#pragma unroll
+            for (int a = 0; a < 16; a++) v[a] = P::pack(P::none(), P::none());
+        }
+        dft_regs<16>(v);
+#pragma unroll
+        for (int a = 0; a < 16; a++) sm[(b * 16 + a) * kCols + c] = (a && R2 > 1) ? cmul(v[a], tw_inner<P, R>(b * a)) : v[a];
+    }
+    __syncthreads();
+    C y[16];
+#pragma unroll
+    for (int e = 0; e < 16 / R2; e++) {
+        const int d = threadIdx.x + 256 * e, a = d / kCols, c = d % kCols;
+#pragma unroll
+        for (int b = 0; b < R2; b++) y[e * R2 + b] = sm[(b * 16 + a) * kCols + c];
+        dft_regs<R2>(y + e * R2);
+    }
+    if constexpr (SRC == 0) {
+#pragma unroll
+        for (int e = 0; e < 16 / R2; e++) {
+            const int d = threadIdx.x + 256 * e, a = d / kCols, c = d % kCols;
+            const uint64_t j = j0 + c;
+            if (j < stride) {
+                const uint64_t k = j & (Ns - 1);
+                C* o = out + (j - k) * R + k;
+#pragma unroll
+                for (int b = 0; b < R2; b++) o[(uint64_t)(a + 16 * b) * Ns] = y[e * R2 + b];
+            }
+        }
+    } else {
+        // first pass (Ns = 1): a column's outputs are consecutive; stored through shared memory, column
+        // by column (one element of padding each)
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 16 / R2; e++) {
+            const int d = threadIdx.x + 256 * e, a = d / kCols, c = d % kCols;
+#pragma unroll
+            for (int b = 0; b < R2; b++) sm[c * (R + 1) + a + 16 * b] = y[e * R2 + b];
+        }
+        __syncthreads();
+        for (int x = threadIdx.x; x < kCols * R; x += 256) {
+            const int c = x / R, k = x % R;
+            if (j0 + c < stride) out[j0 * R + x] = sm[c * (R + 1) + k];
+        }
+    }
+}
+
+// Transforms of at most 16 points: one thread.
+template <class P, int R, int SRC>
+__global__ void k_fft_small(const void* __restrict__ in, typename P::C* __restrict__ out, uint64_t n) {
+    typename P::C v[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) v[r] = fft_input<P, SRC>(in, r, R, n);
+    dft_regs<R>(v);
+#pragma unroll
+    for (int r = 0; r < R; r++) out[r] = v[r];
+}
+
+// E and T = W^k O of the pair (k, H - k), 0 < k <= H / 2.
+template <class P>
+__device__ __forceinline__ void untangle(const typename P::C* __restrict__ Z, uint64_t k, uint64_t H,
+                                         typename P::C& E, typename P::C& T) {
+    using C = typename P::C;
+    const C a = Z[k], b = P::conj(Z[H - k]);
+    E = P::half(cadd(a, b));
+    T = cmul(crot(P::half(csub(a, b))), twiddle<P>(k, 2 * H));  // D / 2i = -i D / 2
+}
+
+// The power spectrum P[0 .. H] of the packed transform Z.
+template <class P>
+__global__ void k_power(uint64_t H, const typename P::C* __restrict__ Z, typename P::S* __restrict__ pw) {
+    const uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (k > H / 2) return;
+    if (k == 0) {
+        const typename P::S s = P::addv(P::re(Z[0]), P::im(Z[0])), d = P::sub(P::re(Z[0]), P::im(Z[0]));
+        pw[0] = P::mul(s, s);
+        pw[H] = P::mul(d, d);
+        return;
+    }
+    typename P::C E, T;
+    untangle<P>(Z, k, H, E, T);
+    pw[k] = P::norm(cadd(E, T));
+    pw[H - k] = P::norm(csub(E, T));
+}
+
+// A[m] = Re FFT(P)[m] / M for m < n, from the packed transform Q of the spectrum.
+template <class P>
+__global__ void k_autocorr(uint64_t H, uint64_t n, const typename P::C* __restrict__ Q, typename P::S* __restrict__ A) {
+    const uint64_t m = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (m > H / 2) return;
+    if (m == 0) {
+        A[0] = P::scaled(P::addv(P::re(Q[0]), P::im(Q[0])), 2 * H);
+        return;
+    }
+    typename P::C E, T;
+    untangle<P>(Q, m, H, E, T);
+    if (m < n) A[m] = P::scaled(P::addv(P::re(E), P::re(T)), 2 * H);
+    if (H - m < n) A[H - m] = P::scaled(P::sub(P::re(E), P::re(T)), 2 * H);
 }
 
 // What the passes over one signal share, on the device.
@@ -665,7 +795,7 @@ __global__ void __launch_bounds__(kSigThreads) k_center(uint64_t n, const float*
     for (int k = 0; k < kSigItems; k++) {
         if (base + k >= n) break;
         run = P::add_s(run, u[k]);
-        x[2 * (base + k)] = u[k];  // the real parts of a complex signal
+        x[base + k] = u[k];
         if constexpr (std::is_same<P, P64>::value) U[base + k + 1] = run.hi + run.lo;
         else U[base + k + 1] = run;
     }
@@ -856,18 +986,29 @@ using namespace rgl;
 // Per-build device workspace (grown on demand) and the host twiddle table.
 namespace {
 struct MomentWs {
-    DevBuf iv, key_a, key_b, val_a, val_b, g, totals, nz, idx, cum, cnt, fa, fb, U, A, sums, state, direct, gl, tmp,
-        tw, mv;
+    DevBuf iv, key_a, key_b, val_a, val_b, g, totals, nz, idx, cum, cnt, fa, fb, pw, U, A, sums, state, direct, gl, tmp,
+        mv;
 };
 std::mutex g_ws_mu;
 MomentWs g_ws[16];  // one workspace per device ordinal
 bool g_tw_ready[64] = {false};
 
+// The constant tables exp(-2 pi i k / 256) of both arithmetics, once per device.
 int upload_twiddles(int device) {
     if (device >= 0 && device < 64 && g_tw_ready[device]) return RGL_OK;
-    double2 tw[16];
-    for (int k = 0; k < 16; k++) tw[k] = make_double2(std::cos(2.0 * M_PI * k / 16.0), -std::sin(2.0 * M_PI * k / 16.0));
-    RGL_CUDA(cudaMemcpyToSymbol(c_tw16, tw, sizeof(tw)));
+    double2 tw[256];
+    float twf[256][4];
+    for (int k = 0; k < 256; k++) {
+        const long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)k / 256.0L;
+        const long double v[2] = {cosl(a), sinl(a)};
+        tw[k] = make_double2((double)v[0], (double)v[1]);
+        for (int h = 0; h < 2; h++) {  // float-float: hi = nearest float, lo = nearest float of the remainder
+            twf[k][2 * h] = (float)v[h];
+            twf[k][2 * h + 1] = (float)(v[h] - (long double)twf[k][2 * h]);
+        }
+    }
+    RGL_CUDA(cudaMemcpyToSymbol(c_tw256, tw, sizeof(tw)));
+    RGL_CUDA(cudaMemcpyToSymbol(c_tw256f, twf, sizeof(twf)));
     if (device >= 0 && device < 64) g_tw_ready[device] = true;
     return RGL_OK;
 }
@@ -927,100 +1068,58 @@ int depth_signal_dev(MomentWs& w, const rgl_interval* h_iv, uint64_t n, uint64_t
     return RGL_OK;
 }
 
-int fft_forward(MomentWs& w, uint64_t M, cudaStream_t st, double2** result) {
-    // ping-pong between fa and fb; input in fa
-    double2* src = w.fa.as<double2>();
-    double2* dst = w.fb.as<double2>();
-    uint64_t Ns = 1;
-    int logm = 0;
-    while ((1ull << logm) < M) logm++;
-    int rem = logm;
-    while (rem > 0) {
-        const int r = rem >= 4 ? 4 : rem;
-        const uint64_t threads = M >> r;
-        switch (r) {
-            case 4: k_fft_pass<16><<<blocks_for(threads), 256, 0, st>>>(src, dst, M, Ns); break;
-            case 3: k_fft_pass<8><<<blocks_for(threads), 256, 0, st>>>(src, dst, M, Ns); break;
-            case 2: k_fft_pass<4><<<blocks_for(threads), 256, 0, st>>>(src, dst, M, Ns); break;
-            default: k_fft_pass<2><<<blocks_for(threads), 256, 0, st>>>(src, dst, M, Ns); break;
-        }
-        Ns <<= r;
-        rem -= r;
-        std::swap(src, dst);
-    }
-    RGL_CUDA(cudaGetLastError());
-    *result = src;
+template <class P, int R2, int SRC>
+int fft_pass(const void* in, typename P::C* out, uint64_t H, uint64_t Ns, uint64_t n, cudaStream_t st) {
+    constexpr int R = 16 * R2, kCols = 256 / R2;
+    constexpr int smem = (SRC ? kCols * (R + 1) : kCols * R) * (int)sizeof(typename P::C);  // 64 to 68 KB
+    RGL_CUDA(cudaFuncSetAttribute(k_fft_pass<P, R2, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_fft_pass<P, R2, SRC><<<(unsigned)((H / R + kCols - 1) / kCols), 256, smem, st>>>(in, out, H, Ns, n);
     return RGL_OK;
 }
 
-}  // namespace
-
-namespace {
-// Float-float value of a long double: hi = nearest float, lo = nearest float of the remainder.
-inline void ff_of(long double v, float* hi, float* lo) {
-    *hi = (float)v;
-    *lo = (float)(v - (long double)*hi);
-}
-
-bool g_tw16f_ready[64] = {false};
-
-// exp(-2 pi i t / M) for t = (c << tb) (coarse table) and t < 2^tb (fine table), float-float, host-made
-// in extended precision; the radix-16 constants once per device.
-int ff_twiddles(MomentWs& w, uint64_t M, int device, int* tb_out) {
-    if (device >= 0 && device < 64 && !g_tw16f_ready[device]) {
-        float h[64];
-        for (int k = 0; k < 16; k++) {
-            const long double a = -2.0L * (long double)M_PI * (long double)k / 16.0L;
-            ff_of(cosl(a), &h[4 * k], &h[4 * k + 1]);
-            ff_of(sinl(a), &h[4 * k + 2], &h[4 * k + 3]);
+// Transform of H packed points; the first pass reads `first` (SRC 1: a real signal of n elements, 2: the
+// spectrum), the others go between w.fa and w.fb.  *result is one of the two.
+template <class P, int SRC>
+int fft_forward(MomentWs& w, const void* first, uint64_t H, uint64_t n, cudaStream_t st,
+                typename P::C** result) {
+    using C = typename P::C;
+    C *dst = w.fa.as<C>(), *src = w.fb.as<C>();
+    int h = 0;
+    while ((1ull << h) < H) h++;
+    if (h <= 4) {
+        switch (h) {
+            case 4: k_fft_small<P, 16, SRC><<<1, 1, 0, st>>>(first, dst, n); break;
+            case 3: k_fft_small<P, 8, SRC><<<1, 1, 0, st>>>(first, dst, n); break;
+            case 2: k_fft_small<P, 4, SRC><<<1, 1, 0, st>>>(first, dst, n); break;
+            default: k_fft_small<P, 2, SRC><<<1, 1, 0, st>>>(first, dst, n); break;
         }
-        RGL_CUDA(cudaMemcpyToSymbol(c_tw16f, h, sizeof(h)));
-        g_tw16f_ready[device] = true;
+        *result = dst;
+        return RGL_OK;
     }
-    int logm = 0;
-    while ((1ull << logm) < M) logm++;
-    const int tb = (logm + 1) / 2;
-    const uint64_t nf = 1ull << tb, nc = (M >> tb) + 1;
-    std::vector<float> h(4 * (nf + nc));
-    const long double pi2 = 2.0L * 3.141592653589793238462643383279502884L;
-    for (uint64_t t = 0; t < nf; t++) {
-        const long double a = -pi2 * (long double)t / (long double)M;
-        ff_of(cosl(a), &h[4 * t], &h[4 * t + 1]);
-        ff_of(sinl(a), &h[4 * t + 2], &h[4 * t + 3]);
-    }
-    for (uint64_t c = 0; c < nc; c++) {
-        const long double a = -pi2 * (long double)(c << tb) / (long double)M;
-        float* q = &h[4 * (nf + c)];
-        ff_of(cosl(a), &q[0], &q[1]);
-        ff_of(sinl(a), &q[2], &q[3]);
-    }
-    RGL_TRY(w.tw.ensure(h.size() * 4));
-    RGL_CUDA(cudaMemcpy(w.tw.p, h.data(), h.size() * 4, cudaMemcpyHostToDevice));
-    *tb_out = tb;
-    return RGL_OK;
-}
-
-int ff_fft_forward(MomentWs& w, uint64_t M, int tb, cudaStream_t st, CFF** result) {
-    CFF* src = reinterpret_cast<CFF*>(w.fa.p);
-    CFF* dst = reinterpret_cast<CFF*>(w.fb.p);
-    const CFF* wf = reinterpret_cast<const CFF*>(w.tw.p);
-    const CFF* wc = wf + (1ull << tb);
+    // radices of 2^4 to 2^8, as even as possible, the larger ones first
+    const int passes = (h + 7) / 8, base = h / passes, more = h % passes;
     uint64_t Ns = 1;
-    int logm = 0;
-    while ((1ull << logm) < M) logm++;
-    int rem = logm;
-    while (rem > 0) {
-        const int r = rem >= 4 ? 4 : rem;
-        const uint64_t threads = M >> r;
-        const unsigned blocks = (unsigned)((threads + 127) / 128);
-        switch (r) {
-            case 4: k_ff_fft_pass<16><<<blocks, 128, 0, st>>>(src, dst, M, Ns, wc, wf, tb); break;
-            case 3: k_ff_fft_pass<8><<<blocks, 128, 0, st>>>(src, dst, M, Ns, wc, wf, tb); break;
-            case 2: k_ff_fft_pass<4><<<blocks, 128, 0, st>>>(src, dst, M, Ns, wc, wf, tb); break;
-            default: k_ff_fft_pass<2><<<blocks, 128, 0, st>>>(src, dst, M, Ns, wc, wf, tb); break;
+    for (int p = 0; p < passes; p++) {
+        const int r = base + (p < more ? 1 : 0);
+        int s = RGL_OK;
+        if (p == 0) {
+            switch (r) {
+                case 8: s = fft_pass<P, 16, SRC>(first, dst, H, Ns, n, st); break;
+                case 7: s = fft_pass<P, 8, SRC>(first, dst, H, Ns, n, st); break;
+                case 6: s = fft_pass<P, 4, SRC>(first, dst, H, Ns, n, st); break;
+                default: s = fft_pass<P, 2, SRC>(first, dst, H, Ns, n, st); break;  // h >= 5: r >= 5
+            }
+        } else {
+            switch (r) {
+                case 8: s = fft_pass<P, 16, 0>(src, dst, H, Ns, n, st); break;
+                case 7: s = fft_pass<P, 8, 0>(src, dst, H, Ns, n, st); break;
+                case 6: s = fft_pass<P, 4, 0>(src, dst, H, Ns, n, st); break;
+                case 5: s = fft_pass<P, 2, 0>(src, dst, H, Ns, n, st); break;
+                default: s = fft_pass<P, 1, 0>(src, dst, H, Ns, n, st); break;
+            }
         }
+        RGL_TRY(s);
         Ns <<= r;
-        rem -= r;
         std::swap(src, dst);
     }
     RGL_CUDA(cudaGetLastError());
@@ -1031,15 +1130,19 @@ int ff_fft_forward(MomentWs& w, uint64_t M, int tb, cudaStream_t st, CFF** resul
 // K5-K7 for the depth signal in w.g (N bins): the moments of the L grid (G points, on the device at
 // w.gl) into `table` and, where given, d_mean / d_var.
 template <class P>
-int moments_dev(MomentWs& w, uint64_t N, uint64_t M, int device, const std::vector<uint64_t>& grid, float2* table,
-                double* d_mean, double* d_var, cudaStream_t st) {
+int moments_dev(MomentWs& w, uint64_t N, const std::vector<uint64_t>& grid, float2* table, double* d_mean,
+                double* d_var, cudaStream_t st) {
     using S = typename P::S;
+    using C = typename P::C;
     using T = typename P::T;
     constexpr bool kFF = std::is_same<P, PFF>::value;
     const uint32_t G = (uint32_t)grid.size();
     const uint64_t nt = (N + kSigTile - 1) / kSigTile, mt = N / kTermTile + 1;  // tiles of g and of the terms (0 .. N)
-    RGL_TRY(w.fa.ensure(M * 16));
-    RGL_TRY(w.fb.ensure(M * 16));
+    uint64_t H = 1;  // packed points: half of the smallest power of two at or above 2 N
+    while (H < N) H <<= 1;
+    RGL_TRY(w.fa.ensure(H * 16));
+    RGL_TRY(w.fb.ensure(H * 16));
+    RGL_TRY(w.pw.ensure((H + 2) * sizeof(S)));
     RGL_TRY(w.U.ensure((N + 2) * sizeof(S)));
     RGL_TRY(w.A.ensure((N + 2) * sizeof(S)));
     RGL_TRY(w.sums.ensure((2 * nt + kTerms * (mt + 1) + 4) * sizeof(T)));
@@ -1051,8 +1154,6 @@ int moments_dev(MomentWs& w, uint64_t N, uint64_t M, int device, const std::vect
     const uint64_t most = first < G ? N - grid[first] + 1 : 0;
     const uint32_t parts = (uint32_t)std::min<uint64_t>(64, (most + 2047) / 2048);
     RGL_TRY(w.direct.ensure(std::max<uint64_t>(1, (uint64_t)(G - first) * parts) * 2 * sizeof(DD)));
-    int tb = 0;
-    if constexpr (kFF) RGL_TRY(ff_twiddles(w, M, device, &tb));
     const float* g = w.g.as<float>();
     const uint64_t* d_grid = w.gl.as<uint64_t>();
     MomentState* ms = w.state.as<MomentState>();
@@ -1069,25 +1170,15 @@ int moments_dev(MomentWs& w, uint64_t N, uint64_t M, int device, const std::vect
         k_u_tiles<<<(unsigned)nt, kSigThreads, 0, st>>>(N, g, ms, usum);
         k_u_tops<<<1, 1024, 0, st>>>(nt, usum);
     }
-    RGL_CUDA(cudaMemsetAsync(w.fa.p, 0, M * 16, st));
-    k_center<P><<<(unsigned)nt, kSigThreads, 0, st>>>(N, g, ms, usum, w.fa.as<S>(), U);
+    S* x = A;  // the signal, read by the transform's first pass
+    k_center<P><<<(unsigned)nt, kSigThreads, 0, st>>>(N, g, ms, usum, x, U);
     // K6: A[m] = Re(FFT(|FFT(u)|^2))[m] / M
-    const double inv_m = 1.0 / (double)M;
-    if constexpr (kFF) {
-        CFF *X = nullptr, *Y = nullptr;
-        RGL_TRY(ff_fft_forward(w, M, tb, st, &X));
-        k_ff_power<<<blocks_for(M), 256, 0, st>>>(M, X);
-        if (X != w.fa.as<CFF>()) RGL_CUDA(cudaMemcpyAsync(w.fa.p, X, M * 16, cudaMemcpyDeviceToDevice, st));
-        RGL_TRY(ff_fft_forward(w, M, tb, st, &Y));
-        k_ff_autocorr<<<blocks_for(N), 256, 0, st>>>(N, Y, (float)inv_m, A);
-    } else {
-        double2 *X = nullptr, *Y = nullptr;
-        RGL_TRY(fft_forward(w, M, st, &X));
-        k_power<<<blocks_for(M), 256, 0, st>>>(M, X);
-        if (X != w.fa.as<double2>()) RGL_CUDA(cudaMemcpyAsync(w.fa.p, X, M * 16, cudaMemcpyDeviceToDevice, st));
-        RGL_TRY(fft_forward(w, M, st, &Y));
-        k_autocorr<<<blocks_for(N), 256, 0, st>>>(N, Y, inv_m, A);
-    }
+    C *Z = nullptr, *Q = nullptr;
+    S* pw = w.pw.as<S>();
+    RGL_TRY((fft_forward<P, 1>(w, x, H, N, st, &Z)));
+    k_power<P><<<blocks_for(H / 2 + 1), 256, 0, st>>>(H, Z, pw);
+    RGL_TRY((fft_forward<P, 2>(w, pw, H, 0, st, &Q)));
+    k_autocorr<P><<<blocks_for(H / 2 + 1), 256, 0, st>>>(H, N, Q, A);
     // K7
     k_term_tiles<P><<<(unsigned)mt, kTermThreads, 0, st>>>(N, mt, A, U, terms);
     k_term_tops<P><<<kTerms, 1024, 0, st>>>(mt, terms, totals);
@@ -1148,8 +1239,6 @@ int rgl_moments_build_ex(rgl_moments* m, uint32_t sid, uint32_t chrom, const rgl
     cudaStream_t st = 0;
     RGL_TRY(upload_twiddles(device));
     RGL_TRY(depth_signal_dev(w, intervals, n, N, bin_size, st));
-    uint64_t M = 1;
-    while (M < 2 * N) M <<= 1;
     // K7 points: the L grid of the store
     const std::vector<uint64_t> grid = moment_grid(N);
     const uint32_t G = (uint32_t)grid.size();
@@ -1159,8 +1248,8 @@ int rgl_moments_build_ex(rgl_moments* m, uint32_t sid, uint32_t chrom, const rgl
     RGL_TRY(w.mv.ensure(G * 16ull + 64));
     double* d_mean = mean_out ? w.mv.as<double>() : nullptr;
     double* d_var = var_out ? w.mv.as<double>() + G : nullptr;
-    if (precision == RGL_MOM_FP32C) RGL_TRY(moments_dev<PFF>(w, N, M, device, grid, table, d_mean, d_var, st));
-    else RGL_TRY(moments_dev<P64>(w, N, M, device, grid, table, d_mean, d_var, st));
+    if (precision == RGL_MOM_FP32C) RGL_TRY(moments_dev<PFF>(w, N, grid, table, d_mean, d_var, st));
+    else RGL_TRY(moments_dev<P64>(w, N, grid, table, d_mean, d_var, st));
     if (mean_out) RGL_CUDA(cudaMemcpyAsync(mean_out, d_mean, G * 8, cudaMemcpyDeviceToHost, st));
     if (var_out) RGL_CUDA(cudaMemcpyAsync(var_out, d_var, G * 8, cudaMemcpyDeviceToHost, st));
     RGL_CUDA(cudaStreamSynchronize(st));
