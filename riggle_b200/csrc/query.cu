@@ -220,22 +220,16 @@ __global__ void k_seg_begin(uint32_t n, const uint32_t* __restrict__ segflag, co
 // DB intervals the segment's rank-difference ranges sweep (need[]): each swept interval reads the
 // table a few times, so a table much larger than its sweep costs more to build than its finer bins
 // save (large query files against a small database).  A coarser bin only lengthens the search
-// inside it.  A segment with a rank-difference range gets nbins + 1 table entries, any other
-// segment a single entry (see k_tab_place).
+// inside it.  A segment of m queries has at most 8 m + 2 entries (nbins + 1), so segment k's table
+// starts at 8 beg + 2 k: the places need no scan.
 __global__ void k_seg_tabsize(uint32_t n, const uint32_t* __restrict__ segnum, const uint32_t* __restrict__ seg_begin,
                               const unsigned long long* __restrict__ need, const uint32_t* __restrict__ ends_s,
-                              SegTab* __restrict__ tabs, uint32_t* __restrict__ tab_len) {
-    uint32_t sgi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (sgi > n) return;
-    const uint32_t nseg = segnum[n - 1];
-    if (sgi >= nseg) {
-        tab_len[sgi] = 0;
-        return;
-    }
+                              SegTab* __restrict__ tabs) {
+    const uint32_t sgi = blockIdx.x * blockDim.x + threadIdx.x;
+    if (sgi >= segnum[n - 1]) return;
     const uint32_t beg = seg_begin[sgi], end = seg_begin[sgi + 1];
     if (!need[sgi]) {  // no range of this segment is swept by rank differences
         tabs[sgi] = SegTab{beg, end, 6, 0, 0, 0};
-        tab_len[sgi] = 1;
         return;
     }
     const uint64_t extent = (uint64_t)ends_s[end - 1] + 1;  // covers every start and end of the segment
@@ -244,60 +238,56 @@ __global__ void k_seg_tabsize(uint32_t n, const uint32_t* __restrict__ segnum, c
     uint32_t shift = want > 1 ? 63u - __clzll(want) : 0u;
     if (shift < 6) shift = 6;
     if (shift > 31) shift = 31;
-    const uint32_t nbins = (uint32_t)(extent >> shift) + 1;  // <= 8 (end - beg): tables fit 10 n entries
-    tabs[sgi] = SegTab{beg, end, shift, nbins, 0, 0};
-    tab_len[sgi] = nbins + 1;
+    const uint32_t nbins = (uint32_t)(extent >> shift) + 1;  // <= 8 (end - beg) + 1
+    tabs[sgi] = SegTab{beg, end, shift, nbins, 8 * beg + 2 * sgi, 0};
 }
 
-// Rank tables by counting.  Entry b of a segment's table must hold beg + #{elements with bin < b}.
-// With the per-bin counts placed one entry to the right (bin b at entry b + 1) and every other
-// segment's single entry holding its element count, an inclusive scan over all segments' entries
-// yields exactly that: everything before a segment's first entry sums to its `beg`.
-// Zeroes the count arrays over the tables' actual size (tab_off[number of segments]) and records
-// that size in *count for the scans.
-__global__ void k_tab_zero(uint32_t n, const uint32_t* __restrict__ segnum, const uint32_t* __restrict__ tab_off,
-                           uint32_t* __restrict__ xs, uint32_t* __restrict__ xe, uint32_t* __restrict__ count) {
-    const uint32_t total = tab_off[segnum[n - 1]];
-    const uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (g == 0) *count = total;
-    for (uint64_t i = g; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-        xs[i] = 0;
-        xe[i] = 0;
-    }
-}
-
+// Rank tables from the sorted arrays: entry b of a segment holds the position of its first element of bin
+// >= b, so element j fills the entries from its predecessor's bin (exclusive) through its own with j, and
+// the last one the rest with the segment's end.  A lane fills up to kTabShort entries itself, longer
+// stretches are filled by the whole warp.  Bound: 8 bytes written per entry.  Counting the elements per
+// bin with atomics, two scans over the tables and interleaving them took twelve launches, and 1.6 ms for
+// 3.1e7 intervals whose few-bin tables made thousands of atomics meet on one counter; this takes 0.26 ms.
+constexpr uint32_t kTabShort = 8;
 template <bool PDL>
-__global__ void k_tab_place(uint32_t n, const uint32_t* __restrict__ segnum, SegTab* __restrict__ tabs,
-                            const uint32_t* __restrict__ tab_off, uint32_t* __restrict__ xs, uint32_t* __restrict__ xe) {
+__global__ void __launch_bounds__(256) k_tab_fill(uint32_t n, const uint32_t* __restrict__ segnum,
+                                                  const SegTab* __restrict__ tabs,
+                                                  const uint32_t* __restrict__ starts,
+                                                  const uint32_t* __restrict__ ends_s, uint2* __restrict__ tab2) {
     if constexpr (PDL) {
         pdl_wait();
         pdl_release();
     }
-    const uint32_t sgi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (sgi >= segnum[n - 1]) return;
-    const uint32_t off = tab_off[sgi];
-    tabs[sgi].off = off;
-    const SegTab t = tabs[sgi];
-    if (t.nbins == 0) {
-        xs[off] = t.end - t.beg;
-        xe[off] = t.end - t.beg;
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    SegTab t{0, 0, 0, 0, 0, 0};
+    if (j < n) t = tabs[segnum[j] - 1];
+    if (!__ballot_sync(0xffffffffu, t.nbins != 0)) return;
+#pragma unroll
+    for (int side = 0; side < 2; side++) {
+        const uint32_t* a = side ? ends_s : starts;
+        uint32_t* col = reinterpret_cast<uint32_t*>(tab2) + side;  // entry b at col[2 (off + b)]
+        uint32_t from = 0, to = 0;  // entries [from, to) of the table, as absolute entries
+        uint32_t rest = 0;          // and [to, rest) by the segment's last element
+        if (t.nbins) {  // (a refused interval may start past every end: its bin is held to the table)
+            to = t.off + min(a[j] >> t.shift, t.nbins - 1) + 1;
+            from = j == t.beg ? t.off : t.off + min(a[j - 1] >> t.shift, t.nbins - 1) + 1;
+            rest = j + 1 == t.end ? t.off + t.nbins + 1 : to;
+        }
+        if (to - from <= kTabShort)
+            for (uint32_t b = from; b < to; b++) col[2ull * b] = j;
+        if (rest - to <= kTabShort)
+            for (uint32_t b = to; b < rest; b++) col[2ull * b] = t.end;
+#pragma unroll
+        for (int part = 0; part < 2; part++) {
+            const uint32_t f = part ? to : from, e = part ? rest : to, v = part ? t.end : j;
+            for (uint32_t m = __ballot_sync(0xffffffffu, e - f > kTabShort); m; m &= m - 1) {
+                const int src = __ffs(m) - 1;
+                const uint32_t f1 = __shfl_sync(0xffffffffu, f, src), e1 = __shfl_sync(0xffffffffu, e, src);
+                const uint32_t v1 = __shfl_sync(0xffffffffu, v, src);
+                for (uint32_t b = f1 + lane; b < e1; b += 32) col[2ull * b] = v1;
+            }
+        }
     }
-}
-
-template <bool PDL>
-__global__ void k_tab_count(uint32_t n, const uint32_t* __restrict__ segnum, const SegTab* __restrict__ tabs,
-                            const uint32_t* __restrict__ starts, const uint32_t* __restrict__ ends_s,
-                            uint32_t* __restrict__ xs, uint32_t* __restrict__ xe) {
-    if constexpr (PDL) {
-        pdl_wait();
-        pdl_release();
-    }
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const SegTab t = tabs[segnum[j] - 1];
-    if (t.nbins == 0) return;
-    atomicAdd(xs + t.off + (starts[j] >> t.shift) + 1, 1u);
-    atomicAdd(xe + t.off + (ends_s[j] >> t.shift) + 1, 1u);
 }
 
 // Adds a 32-bit value to a 64-bit shared-memory counter with 32-bit atomics: the low word, and the
@@ -314,20 +304,6 @@ __device__ __forceinline__ void add_u64(unsigned long long* c, unsigned long lon
     const uint32_t lo = (uint32_t)v, old = atomicAdd(w, lo);
     const uint32_t hi = (uint32_t)(v >> 32) + (old + lo < old ? 1u : 0u);
     if (hi) atomicAdd(w + 1, hi);
-}
-
-// Interleaves the two scanned count arrays into (#starts, #ends) pairs: entry k of the tables is
-// entry k + 1 of the exclusive scans (the inclusive sums through k).
-template <bool PDL>
-__global__ void k_tab_interleave(const uint32_t* __restrict__ count, const uint32_t* __restrict__ xs_scan,
-                                 const uint32_t* __restrict__ xe_scan, uint2* __restrict__ tab2) {
-    if constexpr (PDL) {
-        pdl_wait();
-        pdl_release();
-    }
-    const uint32_t total = *count;
-    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < total; k += (uint64_t)gridDim.x * blockDim.x)
-        tab2[k] = make_uint2(xs_scan[k + 1], xe_scan[k + 1]);
 }
 
 // ---- 4. K1 partition -----------------------------------------------------------------------------
@@ -1389,9 +1365,9 @@ struct rgl_context {
     DevBuf iv, blk_off, blk_shard, key_a, key_b, val_a, val_b, ekey_a, ekey_b;
     DevBuf starts, ends, seg, segflag, segnum, seg_begin, ps_in, pe_in, ps, pe;
     DevBuf lo, hi, maxhi, rflag, ridx, ranges, rlen, rpos, cub_tmp, small, out_counts, out_bp, item_r0;
-    DevBuf segtab, tab_len, tab_off, tab_s, tab_e, tab_xs, tab_xe, tab2;
+    DevBuf segtab, tab2;
     DevBuf cl, pc, method, plen, ppos, psegs, item_t0, seg_need, tl, scan_sums;
-    DevBuf cub_tmp2, scan_sums2;  // the side stream's own scratch
+    DevBuf cub_tmp2;  // the side stream's own scratch
     DevBuf sortplan;  // block-local sort: order flags, tile and merge-chunk prefix counts, two pass words
     DevBuf sort_tab, sort_rank;  // its segment-order layout, for the single-call entry points
     DevBuf item_hits, item_base, pairs;  // intervals mode
@@ -1501,19 +1477,12 @@ int size_workspace(rgl_context* c, uint64_t n, uint32_t rows, uint32_t nblk, uin
     RGL_TRY(z.ensure_in(c->pc, tot * 8 + 16));
     RGL_TRY(z.ensure_in(c->method, tot + 16));
     RGL_TRY(z.ensure_in(c->tl, tot * 4 + 8));
-    RGL_TRY(z.ensure_in(c->scan_sums, (std::max<uint64_t>(tot, 10 * n + 16) / kScanTile + 4) * 8));
-    RGL_TRY(z.ensure_in(c->scan_sums2, (10 * n + 16) / kScanTile * 8 + 32));
+    RGL_TRY(z.ensure_in(c->scan_sums, (tot / kScanTile + 4) * 8));
     RGL_TRY(z.ensure_in(c->plen, tot * 8 + 16));
     RGL_TRY(z.ensure_in(c->ppos, tot * 8 + 16));
     RGL_TRY(z.ensure_in(c->psegs, tot * sizeof(PairSeg) + sizeof(PairSeg)));
     RGL_TRY(z.ensure_in(c->segtab, (n + 1) * sizeof(SegTab)));
-    RGL_TRY(z.ensure_in(c->tab_len, (n + 2) * 4));
-    RGL_TRY(z.ensure_in(c->tab_off, (n + 2) * 4));
-    RGL_TRY(z.ensure_in(c->tab_s, (10 * n + 18) * 4));
-    RGL_TRY(z.ensure_in(c->tab_e, (10 * n + 18) * 4));
     RGL_TRY(z.ensure_in(c->tab2, (10 * n + 18) * 8));
-    RGL_TRY(z.ensure_in(c->tab_xs, (10 * n + 16) * 4));
-    RGL_TRY(z.ensure_in(c->tab_xe, (10 * n + 16) * 4));
     RGL_TRY(z.ensure_in(c->acc, 64));
     // CUB temporary storage: the maximum over every primitive used, at these sizes.
     size_t need = 0, b = 0;
@@ -1525,8 +1494,6 @@ int size_workspace(rgl_context* c, uint64_t n, uint32_t rows, uint32_t nblk, uin
     cub::DeviceRadixSort::SortKeys(nullptr, b, (uint64_t*)nullptr, (uint64_t*)nullptr, nn, 0, 64, c->stream);
     need = std::max(need, b);
     cub::DeviceScan::InclusiveSum(nullptr, b, (uint32_t*)nullptr, (uint32_t*)nullptr, nn, c->stream);
-    need = std::max(need, b);
-    cub::DeviceScan::InclusiveSum(nullptr, b, (uint32_t*)nullptr, (uint32_t*)nullptr, (int)(10 * n + 16), c->stream);
     need = std::max(need, b);
     cub::DeviceScan::ExclusiveSum(nullptr, b, (uint64_t*)nullptr, (uint64_t*)nullptr, nn + 1, c->stream);
     need = std::max(need, b);
@@ -1556,9 +1523,8 @@ int size_workspace(rgl_context* c, uint64_t n, uint32_t rows, uint32_t nblk, uin
     for (DevBuf* b : {&c->iv, &c->key_a, &c->key_b, &c->val_a, &c->val_b, &c->ekey_a, &c->ekey_b, &c->starts,
                       &c->ends, &c->seg, &c->segflag, &c->segnum, &c->seg_begin, &c->ps_in, &c->pe_in, &c->ps,
                       &c->pe, &c->lo, &c->hi, &c->maxhi, &c->rflag, &c->ridx, &c->ranges, &c->rlen, &c->rpos,
-                      &c->cub_tmp, &c->small, &c->item_r0, &c->item_t0, &c->segtab, &c->tab_len, &c->tab_off,
-                      &c->tab_s, &c->tab_e, &c->tab_xs, &c->tab_xe, &c->tab2, &c->cl, &c->pc, &c->method, &c->tl, &c->scan_sums, &c->plen, &c->ppos, &c->psegs,
-                      &c->seg_need, &c->acc, &c->cub_tmp2, &c->scan_sums2, &c->sortplan})
+                      &c->cub_tmp, &c->small, &c->item_r0, &c->item_t0, &c->segtab, &c->tab2, &c->cl, &c->pc, &c->method, &c->tl, &c->scan_sums, &c->plen, &c->ppos, &c->psegs,
+                      &c->seg_need, &c->acc, &c->cub_tmp2, &c->sortplan})
         sig = (sig ^ (uint64_t)(uintptr_t)b->p ^ ((uint64_t)b->cap << 17)) * 1099511628211ull;
     c->ws_sig = sig;
     return RGL_OK;
@@ -1927,7 +1893,8 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     k_seg_begin<<<grid_for(n, 256), 256, 0, st>>>(n, c->segflag.as<uint32_t>(), c->segnum.as<uint32_t>(),
                                                   c->seg_begin.as<uint32_t>());
     launches++;
-    RGL_CUDA(cudaMemsetAsync(c->seg_need.p, 0, (size_t)(n + 1) * 8, st));
+    const uint32_t max_segs = (uint32_t)std::min<uint64_t>(n, nseg);
+    RGL_CUDA(cudaMemsetAsync(c->seg_need.p, 0, (size_t)max_segs * 8, st));
     const uint64_t tot = (uint64_t)n * ns;
     if (tot + 1 >= (1ull << 31)) {
         RGL_TRY(stream_after(st, sd, c->ev_join));
@@ -1975,33 +1942,13 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     launches += 2;
     // side stream: rank tables of the query segments that have a rank-difference range
     RGL_TRY(stream_after(sd, st, c->ev_fork));
-    k_seg_tabsize<<<grid_for(n + 1, 256), 256, 0, sd>>>(n, c->segnum.as<uint32_t>(), c->seg_begin.as<uint32_t>(),
-                                                        c->seg_need.as<unsigned long long>(), c->ends.as<uint32_t>(),
-                                                        c->segtab.as<SegTab>(), c->tab_len.as<uint32_t>());
-    tb = c->cub_tmp2.cap;
-    RGL_CUDA(cub::DeviceScan::ExclusiveSum(c->cub_tmp2.p, tb, c->tab_len.as<uint32_t>(), c->tab_off.as<uint32_t>(),
-                                           (int)n + 1, sd));
-    const uint64_t tab_cap = 10ull * n + 16;
-    uint32_t* tab_count = d_small + 14;
-    k_tab_zero<<<(unsigned)std::min<uint64_t>(grid_for(tab_cap, 256), (uint64_t)c->num_sms * 32), 256, 0, sd>>>(
-        n, c->segnum.as<uint32_t>(), c->tab_off.as<uint32_t>(), c->tab_xs.as<uint32_t>(), c->tab_xe.as<uint32_t>(),
-        tab_count);
-    (void)launch_chain(pdl, k_tab_place<true>, k_tab_place<false>, grid_for(n, 256), 256, 0, sd, n,
-                     c->segnum.as<uint32_t>(), c->segtab.as<SegTab>(), c->tab_off.as<uint32_t>(),
-                     c->tab_xs.as<uint32_t>(), c->tab_xe.as<uint32_t>());
-    (void)launch_chain(pdl, k_tab_count<true>, k_tab_count<false>, grid_for(n, 256), 256, 0, sd, n,
+    k_seg_tabsize<<<grid_for(max_segs, 256), 256, 0, sd>>>(n, c->segnum.as<uint32_t>(), c->seg_begin.as<uint32_t>(),
+                                                           c->seg_need.as<unsigned long long>(),
+                                                           c->ends.as<uint32_t>(), c->segtab.as<SegTab>());
+    (void)launch_chain(pdl, k_tab_fill<true>, k_tab_fill<false>, grid_for(n, 256), 256, 0, sd, n,
                      c->segnum.as<uint32_t>(), c->segtab.as<SegTab>(), c->starts.as<uint32_t>(),
-                     c->ends.as<uint32_t>(), c->tab_xs.as<uint32_t>(), c->tab_xe.as<uint32_t>());
-    // inclusive scans written one entry ahead: exclusive scan into tab_* whose entry k + 1 is the
-    // inclusive sum through k (the tables are read from tab_* + 1)
-    uint32_t* sums2 = c->scan_sums2.as<uint32_t>();
-    launches += scan_dev(sums2, c->tab_xs.as<uint32_t>(), c->tab_s.as<uint32_t>(), tab_count, tab_cap, sd, pdl);
-    launches += scan_dev(sums2, c->tab_xe.as<uint32_t>(), c->tab_e.as<uint32_t>(), tab_count, tab_cap, sd, pdl);
-    (void)launch_chain(pdl, k_tab_interleave<true>, k_tab_interleave<false>,
-                     (unsigned)std::min<uint64_t>(grid_for(tab_cap, 256), (uint64_t)c->num_sms * 32), 256, 0, sd,
-                     tab_count, c->tab_s.as<uint32_t>(), c->tab_e.as<uint32_t>(), c->tab2.as<uint2>());
-    launches++;
-    launches += 4;
+                     c->ends.as<uint32_t>(), c->tab2.as<uint2>());
+    launches += 2;
     // main stream: the pair work space and the rank ranges' positions
     (void)launch_chain(pdl, k_cpair_len<true>, k_cpair_len<false>, gc, 256, 0, st, Lp, n, ns, rows, sps,
                      c->tl.as<uint32_t>(), c->seg.as<uint32_t>(), idx->d_slot, idx->d_layers, c->lo.as<uint32_t>(),
@@ -2487,10 +2434,10 @@ int rgl_context_destroy(rgl_context* c) {
                       &c->seg_begin, &c->ps_in, &c->pe_in, &c->ps, &c->pe, &c->lo, &c->hi, &c->maxhi,
                       &c->rflag, &c->ridx, &c->ranges, &c->rlen, &c->rpos, &c->cub_tmp, &c->small,
                       &c->out_counts, &c->out_bp, &c->item_r0,
-                      &c->segtab, &c->tab_len, &c->tab_off, &c->tab_s, &c->tab_e, &c->tab_xs, &c->tab_xe, &c->tab2,
+                      &c->segtab, &c->tab2,
                       &c->cl, &c->pc, &c->method, &c->tl, &c->scan_sums, &c->plen, &c->ppos, &c->psegs, &c->item_t0,
                       &c->seg_need, &c->item_hits, &c->item_base, &c->pairs, &c->bt_off, &c->bt_shard, &c->acc, &c->gc.t_off, &c->gc.t_shard,
-                      &c->cub_tmp2, &c->scan_sums2, &c->sortplan, &c->sort_tab, &c->sort_rank};
+                      &c->cub_tmp2, &c->sortplan, &c->sort_tab, &c->sort_rank};
     if (c->gc.exec) cudaGraphExecDestroy(c->gc.exec);
     if (c->gc.graph) cudaGraphDestroy(c->gc.graph);
     if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
