@@ -10,11 +10,12 @@
 //      which the rank formulation below needs): block by block when every input block is one
 //      segment (tiles sorted in shared memory, then merge passes; ordered blocks copied through),
 //      else a device-wide radix sort.
-//   3. exclusive u64 prefix sums of the sorted starts and sorted ends (PS, PE).
+//   3. one scan over the sorted queries (k_q_reduce, k_q_apply): segment numbers, prefix sums of the
+//      starts (PS) and the largest end of each segment's earlier queries; the same for the ends (PE).
 //   4. K1 partition: for every (layer slot K, query i) the candidate range of the reference's scan,
 //      [pp(start - max_K), pp(end)) with pp = partition point of the layer's starts
-//      (src/sweep/query.rs:98-105); a segmented max-scan merges them into disjoint ranges per
-//      (K, segment); an exclusive scan of the range lengths lays all ranges end to end.
+//      (src/sweep/query.rs:98-105), k_lohi; the non-empty ones laid out and merged into disjoint
+//      ranges per (K, segment), k_emit; the ranges' unions, methods and places, k_range_*.
 //   5. K2 sweep (k_sweep): a persistent kernel pulls fixed-size chunks of that concatenated range
 //      space from a device counter.  Each thread takes one DB interval d and computes, against the
 //      segment's sorted query starts S and ends E,
@@ -29,7 +30,6 @@
 //      Counts and base pairs are tallied per (row, source) in shared memory when a chunk belongs to
 //      one row, else with global atomics.
 #include <cub/cub.cuh>
-#include <thrust/iterator/counting_iterator.h>
 
 #include <algorithm>
 #include <cstring>
@@ -40,22 +40,19 @@
 
 namespace rgl {
 
+// A range swept by ranks.
 struct RangeDesc {
-    uint32_t db_lo, db_hi;      // DB index range within the layer
-    uint32_t c_first, c_last;   // live runs (compacted positions) whose windows formed the range
-    uint32_t layer_idx;         // index into the layer table
-    uint32_t qrow;              // query row (Q_SID)
-    uint32_t seg;               // query segment (shard, row)
-    uint32_t slot;              // layer slot K
+    uint32_t db_lo;      // its first DB interval within the layer
+    uint32_t layer_idx;  // index into the layer table
+    uint32_t qrow;       // query row (Q_SID)
+    uint32_t seg;        // query segment number
 };
 
-// One query's candidate run for the pair sweep: DB elements [base, base + plen) of its layer.
-struct PairSeg {
+// One query's candidate run for the pair sweep: DB elements from `base` (of the index arrays) on.
+struct __align__(16) PairSeg {
     uint64_t base;
-    uint32_t qs, qe, qrow, shard;
+    uint32_t qs, qe;
 };
-
-enum : uint8_t { M_RANK = 0, M_PAIR = 1 };
 
 // Rank table of one query segment: bin b (width 2^shift bp) holds, at tab2[off + b], the numbers
 // of the segment's sorted starts and ends below b << shift, as absolute positions in the sorted
@@ -177,43 +174,336 @@ __global__ void k_expand_keys(uint32_t n, const rgl_interval* __restrict__ iv, c
     ekey[o] = (seg << 32) | e;
 }
 
-// The sorted start keys into starts, segment ids, segment-start flags and the starts' prefix-sum
-// input (entry n = 0); the sorted end keys into ends and the ends' prefix-sum input.
-__global__ void k_unpack_starts(uint32_t n, const uint64_t* __restrict__ key, uint32_t* __restrict__ starts,
-                                uint32_t* __restrict__ seg, uint32_t* __restrict__ segflag,
-                                uint64_t* __restrict__ ps_in) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > n) return;
-    if (i == n) {
-        ps_in[n] = 0;
-        return;
+// ---- tile prefixes ------------------------------------------------------------------------------------
+// The layout below is made of passes over tiles of a sequence, each with a summary per tile whose prefix
+// the next pass needs.  Every block of that pass sums the summaries before its tile itself, with no launch
+// in between, up to kMaxLook tiles (at most 8 reads a thread); beyond, groups of kGroup tiles are summed
+// (k_group_sums) and every tile's prefix written in its place (k_group_scan), since a block that sums
+// hundreds of them first starts its own reads 3 us late.
+constexpr uint32_t kTileThreads = 256, kMaxLook = 2048, kGroup = 256;
+
+// Summary of a span of the sorted queries: segment starts in it, the largest end since the last of them
+// (since the span's start without one), and the sum of the starts.
+struct QSum {
+    uint32_t heads, emax;
+    uint64_t sum;
+    __device__ __forceinline__ static QSum zero() { return QSum{0u, 0u, 0ull}; }
+    __device__ __forceinline__ static QSum add(const QSum& a, const QSum& b) {
+        return QSum{a.heads + b.heads, b.heads ? b.emax : max(a.emax, b.emax), a.sum + b.sum};
     }
-    const uint64_t k = key[i];
-    const uint32_t s = (uint32_t)k, sg = (uint32_t)(k >> 32);
-    starts[i] = s;
-    seg[i] = sg;
-    segflag[i] = (i == 0 || (uint32_t)(key[i - 1] >> 32) != sg) ? 1u : 0u;
-    ps_in[i] = s;
+};
+// Summary of a span of (slot, query) entries: live runs, ranges that start in it, candidates.
+struct LSum {
+    uint32_t live, ranges;
+    uint64_t cand;
+    __device__ __forceinline__ static LSum zero() { return LSum{0u, 0u, 0ull}; }
+    __device__ __forceinline__ static LSum add(const LSum& a, const LSum& b) {
+        return LSum{a.live + b.live, a.ranges + b.ranges, a.cand + b.cand};
+    }
+};
+// Summary of a span of ranges: positions swept by ranks, candidates swept by pairs, ranges of the former.
+struct RSum {
+    uint64_t rank, pair;
+    uint64_t nrank;
+    __device__ __forceinline__ static RSum zero() { return RSum{0ull, 0ull, 0ull}; }
+    __device__ __forceinline__ static RSum add(const RSum& a, const RSum& b) {
+        return RSum{a.rank + b.rank, a.pair + b.pair, a.nrank + b.nrank};
+    }
+};
+struct ESum {
+    uint64_t sum;
+    __device__ __forceinline__ static ESum zero() { return ESum{0ull}; }
+    __device__ __forceinline__ static ESum add(const ESum& a, const ESum& b) { return ESum{a.sum + b.sum}; }
+};
+template <class T>
+struct TileOp {
+    __device__ __forceinline__ T operator()(const T& a, const T& b) const { return T::add(a, b); }
+};
+
+// v of the lane o above, of any struct of 32-bit words.
+template <class T>
+__device__ __forceinline__ T shfl_down_words(const T& v, int o) {
+    T r;
+    const uint32_t* a = reinterpret_cast<const uint32_t*>(&v);
+    uint32_t* b = reinterpret_cast<uint32_t*>(&r);
+#pragma unroll
+    for (int w = 0; w < (int)(sizeof(T) / 4); w++) b[w] = __shfl_down_sync(0xffffffffu, a[w], o);
+    return r;
 }
-__global__ void k_unpack_ends(uint32_t n, const uint64_t* __restrict__ ekey, uint32_t* __restrict__ ends_s,
-                              uint64_t* __restrict__ pe_in) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > n) return;
-    if (i == n) {
-        pe_in[n] = 0;
-        return;
-    }
-    const uint32_t e = (uint32_t)ekey[i];
-    ends_s[i] = e;
-    pe_in[i] = e;
+// Sum of the lanes' values in order, lane 0's.
+template <class T>
+__device__ __forceinline__ T warp_total(T v) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) v = T::add(v, shfl_down_words(v, o));  // lane 0: lanes 0 .. 2 o - 1, in order
+    return v;
+}
+// Sum of s[0, m), for every thread of the block (kTileThreads threads, contiguous stretches, in order).
+template <class T>
+__device__ __forceinline__ T block_total(const T* __restrict__ s, uint32_t m) {
+    __shared__ T part[kTileThreads / 32];
+    const uint32_t per = (m + kTileThreads - 1) / kTileThreads;
+    T v = T::zero();
+    const uint32_t a = min(threadIdx.x * per, m), b = min(a + per, m);
+    for (uint32_t k = a; k < b; k++) v = T::add(v, s[k]);
+    v = warp_total(v);
+    if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = part[0];
+#pragma unroll
+    for (uint32_t w = 1; w < kTileThreads / 32; w++) v = T::add(v, part[w]);
+    __syncthreads();  // part may be reused by the next call
+    return v;
+}
+// Sum of sums[0, tile); with `scanned`, sums[tile] is that sum already.
+template <class T>
+__device__ __forceinline__ T tile_prefix(const T* __restrict__ sums, int scanned, uint32_t tile) {
+    return scanned ? sums[tile] : block_total(sums, tile);
+}
+// groups[g] = sum of the g-th group's tiles, of nt tiles (or of those of *count elements).
+template <class T>
+__global__ void __launch_bounds__(kTileThreads) k_group_sums(const T* __restrict__ sums, uint32_t nt,
+                                                             const uint32_t* __restrict__ count, uint32_t tile,
+                                                             T* __restrict__ groups) {
+    if (count) nt = (uint32_t)(((uint64_t)*count + tile - 1) / tile);
+    const uint32_t a = blockIdx.x * kGroup;
+    const T v = block_total(sums + a, a < nt ? min(kGroup, nt - a) : 0u);
+    if (threadIdx.x == 0) groups[blockIdx.x] = v;
 }
 
-__global__ void k_seg_begin(uint32_t n, const uint32_t* __restrict__ segflag, const uint32_t* __restrict__ segnum,
-                            uint32_t* __restrict__ seg_begin) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (segflag[i]) seg_begin[segnum[i] - 1] = i;
-    if (i == n - 1) seg_begin[segnum[i]] = n;
+template <class T>
+__device__ __forceinline__ T shfl_up_words(const T& v, int o) {
+    T r;
+    const uint32_t* a = reinterpret_cast<const uint32_t*>(&v);
+    uint32_t* b = reinterpret_cast<uint32_t*>(&r);
+#pragma unroll
+    for (int w = 0; w < (int)(sizeof(T) / 4); w++) b[w] = __shfl_up_sync(0xffffffffu, a[w], o);
+    return r;
+}
+template <class T>
+__device__ __forceinline__ T shfl_words(const T& v, int src) {
+    T r;
+    const uint32_t* a = reinterpret_cast<const uint32_t*>(&v);
+    uint32_t* b = reinterpret_cast<uint32_t*>(&r);
+#pragma unroll
+    for (int w = 0; w < (int)(sizeof(T) / 4); w++) b[w] = __shfl_sync(0xffffffffu, a[w], src);
+    return r;
+}
+template <class T>
+__device__ __forceinline__ T warp_scan(T v, uint32_t lane) {  // inclusive, in order
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T w = shfl_up_words(v, o);
+        if (lane >= (uint32_t)o) v = T::add(w, v);
+    }
+    return v;
+}
+// Exclusive prefix of v over the block's threads, in order (kTileThreads threads).
+template <class T>
+__device__ __forceinline__ T block_exclusive(T v) {
+    __shared__ T part[kTileThreads / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const T inc = warp_scan(v, lane);
+    if (lane == 31) part[warp] = inc;
+    __syncthreads();
+    T ex = shfl_up_words(inc, 1);
+    if (lane == 0) ex = T::zero();
+    T before = T::zero();
+    for (uint32_t w = 0; w < warp; w++) before = T::add(before, part[w]);
+    __syncthreads();  // part may be reused by the next call
+    return T::add(before, ex);
+}
+// Every tile of group blockIdx.x: sums[tile] becomes the sum of all tiles before it.
+template <class T>
+__global__ void __launch_bounds__(kTileThreads) k_group_scan(T* __restrict__ sums, uint32_t nt,
+                                                             const uint32_t* __restrict__ count, uint32_t tile,
+                                                             const T* __restrict__ groups) {
+    static_assert(kGroup == kTileThreads, "one tile a thread");
+    if (count) nt = (uint32_t)(((uint64_t)*count + tile - 1) / tile);
+    const uint32_t k = blockIdx.x * kGroup + threadIdx.x;
+    const T before = block_total(groups, blockIdx.x);
+    const T ex = block_exclusive(k < nt ? sums[k] : T::zero());
+    if (k < nt) sums[k] = T::add(before, ex);
+}
+
+// ---- 3. the sorted queries ------------------------------------------------------------------------------
+// One pass of summaries and one that writes, over the sorted start keys: starts, shards, rows and segment
+// numbers, the first query of every segment, the exclusive prefix sums of the starts (n + 1), and for every
+// query the largest end of the segment's earlier queries (0 for its first), by which the ranges are cut
+// below.  Bound by the 12 bytes read twice and the 28 written per query; four consecutive queries a thread,
+// in 16-byte reads and writes.
+constexpr uint32_t kQItems = 4, kQTile = kTileThreads * kQItems;
+
+// v[0, 4) from / to a[base, base + 4) (base a multiple of 4), below n.
+template <class T>
+__device__ __forceinline__ void load4(const T* __restrict__ a, uint32_t base, uint32_t n, T (&v)[4]) {
+    if (base + 4 <= n) {
+        const uint4* p = reinterpret_cast<const uint4*>(a + base);
+        if constexpr (sizeof(T) == 4) {
+            const uint4 w = p[0];
+            v[0] = w.x, v[1] = w.y, v[2] = w.z, v[3] = w.w;
+        } else {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint4 w = p[h];
+                v[2 * h] = ((uint64_t)w.y << 32) | w.x;
+                v[2 * h + 1] = ((uint64_t)w.w << 32) | w.z;
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) v[j] = base + j < n ? a[base + j] : (T)0;
+}
+template <class T>
+__device__ __forceinline__ void store4(T* __restrict__ a, uint32_t base, uint32_t n, const T (&v)[4]) {
+    if (base + 4 <= n) {
+        uint4* p = reinterpret_cast<uint4*>(a + base);
+        if constexpr (sizeof(T) == 4) p[0] = make_uint4(v[0], v[1], v[2], v[3]);
+        else {
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                p[h] = make_uint4((uint32_t)v[2 * h], (uint32_t)(v[2 * h] >> 32), (uint32_t)v[2 * h + 1],
+                                  (uint32_t)(v[2 * h + 1] >> 32));
+        }
+        return;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++)
+        if (base + j < n) a[base + j] = v[j];
+}
+
+// The summaries of a thread's queries and their sum.
+__device__ __forceinline__ QSum q_items(uint32_t n, uint32_t base, const uint64_t* __restrict__ key,
+                                        const uint32_t* __restrict__ end, uint64_t (&k)[4], uint32_t (&e)[4],
+                                        uint32_t* heads) {
+    load4(key, base, n, k);
+    load4(end, base, n, e);
+    uint32_t prev = (base && base < n) ? (uint32_t)(key[base - 1] >> 32) : 0u;
+    QSum s = QSum::zero();
+    *heads = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < kQItems; j++) {
+        const uint32_t i = base + j, sg = (uint32_t)(k[j] >> 32);
+        const uint32_t h = i < n && (i == 0 || sg != prev) ? 1u : 0u;
+        *heads |= h << j;
+        s = QSum::add(s, QSum{h, e[j], (uint32_t)k[j]});
+        prev = sg;
+    }
+    return s;
+}
+
+template <bool PDL>
+__global__ void __launch_bounds__(kTileThreads) k_q_reduce(uint32_t n, const uint64_t* __restrict__ key,
+                                                           const uint32_t* __restrict__ end,
+                                                           QSum* __restrict__ sums) {
+    if constexpr (PDL) {
+        pdl_wait();
+        pdl_release();
+    }
+    __shared__ QSum part[kTileThreads / 32];
+    uint64_t k[4];
+    uint32_t e[4], heads;
+    const QSum s = warp_total(q_items(n, blockIdx.x * kQTile + threadIdx.x * kQItems, key, end, k, e, &heads));
+    if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        QSum t = part[0];
+#pragma unroll
+        for (uint32_t w = 1; w < kTileThreads / 32; w++) t = QSum::add(t, part[w]);
+        sums[blockIdx.x] = t;
+    }
+}
+
+template <bool PDL>
+__global__ void __launch_bounds__(kTileThreads) k_q_apply(
+    uint32_t n, uint32_t rows, uint32_t seg_per_shard, const uint64_t* __restrict__ key,
+    const uint32_t* __restrict__ end, const QSum* __restrict__ sums, int scanned, uint32_t* __restrict__ starts,
+    uint32_t* __restrict__ shard, uint32_t* __restrict__ row, uint32_t* __restrict__ segnum,
+    uint32_t* __restrict__ seg_begin, uint64_t* __restrict__ ps, uint32_t* __restrict__ emax) {
+    if constexpr (PDL) {
+        pdl_wait();
+        pdl_release();
+    }
+    const uint32_t base = blockIdx.x * kQTile + threadIdx.x * kQItems;
+    uint64_t k[4];
+    uint32_t e[4], heads;
+    const QSum own = q_items(n, base, key, end, k, e, &heads);
+    const QSum before = tile_prefix(sums, scanned, blockIdx.x);
+    QSum run = QSum::add(before, block_exclusive(own));
+    uint32_t st[4], sh[4], rw[4], num[4], em[4];
+    uint64_t pre[4];
+#pragma unroll
+    for (uint32_t j = 0; j < kQItems; j++) {
+        const uint32_t i = base + j, sg = (uint32_t)(k[j] >> 32), h = heads >> j & 1u;
+        st[j] = (uint32_t)k[j];
+        sh[j] = sg / seg_per_shard;
+        rw[j] = rows > 1 ? sg % rows : 0u;
+        pre[j] = run.sum;
+        em[j] = h ? 0u : run.emax;
+        if (h) seg_begin[run.heads] = i;
+        run = QSum::add(run, QSum{h, e[j], st[j]});
+        num[j] = run.heads;
+        if (i + 1 == n) {
+            ps[n] = run.sum;
+            seg_begin[run.heads] = n;
+        }
+    }
+    store4(starts, base, n, st);
+    store4(shard, base, n, sh);
+    if (rows > 1) store4(row, base, n, rw);
+    store4(segnum, base, n, num);
+    store4(emax, base, n, em);
+    store4(ps, base, n, pre);
+}
+
+// The sorted end keys into ends and their exclusive prefix sums (n + 1).
+template <bool PDL>
+__global__ void __launch_bounds__(kTileThreads) k_e_reduce(uint32_t n, const uint64_t* __restrict__ ekey,
+                                                           ESum* __restrict__ sums) {
+    if constexpr (PDL) {
+        pdl_wait();
+        pdl_release();
+    }
+    __shared__ ESum part[kTileThreads / 32];
+    uint64_t k[4];
+    load4(ekey, blockIdx.x * kQTile + threadIdx.x * kQItems, n, k);
+    const ESum s = warp_total(ESum{(k[0] & 0xFFFFFFFFull) + (uint32_t)k[1] + (uint32_t)k[2] + (uint32_t)k[3]});
+    if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        ESum t = part[0];
+#pragma unroll
+        for (uint32_t w = 1; w < kTileThreads / 32; w++) t = ESum::add(t, part[w]);
+        sums[blockIdx.x] = t;
+    }
+}
+template <bool PDL>
+__global__ void __launch_bounds__(kTileThreads) k_e_apply(uint32_t n, const uint64_t* __restrict__ ekey,
+                                                          const ESum* __restrict__ sums, int scanned,
+                                                          uint32_t* __restrict__ ends_s, uint64_t* __restrict__ pe) {
+    if constexpr (PDL) {
+        pdl_wait();
+        pdl_release();
+    }
+    const uint32_t base = blockIdx.x * kQTile + threadIdx.x * kQItems;
+    uint64_t k[4], pre[4], s = 0;
+    uint32_t e[4];
+    load4(ekey, base, n, k);
+#pragma unroll
+    for (uint32_t j = 0; j < kQItems; j++) {
+        e[j] = (uint32_t)k[j];
+        s += e[j];
+    }
+    const ESum before = tile_prefix(sums, scanned, blockIdx.x);
+    uint64_t run = before.sum + block_exclusive(ESum{s}).sum;
+#pragma unroll
+    for (uint32_t j = 0; j < kQItems; j++) {
+        pre[j] = run;
+        run += e[j];
+        if (base + j + 1 == n) pe[n] = run;
+    }
+    store4(ends_s, base, n, e);
+    store4(pe, base, n, pre);
 }
 
 // Bin width per segment: about four bins per query, at least 64 bp, but no more than one bin per 8
@@ -307,294 +597,197 @@ __device__ __forceinline__ void add_u64(unsigned long long* c, unsigned long lon
 }
 
 // ---- 4. K1 partition -----------------------------------------------------------------------------
-// lo/hi of the reference's candidate scan for (slot K, query i), layer-major arrays [K][n].
-__global__ void k_lohi(uint32_t n, uint32_t nslots, uint32_t seg_per_shard, const uint32_t* __restrict__ starts,
-                       const uint32_t* __restrict__ qend, const uint32_t* __restrict__ seg,
-                       const int32_t* __restrict__ slot, const LayerDev* __restrict__ layers,
-                       const uint2* __restrict__ pos, const uint32_t* __restrict__ btab,
-                       uint32_t* __restrict__ lo_out, uint32_t* __restrict__ hi_out, uint32_t* __restrict__ live) {
-    // grid: x over the queries, y over the layer slots (no 64-bit division per thread)
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, K = blockIdx.y;
-    if (i >= n) return;
-    const uint64_t t = (uint64_t)K * n + i;
-    uint32_t shard = seg[i] / seg_per_shard;
-    int32_t li = slot[(uint64_t)shard * nslots + K];
+// Entry (slot K, query i) in the order K, i.  Its candidate run is the reference's scan [lo, hi): lo =
+// partition point of start - max_K, hi = that of end; an entry whose run is empty takes part in nothing.
+// The live entries (the others) merge into disjoint ranges per (K, segment): a live entry starts a range
+// when no earlier run of its row reaches past its lo.  The earlier runs' largest hi is the partition point
+// of the segment's largest end so far, E (k_q_apply), the same for every slot, so that no scan over the
+// entries is needed: with back = start - max_K,
+//     back >= E            starts a range (the partition point is monotone);
+//     E >= end             does not (its run ends at or before the partition point of E);
+//     back < E < end       starts one when no start lies in [back, E), i.e. when the run's first element
+//                          (live: it exists) starts at or after E.
+// Pass 1 (k_lohi) searches, stores [lo, hi) and a flag bit per entry and sums live entries, ranges and
+// candidates per tile of kTileThreads queries of one slot; pass 2 (k_emit) writes the live runs and the
+// ranges at their places.  Pass 1 is bound by its random reads (bucket table and starts): one query a
+// thread, so that the blocks running at once lie close together and the rows of a chromosome find its
+// starts in L2 (eight queries a thread: 0.75 -> 2.0 ms for 48 files against 2e8 intervals).  Before, the
+// flags, a compaction, a segmented running maximum and three scans over the entries took eleven launches
+// (3.9 of the 11 ms of 3.1e7 intervals against 3.2e6).
+__device__ __forceinline__ bool large_counts(uint32_t cnt) { return __any_sync(0xffffffffu, cnt >> 27); }
+
+// Sum of the lanes' counts, in 32 bits unless a count is so large that it may not fit.
+__device__ __forceinline__ uint64_t warp_count(uint32_t cnt) {
+    if (!large_counts(cnt)) return __reduce_add_sync(0xffffffffu, cnt);
+    uint64_t c = cnt;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    return c;
+}
+
+template <bool PDL>
+__global__ void __launch_bounds__(kTileThreads) k_lohi(
+    uint32_t n, uint32_t nslots, const uint32_t* __restrict__ starts, const uint32_t* __restrict__ qend,
+    const uint32_t* __restrict__ emax, const uint32_t* __restrict__ shard, const int32_t* __restrict__ slot,
+    const LayerDev* __restrict__ layers, const uint2* __restrict__ pos, const uint32_t* __restrict__ btab,
+    uint32_t* __restrict__ lo_out, uint32_t* __restrict__ hi_out, uint32_t* __restrict__ flags,
+    LSum* __restrict__ sums) {
+    if constexpr (PDL) {
+        pdl_wait();
+        pdl_release();
+    }
+    __shared__ LSum part[kTileThreads / 32];
+    const uint32_t K = blockIdx.y, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t tile = K * gridDim.x + blockIdx.x;
+    const uint32_t i = blockIdx.x * kTileThreads + threadIdx.x;
     uint32_t lo = 0, hi = 0;
-    if (li >= 0) {
-        LayerDev L = layers[li];
-        const uint2* p = pos + L.off;
-        uint32_t s = starts[i];
-        uint32_t back = s >= L.max_size ? s - L.max_size : 0u;  // saturating_sub, src/sweep/query.rs:98
-        const uint32_t* bt = btab + L.boff;
-        pp_layer2(p, bt, L, back, qend[i], lo, hi);
-        if (hi < lo) hi = lo;
-    }
-    lo_out[t] = lo;
-    hi_out[t] = hi;
-    // the live-run flags of the compaction below (entry n * nslots: the scan's closing zero)
-    live[t] = hi > lo ? 1u : 0u;
-    if (t == 0) live[(uint64_t)n * nslots] = 0u;
-}
-
-// ---- scans whose length is a device count ------------------------------------------------------
-// After the compaction below, the number of entries (live candidate runs, ranges) is known only on
-// the device; these scans read it there, so the pipeline keeps no host synchronisation (and stays
-// graph-capturable) while its work follows the live count instead of the (query, slot) capacity.
-// Exclusive scan of in[0, n) into out[0, n], out[n] = total: per-tile sums, one block scanning the
-// tile sums, per-tile block scans offset by them.  The tile kernels are launched with a grid sized
-// for the SMs and walk the tiles below n grid-stride, so a capacity far above the live count costs
-// no empty blocks.
-constexpr int kScanThreads = 256, kScanItems = 8, kScanTile = kScanThreads * kScanItems;
-
-template <typename Tin, typename Tout, bool PDL>
-__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const Tin* __restrict__ in,
-                                                              const uint32_t* __restrict__ n_ptr,
-                                                              Tout* __restrict__ tile_sums) {
-    if constexpr (PDL) {
-        pdl_wait();
-        pdl_release();
-    }
-    const uint32_t n = *n_ptr;
-    using BR = cub::BlockReduce<Tout, kScanThreads>;
-    __shared__ typename BR::TempStorage tmp;
-    for (uint64_t tile = blockIdx.x; tile * kScanTile < n; tile += gridDim.x) {
-        const uint64_t base = tile * kScanTile;
-        Tout s = 0;
-#pragma unroll
-        for (int k = 0; k < kScanItems; k++) {
-            const uint64_t i = base + (uint64_t)k * kScanThreads + threadIdx.x;
-            if (i < n) s += (Tout)in[i];
+    bool start = false;
+    if (i < n) {
+        const int32_t li = slot[(uint64_t)shard[i] * nslots + K];
+        if (li >= 0) {
+            const LayerDev L = layers[li];
+            const uint2* p = pos + L.off;
+            const uint32_t st = starts[i], en = qend[i], E = emax[i];
+            const uint32_t back = st >= L.max_size ? st - L.max_size : 0u;  // saturating_sub, src/sweep/query.rs:98
+            pp_layer2(p, btab + L.boff, L, back, en, lo, hi);
+            if (hi < lo) hi = lo;
+            if (hi > lo) start = back >= E || (E < en && __ldg(&p[lo].x) >= E);
         }
-        s = BR(tmp).Sum(s);
-        if (threadIdx.x == 0) tile_sums[tile] = s;
-        __syncthreads();  // tmp is reused by the next tile
+        const uint64_t t = (uint64_t)K * n + i;
+        lo_out[t] = lo;
+        hi_out[t] = hi;
     }
-}
-
-template <typename Tout, bool PDL>
-__global__ void __launch_bounds__(1024) k_scan_tops(Tout* __restrict__ tile_sums, const uint32_t* __restrict__ n_ptr,
-                                                    Tout* __restrict__ out) {
-    if constexpr (PDL) {
-        pdl_wait();
-        pdl_release();
+    const uint32_t fl = __ballot_sync(0xffffffffu, start), live = __ballot_sync(0xffffffffu, hi > lo);
+    const uint64_t cand = warp_count(hi - lo);
+    if (lane == 0) {
+        flags[tile * (kTileThreads / 32) + warp] = fl;
+        part[warp] = LSum{(uint32_t)__popc(live), (uint32_t)__popc(fl), cand};
     }
-    const uint32_t n = *n_ptr;
-    const uint32_t nt = (uint32_t)((n + kScanTile - 1) / kScanTile);
-    using BS = cub::BlockScan<Tout, 1024>;
-    __shared__ typename BS::TempStorage tmp;
-    Tout run = 0;
-    for (uint32_t b0 = 0; b0 < nt; b0 += 1024) {
-        const uint32_t b = b0 + threadIdx.x;
-        Tout v = b < nt ? tile_sums[b] : (Tout)0, ex, agg;
-        BS(tmp).ExclusiveSum(v, ex, agg);
-        if (b < nt) tile_sums[b] = run + ex;
-        run += agg;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[n] = run;
-}
-
-template <typename Tin, typename Tout, bool PDL>
-__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const Tin* __restrict__ in, Tout* __restrict__ out,
-                                                             const uint32_t* __restrict__ n_ptr,
-                                                             const Tout* __restrict__ tile_off) {
-    if constexpr (PDL) {
-        pdl_wait();
-        pdl_release();
-    }
-    const uint32_t n = *n_ptr;
-    using BL = cub::BlockLoad<Tout, kScanThreads, kScanItems, cub::BLOCK_LOAD_WARP_TRANSPOSE>;
-    using BSt = cub::BlockStore<Tout, kScanThreads, kScanItems, cub::BLOCK_STORE_WARP_TRANSPOSE>;
-    using BS = cub::BlockScan<Tout, kScanThreads>;
-    __shared__ union {
-        typename BL::TempStorage load;
-        typename BSt::TempStorage store;
-        typename BS::TempStorage scan;
-    } tmp;
-    for (uint64_t tile = blockIdx.x; tile * kScanTile < n; tile += gridDim.x) {
-        const uint64_t base = tile * kScanTile;
-        const int valid = (int)((uint64_t)n - base < (uint64_t)kScanTile ? (uint64_t)n - base : (uint64_t)kScanTile);
-        Tout v[kScanItems];
-        BL(tmp.load).Load(in + base, v, valid, (Tout)0);
-        __syncthreads();
-        BS(tmp.scan).ExclusiveSum(v, v);
-        const Tout off = tile_off[tile];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        LSum s = part[0];
 #pragma unroll
-        for (int k = 0; k < kScanItems; k++) v[k] += off;
-        __syncthreads();
-        BSt(tmp.store).Store(out + base, v, valid);
-        __syncthreads();  // tmp is reused by the next tile
+        for (uint32_t w = 1; w < kTileThreads / 32; w++) s = LSum::add(s, part[w]);
+        sums[tile] = s;
     }
 }
 
-// ---- running maximum of hi over the live runs of each (slot, segment) row -----------------------
-// maxc[c] = max of hi over the live entries of entry c's row up to c.  Empty entries never raise the
-// running maximum past a later entry's lo (see 4b), so the maximum over live entries alone decides
-// every range exactly as the maximum over all entries would.  A segmented scan over the L live
-// entries (a device count): per-tile summaries (head seen, maximum since the last head), one block
-// scanning them into each tile's carry, per-tile block scans with the carry.
-struct SegMax {
-    uint32_t f, v;  // f: the span holds a row start; v: maximum since the span's last row start
-};
-struct SegMaxOp {
-    __device__ __forceinline__ SegMax operator()(const SegMax& a, const SegMax& b) const {
-        return SegMax{a.f | b.f, b.f ? b.v : max(a.v, b.v)};
+// Live run c: its query's candidates psegs[c], the candidates before it pc[c], its range cr[c] and uhi[c],
+// the end of the union of its range's runs through it (written only where the run may be its range's last).
+// Range r: rt[r] = (its first live run, that run's entry K n + i).  The last block writes the totals: L, R
+// and pc[L].
+__device__ __forceinline__ uint32_t pp_layer(const uint2* __restrict__ pos, const uint32_t* __restrict__ btab,
+                                             const LayerDev& L, uint32_t x) {
+    const uint32_t b = x >> L.bshift;
+    if (b >= L.nb - 1) return (uint32_t)L.n;
+    uint32_t lo = __ldg(btab + b), hi = __ldg(btab + b + 1);
+    while (lo < hi) {
+        const uint32_t m = lo + ((hi - lo) >> 1);
+        if (__ldg(&pos[m].x) < x) lo = m + 1; else hi = m;
     }
-};
-
-// Live entry c as a scan item: its hi and whether it starts a (slot, segment) row.
-__device__ __forceinline__ SegMax segmax_item(uint64_t c, const uint32_t* __restrict__ tl, uint32_t n,
-                                              const uint32_t* __restrict__ segnum, const uint32_t* __restrict__ hi) {
-    const uint32_t t = tl[c];
-    bool head = c == 0;
-    if (!head) {
-        const uint32_t tp = tl[c - 1];
-        head = (tp / n != t / n) || (segnum[tp % n] != segnum[t % n]);
-    }
-    return SegMax{head ? 1u : 0u, hi[t]};
+    return lo;
 }
 
-template <bool PDL>
-__global__ void __launch_bounds__(kScanThreads) k_segmax_reduce(const uint32_t* __restrict__ Lp, uint32_t n,
-                                                                const uint32_t* __restrict__ tl,
-                                                                const uint32_t* __restrict__ segnum,
-                                                                const uint32_t* __restrict__ hi,
-                                                                unsigned long long* __restrict__ tile_sums) {
-    if constexpr (PDL) {
-        pdl_wait();
-        pdl_release();
-    }
-    const uint32_t L = *Lp;
-    using BS = cub::BlockScan<SegMax, kScanThreads>;
-    __shared__ typename BS::TempStorage tmp;
-    for (uint64_t tile = blockIdx.x; tile * kScanTile < L; tile += gridDim.x) {
-        const uint64_t base = tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-        SegMax v[kScanItems];
+// Inclusive sums of the lanes' counts, in 32 bits as warp_count.
+__device__ __forceinline__ uint64_t warp_inclusive(uint32_t cnt, uint32_t lane) {
+    if (!large_counts(cnt)) {
+        uint32_t inc = cnt;
 #pragma unroll
-        for (int k = 0; k < kScanItems; k++)
-            v[k] = base + k < L ? segmax_item(base + k, tl, n, segnum, hi) : SegMax{0u, 0u};
-        SegMax agg;
-        BS(tmp).InclusiveScan(v, v, SegMaxOp(), agg);
-        if (threadIdx.x == 0) tile_sums[tile] = ((unsigned long long)agg.f << 32) | agg.v;
-        __syncthreads();  // tmp is reused by the next tile
-    }
-}
-
-// tile_sums[t] <- the running maximum carried into tile t (the value before its first row start).
-template <bool PDL>
-__global__ void __launch_bounds__(1024) k_segmax_tops(const uint32_t* __restrict__ Lp,
-                                                      unsigned long long* __restrict__ tile_sums) {
-    if constexpr (PDL) {
-        pdl_wait();
-        pdl_release();
-    }
-    const uint32_t L = *Lp;
-    const uint32_t nt = (uint32_t)((L + kScanTile - 1) / kScanTile);
-    using BS = cub::BlockScan<SegMax, 1024>;
-    __shared__ typename BS::TempStorage tmp;
-    SegMax run{0u, 0u};
-    for (uint32_t b0 = 0; b0 < nt; b0 += 1024) {
-        const uint32_t b = b0 + threadIdx.x;
-        const unsigned long long w = b < nt ? tile_sums[b] : 0ull;
-        SegMax v{(uint32_t)(w >> 32), (uint32_t)w}, ex, agg;
-        BS(tmp).ExclusiveScan(v, ex, SegMax{0u, 0u}, SegMaxOp(), agg);
-        const SegMax carry = threadIdx.x ? SegMaxOp()(run, ex) : run;
-        __syncthreads();  // every thread has read its summary before any is overwritten
-        if (b < nt) tile_sums[b] = carry.v;
-        run = SegMaxOp()(run, agg);
-        __syncthreads();
-    }
-}
-
-template <bool PDL>
-__global__ void __launch_bounds__(kScanThreads) k_segmax_apply(const uint32_t* __restrict__ Lp, uint32_t n,
-                                                               const uint32_t* __restrict__ tl,
-                                                               const uint32_t* __restrict__ segnum,
-                                                               const uint32_t* __restrict__ hi,
-                                                               const unsigned long long* __restrict__ carry,
-                                                               uint32_t* __restrict__ maxc) {
-    if constexpr (PDL) {
-        pdl_wait();
-        pdl_release();
-    }
-    const uint32_t L = *Lp;
-    using BS = cub::BlockScan<SegMax, kScanThreads>;
-    __shared__ typename BS::TempStorage tmp;
-    for (uint64_t tile = blockIdx.x; tile * kScanTile < L; tile += gridDim.x) {
-        const uint64_t base = tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-        SegMax v[kScanItems];
-#pragma unroll
-        for (int k = 0; k < kScanItems; k++)
-            v[k] = base + k < L ? segmax_item(base + k, tl, n, segnum, hi) : SegMax{0u, 0u};
-        if (threadIdx.x == 0 && !v[0].f) v[0].v = max(v[0].v, (uint32_t)carry[tile]);
-        BS(tmp).InclusiveScan(v, v, SegMaxOp());
-#pragma unroll
-        for (int k = 0; k < kScanItems; k++)
-            if (base + k < L) maxc[base + k] = v[k].v;
-        __syncthreads();  // tmp is reused by the next tile
-    }
-}
-
-// ---- 4b. live candidate runs -------------------------------------------------------------------
-// An entry (K, i) whose run [lo, hi) is empty takes part in nothing: with starts sorted, lo is
-// non-decreasing within a (K, segment) row, so an empty run's hi (= its lo) never exceeds a later
-// entry's lo and can neither merge nor split ranges.  The live entries are compacted (tl[c] = t,
-// c < L, by a flagged selection) and everything after this works on them.  k_lohi writes the live
-// flags with lo and hi.
-
-// Range starts among the live runs: the first live run of a (K, segment) row, or one whose lo is
-// past the running maximum of hi over the row's earlier live runs (maxhi[c - 1]); cl = the run's
-// candidate count.
-template <bool PDL>
-__global__ void k_crange_flags(const uint32_t* __restrict__ Lp, uint32_t n, const uint32_t* __restrict__ tl,
-                               const uint32_t* __restrict__ segnum, const uint32_t* __restrict__ lo,
-                               const uint32_t* __restrict__ hi, const uint32_t* __restrict__ maxhi,
-                               uint32_t* __restrict__ cflag, uint64_t* __restrict__ ccl) {
-    if constexpr (PDL) {
-        pdl_wait();
-        pdl_release();
-    }
-    const uint32_t L = *Lp;
-    for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < L; c += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t t = tl[c];
-        bool start = c == 0;
-        if (!start) {
-            const uint32_t tp = tl[c - 1];
-            start = (tp / n != t / n) || (segnum[tp % n] != segnum[t % n]) || (lo[t] >= maxhi[c - 1]);
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t w = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= (uint32_t)o) inc += w;
         }
-        cflag[c] = start ? 1u : 0u;
-        ccl[c] = (uint64_t)(hi[t] - lo[t]);
+        return inc;
     }
+    uint64_t inc = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t w = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += w;
+    }
+    return inc;
 }
 
-template <bool PDL>
-__global__ void k_crange_emit(const uint32_t* __restrict__ Lp, uint32_t n, uint32_t nslots, uint32_t rows,
-                              uint32_t seg_per_shard, const uint32_t* __restrict__ tl, const uint32_t* __restrict__ seg,
-                              const uint32_t* __restrict__ segnum, const int32_t* __restrict__ slot,
-                              const uint32_t* __restrict__ lo, const uint32_t* __restrict__ maxhi,
-                              const uint32_t* __restrict__ cflag, const uint32_t* __restrict__ cridx,
-                              RangeDesc* __restrict__ ranges) {
+// What the runs carry beside their queries: nothing, the row (several-row sweeps), or shard and row
+// (shard * rows + row; the pair list).
+enum : int { RUN_PLAIN = 0, RUN_ROW = 1, RUN_SHARD_ROW = 2 };
+
+// A block takes ITEMS of k_lohi's tiles of its slot (tiles of them: per_slot).
+template <int ITEMS, bool PDL>
+__global__ void __launch_bounds__(kTileThreads) k_emit(
+    uint32_t n, uint32_t nslots, uint32_t rows, uint32_t per_slot, int tag, const uint32_t* __restrict__ starts,
+    const uint32_t* __restrict__ qend, const uint32_t* __restrict__ emax, const uint32_t* __restrict__ shard,
+    const uint32_t* __restrict__ row, const int32_t* __restrict__ slot, const LayerDev* __restrict__ layers,
+    const uint2* __restrict__ pos, const uint32_t* __restrict__ btab, const uint32_t* __restrict__ lo_in,
+    const uint32_t* __restrict__ hi_in, const uint32_t* __restrict__ flags, const LSum* __restrict__ sums, int scanned,
+    PairSeg* __restrict__ psegs, uint32_t* __restrict__ prow,
+    uint64_t* __restrict__ pc, uint32_t* __restrict__ cr, uint32_t* __restrict__ uhi, uint2* __restrict__ rt,
+    uint32_t* __restrict__ Lp, uint32_t* __restrict__ Rp) {
     if constexpr (PDL) {
         pdl_wait();
         pdl_release();
     }
-    const uint32_t L = *Lp;
-    for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < L; c += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t t = tl[c], K = t / n, i = t % n;
-        const uint32_t f = cflag[c];
-        const uint32_t r = cridx[c] + f - 1;  // inclusive range index
-        if (f) {
-            const uint32_t sg = seg[i];
-            ranges[r].db_lo = lo[t];
-            ranges[r].c_first = (uint32_t)c;
-            ranges[r].layer_idx = (uint32_t)slot[(uint64_t)(sg / seg_per_shard) * nslots + K];
-            ranges[r].qrow = sg % rows;
-            ranges[r].seg = segnum[i] - 1;
-            ranges[r].slot = K;
-        }
-        if (c + 1 == L || cflag[c + 1]) {
-            ranges[r].c_last = (uint32_t)c;
-            ranges[r].db_hi = maxhi[c];
+    constexpr uint32_t kWarps = kTileThreads / 32, kChunks = kWarps * ITEMS;  // chunks of 32 entries, in order
+    static_assert(kChunks <= 32, "one chunk a lane");
+    __shared__ LSum chunk[kChunks];
+    const uint32_t K = blockIdx.y, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t tile0 = K * per_slot + blockIdx.x * ITEMS;
+    uint32_t lo[ITEMS], cnt[ITEMS], fl[ITEMS], sh[ITEMS], qs[ITEMS], qe[ITEMS], E[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) {
+        const uint32_t x = blockIdx.x * ITEMS + k, i = x * kTileThreads + threadIdx.x;
+        const uint64_t t = (uint64_t)K * n + i;
+        const bool in = x < per_slot && i < n;
+        lo[k] = in ? lo_in[t] : 0u;
+        cnt[k] = (in ? hi_in[t] : 0u) - lo[k];
+        fl[k] = x < per_slot ? flags[(tile0 + k) * kWarps + warp] : 0u;
+        const bool live = cnt[k] != 0;
+        sh[k] = live ? shard[i] : 0u;
+        qs[k] = live ? starts[i] : 0u;
+        qe[k] = live ? qend[i] : 0u;
+        E[k] = live ? emax[i] : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) {
+        const uint64_t total = warp_count(cnt[k]);
+        const uint32_t live = __popc(__ballot_sync(0xffffffffu, cnt[k] != 0));
+        if (lane == 0) chunk[k * kWarps + warp] = LSum{live, (uint32_t)__popc(fl[k]), total};
+    }
+    const LSum before = tile_prefix(sums, scanned, tile0);
+    __syncthreads();
+    // the chunks' prefixes, by every warp for itself: lane h holds chunk h's
+    const LSum inc_chunk = LSum::add(before, warp_scan(lane < kChunks ? chunk[lane] : LSum::zero(), lane));
+    LSum ex_chunk = shfl_up_words(inc_chunk, 1);
+    if (lane == 0) ex_chunk = before;
+    if (K + 1 == gridDim.y && blockIdx.x + 1 == gridDim.x && threadIdx.x == 31) {
+        *Lp = inc_chunk.live;
+        *Rp = inc_chunk.ranges;
+        pc[inc_chunk.live] = inc_chunk.cand;
+    }
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) {
+        const uint32_t live = __ballot_sync(0xffffffffu, cnt[k] != 0);
+        const LSum at = shfl_words(ex_chunk, k * kWarps + warp);
+        if (!live) continue;
+        const uint64_t inc = warp_inclusive(cnt[k], lane);
+        if (!cnt[k]) continue;
+        const uint32_t i = (blockIdx.x * ITEMS + k) * kTileThreads + threadIdx.x;
+        const uint32_t c = at.live + __popc(live & ((1u << lane) - 1u));
+        const int32_t li = slot[(uint64_t)sh[k] * nslots + K];
+        psegs[c] = PairSeg{layers[li].off + lo[k], qs[k], qe[k]};
+        if (tag) prow[c] = (rows > 1 ? row[i] : 0u) + (tag == RUN_SHARD_ROW ? sh[k] * rows : 0u);
+        pc[c] = at.cand + inc - cnt[k];
+        cr[c] = at.ranges + __popc(fl[k] & ((2u << lane) - 1u)) - 1;  // the range it starts or continues
+        if (fl[k] >> lane & 1u) rt[at.ranges + __popc(fl[k] & ((1u << lane) - 1u))] = make_uint2(c, K * n + i);
+        // its range's last run unless the next live entry of the chunk goes on with the range
+        const uint32_t later = live & ~((2u << lane) - 1u);
+        if (!later || (fl[k] & later & (0u - later))) {
+            uint32_t end = lo[k] + cnt[k];
+            if (E[k] > qe[k]) {  // an earlier query reaches further
+                const LayerDev Ld = layers[li];
+                end = pp_layer(pos + Ld.off, btab + Ld.boff, Ld, E[k]);
+            }
+            uhi[c] = end;
         }
     }
 }
@@ -602,81 +795,191 @@ __global__ void k_crange_emit(const uint32_t* __restrict__ Lp, uint32_t n, uint3
 // Per range: the reference's candidate count (sum over its runs of hi - lo) against the size of the
 // union.  Where the two are close (narrow layers) the pair sweep reads each candidate once with
 // trivial per-pair work; where candidate windows overlap heavily (broad layers) the rank sweep reads
-// each union element once.  rlen = union length of rank ranges (the rank work space); the union of
-// every range is summed into *union_total (the swept count of the metric).
+// each union element once.  The unions of all ranges are summed into *union_total (the swept count of the
+// metric), those swept by ranks per segment into seg_need.
+constexpr uint32_t kRItems = 4, kRTile = kTileThreads * kRItems;
+
 template <bool PDL>
-__global__ void __launch_bounds__(256) k_crange_method(const uint32_t* __restrict__ Lp, const uint32_t* __restrict__ cridx,
-                                const RangeDesc* __restrict__ ranges, const uint64_t* __restrict__ cpc,
-                                uint32_t pair_ratio, uint8_t* __restrict__ method, uint64_t* __restrict__ rlen,
-                                unsigned long long* __restrict__ seg_need, uint32_t* __restrict__ R_out,
-                                unsigned long long* __restrict__ union_total) {
+__global__ void __launch_bounds__(kTileThreads) k_range_reduce(
+    const uint32_t* __restrict__ Lp, const uint32_t* __restrict__ Rp, uint32_t n, const uint2* __restrict__ rt,
+    const uint64_t* __restrict__ pc, const uint32_t* __restrict__ uhi, const uint32_t* __restrict__ lo,
+    const uint32_t* __restrict__ segnum, uint32_t pair_ratio, uint32_t* __restrict__ ulen,
+    unsigned long long* __restrict__ seg_need, unsigned long long* __restrict__ union_total,
+    RSum* __restrict__ sums) {
     if constexpr (PDL) {
         pdl_wait();
         pdl_release();
     }
-    const uint32_t R = cridx[*Lp];
-    const uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (g == 0) *R_out = R;
-    unsigned long long acc = 0;
-    for (uint64_t r = g; r < R; r += (uint64_t)gridDim.x * blockDim.x) {
-        const RangeDesc rd = ranges[r];
-        const uint64_t len = rd.db_hi - rd.db_lo;
-        const uint64_t cand = cpc[rd.c_last + 1] - cpc[rd.c_first];
-        const uint8_t m = (cand <= (uint64_t)pair_ratio * len) ? M_PAIR : M_RANK;
-        method[r] = m;
-        if (m == M_RANK && len) atomicAdd(&seg_need[rd.seg], (unsigned long long)len);  // rank-swept positions
-        rlen[r] = m == M_RANK ? len : 0;
-        acc += len;
+    __shared__ RSum part[kTileThreads / 32];
+    const uint32_t L = *Lp, R = *Rp, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    unsigned long long uni = 0;
+    for (uint64_t tile = blockIdx.x; tile * kRTile < R; tile += gridDim.x) {
+        RSum s = RSum::zero();
+        uint2 f[kRItems];
+        uint32_t c1[kRItems];
+#pragma unroll
+        for (uint32_t k = 0; k < kRItems; k++) {
+            const uint64_t r = tile * kRTile + k * kTileThreads + threadIdx.x;
+            f[k] = r < R ? rt[r] : make_uint2(0, 0);
+            c1[k] = r + 1 < R ? rt[r + 1].x : L;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kRItems; k++) {
+            const uint64_t r = tile * kRTile + k * kTileThreads + threadIdx.x;
+            if (r >= R) continue;
+            const uint64_t cand = pc[c1[k]] - pc[f[k].x];
+            const uint32_t len = uhi[c1[k] - 1] - lo[f[k].y];
+            ulen[r] = len;
+            uni += len;
+            if (cand <= (uint64_t)pair_ratio * len) s.pair += cand;
+            else {
+                s.rank += len;
+                s.nrank++;
+                atomicAdd(&seg_need[segnum[f[k].y % n] - 1], (unsigned long long)len);  // rank-swept positions
+            }
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            s.pair += __shfl_down_sync(0xffffffffu, s.pair, o);
+            s.rank += __shfl_down_sync(0xffffffffu, s.rank, o);
+            s.nrank += __shfl_down_sync(0xffffffffu, s.nrank, o);
+        }
+        if (lane == 0) part[warp] = s;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (uint32_t w = 1; w < kTileThreads / 32; w++) s = RSum::add(s, part[w]);
+            sums[tile] = s;
+        }
+        __syncthreads();  // part is reused
     }
-    // one atomic per block on the shared total
-    using BR = cub::BlockReduce<unsigned long long, 256>;
-    __shared__ typename BR::TempStorage tmp;
-    acc = BR(tmp).Sum(acc);
-    if (threadIdx.x == 0 && acc) atomicAdd(union_total, acc);
+    // one atomic per warp on the shared total
+#pragma unroll
+    for (int o = 16; o; o >>= 1) uni += __shfl_down_sync(0xffffffffu, uni, o);
+    if (lane == 0 && uni) atomicAdd(union_total, uni);
 }
 
-// Pair work space: each live run of a pair range contributes its candidates.
+// The rank work space: range q of those swept by ranks covers positions [rpos[q], rpos[q + 1]).  For the
+// pair work space every range gets rpair[r]: kRankRange | the pair candidates before it, for a range
+// swept by ranks (its runs take no room there), or the candidates of the rank ranges before it, for one
+// swept by pairs (to be taken off its runs' pc).  The totals go to the counter block.
+constexpr uint64_t kRankRange = 1ull << 63;
 template <bool PDL>
-__global__ void k_cpair_len(const uint32_t* __restrict__ Lp, uint32_t n, uint32_t nslots, uint32_t rows,
-                            uint32_t seg_per_shard, const uint32_t* __restrict__ tl, const uint32_t* __restrict__ seg,
-                            const int32_t* __restrict__ slot, const LayerDev* __restrict__ layers,
-                            const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi,
-                            const uint32_t* __restrict__ cflag, const uint32_t* __restrict__ cridx,
-                            const uint8_t* __restrict__ method, const uint32_t* __restrict__ starts,
-                            const uint32_t* __restrict__ qend, uint64_t* __restrict__ plen,
-                            PairSeg* __restrict__ psegs) {
+__global__ void __launch_bounds__(kTileThreads) k_range_apply(
+    const uint32_t* __restrict__ Lp, const uint32_t* __restrict__ Rp, uint32_t n, uint32_t nslots, uint32_t rows,
+    const uint2* __restrict__ rt, const uint64_t* __restrict__ pc, const uint32_t* __restrict__ ulen,
+    const uint32_t* __restrict__ lo, const uint32_t* __restrict__ shard, const uint32_t* __restrict__ row,
+    const uint32_t* __restrict__ segnum, const int32_t* __restrict__ slot, uint32_t pair_ratio,
+    const RSum* __restrict__ sums, int scanned, RangeDesc* __restrict__ ranges,
+    uint64_t* __restrict__ rpos, uint64_t* __restrict__ rpair, uint64_t* __restrict__ ppos,
+    uint32_t* __restrict__ rank_count, unsigned long long* __restrict__ totals) {
+    if constexpr (PDL) {
+        pdl_wait();
+        pdl_release();
+    }
+    constexpr uint32_t kWarps = kTileThreads / 32, kChunks = kWarps * kRItems;
+    __shared__ RSum chunk[kChunks];
+    const uint32_t L = *Lp, R = *Rp, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (R == 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+        rpos[0] = 0;
+        ppos[0] = 0;
+        *rank_count = 0;
+        totals[0] = 0;
+        totals[1] = 0;
+    }
+    for (uint64_t tile = blockIdx.x; tile * kRTile < R; tile += gridDim.x) {
+        uint64_t first[kRItems], cand[kRItems];
+        uint32_t len[kRItems], ent[kRItems];
+#pragma unroll
+        for (uint32_t k = 0; k < kRItems; k++) {
+            const uint64_t r = tile * kRTile + k * kTileThreads + threadIdx.x;
+            const uint2 f = r < R ? rt[r] : make_uint2(0, 0);
+            const uint32_t c1 = r < R ? (r + 1 < R ? rt[r + 1].x : L) : 0u;
+            ent[k] = f.y;
+            first[k] = pc[f.x];
+            cand[k] = pc[c1] - first[k];
+            len[k] = r < R ? ulen[r] : 0u;
+        }
+        uint32_t rank = 0;  // bit k: range k of this thread is swept by ranks
+#pragma unroll
+        for (uint32_t k = 0; k < kRItems; k++) {
+            const uint64_t r = tile * kRTile + k * kTileThreads + threadIdx.x;
+            if (r >= R) cand[k] = 0;
+            else if (cand[k] > (uint64_t)pair_ratio * len[k]) rank |= 1u << k;
+            RSum s = RSum::zero();
+            if (__any_sync(0xffffffffu, rank >> k & 1u)) {
+                s = rank >> k & 1u ? RSum{len[k], 0ull, 1ull} : RSum{0ull, cand[k], 0ull};
+                s = warp_total(s);
+            } else {
+                s.pair = cand[k];
+#pragma unroll
+                for (int o = 16; o; o >>= 1) s.pair += __shfl_down_sync(0xffffffffu, s.pair, o);
+            }
+            if (lane == 0) chunk[k * kWarps + warp] = s;
+        }
+        const RSum before = tile_prefix(sums, scanned, (uint32_t)tile);
+        __syncthreads();
+        static_assert(kChunks == 32, "one chunk a lane");
+        const RSum mine = chunk[lane];
+        RSum ex_chunk = shfl_up_words(warp_scan(mine, lane), 1);  // lane h: the chunks before h
+        ex_chunk = lane ? RSum::add(before, ex_chunk) : before;
+#pragma unroll
+        for (uint32_t k = 0; k < kRItems; k++) {
+            const uint64_t r = tile * kRTile + k * kTileThreads + threadIdx.x;
+            const RSum at = shfl_words(ex_chunk, k * kWarps + warp);
+            const bool by_rank = rank >> k & 1u;
+            const RSum own = by_rank ? RSum{len[k], 0ull, 1ull} : RSum{0ull, cand[k], 0ull};
+            RSum inc = own;
+            if (__any_sync(0xffffffffu, by_rank)) inc = warp_scan(own, lane);
+            else {
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint64_t w = __shfl_up_sync(0xffffffffu, inc.pair, o);
+                    if (lane >= (uint32_t)o) inc.pair += w;
+                }
+            }
+            inc = RSum::add(at, inc);
+            if (r >= R) continue;
+            if (by_rank) {
+                const uint32_t K = ent[k] / n, i = ent[k] % n;
+                const uint64_t q = inc.nrank - 1;
+                rpair[r] = kRankRange | inc.pair;
+                rpos[q] = inc.rank - len[k];
+                ranges[q] = RangeDesc{lo[ent[k]], (uint32_t)slot[(uint64_t)shard[i] * nslots + K],
+                                      rows > 1 ? row[i] : 0u, segnum[i] - 1};
+            } else {
+                rpair[r] = first[k] - (inc.pair - cand[k]);
+            }
+            if (r + 1 == R) {
+                rpos[inc.nrank] = inc.rank;
+                ppos[L] = inc.pair;
+                *rank_count = (uint32_t)inc.nrank;
+                totals[0] = inc.rank;
+                totals[1] = inc.pair;
+            }
+        }
+        __syncthreads();  // chunk is reused
+    }
+}
+
+// Pair work space: live run c's candidates begin at ppos[c].
+template <bool PDL>
+__global__ void k_run_pos(const uint32_t* __restrict__ Lp, const uint32_t* __restrict__ cr,
+                          const uint64_t* __restrict__ pc, const uint64_t* __restrict__ rpair,
+                          uint64_t* __restrict__ ppos) {
     if constexpr (PDL) {
         pdl_wait();
         pdl_release();
     }
     const uint32_t L = *Lp;
     for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < L; c += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t t = tl[c], K = t / n, i = t % n;
-        const uint32_t r = cridx[c] + cflag[c] - 1;
-        uint64_t len = 0;
-        if (method[r] == M_PAIR) {
-            const uint32_t sg = seg[i];
-            const int32_t li = slot[(uint64_t)(sg / seg_per_shard) * nslots + K];
-            len = hi[t] - lo[t];
-            psegs[c] = PairSeg{layers[li].off + lo[t], starts[i], qend[i], sg % rows, sg / seg_per_shard};
-        }
-        plen[c] = len;
-    }
-}
-
-// Totals of the rank and pair work spaces (stats): small[10..11] = rpos[R], small[12..13] = ppos[L].
-__global__ void k_totals(uint32_t* __restrict__ small, const uint64_t* __restrict__ rpos,
-                         const uint64_t* __restrict__ ppos) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        unsigned long long* s64 = reinterpret_cast<unsigned long long*>(small);
-        s64[5] = rpos[small[9]];
-        s64[6] = ppos[small[8]];
+        const uint64_t v = rpair[cr[c]];
+        ppos[c] = v & kRankRange ? v & ~kRankRange : pc[c] - v;
     }
 }
 
 struct SweepParams {
     const uint64_t* rpos;   // exclusive scan of rank-range lengths, R + 1 entries; rpos[R] = total
-    const uint32_t* rcount; // R (device): ranges
+    const uint32_t* rcount; // R (device): ranges swept by ranks
     const uint32_t* pcount; // L (device): live candidate runs
     const RangeDesc* ranges;
     const LayerDev* layers;
@@ -692,6 +995,7 @@ struct SweepParams {
     const uint32_t* item_r0; // first range of each work item (items < item_cap)
     const uint64_t* ppos;    // pair work space: exclusive scan of candidate runs, L + 1 entries
     const PairSeg* psegs;
+    const uint32_t* prow;    // rows of the runs (several-row sweeps)
     const uint32_t* item_t0; // first run of each pair work item
     const SegTab* segtabs;   // per query segment
     const uint2* tab2;       // rank tables, bin b = (#starts, #ends) below b << shift
@@ -765,10 +1069,9 @@ __device__ __forceinline__ uint32_t range_advance(const uint64_t* __restrict__ r
 // Work-item partition: item i covers positions [i * chunk, (i + 1) * chunk) of the concatenated
 // ranges; item_r0[i] = the range holding its first position (last r with rpos[r] <= i * chunk),
 // found by binary search over the range offsets.  One launch serves the rank ranges (rpos, *Rp
-// ranges) and the pair runs (ppos, *Lp runs), grid-stride over the items of both, and records the
-// two position totals in the counter block (64-bit words 5 and 6).
+// ranges) and the pair runs (ppos, *Lp runs), grid-stride over the items of both.
 template <bool PDL>
-__global__ void k_item_ranges(uint32_t* __restrict__ small, const uint32_t* __restrict__ Rp,
+__global__ void k_item_ranges(const uint32_t* __restrict__ Rp,
                               const uint64_t* __restrict__ rpos, const uint32_t* __restrict__ Lp,
                               const uint64_t* __restrict__ ppos, uint32_t chunk, uint32_t spread, uint64_t item_cap,
                               uint32_t* __restrict__ item_r0, uint32_t* __restrict__ item_t0) {
@@ -779,11 +1082,6 @@ __global__ void k_item_ranges(uint32_t* __restrict__ small, const uint32_t* __re
     const uint32_t R = *Rp, L = *Lp;
     const uint64_t rtot = rpos[R], ptot = ppos[L];
     const uint64_t g0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (g0 == 0) {
-        unsigned long long* s64 = reinterpret_cast<unsigned long long*>(small);
-        s64[5] = rtot;
-        s64[6] = ptot;
-    }
     const uint32_t rc = item_size(rtot, chunk, spread), pc = item_size(ptot, chunk, spread);
     const uint64_t ri = min((rtot + rc - 1) / rc, item_cap);
     const uint64_t pi = min((ptot + pc - 1) / pc, item_cap);
@@ -886,19 +1184,20 @@ constexpr uint32_t kCtaItems = 8;  // warps of a 256-thread block
 // The row of the middle of block item ci (its warp item ci * kCtaItems + kCtaItems / 2, or the last
 // item), from the first range (RANK) or run of that warp item: the row the block's histogram serves.
 template <bool RANK>
-__device__ __forceinline__ uint32_t cta_item_row(const SweepParams& P, uint64_t ci, uint64_t items, uint32_t rcap) {
+__device__ __forceinline__ uint32_t cta_item_row(const SweepParams& P, uint32_t chunk, uint64_t ci, uint64_t items,
+                                                 uint32_t rcap) {
     const uint64_t wi = min(ci * kCtaItems + kCtaItems / 2, items - 1);
     const uint64_t* off = RANK ? P.rpos : P.ppos;
     uint32_t r;
     if (wi < P.item_cap) {
         r = __ldg((RANK ? P.item_r0 : P.item_t0) + wi);
     } else {
-        const uint64_t p = wi * P.chunk;
+        const uint64_t p = wi * chunk;
         uint64_t lo = 0, hi = rcap;
         while (lo < hi) { uint64_t m = (lo + hi + 1) >> 1; if (__ldg(off + m) <= p) lo = m; else hi = m - 1; }
         r = (uint32_t)lo;
     }
-    return RANK ? P.ranges[r].qrow : P.psegs[r].qrow;
+    return RANK ? P.ranges[r].qrow : __ldg(P.prow + r);
 }
 
 // The outer loop of the several-row sweeps.  Blocks pull block items (kCtaItems warp items) from the
@@ -908,8 +1207,8 @@ __device__ __forceinline__ uint32_t cta_item_row(const SweepParams& P, uint64_t 
 // added to the outputs and cleared (and once more at the end).  item_fn(warp_item, row) walks one
 // warp item; flush_fn(row) adds and clears the histogram.
 template <bool RANK, typename ItemFn, typename FlushFn>
-__device__ __forceinline__ void multi_row_loop(const SweepParams& P, uint64_t items, uint32_t rcap, ItemFn item_fn,
-                                               FlushFn flush_fn) {
+__device__ __forceinline__ void multi_row_loop(const SweepParams& P, uint32_t chunk, uint64_t items, uint32_t rcap,
+                                               ItemFn item_fn, FlushFn flush_fn) {
     __shared__ uint32_t s_ctl[2];
     constexpr uint32_t kNone = 0xFFFFFFFFu;
     uint32_t cur = kNone;  // the row the histogram holds (block-uniform)
@@ -917,7 +1216,7 @@ __device__ __forceinline__ void multi_row_loop(const SweepParams& P, uint64_t it
         if (threadIdx.x == 0) {
             const uint32_t ci = atomicAdd(P.queue, 1u);
             s_ctl[0] = ci;
-            if ((uint64_t)ci * kCtaItems < items) s_ctl[1] = cta_item_row<RANK>(P, ci, items, rcap);
+            if ((uint64_t)ci * kCtaItems < items) s_ctl[1] = cta_item_row<RANK>(P, chunk, ci, items, rcap);
         }
         __syncthreads();
         const uint64_t ci = s_ctl[0];
@@ -961,15 +1260,18 @@ __device__ __forceinline__ void flush_row(const SweepParams& P, uint32_t row, ui
 
 constexpr uint32_t kUnroll = 2;      // DB intervals per lane per step of the rank sweep
 constexpr uint32_t kPairUnroll = 4;  // candidates per lane per step of the pair sweep
+// Run boundaries inside a step up to which they are counted one by one (nine instructions each); beyond,
+// pairs_step_dense (a hundred and fifty or so for any number, and a call).
+constexpr uint32_t kFewBounds = 16;
 
 // One work item of the rank sweep: positions [item * chunk, (item + 1) * chunk) of the concatenated
 // rank ranges, walked by one warp.
 template <bool WITH_BP, bool MULTI>
-__device__ __forceinline__ void sweep_item(const SweepParams& P, uint32_t item, uint32_t lane, uint32_t rcap,
+__device__ __forceinline__ void sweep_item(const SweepParams& P, uint32_t chunk, uint32_t item, uint32_t lane, uint32_t rcap,
                                            uint64_t total, uint32_t* s_cnt, unsigned long long* s_bp,
                                            uint32_t cta_row) {
-    const uint64_t p0 = (uint64_t)item * P.chunk;
-    const uint64_t p1 = min(p0 + P.chunk, total);
+    const uint64_t p0 = (uint64_t)item * chunk;
+    const uint64_t p1 = min(p0 + chunk, total);
     uint32_t r0;
     if (item < P.item_cap) {
         r0 = __ldg(P.item_r0 + item);
@@ -1026,7 +1328,7 @@ __device__ __forceinline__ void sweep_item(const SweepParams& P, uint32_t item, 
 }
 
 template <bool WITH_BP, bool MULTI>
-__global__ void __launch_bounds__(256, 5) k_sweep(SweepParams P) {
+__global__ void __launch_bounds__(256, 5) k_sweep(const __grid_constant__ SweepParams P) {
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned long long* s_bp = reinterpret_cast<unsigned long long*>(smem);
     uint32_t* s_cnt = reinterpret_cast<uint32_t*>(smem + (WITH_BP ? (size_t)P.D * 8 : 0));
@@ -1034,7 +1336,7 @@ __global__ void __launch_bounds__(256, 5) k_sweep(SweepParams P) {
 
     const uint32_t rcap = *P.rcount;
     const uint64_t total = P.rpos[rcap];
-    P.chunk = item_size(total, P.chunk, P.spread);
+    const uint32_t chunk = item_size(total, P.chunk, P.spread);
     if (P.smem_tally) {
         for (uint32_t k = threadIdx.x; k < P.D; k += blockDim.x) {
             s_cnt[k] = 0;
@@ -1045,11 +1347,11 @@ __global__ void __launch_bounds__(256, 5) k_sweep(SweepParams P) {
     if constexpr (MULTI) {
         // several rows: blocks pull block items (kCtaItems warp items each); the block's histogram
         // serves the row of the current item and is added to the outputs on a row change
-        const uint64_t items = (total + P.chunk - 1) / P.chunk;
+        const uint64_t items = (total + chunk - 1) / chunk;
         multi_row_loop<true>(
-            P, items, rcap,
+            P, chunk, items, rcap,
             [&](uint32_t item, uint32_t row) {
-                sweep_item<WITH_BP, true>(P, item, lane, rcap, total, s_cnt, s_bp, row);
+                sweep_item<WITH_BP, true>(P, chunk, item, lane, rcap, total, s_cnt, s_bp, row);
             },
             [&](uint32_t row) { flush_row<WITH_BP>(P, row, s_cnt, s_bp); });
     } else {
@@ -1063,8 +1365,8 @@ __global__ void __launch_bounds__(256, 5) k_sweep(SweepParams P) {
             uint32_t item = 0;
             if (lane == 0) item = atomicAdd(P.queue, 1u);
             item = __shfl_sync(0xffffffffu, item, 0);
-            if ((uint64_t)item * P.chunk >= total) break;
-            sweep_item<WITH_BP, false>(P, item, lane, rcap, total, s_cnt, s_bp, 0u);
+            if ((uint64_t)item * chunk >= total) break;
+            sweep_item<WITH_BP, false>(P, chunk, item, lane, rcap, total, s_cnt, s_bp, 0u);
         }
         if (P.smem_tally) {
             __syncthreads();
@@ -1080,47 +1382,91 @@ __global__ void __launch_bounds__(256, 5) k_sweep(SweepParams P) {
 // adds 1 and min(ends) - max(starts) to cell (qrow, sid) — in the block's shared histograms (SMEM,
 // one query row) or in the output matrix.
 template <bool WITH_BP, bool SMEM, int MULTI>
-__device__ __forceinline__ void pair_tally(const SweepParams& P, uint32_t qs, uint32_t qe, uint32_t qrow, uint2 d,
-                                           uint32_t sid, uint32_t* s_cnt, unsigned long long* s_bp,
-                                           uint32_t cta_row) {
+__device__ __forceinline__ void pair_tally(uint32_t* counts, unsigned long long* bp, uint32_t D, uint32_t qs,
+                                           uint32_t qe, uint32_t qrow, uint2 d, uint32_t sid, uint32_t* s_cnt,
+                                           unsigned long long* s_bp, uint32_t cta_row) {
     if (d.y <= qs) return;
     if (SMEM && (!MULTI || qrow == cta_row)) {
         atomicAdd(&s_cnt[sid], 1u);
         if (WITH_BP) add_u64_lo(&s_bp[sid], min(qe, d.y) - max(qs, d.x));
     } else {
-        const uint64_t cell = (uint64_t)qrow * P.D + sid;
-        atomicAdd(&P.counts[cell], 1u);
-        if (WITH_BP) atomicAdd(&P.bp[cell], (unsigned long long)(min(qe, d.y) - max(qs, d.x)));
+        const uint64_t cell = (uint64_t)qrow * D + sid;
+        atomicAdd(&counts[cell], 1u);
+        if (WITH_BP) atomicAdd(&bp[cell], (unsigned long long)(min(qe, d.y) - max(qs, d.x)));
     }
 }
 
-// One step of the pair sweep position by position, each position's run found on its own by a
-// galloping search from t.  Kept out of line: it runs only when a step holds 32 or more run
-// boundaries (a stretch of empty runs), and inlined its registers would count against the whole
-// kernel.
+// One step of the pair sweep (positions pb + [0, span], the first of them in run t) over many short runs:
+// the boundaries inside the step are counted per position in shared memory (`cntr`, 128 words of the warp's
+// own) and the counts summed along the step, which gives every position's run; its descriptor, element and
+// tally follow with all four positions of a lane in flight.  A stretch of more than kDenseGroups x 32
+// boundaries (empty runs of ranges swept by ranks) is searched position by position instead.
+// Kept out of line: inlined its registers would count against the whole kernel.
+// Files of 1e6 intervals against 3.2e6 have about two candidates a run: 52e9 candidates/s with a search per
+// position, 1.3e11 so.
+constexpr int kDenseGroups = 16;
 template <bool WITH_BP, bool SMEM, int MULTI>
-__device__ __noinline__ void pairs_step_slow(const uint64_t* __restrict__ ppos, const PairSeg* __restrict__ psegs,
-                                             const uint2* __restrict__ pos, const uint32_t* __restrict__ sidv,
-                                             uint32_t* counts, unsigned long long* bp, uint32_t D, uint32_t t,
-                                             uint32_t rcap, uint64_t pb, uint32_t span, uint32_t lane,
-                                             uint32_t* s_cnt, unsigned long long* s_bp, uint32_t cta_row) {
-    for (uint32_t o = lane; o <= span; o += 32) {
-        const uint64_t pj = pb + o;
-        const uint32_t tt = range_advance(ppos, t, rcap, pj);
-        const PairSeg q = psegs[tt];
-        const uint64_t di = q.base + (pj - __ldg(ppos + tt));
-        const uint2 d = __ldg(pos + di);
-        const uint32_t sid = __ldg(sidv + di);
-        if (d.y <= q.qs) continue;
-        if (SMEM && (!MULTI || q.qrow == cta_row)) {
-            atomicAdd(&s_cnt[sid], 1u);
-            if (WITH_BP) add_u64_lo(&s_bp[sid], min(q.qe, d.y) - max(q.qs, d.x));
-        } else {
-            const uint64_t cell = (uint64_t)q.qrow * D + sid;
-            atomicAdd(&counts[cell], 1u);
-            if (WITH_BP) atomicAdd(&bp[cell], (unsigned long long)(min(q.qe, d.y) - max(q.qs, d.x)));
-        }
+__device__ __noinline__ void pairs_step_dense(const uint64_t* __restrict__ ppos, const PairSeg* __restrict__ psegs,
+                                              const uint32_t* __restrict__ prow, const uint2* __restrict__ pos,
+                                              const uint32_t* __restrict__ sidv, uint32_t* counts,
+                                              unsigned long long* bp, uint32_t D, uint32_t t, uint32_t rcap,
+                                              uint64_t pb, uint32_t span, uint32_t lane, uint32_t* cntr,
+                                              uint32_t* s_cnt, unsigned long long* s_bp, uint32_t cta_row) {
+    reinterpret_cast<uint4*>(cntr)[lane] = make_uint4(0, 0, 0, 0);
+    __syncwarp();
+    bool all = false;
+    for (int g = 0; g < kDenseGroups && !all; g++) {
+        const uint64_t k = (uint64_t)t + 1 + 32 * g + lane;
+        const uint64_t B = k <= rcap ? __ldg(ppos + k) : ~0ull;
+        const bool in = B - pb <= span;  // B > pb: run t holds pb
+        if (in) atomicAdd(&cntr[(uint32_t)(B - pb)], 1u);
+        all = __any_sync(0xffffffffu, !in);
     }
+    __syncwarp();
+    if (all) {  // counts into sums along the step
+        uint4 c = reinterpret_cast<uint4*>(cntr)[lane];
+        c.y += c.x;
+        c.z += c.y;
+        c.w += c.z;
+        uint32_t inc = c.w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t w = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= (uint32_t)o) inc += w;
+        }
+        inc -= c.w;
+        reinterpret_cast<uint4*>(cntr)[lane] = make_uint4(c.x + inc, c.y + inc, c.z + inc, c.w + inc);
+    } else {
+#pragma unroll 1
+        for (uint32_t o = lane; o <= span; o += 32) cntr[o] = range_advance(ppos, t, rcap, pb + o) - t;
+    }
+    __syncwarp();
+    constexpr uint32_t U = MULTI ? kPairUnroll : kPairUnroll / 2;  // the one-row sweep has 32 registers a thread
+#pragma unroll 1
+    for (uint32_t o0 = lane; o0 <= span; o0 += 32 * U) {
+        uint2 d[U], q[U];
+        uint32_t sid[U], row[U];
+#pragma unroll
+        for (uint32_t j = 0; j < U; j++) {
+            const uint32_t o = o0 + 32 * j;
+            d[j] = make_uint2(0, 0);  // never a hit: d.y = 0 <= qs
+            q[j] = make_uint2(0, 0);
+            sid[j] = row[j] = 0;
+            if (o <= span) {
+                const uint32_t run = t + cntr[o];
+                const uint4 w = __ldg(reinterpret_cast<const uint4*>(psegs + run));
+                const uint64_t di = (((uint64_t)w.y << 32) | w.x) + (pb + o - __ldg(ppos + run));
+                q[j] = make_uint2(w.z, w.w);
+                d[j] = __ldg(pos + di);
+                sid[j] = __ldg(sidv + di);
+                if ((!SMEM || MULTI) && prow) row[j] = __ldg(prow + run);
+            }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < U; j++)
+            pair_tally<WITH_BP, SMEM, MULTI>(counts, bp, D, q[j].x, q[j].y, row[j], d[j], sid[j], s_cnt, s_bp, cta_row);
+    }
+    __syncwarp();  // cntr is reused by the next step
 }
 
 // The pair sweep: the reference's scan (src/sweep/query.rs:104-115) over the candidate runs of the
@@ -1140,11 +1486,11 @@ __device__ __noinline__ void pairs_step_slow(const uint64_t* __restrict__ ppos, 
 // One work item of the pair sweep (positions [item * chunk, (item + 1) * chunk) of the concatenated
 // candidate runs), walked by one warp.
 template <bool WITH_BP, bool SMEM, int MULTI>
-__device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t item, uint32_t lane, uint32_t rcap,
-                                           uint64_t total, uint32_t* s_cnt, unsigned long long* s_bp,
-                                           uint32_t cta_row) {
-    const uint64_t p0 = (uint64_t)item * P.chunk;
-    const uint64_t p1 = min(p0 + P.chunk, total);
+__device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t chunk, uint32_t item, uint32_t lane, uint32_t rcap,
+                                           uint64_t total, uint32_t* cntr, uint32_t* s_cnt,
+                                           unsigned long long* s_bp, uint32_t cta_row) {
+    const uint64_t p0 = (uint64_t)item * chunk;
+    const uint64_t p1 = min(p0 + chunk, total);
     uint32_t t;
     if (item < P.item_cap) {
         t = __ldg(P.item_t0 + item);
@@ -1155,6 +1501,8 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t item, 
     }
     uint64_t rlo = __ldg(P.ppos + t), rhi = __ldg(P.ppos + t + 1);
     PairSeg ps = P.psegs[t];
+    const bool rowed = (!SMEM || MULTI) && P.rows > 1;
+    uint32_t prow = rowed ? __ldg(P.prow + t) : 0u;
     for (uint64_t pb = p0; pb < p1; pb += 32 * kPairUnroll) {
         const uint64_t pend = min(pb + 32 * kPairUnroll, p1) - 1;
         const uint32_t span = (uint32_t)(pend - pb);
@@ -1163,6 +1511,7 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t item, 
             rlo = __ldg(P.ppos + t);
             rhi = __ldg(P.ppos + t + 1);
             ps = P.psegs[t];
+            if (rowed) prow = __ldg(P.prow + t);
         }
         const uint64_t base0 = ps.base - rlo + pb;  // element of offset 0 when it lies in run t
         if (pend < rhi) {
@@ -1181,7 +1530,7 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t item, 
             }
 #pragma unroll
             for (uint32_t j = 0; j < kPairUnroll; j++)
-                pair_tally<WITH_BP, SMEM, MULTI>(P, ps.qs, ps.qe, ps.qrow, d[j], sid[j], s_cnt, s_bp, cta_row);
+                pair_tally<WITH_BP, SMEM, MULTI>(P.counts, P.bp, P.D, ps.qs, ps.qe, prow, d[j], sid[j], s_cnt, s_bp, cta_row);
             continue;
         }
         // lane l: boundary ppos[t + 1 + l] as an offset from pb (> 0, since run t holds pb);
@@ -1189,9 +1538,9 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t item, 
         const uint64_t B = (uint64_t)t + 1 + lane <= rcap ? __ldg(P.ppos + t + 1 + lane) : ~0ull;
         const uint32_t rel = B - pb < 0xffffffffull ? (uint32_t)(B - pb) : 0xffffffffu;
         const uint32_t nb = __popc(__ballot_sync(0xffffffffu, rel <= span));
-        if (nb == 32) {
-            pairs_step_slow<WITH_BP, SMEM, MULTI>(P.ppos, P.psegs, P.pos, P.sid, P.counts, P.bp, P.D, t, rcap, pb, span,
-                                           lane, s_cnt, s_bp, cta_row);
+        if (nb > kFewBounds) {
+            pairs_step_dense<WITH_BP, SMEM, MULTI>(P.ppos, P.psegs, rowed ? P.prow : nullptr, P.pos, P.sid, P.counts,
+                                                   P.bp, P.D, t, rcap, pb, span, lane, cntr, s_cnt, s_bp, cta_row);
             continue;  // the next step starts past rhi: range_advance finds its run
         }
         uint32_t k[kPairUnroll];  // position lane + 32 j lies in run t + k[j]
@@ -1221,9 +1570,8 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t item, 
 #pragma unroll
         for (uint32_t j = 0; j < kPairUnroll; j++) {
             const PairSeg* q = P.psegs + t + k[j];
-            pair_tally<WITH_BP, SMEM, MULTI>(P, __ldg(&q->qs), __ldg(&q->qe),
-                                             (SMEM && !MULTI) ? 0u : __ldg(&q->qrow), d[j], sid[j], s_cnt, s_bp,
-                                             cta_row);
+            pair_tally<WITH_BP, SMEM, MULTI>(P.counts, P.bp, P.D, __ldg(&q->qs), __ldg(&q->qe), rowed ? __ldg(P.prow + t + k[j]) : 0u,
+                                             d[j], sid[j], s_cnt, s_bp, cta_row);
         }
         // the run of the next step's first position pend + 1, from the boundaries in hand (at
         // least one boundary, ppos[t + 1] <= pend, lies at or below it)
@@ -1233,19 +1581,22 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t item, 
             rlo = __ldg(P.ppos + t);
             rhi = __ldg(P.ppos + t + 1);
             ps = P.psegs[t];
+            if (rowed) prow = __ldg(P.prow + t);
         }
     }
 }
 
 template <bool WITH_BP, bool SMEM, int MULTI>
-__global__ void __launch_bounds__(256, MULTI ? 6 : 8) k_pairs(SweepParams P) {
+__global__ void __launch_bounds__(256, MULTI ? 6 : 8) k_pairs(const __grid_constant__ SweepParams P) {
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned long long* s_bp = reinterpret_cast<unsigned long long*>(smem);
     uint32_t* s_cnt = reinterpret_cast<uint32_t*>(smem + (WITH_BP ? (size_t)P.D * 8 : 0));
+    __shared__ __align__(16) uint32_t s_cntr[8][32 * kPairUnroll];  // pairs_step_dense, one row per warp
+    uint32_t* cntr = s_cntr[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t rcap = *P.pcount;
     const uint64_t total = P.ppos[rcap];
-    P.chunk = item_size(total, P.chunk, P.spread);
+    const uint32_t chunk = item_size(total, P.chunk, P.spread);
     if (SMEM)
         for (uint32_t k = threadIdx.x; k < P.D; k += blockDim.x) {
             s_cnt[k] = 0;
@@ -1254,11 +1605,11 @@ __global__ void __launch_bounds__(256, MULTI ? 6 : 8) k_pairs(SweepParams P) {
     __syncthreads();
     if constexpr (MULTI) {
         // several rows: block items, the histogram serves one row at a time (as k_sweep)
-        const uint64_t items = (total + P.chunk - 1) / P.chunk;
+        const uint64_t items = (total + chunk - 1) / chunk;
         multi_row_loop<false>(
-            P, items, rcap,
+            P, chunk, items, rcap,
             [&](uint32_t item, uint32_t row) {
-                pairs_item<WITH_BP, true, 1>(P, item, lane, rcap, total, s_cnt, s_bp, row);
+                pairs_item<WITH_BP, true, 1>(P, chunk, item, lane, rcap, total, cntr, s_cnt, s_bp, row);
             },
             [&](uint32_t row) { flush_row<WITH_BP>(P, row, s_cnt, s_bp); });
     } else {
@@ -1266,8 +1617,8 @@ __global__ void __launch_bounds__(256, MULTI ? 6 : 8) k_pairs(SweepParams P) {
             uint32_t item = 0;
             if (lane == 0) item = atomicAdd(P.queue, 1u);
             item = __shfl_sync(0xffffffffu, item, 0);
-            if ((uint64_t)item * P.chunk >= total) break;
-            pairs_item<WITH_BP, SMEM, 0>(P, item, lane, rcap, total, s_cnt, s_bp, 0u);
+            if ((uint64_t)item * chunk >= total) break;
+            pairs_item<WITH_BP, SMEM, 0>(P, chunk, item, lane, rcap, total, cntr, s_cnt, s_bp, 0u);
         }
         if (SMEM) {
             __syncthreads();
@@ -1288,8 +1639,10 @@ __global__ void __launch_bounds__(256, MULTI ? 6 : 8) k_pairs(SweepParams P) {
 template <bool EMIT>
 __global__ void __launch_bounds__(256) k_pair_list(const uint64_t* __restrict__ ppos,
                                                    const uint32_t* __restrict__ pcount,
-                                                   const PairSeg* __restrict__ psegs, const uint2* __restrict__ pos,
-                                                   const uint32_t* __restrict__ sid, uint64_t items, uint32_t chunk,
+                                                   const PairSeg* __restrict__ psegs,
+                                                   const uint32_t* __restrict__ prow, uint32_t rows,
+                                                   const uint2* __restrict__ pos, const uint32_t* __restrict__ sid,
+                                                   uint64_t items, uint32_t chunk,
                                                    uint64_t* __restrict__ item_hits,
                                                    const uint64_t* __restrict__ item_base, rgl_pair* __restrict__ out) {
     const uint32_t lane = threadIdx.x & 31u;
@@ -1333,9 +1686,10 @@ __global__ void __launch_bounds__(256) k_pair_list(const uint64_t* __restrict__ 
                 r.query_end = ps.qe;
                 r.db_start = d.x;
                 r.db_end = d.y;
-                r.row = ps.qrow;
+                const uint32_t sr = __ldg(prow + t);  // shard * rows + row
+                r.row = sr % rows;
                 r.sid = __ldg(sid + di);
-                r.shard = ps.shard;
+                r.shard = sr / rows;
                 r.intersection_bp = min(ps.qe, d.y) - max(ps.qs, d.x);
                 out[base + done + rank] = r;
             }
@@ -1363,10 +1717,11 @@ struct rgl_context {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int num_sms = 148;
     DevBuf iv, blk_off, blk_shard, key_a, key_b, val_a, val_b, ekey_a, ekey_b;
-    DevBuf starts, ends, seg, segflag, segnum, seg_begin, ps_in, pe_in, ps, pe;
-    DevBuf lo, hi, maxhi, rflag, ridx, ranges, rlen, rpos, cub_tmp, small, out_counts, out_bp, item_r0;
+    DevBuf starts, ends, shard, row, segnum, seg_begin, ps, pe, emax;
+    DevBuf lo, hi, flags, ranges, rpos, cub_tmp, small, out_counts, out_bp, item_r0;
     DevBuf segtab, tab2;
-    DevBuf cl, pc, method, plen, ppos, psegs, item_t0, seg_need, tl, scan_sums;
+    DevBuf pc, cr, uhi, rt, ulen, rpair, ppos, psegs, prow, item_t0, seg_need;
+    DevBuf sums, esums;  // tile summaries, of the main and of the side stream
     DevBuf cub_tmp2;  // the side stream's own scratch
     DevBuf sortplan;  // block-local sort: order flags, tile and merge-chunk prefix counts, two pass words
     DevBuf sort_tab, sort_rank;  // its segment-order layout, for the single-call entry points
@@ -1453,60 +1808,45 @@ int size_workspace(rgl_context* c, uint64_t n, uint32_t rows, uint32_t nblk, uin
     RGL_TRY(z.ensure_in(c->ekey_b, n * 8 + 8));
     RGL_TRY(z.ensure_in(c->starts, n * 4 + 4));
     RGL_TRY(z.ensure_in(c->ends, n * 4 + 4));
-    RGL_TRY(z.ensure_in(c->seg, n * 4 + 4));
-    RGL_TRY(z.ensure_in(c->segflag, n * 4 + 4));
+    RGL_TRY(z.ensure_in(c->shard, n * 4 + 4));
+    RGL_TRY(z.ensure_in(c->row, n * 4 + 4));
     RGL_TRY(z.ensure_in(c->segnum, n * 4 + 4));
     RGL_TRY(z.ensure_in(c->seg_begin, n * 4 + 4));
     RGL_TRY(z.ensure_in(c->seg_need, n * 8 + 8));
-    RGL_TRY(z.ensure_in(c->ps_in, n * 8 + 16));
-    RGL_TRY(z.ensure_in(c->pe_in, n * 8 + 16));
     RGL_TRY(z.ensure_in(c->ps, n * 8 + 16));
     RGL_TRY(z.ensure_in(c->pe, n * 8 + 16));
     RGL_TRY(z.ensure_in(c->lo, tot * 4 + 4));
     RGL_TRY(z.ensure_in(c->hi, tot * 4 + 4));
-    RGL_TRY(z.ensure_in(c->maxhi, tot * 4 + 4));
-    RGL_TRY(z.ensure_in(c->rflag, tot * 4 + 8));
-    RGL_TRY(z.ensure_in(c->ridx, tot * 4 + 8));
-    RGL_TRY(z.ensure_in(c->ranges, tot * sizeof(RangeDesc) + sizeof(RangeDesc)));
-    RGL_TRY(z.ensure_in(c->rlen, tot * 8 + 16));
-    RGL_TRY(z.ensure_in(c->rpos, tot * 8 + 16));
+    RGL_TRY(z.ensure_in(c->flags, tot / 8 + ns * 32 + 64));
+    RGL_TRY(z.ensure_in(c->ranges, (tot / 2 + 2) * sizeof(RangeDesc)));  // a range swept by ranks has two runs or more
+    RGL_TRY(z.ensure_in(c->rpos, (tot / 2 + 2) * 8));
     RGL_TRY(z.ensure_in(c->small, 256));
     RGL_TRY(z.ensure_in(c->item_r0, kItemCap * 4));
     RGL_TRY(z.ensure_in(c->item_t0, kItemCap * 4));
-    RGL_TRY(z.ensure_in(c->cl, tot * 8 + 16));
+    RGL_TRY(z.ensure_in(c->emax, n * 4 + 4));
     RGL_TRY(z.ensure_in(c->pc, tot * 8 + 16));
-    RGL_TRY(z.ensure_in(c->method, tot + 16));
-    RGL_TRY(z.ensure_in(c->tl, tot * 4 + 8));
-    RGL_TRY(z.ensure_in(c->scan_sums, (tot / kScanTile + 4) * 8));
-    RGL_TRY(z.ensure_in(c->plen, tot * 8 + 16));
+    RGL_TRY(z.ensure_in(c->cr, tot * 4 + 4));
+    RGL_TRY(z.ensure_in(c->uhi, tot * 4 + 4));
+    RGL_TRY(z.ensure_in(c->rt, tot * 8 + 8));
+    RGL_TRY(z.ensure_in(c->ulen, tot * 4 + 4));
+    RGL_TRY(z.ensure_in(c->rpair, tot * 8 + 8));
+    RGL_TRY(z.ensure_in(c->sums, (tot / kTileThreads + tot / kTileThreads / kGroup + 3 * ns + n / kQTile + 8) * sizeof(RSum)));
+    RGL_TRY(z.ensure_in(c->esums, (n / kQTile + n / kQTile / kGroup + 4) * sizeof(ESum)));
     RGL_TRY(z.ensure_in(c->ppos, tot * 8 + 16));
     RGL_TRY(z.ensure_in(c->psegs, tot * sizeof(PairSeg) + sizeof(PairSeg)));
+    RGL_TRY(z.ensure_in(c->prow, tot * 4 + 4));
     RGL_TRY(z.ensure_in(c->segtab, (n + 1) * sizeof(SegTab)));
     RGL_TRY(z.ensure_in(c->tab2, (10 * n + 18) * 8));
     RGL_TRY(z.ensure_in(c->acc, 64));
     // CUB temporary storage: the maximum over every primitive used, at these sizes.
     size_t need = 0, b = 0;
     int nn = (int)std::max<uint64_t>(n, 1);
-    int nt = (int)std::max<uint64_t>(tot + 1, 1);
     cub::DeviceRadixSort::SortPairs(nullptr, b, (uint64_t*)nullptr, (uint64_t*)nullptr, (uint32_t*)nullptr,
                                     (uint32_t*)nullptr, nn, 0, 64, c->stream);
     need = std::max(need, b);
     cub::DeviceRadixSort::SortKeys(nullptr, b, (uint64_t*)nullptr, (uint64_t*)nullptr, nn, 0, 64, c->stream);
     need = std::max(need, b);
-    cub::DeviceScan::InclusiveSum(nullptr, b, (uint32_t*)nullptr, (uint32_t*)nullptr, nn, c->stream);
-    need = std::max(need, b);
     cub::DeviceScan::ExclusiveSum(nullptr, b, (uint64_t*)nullptr, (uint64_t*)nullptr, nn + 1, c->stream);
-    need = std::max(need, b);
-    cub::DeviceScan::ExclusiveSum(nullptr, b, (uint32_t*)nullptr, (uint32_t*)nullptr, nt, c->stream);
-    need = std::max(need, b);
-    cub::DeviceSelect::Flagged(nullptr, b, thrust::counting_iterator<uint32_t>(0), (const uint32_t*)nullptr,
-                               (uint32_t*)nullptr, (uint32_t*)nullptr, nt, c->stream);
-    need = std::max(need, b);
-    cub::DeviceScan::ExclusiveSum(nullptr, b, (uint32_t*)nullptr, (uint32_t*)nullptr, nn + 1, c->stream);
-    need = std::max(need, b);
-    cub::DeviceReduce::Sum(nullptr, b, (uint64_t*)nullptr, (uint64_t*)nullptr, nt, c->stream);
-    need = std::max(need, b);
-    cub::DeviceScan::ExclusiveSum(nullptr, b, (uint64_t*)nullptr, (uint64_t*)nullptr, nt, c->stream);
     need = std::max(need, b);
     RGL_TRY(z.ensure_in(c->cub_tmp, need + 256));
     RGL_TRY(z.ensure_in(c->cub_tmp2, need + 256));
@@ -1521,10 +1861,10 @@ int size_workspace(rgl_context* c, uint64_t n, uint32_t rows, uint32_t nblk, uin
     c->ws_ready = true;
     uint64_t sig = 1469598103934665603ull;
     for (DevBuf* b : {&c->iv, &c->key_a, &c->key_b, &c->val_a, &c->val_b, &c->ekey_a, &c->ekey_b, &c->starts,
-                      &c->ends, &c->seg, &c->segflag, &c->segnum, &c->seg_begin, &c->ps_in, &c->pe_in, &c->ps,
-                      &c->pe, &c->lo, &c->hi, &c->maxhi, &c->rflag, &c->ridx, &c->ranges, &c->rlen, &c->rpos,
-                      &c->cub_tmp, &c->small, &c->item_r0, &c->item_t0, &c->segtab, &c->tab2, &c->cl, &c->pc, &c->method, &c->tl, &c->scan_sums, &c->plen, &c->ppos, &c->psegs,
-                      &c->seg_need, &c->acc, &c->cub_tmp2, &c->sortplan})
+                      &c->ends, &c->shard, &c->row, &c->segnum, &c->seg_begin, &c->ps, &c->pe, &c->emax, &c->lo, &c->hi,
+                      &c->flags, &c->ranges, &c->rpos, &c->cub_tmp, &c->small, &c->item_r0, &c->item_t0, &c->segtab,
+                      &c->tab2, &c->pc, &c->cr, &c->uhi, &c->rt, &c->ulen, &c->rpair, &c->sums, &c->esums, &c->ppos,
+                      &c->psegs, &c->prow, &c->seg_need, &c->acc, &c->cub_tmp2, &c->sortplan})
         sig = (sig ^ (uint64_t)(uintptr_t)b->p ^ ((uint64_t)b->cap << 17)) * 1099511628211ull;
     c->ws_sig = sig;
     return RGL_OK;
@@ -1608,7 +1948,6 @@ int finish(rgl_context* c, const Launch& L, rgl_query_stats* stats) {
     return RGL_OK;
 }
 
-// Exclusive scan of in[0, *n_ptr) into out (with out[n] = total), n <= cap; returns the launches.
 // Launches a short kernel of a pipeline chain: with `pdl` its PDL variant (which begins with
 // pdl_wait()) with programmatic stream serialization, so that it may be scheduled while the previous
 // grid of the stream is finishing; else its plain variant.  PDL is used for small runs, where the
@@ -1633,17 +1972,11 @@ cudaError_t launch_chain(bool pdl, void (*with_pdl)(K...), void (*plain)(K...), 
     return cudaLaunchKernelEx(&cfg, with_pdl, std::forward<A>(args)...);
 }
 
-// `sums` holds cap / kScanTile + 1 tile sums (one buffer per stream that scans concurrently).
-template <typename Tin, typename Tout>
-uint32_t scan_dev(Tout* sums, const Tin* in, Tout* out, const uint32_t* n_ptr, uint64_t cap, cudaStream_t st,
-                  bool pdl) {
-    const unsigned grid = (unsigned)std::min<uint64_t>(cap / kScanTile + 1, 148ull * 8);
-    (void)launch_chain(pdl, k_scan_reduce<Tin, Tout, true>, k_scan_reduce<Tin, Tout, false>, grid, kScanThreads, 0,
-                     st, in, n_ptr, sums);
-    (void)launch_chain(pdl, k_scan_tops<Tout, true>, k_scan_tops<Tout, false>, 1, 1024, 0, st, sums, n_ptr, out);
-    (void)launch_chain(pdl, k_scan_apply<Tin, Tout, true>, k_scan_apply<Tin, Tout, false>, grid, kScanThreads, 0, st,
-                     in, out, n_ptr, sums);
-    return 3;
+// Tile summaries into exclusive prefixes (nt tiles, or those of *count elements), by groups of kGroup.
+template <class T>
+void scan_groups(T* sums, uint32_t nt, const uint32_t* count, uint32_t tile, T* groups, uint32_t ng, cudaStream_t st) {
+    k_group_sums<T><<<ng, kTileThreads, 0, st>>>(sums, nt, count, tile, groups);
+    k_group_scan<T><<<ng, kTileThreads, 0, st>>>(sums, nt, count, tile, groups);
 }
 
 // `to` waits for everything enqueued on `from` so far.
@@ -1800,6 +2133,7 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
         if (mode.reset_err) RGL_CUDA(cudaMemcpyAsync(c->h_small, d_small, 4, cudaMemcpyDeviceToHost, st));
         return RGL_OK;
     }
+    if (!rows) return fail(RGL_ERR_INVALID_ARGUMENT, "a query interval's sid >= num_rows");
     // key width: segment = shard * rows + row
     const uint32_t rb = in.region_bits;
     if (rb && (rb < 16 || rb > 31)) return fail(RGL_ERR_INVALID_ARGUMENT, "region bits must be in [16, 31]");
@@ -1874,72 +2208,63 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
                                                  32 + segbits, st));
     }
     // the side stream goes on with the ends (their prefix sums), the main one with the starts
-    k_unpack_ends<<<grid_for(n + 1, 256), 256, 0, sd>>>(n, c->ekey_b.as<uint64_t>(), c->ends.as<uint32_t>(),
-                                                        c->pe_in.as<uint64_t>());
-    tb = c->cub_tmp2.cap;
-    RGL_CUDA(cub::DeviceScan::ExclusiveSum(c->cub_tmp2.p, tb, c->pe_in.as<uint64_t>(), c->pe.as<uint64_t>(),
-                                           (int)n + 1, sd));
-    k_unpack_starts<<<grid_for(n + 1, 256), 256, 0, st>>>(n, c->key_b.as<uint64_t>(), c->starts.as<uint32_t>(),
-                                                          c->seg.as<uint32_t>(), c->segflag.as<uint32_t>(),
-                                                          c->ps_in.as<uint64_t>());
-    launches += 2;
-    RGL_TRY(stream_after(sd, st, c->ev_fork));
-    tb = c->cub_tmp2.cap;
-    RGL_CUDA(cub::DeviceScan::ExclusiveSum(c->cub_tmp2.p, tb, c->ps_in.as<uint64_t>(), c->ps.as<uint64_t>(),
-                                           (int)n + 1, sd));
-    tb = c->cub_tmp.cap;
-    RGL_CUDA(cub::DeviceScan::InclusiveSum(c->cub_tmp.p, tb, c->segflag.as<uint32_t>(), c->segnum.as<uint32_t>(),
-                                           (int)n, st));
-    k_seg_begin<<<grid_for(n, 256), 256, 0, st>>>(n, c->segflag.as<uint32_t>(), c->segnum.as<uint32_t>(),
-                                                  c->seg_begin.as<uint32_t>());
-    launches++;
-    const uint32_t max_segs = (uint32_t)std::min<uint64_t>(n, nseg);
-    RGL_CUDA(cudaMemsetAsync(c->seg_need.p, 0, (size_t)max_segs * 8, st));
     const uint64_t tot = (uint64_t)n * ns;
     if (tot + 1 >= (1ull << 31)) {
         RGL_TRY(stream_after(st, sd, c->ev_join));
         return fail(RGL_ERR_INVALID_ARGUMENT, "query intervals x layer slots must be < 2^31 per run");
     }
-    k_lohi<<<dim3(grid_for(n, 256), ns), 256, 0, st>>>(n, ns, sps, c->starts.as<uint32_t>(), c->val_b.as<uint32_t>(),
-                                                c->seg.as<uint32_t>(), idx->d_slot, idx->d_layers, idx->d_pos,
-                                                idx->d_btab, c->lo.as<uint32_t>(), c->hi.as<uint32_t>(),
-                                                c->rflag.as<uint32_t>());
-    launches++;
-    // live runs: compaction of the (K, query) entries with a non-empty candidate run (flags from
-    // k_lohi) in one pass: tl[c] = t of the c-th live entry, *Lp = their number
-    uint32_t* Lp = d_small + 8;  // live runs L
-    uint32_t* Rp = d_small + 9;  // ranges R
-    tb = c->cub_tmp.cap;
-    RGL_CUDA(cub::DeviceSelect::Flagged(c->cub_tmp.p, tb, thrust::counting_iterator<uint32_t>(0),
-                                        c->rflag.as<uint32_t>(), c->tl.as<uint32_t>(), Lp, (int)tot, st));
-    {  // running max of hi along every (slot, segment) row, over the live runs: maxhi[c]
-        unsigned long long* sums = c->scan_sums.as<unsigned long long>();
-        const unsigned g = (unsigned)std::min<uint64_t>(tot / kScanTile + 1, 148ull * 8);
-        (void)launch_chain(pdl, k_segmax_reduce<true>, k_segmax_reduce<false>, g, kScanThreads, 0, st, Lp, n,
-                           c->tl.as<uint32_t>(), c->segnum.as<uint32_t>(), c->hi.as<uint32_t>(), sums);
-        (void)launch_chain(pdl, k_segmax_tops<true>, k_segmax_tops<false>, 1, 1024, 0, st, Lp, sums);
-        (void)launch_chain(pdl, k_segmax_apply<true>, k_segmax_apply<false>, g, kScanThreads, 0, st, Lp, n,
-                           c->tl.as<uint32_t>(), c->segnum.as<uint32_t>(), c->hi.as<uint32_t>(), sums,
-                           c->maxhi.as<uint32_t>());
-        launches += 3;
-    }
-    // ranges over the live runs, their candidate counts and methods
-    const unsigned gc = (unsigned)std::min<uint64_t>(grid_for(tot, 256), (uint64_t)c->num_sms * 32);
-    (void)launch_chain(pdl, k_crange_flags<true>, k_crange_flags<false>, gc, 256, 0, st, Lp, n, c->tl.as<uint32_t>(),
-                     c->segnum.as<uint32_t>(), c->lo.as<uint32_t>(), c->hi.as<uint32_t>(), c->maxhi.as<uint32_t>(),
-                     c->rflag.as<uint32_t>(), c->cl.as<uint64_t>());
-    launches++;
-    launches += scan_dev(c->scan_sums.as<uint32_t>(), c->rflag.as<uint32_t>(), c->ridx.as<uint32_t>(), Lp, tot, st, pdl);
-    launches += scan_dev(c->scan_sums.as<uint64_t>(), c->cl.as<uint64_t>(), c->pc.as<uint64_t>(), Lp, tot, st, pdl);
-    (void)launch_chain(pdl, k_crange_emit<true>, k_crange_emit<false>, gc, 256, 0, st, Lp, n, ns, rows, sps,
-                     c->tl.as<uint32_t>(), c->seg.as<uint32_t>(), c->segnum.as<uint32_t>(), idx->d_slot,
-                     c->lo.as<uint32_t>(), c->maxhi.as<uint32_t>(), c->rflag.as<uint32_t>(), c->ridx.as<uint32_t>(),
-                     c->ranges.as<RangeDesc>());
-    (void)launch_chain(pdl, k_crange_method<true>, k_crange_method<false>, gc, 256, 0, st, Lp, c->ridx.as<uint32_t>(),
-                     c->ranges.as<RangeDesc>(), c->pc.as<uint64_t>(), L.pair_ratio, c->method.as<uint8_t>(),
-                     c->rlen.as<uint64_t>(), c->seg_need.as<unsigned long long>(), Rp,
-                     reinterpret_cast<unsigned long long*>(d_small + 4));
-    launches += 2;
+    const uint32_t qt = (n + kQTile - 1) / kQTile;
+    const uint32_t qg = qt > kMaxLook ? (qt + kGroup - 1) / kGroup : 0u;  // groups of tiles, if any
+    ESum* eg = qg ? c->esums.as<ESum>() + qt : nullptr;
+    QSum* qgs = qg ? c->sums.as<QSum>() + qt : nullptr;
+    (void)launch_chain(pdl, k_e_reduce<true>, k_e_reduce<false>, qt, kTileThreads, 0, sd, n,
+                       c->ekey_b.as<uint64_t>(), c->esums.as<ESum>());
+    if (qg) scan_groups(c->esums.as<ESum>(), qt, nullptr, 0, eg, qg, sd);
+    (void)launch_chain(pdl, k_e_apply<true>, k_e_apply<false>, qt, kTileThreads, 0, sd, n, c->ekey_b.as<uint64_t>(),
+                       c->esums.as<ESum>(), (int)(qg != 0), c->ends.as<uint32_t>(), c->pe.as<uint64_t>());
+    (void)launch_chain(pdl, k_q_reduce<true>, k_q_reduce<false>, qt, kTileThreads, 0, st, n,
+                       c->key_b.as<uint64_t>(), c->val_b.as<uint32_t>(), c->sums.as<QSum>());
+    if (qg) scan_groups(c->sums.as<QSum>(), qt, nullptr, 0, qgs, qg, st);
+    (void)launch_chain(pdl, k_q_apply<true>, k_q_apply<false>, qt, kTileThreads, 0, st, n, rows, sps,
+                       c->key_b.as<uint64_t>(), c->val_b.as<uint32_t>(), c->sums.as<QSum>(), (int)(qg != 0),
+                       c->starts.as<uint32_t>(), c->shard.as<uint32_t>(), c->row.as<uint32_t>(), c->segnum.as<uint32_t>(), c->seg_begin.as<uint32_t>(),
+                       c->ps.as<uint64_t>(), c->emax.as<uint32_t>());
+    launches += qg ? 8 : 4;
+    const uint32_t max_segs = (uint32_t)std::min<uint64_t>(n, nseg);
+    RGL_CUDA(cudaMemsetAsync(c->seg_need.p, 0, (size_t)max_segs * 8, st));
+    uint32_t* Lp = d_small + 8;   // live runs L
+    uint32_t* Rp = d_small + 9;   // ranges R
+    uint32_t* RRp = d_small + 14;  // ranges swept by ranks
+    // partition points, live runs and ranges.  k_emit takes four tiles a block, one where that would leave
+    // fewer blocks than the SMs hold at once (8 each)
+    const dim3 lgrid(grid_for(n, kTileThreads), ns);
+    const uint32_t lt = lgrid.x * ns, lg = lt > kMaxLook ? (lt + kGroup - 1) / kGroup : 0u;
+    LSum* lsums = c->sums.as<LSum>();
+    LSum* lgs = lg ? lsums + lt : nullptr;
+    (void)launch_chain(pdl, k_lohi<true>, k_lohi<false>, lgrid, kTileThreads, 0, st, n, ns, c->starts.as<uint32_t>(),
+                       c->val_b.as<uint32_t>(), c->emax.as<uint32_t>(), c->shard.as<uint32_t>(), idx->d_slot,
+                       idx->d_layers, idx->d_pos, idx->d_btab, c->lo.as<uint32_t>(), c->hi.as<uint32_t>(),
+                       c->flags.as<uint32_t>(), lsums);
+    if (lg) scan_groups(lsums, lt, nullptr, 0, lgs, lg, st);
+    const bool wide = lt >= (uint32_t)c->num_sms * 32;
+    const int tag = mode.no_sweep ? RUN_SHARD_ROW : rows > 1 ? RUN_ROW : RUN_PLAIN;
+    (void)launch_chain(pdl, wide ? k_emit<4, true> : k_emit<1, true>, wide ? k_emit<4, false> : k_emit<1, false>,
+                       dim3(wide ? (lgrid.x + 3) / 4 : lgrid.x, ns), kTileThreads, 0, st, n, ns, rows, lgrid.x, tag,
+                       c->starts.as<uint32_t>(), c->val_b.as<uint32_t>(), c->emax.as<uint32_t>(),
+                       c->shard.as<uint32_t>(), c->row.as<uint32_t>(), idx->d_slot, idx->d_layers, idx->d_pos,
+                       idx->d_btab, c->lo.as<uint32_t>(), c->hi.as<uint32_t>(), c->flags.as<uint32_t>(), lsums, (int)(lg != 0),
+                       c->psegs.as<PairSeg>(), c->prow.as<uint32_t>(), c->pc.as<uint64_t>(), c->cr.as<uint32_t>(),
+                       c->uhi.as<uint32_t>(), c->rt.as<uint2>(), Lp, Rp);
+    // the ranges' unions, methods and places; R is a device count, at most tot
+    const unsigned rgrid = (unsigned)std::min<uint64_t>(tot / kRTile + 1, (uint64_t)c->num_sms * 16);
+    RSum* rsums = c->sums.as<RSum>();
+    const uint32_t rtl = (uint32_t)(tot / kRTile + 1), rg = rtl > kMaxLook ? (rtl + kGroup - 1) / kGroup : 0u;
+    RSum* rgs = rg ? rsums + rtl : nullptr;
+    (void)launch_chain(pdl, k_range_reduce<true>, k_range_reduce<false>, rgrid, kTileThreads, 0, st, Lp, Rp, n,
+                       c->rt.as<uint2>(), c->pc.as<uint64_t>(), c->uhi.as<uint32_t>(), c->lo.as<uint32_t>(),
+                       c->segnum.as<uint32_t>(), L.pair_ratio, c->ulen.as<uint32_t>(),
+                       c->seg_need.as<unsigned long long>(), reinterpret_cast<unsigned long long*>(d_small + 4), rsums);
+    launches += lg ? 5 : 3;
     // side stream: rank tables of the query segments that have a rank-difference range
     RGL_TRY(stream_after(sd, st, c->ev_fork));
     k_seg_tabsize<<<grid_for(max_segs, 256), 256, 0, sd>>>(n, c->segnum.as<uint32_t>(), c->seg_begin.as<uint32_t>(),
@@ -1949,18 +2274,18 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
                      c->segnum.as<uint32_t>(), c->segtab.as<SegTab>(), c->starts.as<uint32_t>(),
                      c->ends.as<uint32_t>(), c->tab2.as<uint2>());
     launches += 2;
-    // main stream: the pair work space and the rank ranges' positions
-    (void)launch_chain(pdl, k_cpair_len<true>, k_cpair_len<false>, gc, 256, 0, st, Lp, n, ns, rows, sps,
-                     c->tl.as<uint32_t>(), c->seg.as<uint32_t>(), idx->d_slot, idx->d_layers, c->lo.as<uint32_t>(),
-                     c->hi.as<uint32_t>(), c->rflag.as<uint32_t>(), c->ridx.as<uint32_t>(), c->method.as<uint8_t>(),
-                     c->starts.as<uint32_t>(), c->val_b.as<uint32_t>(), c->plen.as<uint64_t>(),
-                     c->psegs.as<PairSeg>());
-    launches++;
-    launches += scan_dev(c->scan_sums.as<uint64_t>(), c->rlen.as<uint64_t>(), c->rpos.as<uint64_t>(), Rp, tot, st, pdl);
-    launches += scan_dev(c->scan_sums.as<uint64_t>(), c->plen.as<uint64_t>(), c->ppos.as<uint64_t>(), Lp, tot, st, pdl);
+    // main stream: the two work spaces
+    if (rg) scan_groups(rsums, 0, Rp, kRTile, rgs, rg, st);
+    (void)launch_chain(pdl, k_range_apply<true>, k_range_apply<false>, rgrid, kTileThreads, 0, st, Lp, Rp, n, ns, rows,
+                       c->rt.as<uint2>(), c->pc.as<uint64_t>(), c->ulen.as<uint32_t>(), c->lo.as<uint32_t>(),
+                       c->shard.as<uint32_t>(), c->row.as<uint32_t>(), c->segnum.as<uint32_t>(), idx->d_slot, L.pair_ratio, rsums, (int)(rg != 0),
+                       c->ranges.as<RangeDesc>(), c->rpos.as<uint64_t>(), c->rpair.as<uint64_t>(),
+                       c->ppos.as<uint64_t>(), RRp, reinterpret_cast<unsigned long long*>(d_small + 10));
+    const unsigned gc = (unsigned)std::min<uint64_t>(grid_for(tot, 256), (uint64_t)c->num_sms * 32);
+    (void)launch_chain(pdl, k_run_pos<true>, k_run_pos<false>, gc, 256, 0, st, Lp, c->cr.as<uint32_t>(),
+                       c->pc.as<uint64_t>(), c->rpair.as<uint64_t>(), c->ppos.as<uint64_t>());
+    launches += rg ? 4 : 2;
     if (mode.no_sweep) {
-        k_totals<<<1, 32, 0, st>>>(d_small, c->rpos.as<uint64_t>(), c->ppos.as<uint64_t>());
-        launches++;
         RGL_TRY(stream_after(st, sd, c->ev_join));
         c->last_tot = tot;
         c->last_launches = launches;
@@ -1969,7 +2294,7 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
         return RGL_OK;
     }
     (void)launch_chain(pdl, k_item_ranges<true>, k_item_ranges<false>, (unsigned)(c->num_sms * 8), 256, 0, st,
-                     d_small, Rp, c->rpos.as<uint64_t>(), Lp, c->ppos.as<uint64_t>(), L.chunk, L.spread, kItemCap,
+                     RRp, c->rpos.as<uint64_t>(), Lp, c->ppos.as<uint64_t>(), L.chunk, L.spread, kItemCap,
                      c->item_r0.as<uint32_t>(), c->item_t0.as<uint32_t>());
     launches++;
     SweepParams P;
@@ -1977,11 +2302,12 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     P.item_t0 = c->item_t0.as<uint32_t>();
     P.ppos = c->ppos.as<uint64_t>();
     P.psegs = c->psegs.as<PairSeg>();
+    P.prow = c->prow.as<uint32_t>();
     P.segtabs = c->segtab.as<SegTab>();
     P.tab2 = c->tab2.as<uint2>();
     P.item_cap = kItemCap;
     P.rpos = c->rpos.as<uint64_t>();
-    P.rcount = Rp;
+    P.rcount = RRp;
     P.pcount = Lp;
     P.ranges = c->ranges.as<RangeDesc>();
     P.layers = idx->d_layers;
@@ -2430,14 +2756,12 @@ int rgl_context_destroy(rgl_context* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->side) cudaStreamSynchronize(c->side);
     DevBuf* bufs[] = {&c->iv, &c->blk_off, &c->blk_shard, &c->key_a, &c->key_b, &c->val_a, &c->val_b,
-                      &c->ekey_a, &c->ekey_b, &c->starts, &c->ends, &c->seg, &c->segflag, &c->segnum,
-                      &c->seg_begin, &c->ps_in, &c->pe_in, &c->ps, &c->pe, &c->lo, &c->hi, &c->maxhi,
-                      &c->rflag, &c->ridx, &c->ranges, &c->rlen, &c->rpos, &c->cub_tmp, &c->small,
-                      &c->out_counts, &c->out_bp, &c->item_r0,
-                      &c->segtab, &c->tab2,
-                      &c->cl, &c->pc, &c->method, &c->tl, &c->scan_sums, &c->plen, &c->ppos, &c->psegs, &c->item_t0,
-                      &c->seg_need, &c->item_hits, &c->item_base, &c->pairs, &c->bt_off, &c->bt_shard, &c->acc, &c->gc.t_off, &c->gc.t_shard,
-                      &c->cub_tmp2, &c->sortplan, &c->sort_tab, &c->sort_rank};
+                      &c->ekey_a, &c->ekey_b, &c->starts, &c->ends, &c->shard, &c->row, &c->segnum, &c->seg_begin, &c->ps,
+                      &c->pe, &c->emax, &c->lo, &c->hi, &c->flags, &c->ranges, &c->rpos, &c->cub_tmp, &c->small,
+                      &c->out_counts, &c->out_bp, &c->item_r0, &c->segtab, &c->tab2, &c->pc, &c->cr, &c->uhi, &c->rt,
+                      &c->ulen, &c->rpair, &c->sums, &c->esums, &c->ppos, &c->psegs, &c->prow, &c->item_t0, &c->seg_need,
+                      &c->item_hits, &c->item_base, &c->pairs, &c->bt_off, &c->bt_shard, &c->acc, &c->gc.t_off,
+                      &c->gc.t_shard, &c->cub_tmp2, &c->sortplan, &c->sort_tab, &c->sort_rank};
     if (c->gc.exec) cudaGraphExecDestroy(c->gc.exec);
     if (c->gc.graph) cudaGraphDestroy(c->gc.graph);
     if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
@@ -2881,8 +3205,8 @@ int rgl_query_pairs(rgl_context* c, const rgl_query_batch* b, uint64_t capacity,
     RGL_TRY(c->cub_tmp.ensure(tb + 256));
     const unsigned grid = (unsigned)std::min<uint64_t>((items * 32 + 255) / 256, (uint64_t)c->num_sms * 16);
     RGL_CUDA(cudaMemsetAsync(c->item_hits.as<uint64_t>() + items, 0, 8, st));
-    k_pair_list<false><<<grid, 256, 0, st>>>(c->ppos.as<uint64_t>(), Lp, c->psegs.as<PairSeg>(), c->idx->d_pos,
-                                             c->idx->d_sid, items, chunk, c->item_hits.as<uint64_t>(), nullptr,
+    k_pair_list<false><<<grid, 256, 0, st>>>(c->ppos.as<uint64_t>(), Lp, c->psegs.as<PairSeg>(),
+                                             c->prow.as<uint32_t>(), b->num_rows, c->idx->d_pos, c->idx->d_sid, items, chunk, c->item_hits.as<uint64_t>(), nullptr,
                                              nullptr);
     tb = c->cub_tmp.cap;
     RGL_CUDA(cub::DeviceScan::ExclusiveSum(c->cub_tmp.p, tb, c->item_hits.as<uint64_t>(), c->item_base.as<uint64_t>(),
@@ -2894,8 +3218,8 @@ int rgl_query_pairs(rgl_context* c, const rgl_query_batch* b, uint64_t capacity,
     if (!pairs || !hits) return RGL_OK;
     if (capacity < hits) return fail(RGL_ERR_INVALID_ARGUMENT, "pair capacity too small (needs " + std::to_string(hits) + ")");
     RGL_TRY(c->pairs.ensure(hits * sizeof(rgl_pair)));
-    k_pair_list<true><<<grid, 256, 0, st>>>(c->ppos.as<uint64_t>(), Lp, c->psegs.as<PairSeg>(), c->idx->d_pos,
-                                            c->idx->d_sid, items, chunk, nullptr, c->item_base.as<uint64_t>(),
+    k_pair_list<true><<<grid, 256, 0, st>>>(c->ppos.as<uint64_t>(), Lp, c->psegs.as<PairSeg>(),
+                                            c->prow.as<uint32_t>(), b->num_rows, c->idx->d_pos, c->idx->d_sid, items, chunk, nullptr, c->item_base.as<uint64_t>(),
                                             c->pairs.as<rgl_pair>());
     RGL_CUDA(cudaGetLastError());
     RGL_CUDA(cudaMemcpyAsync(pairs, c->pairs.p, hits * sizeof(rgl_pair), cudaMemcpyDeviceToHost, st));
