@@ -4,6 +4,7 @@
 #include <type_traits>
 
 #include "block_sort.cuh"
+#include "pdl.cuh"
 
 namespace rgl {
 namespace {
@@ -21,8 +22,13 @@ __device__ inline uint32_t find_block(const uint32_t* __restrict__ pre, uint32_t
 // Exclusive prefix counts of the blocks' tiles and merge chunks, by one thread block: each thread
 // sums a contiguous stretch of blocks, a block scan of the stretch totals gives each stretch its
 // offset, and the stretch is written.
+template <bool PDL>
 __global__ void __launch_bounds__(1024) k_sort_plan(uint32_t nblk, const uint64_t* __restrict__ blk_off,
                                                     uint32_t* __restrict__ tile_pre, uint32_t* __restrict__ chunk_pre) {
+    if constexpr (PDL) {
+        pdl_wait();
+        pdl_release();
+    }
     __shared__ uint32_t pt[1024], pc[1024];
     const uint32_t t = threadIdx.x;
     const uint32_t per = (nblk + 1023) / 1024;
@@ -69,13 +75,17 @@ struct BlockSortTypes {
 // The tiles of ordered blocks, copied to the output (one tile per thread block, coalesced; the
 // tiles of other blocks return at once).  Few registers, so the copy runs at full occupancy instead
 // of in the sort's register-heavy blocks.
-template <bool VALUES>
+template <bool VALUES, bool PDL>
 __global__ void __launch_bounds__(kBsThreads) k_tile_copy(uint32_t nblk, const uint64_t* __restrict__ blk_off,
                                                             const uint32_t* __restrict__ tile_pre,
                                                             const uint32_t* __restrict__ unsorted,
                                                             const uint64_t* __restrict__ kin,
                                                             const uint32_t* __restrict__ vin, uint64_t* __restrict__ kout,
                                                             uint32_t* __restrict__ vout) {
+    if constexpr (PDL) {
+        pdl_wait();
+        pdl_release();
+    }
     const uint32_t tile = blockIdx.x;
     if (tile >= __ldg(tile_pre + nblk)) return;
     const uint32_t blk = find_block(tile_pre, nblk, tile);
@@ -96,7 +106,7 @@ __global__ void __launch_bounds__(kBsThreads) k_tile_copy(uint32_t nblk, const u
 // unsorted[b] != 0: block b is not in order (only such blocks are sorted here).  Output: `out` when
 // the block needs an even number of merge passes, else in place (`in`); *maxp: the most merge
 // passes any of these blocks needs.
-template <bool VALUES>
+template <bool VALUES, bool PDL>
 __global__ void __launch_bounds__(kBsThreads) k_tile_sort(uint32_t nblk, const uint64_t* __restrict__ blk_off,
                                                             const uint32_t* __restrict__ tile_pre,
                                                             const uint32_t* __restrict__ unsorted, uint64_t* kin,
@@ -105,6 +115,10 @@ __global__ void __launch_bounds__(kBsThreads) k_tile_sort(uint32_t nblk, const u
     using T = BlockSortTypes<VALUES>;
     extern __shared__ __align__(16) unsigned char bs_smem[];
     typename T::Smem& sm = *reinterpret_cast<typename T::Smem*>(bs_smem);
+    if constexpr (PDL) {
+        pdl_wait();
+        pdl_release();
+    }
     const uint32_t tile = blockIdx.x;
     if (tile >= __ldg(tile_pre + nblk)) return;
     const uint32_t blk = find_block(tile_pre, nblk, tile);
@@ -176,7 +190,7 @@ __device__ inline uint32_t merge_split(const K* a, uint32_t na, const K* b, uint
 // chunks; CTAs past the last chunk, of ordered blocks or of blocks needing fewer passes return).
 // A block needing p passes reads buffer A at pass q when p - q + 1 is odd, else B, and writes the
 // other one.
-template <bool VALUES>
+template <bool VALUES, bool PDL>
 __global__ void __launch_bounds__(kMergeThreads) k_merge_pass(uint32_t q, uint32_t nblk,
                                                               const uint64_t* __restrict__ blk_off,
                                                               const uint32_t* __restrict__ chunk_pre,
@@ -186,6 +200,10 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_pass(uint32_t q, uint32
     __shared__ uint32_t sk[kMergeChunk], sv[VALUES ? kMergeChunk : 1];
     __shared__ uint32_t ok[kMergeChunk], ov[VALUES ? kMergeChunk : 1];
     __shared__ uint32_t s_split[2];
+    if constexpr (PDL) {
+        pdl_wait();
+        pdl_release();
+    }
     if (q > *maxp) return;  // no block out of order needs this pass
     const uint32_t chunk = blockIdx.x;
     if (chunk >= __ldg(chunk_pre + nblk)) return;
@@ -249,21 +267,22 @@ static_assert(block_sort_smem<true>() <= 48 * 1024 && block_sort_smem<false>() <
 template <bool VALUES>
 uint32_t enqueue_t(uint32_t nblk, const uint64_t* off, uint64_t tiles, uint64_t chunks, uint32_t passes,
                    uint32_t* tile_pre, uint32_t* chunk_pre, const uint32_t* unsorted, uint64_t* ka, uint32_t* va,
-                   uint64_t* kb, uint32_t* vb, uint32_t* maxp, cudaStream_t st, bool plan) {
+                   uint64_t* kb, uint32_t* vb, uint32_t* maxp, cudaStream_t st, bool plan, bool pdl) {
     uint32_t launches = 0;
     if (plan) {
-        k_sort_plan<<<1, 1024, 0, st>>>(nblk, off, tile_pre, chunk_pre);
+        (void)launch_chain(pdl, k_sort_plan<true>, k_sort_plan<false>, 1, 1024, 0, st, nblk, off, tile_pre, chunk_pre);
         launches++;
     }
     if (!tiles) return launches;
-    cudaMemsetAsync(maxp, 0, 4, st);
-    k_tile_copy<VALUES><<<(unsigned)tiles, kBsThreads, 0, st>>>(nblk, off, tile_pre, unsorted, ka, va, kb, vb);
-    k_tile_sort<VALUES><<<(unsigned)tiles, kBsThreads, block_sort_smem<VALUES>(), st>>>(nblk, off, tile_pre, unsorted,
-                                                                                      ka, va, kb, vb, maxp);
+    // (the sort of keys alone opens the side stream's chain, after an event wait: a plain launch)
+    (void)launch_chain(pdl && VALUES, k_tile_copy<VALUES, true>, k_tile_copy<VALUES, false>, (unsigned)tiles, kBsThreads, 0, st,
+                       nblk, off, tile_pre, unsorted, ka, va, kb, vb);
+    (void)launch_chain(pdl, k_tile_sort<VALUES, true>, k_tile_sort<VALUES, false>, (unsigned)tiles, kBsThreads,
+                       block_sort_smem<VALUES>(), st, nblk, off, tile_pre, unsorted, ka, va, kb, vb, maxp);
     launches += 2;
     for (uint32_t q = 1; q <= passes && chunks; q++) {
-        k_merge_pass<VALUES><<<(unsigned)chunks, kMergeThreads, 0, st>>>(q, nblk, off, chunk_pre, unsorted, ka, va, kb,
-                                                                       vb, maxp);
+        (void)launch_chain(pdl, k_merge_pass<VALUES, true>, k_merge_pass<VALUES, false>, (unsigned)chunks,
+                           kMergeThreads, 0, st, q, nblk, off, chunk_pre, unsorted, ka, va, kb, vb, maxp);
         launches++;
     }
     return launches;
@@ -273,11 +292,12 @@ uint32_t enqueue_t(uint32_t nblk, const uint64_t* off, uint64_t tiles, uint64_t 
 
 uint32_t block_sort_enqueue(uint32_t nblk, const uint64_t* off, uint64_t tiles, uint64_t chunks, uint32_t passes,
                             uint32_t* tile_pre, uint32_t* chunk_pre, const uint32_t* unsorted, uint64_t* ka,
-                            uint32_t* va, uint64_t* kb, uint32_t* vb, uint32_t* maxp, cudaStream_t st, bool plan) {
+                            uint32_t* va, uint64_t* kb, uint32_t* vb, uint32_t* maxp, cudaStream_t st, bool plan,
+                            bool pdl) {
     return va ? enqueue_t<true>(nblk, off, tiles, chunks, passes, tile_pre, chunk_pre, unsorted, ka, va, kb, vb, maxp,
-                                st, plan)
+                                st, plan, pdl)
               : enqueue_t<false>(nblk, off, tiles, chunks, passes, tile_pre, chunk_pre, unsorted, ka, nullptr, kb,
-                                 nullptr, maxp, st, plan);
+                                 nullptr, maxp, st, plan, pdl);
 }
 
 }  // namespace rgl

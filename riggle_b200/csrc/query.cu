@@ -37,6 +37,7 @@
 
 #include "block_sort.cuh"
 #include "internal.h"
+#include "pdl.cuh"
 
 namespace rgl {
 
@@ -66,15 +67,6 @@ struct SegTab {
 };
 
 enum : uint32_t { ERR_BAD_INTERVAL = 1u, ERR_BAD_ROW = 2u };
-
-// Programmatic dependent launch.  The short kernels of the pipeline's chains have a PDL variant
-// (template flag PDL) that starts with pdl_wait(): it returns once the grid launched before it on
-// the stream has completed and its memory is visible, so nothing is read or written before it.
-// pdl_release() lets the next grid of the stream be scheduled before this one finishes; that grid
-// still waits in pdl_wait() for this one to complete.  Large runs launch the variants without
-// either instruction.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- small device helpers ----------------------------------------------------------------------
 __device__ __forceinline__ uint32_t lb_u32(const uint32_t* __restrict__ a, uint32_t lo, uint32_t hi, uint32_t x) {
@@ -126,12 +118,32 @@ __device__ __forceinline__ void pp_layer2(const uint2* __restrict__ pos, const u
 }
 
 // ---- 1. keys ------------------------------------------------------------------------------------
+// Zeroes the words of up to five regions (the run's counters, outputs, sort flags and per-segment sums):
+// one launch instead of a memset each (7 of them, 4 us of stream time each).
+struct ClearList {
+    static constexpr int kMax = 5;
+    uint32_t* p[kMax];
+    uint64_t words[kMax];
+    int count;
+};
+__global__ void __launch_bounds__(256) k_clear(ClearList list) {
+    for (int r = 0; r < list.count; r++)
+        for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < list.words[r];
+             i += (uint64_t)gridDim.x * blockDim.x)
+            list.p[r][i] = 0u;
+}
+
+template <bool PDL>
 __global__ void k_expand_keys(uint32_t n, const rgl_interval* __restrict__ iv, const uint64_t* __restrict__ blk_off,
                               const uint32_t* __restrict__ blk_shard, const uint32_t* __restrict__ blk_row,
                               int row_from_block, uint32_t nblk, uint32_t rows, uint32_t row_base, uint32_t rb,
                               uint64_t* __restrict__ key, uint32_t* __restrict__ val, uint64_t* __restrict__ ekey,
                               uint32_t* __restrict__ err, uint32_t* __restrict__ unsorted,
                               const uint64_t* __restrict__ sdst, const uint32_t* __restrict__ sidx) {
+    if constexpr (PDL) {
+        pdl_wait();
+        pdl_release();
+    }
     // block b with blk_off[b] <= i < blk_off[b+1]: one search per thread block, for its first
     // element, then a short walk (256 consecutive elements span few blocks)
     __shared__ uint32_t s_b0;
@@ -1337,6 +1349,8 @@ __global__ void __launch_bounds__(256, 5) k_sweep(const __grid_constant__ SweepP
     const uint32_t rcap = *P.rcount;
     const uint64_t total = P.rpos[rcap];
     const uint32_t chunk = item_size(total, P.chunk, P.spread);
+    // a block with no item for any of its warps (every warp pulls on until the items run out)
+    if ((uint64_t)blockIdx.x * kCtaItems * chunk >= total) return;
     if (P.smem_tally) {
         for (uint32_t k = threadIdx.x; k < P.D; k += blockDim.x) {
             s_cnt[k] = 0;
@@ -1597,6 +1611,7 @@ __global__ void __launch_bounds__(256, MULTI ? 6 : 8) k_pairs(const __grid_const
     const uint32_t rcap = *P.pcount;
     const uint64_t total = P.ppos[rcap];
     const uint32_t chunk = item_size(total, P.chunk, P.spread);
+    if ((uint64_t)blockIdx.x * kCtaItems * chunk >= total) return;  // as k_sweep
     if (SMEM)
         for (uint32_t k = threadIdx.x; k < P.D; k += blockDim.x) {
             s_cnt[k] = 0;
@@ -1948,30 +1963,6 @@ int finish(rgl_context* c, const Launch& L, rgl_query_stats* stats) {
     return RGL_OK;
 }
 
-// Launches a short kernel of a pipeline chain: with `pdl` its PDL variant (which begins with
-// pdl_wait()) with programmatic stream serialization, so that it may be scheduled while the previous
-// grid of the stream is finishing; else its plain variant.  PDL is used for small runs, where the
-// launch latency between the short kernels of a chain is a visible share of the run.
-template <typename... K, typename... A>
-cudaError_t launch_chain(bool pdl, void (*with_pdl)(K...), void (*plain)(K...), dim3 grid, dim3 block, size_t smem,
-                         cudaStream_t st, A&&... args) {
-    if (!pdl) {
-        plain<<<grid, block, smem, st>>>(std::forward<A>(args)...);  // errors surface at the next check
-        return cudaSuccess;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, with_pdl, std::forward<A>(args)...);
-}
-
 // Tile summaries into exclusive prefixes (nt tiles, or those of *count elements), by groups of kGroup.
 template <class T>
 void scan_groups(T* sums, uint32_t nt, const uint32_t* count, uint32_t tile, T* groups, uint32_t ng, cudaStream_t st) {
@@ -2119,13 +2110,26 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     const bool pdl = in.n <= kPdlMaxIntervals;
 
     uint32_t* d_small = c->small.as<uint32_t>();  // [0] error bits, [1] queue, [2..] scratch
-    if (mode.reset_err) RGL_CUDA(cudaMemsetAsync(d_small, 0, 64, st));
-    else RGL_CUDA(cudaMemsetAsync(d_small + 1, 0, 60, st));
+    ClearList clear{};
+    auto to_clear = [&](void* p, uint64_t words) {
+        if (p && words) {
+            clear.p[clear.count] = static_cast<uint32_t*>(p);
+            clear.words[clear.count++] = words;
+        }
+    };
+    auto run_clear = [&] {
+        uint64_t most = 0;
+        for (int r = 0; r < clear.count; r++) most = std::max(most, clear.words[r]);
+        k_clear<<<(unsigned)std::min<uint64_t>(grid_for(most, 256), (uint64_t)c->num_sms * 16), 256, 0, st>>>(clear);
+    };
+    if (mode.reset_err) to_clear(d_small, 16);
+    else to_clear(d_small + 1, 15);
     if (mode.zero_out) {
-        if (d_counts) RGL_CUDA(cudaMemsetAsync(d_counts, 0, (size_t)rows * D * 4, st));
-        if (d_bp) RGL_CUDA(cudaMemsetAsync(d_bp, 0, (size_t)rows * D * 8, st));
+        to_clear(d_counts, (uint64_t)rows * D);
+        to_clear(d_bp, (uint64_t)rows * D * 2);
     }
     if (n == 0 || ns == 0) {
+        run_clear();
         c->last_n = 0;
         c->last_tot = 0;
         c->last_launches = 0;
@@ -2169,36 +2173,37 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
         sort_dst = sort_off + nb1;
         sort_idx = c->sort_rank.as<uint32_t>();
     }
-    // block-local sort: per-block order flags ([0, nblk) starts, [nblk, 2 nblk) ends), then the
-    // tile and merge-chunk prefix counts
+    // block-local sort: per-block order flags ([0, nblk) starts, [nblk, 2 nblk) ends), the two sorts'
+    // pass words, then the tile and merge-chunk prefix counts
     uint32_t* d_unsorted = c->sortplan.as<uint32_t>();
-    uint32_t* d_tile_pre = d_unsorted + 2ull * in.nblk;
+    uint32_t* d_maxp = d_unsorted + 2ull * in.nblk;
+    uint32_t* d_tile_pre = d_maxp + 2;
     uint32_t* d_chunk_pre = d_tile_pre + in.nblk + 1;
-    if (in.block_local) RGL_CUDA(cudaMemsetAsync(d_unsorted, 0, 2ull * in.nblk * 4, st));
-    k_expand_keys<<<grid_for(n, 256), 256, 0, st>>>(n, in.iv, in.blk_off, in.blk_shard, in.blk_row,
-                                                    in.row_from_block, in.nblk, rows, in.row_base, rb,
-                                                    c->key_a.as<uint64_t>(), c->val_a.as<uint32_t>(),
-                                                    c->ekey_a.as<uint64_t>(), d_small,
-                                                    in.block_local ? d_unsorted : nullptr,
-                                                    in.block_local ? sort_dst : nullptr,
-                                                    in.block_local ? sort_idx : nullptr);
-    launches++;
+    if (in.block_local) to_clear(d_unsorted, 2ull * in.nblk + 2);
+    const uint32_t max_segs = (uint32_t)std::min<uint64_t>(n, nseg);
+    to_clear(c->seg_need.p, 2ull * max_segs);
+    run_clear();
+    (void)launch_chain(pdl, k_expand_keys<true>, k_expand_keys<false>, grid_for(n, 256), 256, 0, st, n, in.iv,
+                       in.blk_off, in.blk_shard, in.blk_row, in.row_from_block, in.nblk, rows, in.row_base, rb,
+                       c->key_a.as<uint64_t>(), c->val_a.as<uint32_t>(), c->ekey_a.as<uint64_t>(), d_small,
+                       in.block_local ? d_unsorted : nullptr, in.block_local ? sort_dst : nullptr,
+                       in.block_local ? sort_idx : nullptr);
+    launches += 2;
     // the sort's view of the blocks: their offsets in the layout the keys were written in
     const uint64_t* soff = sort_dst ? sort_off : in.blk_off;
     const uint32_t passes = in.block_local ? sort_passes(in.ls.max_block) : 0u;
     if (in.block_local)  // the plan (before the fork), then the end keys here and the start keys there
         launches += block_sort_enqueue(in.nblk, soff, 0, 0, 0, d_tile_pre, d_chunk_pre, nullptr, nullptr, nullptr,
-                                       nullptr, nullptr, nullptr, st, true);
+                                       nullptr, nullptr, nullptr, st, true, pdl);
     RGL_TRY(stream_after(sd, st, c->ev_fork));
     size_t tb = c->cub_tmp2.cap;
     if (in.block_local) {
         launches += block_sort_enqueue(in.nblk, soff, in.ls.tiles, in.ls.chunks, passes, d_tile_pre, d_chunk_pre,
                                        d_unsorted + in.nblk, c->ekey_a.as<uint64_t>(), nullptr,
-                                       c->ekey_b.as<uint64_t>(), nullptr, d_chunk_pre + in.nblk + 2, sd, false);
+                                       c->ekey_b.as<uint64_t>(), nullptr, d_maxp + 1, sd, false, pdl);
         launches += block_sort_enqueue(in.nblk, soff, in.ls.tiles, in.ls.chunks, passes, d_tile_pre, d_chunk_pre,
                                        d_unsorted, c->key_a.as<uint64_t>(), c->val_a.as<uint32_t>(),
-                                       c->key_b.as<uint64_t>(), c->val_b.as<uint32_t>(), d_chunk_pre + in.nblk + 1, st,
-                                       false);
+                                       c->key_b.as<uint64_t>(), c->val_b.as<uint32_t>(), d_maxp, st, false, pdl);
     } else {
         RGL_CUDA(cub::DeviceRadixSort::SortKeys(c->cub_tmp2.p, tb, c->ekey_a.as<uint64_t>(), c->ekey_b.as<uint64_t>(),
                                                 (int)n, 0, 32 + segbits, sd));
@@ -2230,8 +2235,6 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
                        c->starts.as<uint32_t>(), c->shard.as<uint32_t>(), c->row.as<uint32_t>(), c->segnum.as<uint32_t>(), c->seg_begin.as<uint32_t>(),
                        c->ps.as<uint64_t>(), c->emax.as<uint32_t>());
     launches += qg ? 8 : 4;
-    const uint32_t max_segs = (uint32_t)std::min<uint64_t>(n, nseg);
-    RGL_CUDA(cudaMemsetAsync(c->seg_need.p, 0, (size_t)max_segs * 8, st));
     uint32_t* Lp = d_small + 8;   // live runs L
     uint32_t* Rp = d_small + 9;   // ranges R
     uint32_t* RRp = d_small + 14;  // ranges swept by ranks

@@ -786,6 +786,7 @@ static int enqueue_batch_groups(rgl_context* ctx, rgl_moments* m, StatsScratch* 
             uint32_t* tile_heads = unsorted + nblk;
             uint32_t* tile_off = tile_heads + tiles + 1;
             RGL_CUDA(cudaMemsetAsync(unsorted, 0x01, nblk * 4ull, st));
+            RGL_CUDA(cudaMemsetAsync(tile_off + tiles + 1, 0, 4, st));  // the sort's pass word
             block_sort_enqueue(nblk, d_boff, tiles, chunks, sort_passes(max_block), tile_pre, chunk_pre, unsorted,
                                sc->key_a.as<uint64_t>(), sc->len_a.as<uint32_t>(), sc->key_b.as<uint64_t>(),
                                sc->len_b.as<uint32_t>(), tile_off + tiles + 1, st, true);
