@@ -63,12 +63,17 @@ __global__ void __launch_bounds__(1024) k_sort_plan(uint32_t nblk, const uint64_
     }
 }
 
-template <bool VALUES>
+// What a block is sorted by: the low word of its keys, or (WIDE) the whole key.
+template <bool WIDE>
+using SortKey = typename std::conditional<WIDE, uint64_t, uint32_t>::type;
+
+template <bool VALUES, bool WIDE>
 struct BlockSortTypes {
-    using Sort = cub::BlockRadixSort<uint32_t, kBsThreads, kBsItems, typename std::conditional<VALUES, uint32_t, cub::NullType>::type>;
+    using K = SortKey<WIDE>;
+    using Sort = cub::BlockRadixSort<K, kBsThreads, kBsItems, typename std::conditional<VALUES, uint32_t, cub::NullType>::type>;
     union Smem {
         typename Sort::TempStorage sort;
-        uint32_t last[kBsThreads];
+        K last[kBsThreads];
     };
 };
 
@@ -106,13 +111,14 @@ __global__ void __launch_bounds__(kBsThreads) k_tile_copy(uint32_t nblk, const u
 // unsorted[b] != 0: block b is not in order (only such blocks are sorted here).  Output: `out` when
 // the block needs an even number of merge passes, else in place (`in`); *maxp: the most merge
 // passes any of these blocks needs.
-template <bool VALUES, bool PDL>
+template <bool VALUES, bool WIDE, bool PDL>
 __global__ void __launch_bounds__(kBsThreads) k_tile_sort(uint32_t nblk, const uint64_t* __restrict__ blk_off,
                                                             const uint32_t* __restrict__ tile_pre,
                                                             const uint32_t* __restrict__ unsorted, uint64_t* kin,
                                                             uint32_t* vin, uint64_t* __restrict__ kout,
                                                             uint32_t* __restrict__ vout, uint32_t* __restrict__ maxp) {
-    using T = BlockSortTypes<VALUES>;
+    using T = BlockSortTypes<VALUES, WIDE>;
+    using K = SortKey<WIDE>;
     extern __shared__ __align__(16) unsigned char bs_smem[];
     typename T::Smem& sm = *reinterpret_cast<typename T::Smem*>(bs_smem);
     if constexpr (PDL) {
@@ -131,31 +137,39 @@ __global__ void __launch_bounds__(kBsThreads) k_tile_sort(uint32_t nblk, const u
     if (threadIdx.x == 0 && tile == tile_pre[blk] && passes) atomicMax(maxp, passes);
     uint64_t* ko = (passes & 1u) ? kin : kout;
     uint32_t* vo = (passes & 1u) ? vin : vout;
-    const uint64_t hi = kin[base] & 0xFFFFFFFF00000000ull;  // the block's segment, in the high word
-    uint32_t k[kBsItems], v[kBsItems];
-    uint32_t any = 0;
+    const uint64_t first = kin[base];
+    const uint64_t hi = WIDE ? 0ull : first & 0xFFFFFFFF00000000ull;  // the block's segment, in the high word
+    K k[kBsItems];
+    uint32_t v[kBsItems];
+    K any = 0;
     bool ok = true;
 #pragma unroll
     for (int j = 0; j < kBsItems; j++) {
         const uint32_t i = threadIdx.x * kBsItems + j;  // blocked: thread t holds [16 t, 16 t + 16)
-        k[j] = i < cnt ? (uint32_t)kin[base + i] : 0xFFFFFFFFu;  // padding sorts last
+        k[j] = i < cnt ? (K)kin[base + i] : ~(K)0;  // padding sorts last
         v[j] = (VALUES && i < cnt) ? vin[base + i] : 0u;
-        any |= i < cnt ? k[j] : 0u;
+        any |= i < cnt ? (WIDE ? k[j] ^ (K)first : k[j]) : (K)0;
         if (j) ok = ok && k[j - 1] <= k[j];
     }
-    __shared__ uint32_t s_bits;  // bitwise OR of the tile's keys
+    __shared__ uint32_t s_bits[2];  // bitwise OR of the tile's keys (WIDE: of their differences from the first)
     sm.last[threadIdx.x] = k[kBsItems - 1];
-    if (threadIdx.x == 0) s_bits = 0;
+    if (threadIdx.x < 2) s_bits[threadIdx.x] = 0;
     __syncthreads();
     if (threadIdx.x) ok = ok && sm.last[threadIdx.x - 1] <= k[0];
-    any = __reduce_or_sync(0xffffffffu, any);
-    if ((threadIdx.x & 31u) == 0) atomicOr(&s_bits, any);
+    const uint32_t any_lo = __reduce_or_sync(0xffffffffu, (uint32_t)any);
+    const uint32_t any_hi = WIDE ? __reduce_or_sync(0xffffffffu, (uint32_t)((uint64_t)any >> 32)) : 0u;
+    if ((threadIdx.x & 31u) == 0) {
+        atomicOr(&s_bits[0], any_lo);
+        if (WIDE) atomicOr(&s_bits[1], any_hi);
+    }
     // also orders every read of the tile before the in-place writes below, and the atomicOr
     // before the read of s_bits
     const bool sorted = __syncthreads_and(ok);
-    const uint32_t bits = s_bits;
+    const uint32_t blo = s_bits[0], bhi = s_bits[1];
     if (!sorted) {
-        const int end_bit = bits ? 32 - __clz(bits) : 1;
+        // padding differs from every key in all sorted bits' order only if a bit above them is sorted too:
+        // its all-ones low bits keep it last among equals by its position (the sort is stable)
+        const int end_bit = bhi ? 64 - __clz(bhi) : blo ? 32 - __clz(blo) : 1;
         if constexpr (VALUES)
             typename T::Sort(sm.sort).Sort(k, v, 0, end_bit);
         else
@@ -171,17 +185,17 @@ __global__ void __launch_bounds__(kBsThreads) k_tile_sort(uint32_t nblk, const u
     }
 }
 
-template <bool VALUES>
-constexpr size_t block_sort_smem() { return sizeof(typename BlockSortTypes<VALUES>::Smem); }
+template <bool VALUES, bool WIDE>
+constexpr size_t block_sort_smem() { return sizeof(typename BlockSortTypes<VALUES, WIDE>::Smem); }
 
 // Merge-path split of output diagonal d of runs a (na keys) and b (nb keys): the number of the d
 // first outputs that come from a, ties going to a (stability).
-template <class K>
-__device__ inline uint32_t merge_split(const K* a, uint32_t na, const K* b, uint32_t nb, uint32_t d) {
+template <class K, class A>
+__device__ inline uint32_t merge_split(const A* a, uint32_t na, const A* b, uint32_t nb, uint32_t d) {
     uint32_t lo = d > nb ? d - nb : 0u, hi = min(d, na);
     while (lo < hi) {
         const uint32_t m = (lo + hi) >> 1;
-        if ((uint32_t)a[m] <= (uint32_t)b[d - 1 - m]) lo = m + 1; else hi = m;
+        if ((K)a[m] <= (K)b[d - 1 - m]) lo = m + 1; else hi = m;
     }
     return lo;
 }
@@ -190,15 +204,16 @@ __device__ inline uint32_t merge_split(const K* a, uint32_t na, const K* b, uint
 // chunks; CTAs past the last chunk, of ordered blocks or of blocks needing fewer passes return).
 // A block needing p passes reads buffer A at pass q when p - q + 1 is odd, else B, and writes the
 // other one.
-template <bool VALUES, bool PDL>
+template <bool VALUES, bool WIDE, bool PDL>
 __global__ void __launch_bounds__(kMergeThreads) k_merge_pass(uint32_t q, uint32_t nblk,
                                                               const uint64_t* __restrict__ blk_off,
                                                               const uint32_t* __restrict__ chunk_pre,
                                                               const uint32_t* __restrict__ unsorted, uint64_t* ka,
                                                               uint32_t* va, uint64_t* kb, uint32_t* vb,
                                                               const uint32_t* __restrict__ maxp) {
-    __shared__ uint32_t sk[kMergeChunk], sv[VALUES ? kMergeChunk : 1];
-    __shared__ uint32_t ok[kMergeChunk], ov[VALUES ? kMergeChunk : 1];
+    using K = SortKey<WIDE>;
+    __shared__ K sk[kMergeChunk];
+    __shared__ uint32_t sv[VALUES ? kMergeChunk : 1];
     __shared__ uint32_t s_split[2];
     if constexpr (PDL) {
         pdl_wait();
@@ -223,7 +238,7 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_pass(uint32_t q, uint32
     const uint32_t pa = (uint32_t)(((uint64_t)o0 / (2ull * L)) * 2ull * L);  // start of the run pair
     const uint32_t na = min(L, cnt - pa), nb = cnt - pa > L ? min(L, cnt - pa - L) : 0u;
     const uint32_t d0 = o0 - pa, d1 = o1 - pa;
-    const uint64_t hi = ks[0] & 0xFFFFFFFF00000000ull;
+    const uint64_t hi = WIDE ? 0ull : ks[0] & 0xFFFFFFFF00000000ull;
     if (nb == 0) {  // a lone run: copy
         for (uint32_t x = o0 + threadIdx.x; x < o1; x += kMergeThreads) {
             kd[x] = ks[x];
@@ -233,7 +248,7 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_pass(uint32_t q, uint32
     }
     const uint64_t* A = ks + pa;
     const uint64_t* B = ks + pa + L;
-    if (threadIdx.x < 2) s_split[threadIdx.x] = merge_split(A, na, B, nb, threadIdx.x ? d1 : d0);
+    if (threadIdx.x < 2) s_split[threadIdx.x] = merge_split<K>(A, na, B, nb, threadIdx.x ? d1 : d0);
     __syncthreads();
     const uint32_t i0 = s_split[0], i1 = s_split[1];
     const uint32_t j0 = d0 - i0, j1 = d1 - i1;
@@ -241,30 +256,41 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_pass(uint32_t q, uint32
     for (uint32_t x = threadIdx.x; x < tot; x += kMergeThreads) {
         const bool in_a = x < ca;
         const uint32_t src = in_a ? pa + i0 + x : pa + L + j0 + (x - ca);
-        sk[x] = (uint32_t)ks[src];
+        sk[x] = (K)ks[src];
         if (VALUES) sv[x] = vs[src];
     }
     __syncthreads();
     // each thread merges kMergeItems outputs from its own split of the staged windows
     const uint32_t dd = min((uint32_t)threadIdx.x * kMergeItems, tot);
-    uint32_t ia = merge_split(sk, ca, sk + ca, cb, dd), ib = dd - ia;
-    for (uint32_t m = 0; m < (uint32_t)kMergeItems && dd + m < tot; m++) {
+    uint32_t ia = merge_split<K>(sk, ca, sk + ca, cb, dd), ib = dd - ia;
+    K mk[kMergeItems];
+    uint32_t mv[VALUES ? kMergeItems : 1];
+#pragma unroll
+    for (uint32_t m = 0; m < (uint32_t)kMergeItems; m++) {
+        if (dd + m >= tot) break;
         const bool take_a = ib >= cb || (ia < ca && sk[ia] <= sk[ca + ib]);
         const uint32_t from = take_a ? ia++ : ca + ib++;
-        ok[dd + m] = sk[from];
-        if (VALUES) ov[dd + m] = sv[from];
+        mk[m] = sk[from];
+        if (VALUES) mv[m] = sv[from];
+    }
+    __syncthreads();  // the staged windows have been read: the outputs take their place
+#pragma unroll
+    for (uint32_t m = 0; m < (uint32_t)kMergeItems; m++) {
+        if (dd + m >= tot) break;
+        sk[dd + m] = mk[m];
+        if (VALUES) sv[dd + m] = mv[m];
     }
     __syncthreads();
     for (uint32_t x = threadIdx.x; x < tot; x += kMergeThreads) {
-        kd[o0 + x] = hi | ok[x];
-        if (VALUES) vd[o0 + x] = ov[x];
+        kd[o0 + x] = hi | sk[x];
+        if (VALUES) vd[o0 + x] = sv[x];
     }
 }
 
-static_assert(block_sort_smem<true>() <= 48 * 1024 && block_sort_smem<false>() <= 48 * 1024,
+static_assert(block_sort_smem<true, true>() <= 48 * 1024 && block_sort_smem<false, true>() <= 48 * 1024,
               "the tile sort runs without a shared-memory opt-in");
 
-template <bool VALUES>
+template <bool VALUES, bool WIDE>
 uint32_t enqueue_t(uint32_t nblk, const uint64_t* off, uint64_t tiles, uint64_t chunks, uint32_t passes,
                    uint32_t* tile_pre, uint32_t* chunk_pre, const uint32_t* unsorted, uint64_t* ka, uint32_t* va,
                    uint64_t* kb, uint32_t* vb, uint32_t* maxp, cudaStream_t st, bool plan, bool pdl) {
@@ -277,11 +303,11 @@ uint32_t enqueue_t(uint32_t nblk, const uint64_t* off, uint64_t tiles, uint64_t 
     // (the sort of keys alone opens the side stream's chain, after an event wait: a plain launch)
     (void)launch_chain(pdl && VALUES, k_tile_copy<VALUES, true>, k_tile_copy<VALUES, false>, (unsigned)tiles, kBsThreads, 0, st,
                        nblk, off, tile_pre, unsorted, ka, va, kb, vb);
-    (void)launch_chain(pdl, k_tile_sort<VALUES, true>, k_tile_sort<VALUES, false>, (unsigned)tiles, kBsThreads,
-                       block_sort_smem<VALUES>(), st, nblk, off, tile_pre, unsorted, ka, va, kb, vb, maxp);
+    (void)launch_chain(pdl, k_tile_sort<VALUES, WIDE, true>, k_tile_sort<VALUES, WIDE, false>, (unsigned)tiles,
+                       kBsThreads, block_sort_smem<VALUES, WIDE>(), st, nblk, off, tile_pre, unsorted, ka, va, kb, vb, maxp);
     launches += 2;
     for (uint32_t q = 1; q <= passes && chunks; q++) {
-        (void)launch_chain(pdl, k_merge_pass<VALUES, true>, k_merge_pass<VALUES, false>, (unsigned)chunks,
+        (void)launch_chain(pdl, k_merge_pass<VALUES, WIDE, true>, k_merge_pass<VALUES, WIDE, false>, (unsigned)chunks,
                            kMergeThreads, 0, st, q, nblk, off, chunk_pre, unsorted, ka, va, kb, vb, maxp);
         launches++;
     }
@@ -293,11 +319,13 @@ uint32_t enqueue_t(uint32_t nblk, const uint64_t* off, uint64_t tiles, uint64_t 
 uint32_t block_sort_enqueue(uint32_t nblk, const uint64_t* off, uint64_t tiles, uint64_t chunks, uint32_t passes,
                             uint32_t* tile_pre, uint32_t* chunk_pre, const uint32_t* unsorted, uint64_t* ka,
                             uint32_t* va, uint64_t* kb, uint32_t* vb, uint32_t* maxp, cudaStream_t st, bool plan,
-                            bool pdl) {
-    return va ? enqueue_t<true>(nblk, off, tiles, chunks, passes, tile_pre, chunk_pre, unsorted, ka, va, kb, vb, maxp,
-                                st, plan, pdl)
-              : enqueue_t<false>(nblk, off, tiles, chunks, passes, tile_pre, chunk_pre, unsorted, ka, nullptr, kb,
-                                 nullptr, maxp, st, plan, pdl);
+                            bool pdl, bool wide) {
+    auto run = [&](auto enqueue) {
+        return enqueue(nblk, off, tiles, chunks, passes, tile_pre, chunk_pre, unsorted, ka, va, kb, vb, maxp, st, plan,
+                       pdl);
+    };
+    if (va) return wide ? run(enqueue_t<true, true>) : run(enqueue_t<true, false>);
+    return wide ? run(enqueue_t<false, true>) : run(enqueue_t<false, false>);
 }
 
 }  // namespace rgl

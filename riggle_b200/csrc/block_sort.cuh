@@ -1,6 +1,7 @@
 // Block-local sort of 64-bit keys (and optional 32-bit values), shared by the query pipeline and the
 // batched stats stage.  Every block of the input holds keys with one common high word (the block's
-// segment); each block is sorted by the low word, stably, independently of the others.
+// segment) and is sorted by the low word, or (wide) keys of several segments that no other block shares,
+// and is sorted by the whole key; stably, and independently of the other blocks.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -50,11 +51,12 @@ __host__ __device__ inline uint32_t merge_chunks(uint64_t cnt) {
 // merge_chunks, sort_passes of the largest block).  (ka, va) is the input and scratch, (kb, vb) the
 // output; va and vb null: keys alone.  maxp: one device word of scratch (the most merge passes an
 // out-of-order block needs; passes beyond it return at once), its own for each concurrent sort, zero
-// before the call.  pdl: programmatic dependent launches (see pdl.cuh).
+// before the call.  pdl: programmatic dependent launches (see pdl.cuh).  wide: a block's keys differ in
+// their high words too (rows of several files in one block) and are sorted by the whole key.
 // Returns the number of kernels launched.
 uint32_t block_sort_enqueue(uint32_t nblk, const uint64_t* off, uint64_t tiles, uint64_t chunks, uint32_t passes,
                             uint32_t* tile_pre, uint32_t* chunk_pre, const uint32_t* unsorted, uint64_t* ka,
                             uint32_t* va, uint64_t* kb, uint32_t* vb, uint32_t* maxp, cudaStream_t st, bool plan,
-                            bool pdl = false);
+                            bool pdl = false, bool wide = false);
 
 }  // namespace rgl

@@ -139,7 +139,7 @@ __global__ void k_expand_keys(uint32_t n, const rgl_interval* __restrict__ iv, c
                               int row_from_block, uint32_t nblk, uint32_t rows, uint32_t row_base, uint32_t rb,
                               uint64_t* __restrict__ key, uint32_t* __restrict__ val, uint64_t* __restrict__ ekey,
                               uint32_t* __restrict__ err, uint32_t* __restrict__ unsorted,
-                              const uint64_t* __restrict__ sdst, const uint32_t* __restrict__ sidx) {
+                              const uint64_t* __restrict__ sdst, const uint32_t* __restrict__ sidx, int wide) {
     if constexpr (PDL) {
         pdl_wait();
         pdl_release();
@@ -165,17 +165,25 @@ __global__ void k_expand_keys(uint32_t n, const rgl_interval* __restrict__ iv, c
     // layout) or in place; order flags of the block's rank k in that layout: starts (ends) out of
     // order -> unsorted[k] (unsorted[nblk + k]) = 1
     const uint64_t o = sdst ? sdst[lo] + (i - blk_off[lo]) : (uint64_t)i;
-    if (unsorted && i > blk_off[lo]) {
-        const uint32_t k = sidx ? sidx[lo] : lo;
-        if (w[0] < w[-3]) unsorted[k] = 1u;
-        if (w[1] < w[-2]) unsorted[nblk + k] = 1u;
-    }
     // the row is the interval's sid, or with row_from_block its block's row (sid ignored)
     const uint32_t row = row_from_block ? blk_row[lo] : w[2];
+    if (unsorted && i > blk_off[lo]) {
+        const uint32_t k = sidx ? sidx[lo] : lo;
+        const uint32_t before = wide ? w[-1] : row;  // (wide: rows come from the intervals)
+        if (row < before || (row == before && w[0] < w[-3])) unsorted[k] = 1u;
+        if (row < before || (row == before && w[1] < w[-2])) unsorted[nblk + k] = 1u;
+    }
     uint32_t s = w[0], e = w[1], q = row - row_base;  // rows below row_base wrap to >= rows
     uint32_t bad = 0;
     if (s >= e) bad |= ERR_BAD_INTERVAL;
-    if (q >= rows || (blk_row && row != blk_row[lo])) { bad |= ERR_BAD_ROW; q = 0; }
+    if (q >= rows || (blk_row && row != blk_row[lo])) {
+        bad |= ERR_BAD_ROW;
+        q = 0;
+        if (wide && unsorted) {  // its key goes by row 0 now: out of order
+            const uint32_t k = sidx ? sidx[lo] : lo;
+            unsorted[k] = unsorted[nblk + k] = 1u;
+        }
+    }
     if (bad) atomicOr(err, bad);
     // segment = (shard, region, row): with regions (rb > 0) a row's intervals on a shard are cut
     // into 2^rb-bp regions of their starts, so that the rows' work on one region lies together
@@ -1979,6 +1987,7 @@ int stream_after(cudaStream_t to, cudaStream_t from, cudaEvent_t e) {
 
 // Shape of a run's block-local key sort, from the host's block offsets.
 struct LocalSort {
+    bool wide = false;       // blocks of several rows (one per shard): sorted by the whole key
     uint64_t max_block = 0;  // the largest block: sets the number of merge passes
     uint64_t tiles = 0;      // tiles of kBlockSortCap intervals over all blocks
     uint64_t chunks = 0;     // merge chunks of the blocks of more than one tile
@@ -2011,15 +2020,17 @@ struct PipeIn {
 };
 
 // Whether a run's blocks allow the block-local key sort: with one row, or rows taken from the
-// blocks, every block is one segment, and they must be distinct.  off: nblk + 1 host offsets; row:
-// the blocks' rows (null: row 0 of one row).  *ls receives the shape of the sort.
+// blocks, every block is one segment, and they must be distinct; blocks of several rows hold the
+// segments of one shard, and the shards must be distinct (a wide sort: 37 rows in 24 blocks of sorted
+// files took two device-wide radix sorts, 12 passes of 9 us).  off: nblk + 1 host offsets; row:
+// the blocks' rows (null: from the intervals).  *ls receives the shape of the sort.
 bool blocks_local(uint32_t nblk, const uint64_t* off, const uint32_t* shard, const uint32_t* row, uint32_t rows,
                   uint32_t row_base, LocalSort* ls) {
     *ls = LocalSort();
-    if (!row && rows != 1) return false;
     std::vector<std::pair<uint64_t, uint32_t>> segs;  // (segment, block) of the non-empty blocks
     segs.reserve(nblk);
     LocalSort t;
+    t.wide = !row && rows != 1;
     bool ordered = true;
     for (uint32_t b = 0; b < nblk; b++) {
         const uint64_t cnt = off[b + 1] - off[b];
@@ -2187,7 +2198,7 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
                        in.blk_off, in.blk_shard, in.blk_row, in.row_from_block, in.nblk, rows, in.row_base, rb,
                        c->key_a.as<uint64_t>(), c->val_a.as<uint32_t>(), c->ekey_a.as<uint64_t>(), d_small,
                        in.block_local ? d_unsorted : nullptr, in.block_local ? sort_dst : nullptr,
-                       in.block_local ? sort_idx : nullptr);
+                       in.block_local ? sort_idx : nullptr, (int)(in.block_local && in.ls.wide));
     launches += 2;
     // the sort's view of the blocks: their offsets in the layout the keys were written in
     const uint64_t* soff = sort_dst ? sort_off : in.blk_off;
@@ -2200,10 +2211,11 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     if (in.block_local) {
         launches += block_sort_enqueue(in.nblk, soff, in.ls.tiles, in.ls.chunks, passes, d_tile_pre, d_chunk_pre,
                                        d_unsorted + in.nblk, c->ekey_a.as<uint64_t>(), nullptr,
-                                       c->ekey_b.as<uint64_t>(), nullptr, d_maxp + 1, sd, false, pdl);
+                                       c->ekey_b.as<uint64_t>(), nullptr, d_maxp + 1, sd, false, pdl, in.ls.wide);
         launches += block_sort_enqueue(in.nblk, soff, in.ls.tiles, in.ls.chunks, passes, d_tile_pre, d_chunk_pre,
                                        d_unsorted, c->key_a.as<uint64_t>(), c->val_a.as<uint32_t>(),
-                                       c->key_b.as<uint64_t>(), c->val_b.as<uint32_t>(), d_maxp, st, false, pdl);
+                                       c->key_b.as<uint64_t>(), c->val_b.as<uint32_t>(), d_maxp, st, false, pdl,
+                                       in.ls.wide);
     } else {
         RGL_CUDA(cub::DeviceRadixSort::SortKeys(c->cub_tmp2.p, tb, c->ekey_a.as<uint64_t>(), c->ekey_b.as<uint64_t>(),
                                                 (int)n, 0, 32 + segbits, sd));
@@ -2477,6 +2489,7 @@ struct BatchPlan {
         in.ls.max_block = ls[k].max_block;  // the layout goes by the device tables below
         in.ls.tiles = ls[k].tiles;
         in.ls.chunks = ls[k].chunks;
+        in.ls.wide = ls[k].wide;
         if (local[k] && !ls[k].dst.empty()) {
             in.sort_off = d_off + off.size() + sb.tab_at;
             in.sort_dst = d_off + 2 * off.size() + sb.tab_at;
