@@ -256,6 +256,11 @@ typedef struct rgl_pair {
 int rgl_query_pairs(rgl_context* ctx, const rgl_query_batch* batch, uint64_t capacity, rgl_pair* pairs,
                     uint64_t* out_count);
 
+/* The same with one run of the batch: alloc(user, count) is called once the number of pairs is known (not
+ * for none) and returns where they go, room for `count` of them (NULL: RGL_ERR_OOM). */
+int rgl_query_pairs_alloc(rgl_context* ctx, const rgl_query_batch* batch, rgl_pair* (*alloc)(void* user, uint64_t count),
+                          void* user, uint64_t* out_count);
+
 /* ---- Batched form: many query files in one call -------------------------------------------------
  * Replaces query_database's loop over batches of query files (src/tasks/query/mod.rs:182-307) for a
  * whole set of files at once; the reference has no single entry point for it.  Block b holds

@@ -116,6 +116,7 @@ class TuneTrial(C.Structure):
 
 
 FREE_MEMORY_FN = C.CFUNCTYPE(C.c_uint64, C.c_void_p)
+PAIR_ALLOC_FN = C.CFUNCTYPE(C.c_void_p, C.c_void_p, C.c_uint64)
 
 
 class ServerOpts(C.Structure):
@@ -193,6 +194,7 @@ _SIGS = {
     "rgl_query_counts_device": (C.c_int, [_P, C.c_uint32, C.c_uint32, _P, _P, _P, C.POINTER(QueryOpts), _P, _P,
                                           C.POINTER(QueryStats)]),
     "rgl_query_pairs": (C.c_int, [_P, C.POINTER(QueryBatch), C.c_uint64, _P, C.POINTER(C.c_uint64)]),
+    "rgl_query_pairs_alloc": (C.c_int, [_P, C.POINTER(QueryBatch), PAIR_ALLOC_FN, _P, C.POINTER(C.c_uint64)]),
     "rgl_query_batch_device": (C.c_int, [_P, C.POINTER(BatchDesc), C.POINTER(BatchOpts), _P, _P,
                                          C.POINTER(BatchStats)]),
     "rgl_query_batch_host": (C.c_int, [_P, C.POINTER(BatchDesc), _P, C.POINTER(BatchOpts), _P, _P,

@@ -17,6 +17,12 @@ def _ptr(a):
     return C.c_void_p(a.ctypes.data) if a is not None and a.size else None
 
 
+# rgl_query_shard, as a numpy record (filled faster than the ctypes structure, 24 of them a call)
+_SHARD = np.dtype([("name", np.uint64), ("id", np.uint32), ("pad", np.uint32), ("count", np.uint64),
+                   ("intervals", np.uint64)])
+assert _SHARD.itemsize == C.sizeof(_lib.QueryShard)
+
+
 class LayerConfig:
     """LayerConfig (src/io/meta.rs:23-90)."""
 
@@ -198,16 +204,22 @@ class Context:
 
     @staticmethod
     def _batch(shards, num_rows, keep):
-        arr = (_lib.QueryShard * max(1, len(shards)))()
+        arr = np.zeros(max(1, len(shards)), _SHARD)
         for i, (k, ivs) in enumerate(shards.items()):
-            ivs = np.ascontiguousarray(ivs, dtype=np.uint32).reshape(-1, 3)
+            if not (type(ivs) is np.ndarray and ivs.dtype == np.uint32 and ivs.ndim == 2 and ivs.shape[1] == 3
+                    and ivs.flags.c_contiguous):
+                ivs = np.ascontiguousarray(ivs, dtype=np.uint32).reshape(-1, 3)
             keep.append(ivs)
+            n = len(ivs)
+            name = 0
             if isinstance(k, str):
-                arr[i] = _lib.QueryShard(k.encode(), 0, len(ivs), _ptr(ivs))
-            else:
-                arr[i] = _lib.QueryShard(None, int(k), len(ivs), _ptr(ivs))
+                name = C.c_char_p(k.encode())
+                keep.append(name)
+                name, k = C.cast(name, C.c_void_p).value, 0
+            arr[i] = (name, int(k), 0, n, ivs.__array_interface__["data"][0] if n else 0)
         keep.append(arr)
-        return _lib.QueryBatch(int(num_rows), len(shards), arr)
+        return _lib.QueryBatch(int(num_rows), len(shards),
+                               C.cast(arr.__array_interface__["data"][0], C.POINTER(_lib.QueryShard)))
 
     def query_pairs(self, shards, num_rows):
         """`--intervals` mode: every overlapping pair as uint32[n, 8] records (query_start, query_end,
@@ -215,11 +227,14 @@ class Context:
         keep = []
         batch = self._batch(shards, num_rows, keep)
         n = C.c_uint64()
-        check(load().rgl_query_pairs(self._h, C.byref(batch), 0, None, C.byref(n)))
-        out = np.empty((n.value, 8), np.uint32)
-        if n.value:
-            check(load().rgl_query_pairs(self._h, C.byref(batch), n.value, _ptr(out), C.byref(n)))
-        return out
+        out = [np.empty((0, 8), np.uint32)]
+
+        def place(_, count):  # called once, when the number of pairs is known
+            out[0] = np.empty((count, 8), np.uint32)
+            return out[0].ctypes.data
+
+        check(load().rgl_query_pairs_alloc(self._h, C.byref(batch), _lib.PAIR_ALLOC_FN(place), None, C.byref(n)))
+        return out[0]
 
     def query_batch_device(self, batch, d_counts, d_bp=None, graph=False, tuned=False, sub_batch=0, chunk=0,
                            ctas_per_sm=0, pair_ratio=0, counts_only=False, stats=True, region_bits=0,

@@ -1751,6 +1751,7 @@ struct rgl_context {
     DevBuf item_hits, item_base, pairs;  // intervals mode
     DevBuf bt_off, bt_shard, acc;  // batched form: sub-batch block tables (offsets; shards then rows), stats
     uint32_t* h_small = nullptr;  // pinned mirror of `small`
+    unsigned char* h_io = nullptr;  // pinned staging of the host entry points (kHostIoBytes)
     unsigned long long* h_acc = nullptr;  // pinned mirror of `acc`
     uint64_t ws_sig = 0;          // changes whenever a workspace buffer is reallocated
     // the CUDA graph of the last batch run with RGL_BF_GRAPH, replayed while the batch is unchanged
@@ -1815,7 +1816,7 @@ int size_workspace(rgl_context* c, uint64_t n, uint32_t rows, uint32_t nblk, uin
             return RGL_OK;
         }
     } z{plan};
-    RGL_TRY(z.ensure_in(c->iv, n * sizeof(rgl_interval) + 16));
+    RGL_TRY(z.ensure_in(c->iv, n * sizeof(rgl_interval) + (nblk + 1ull) * 32 + 64));  // and the block tables
     RGL_TRY(z.ensure_in(c->blk_off, (nblk + 1) * 8ull));
     RGL_TRY(z.ensure_in(c->blk_shard, (nblk + 1) * 4ull));
     RGL_TRY(z.ensure_in(c->sortplan, (4ull * nblk + 8) * 4));
@@ -1875,7 +1876,7 @@ int size_workspace(rgl_context* c, uint64_t n, uint32_t rows, uint32_t nblk, uin
     RGL_TRY(z.ensure_in(c->cub_tmp2, need + 256));
     if (rows) {
         RGL_TRY(z.ensure_in(c->out_counts, (uint64_t)rows * idx->num_sources * 4 + 16));
-        RGL_TRY(z.ensure_in(c->out_bp, (uint64_t)rows * idx->num_sources * 8 + 16));
+        RGL_TRY(z.ensure_in(c->out_bp, (uint64_t)rows * idx->num_sources * 12 + 32));  // both, see HostIO
     }
     if (plan) return RGL_OK;
     c->res_n = std::max(c->res_n, n);
@@ -2415,16 +2416,68 @@ int resolve_blocks(rgl_context* c, const rgl_query_batch* b, std::vector<uint32_
     return RGL_OK;
 }
 
-// Copies the blocks' host intervals into the context's interval buffer at offsets off, one copy per
-// run of blocks that lie back to back in host memory (a file read into one buffer).
-int copy_blocks(rgl_context* c, const std::vector<const rgl_query_shard*>& blocks, const std::vector<uint64_t>& off,
-                cudaStream_t st) {
-    for (size_t i = 0; i < blocks.size();) {
-        size_t j = i + 1;
-        while (j < blocks.size() && blocks[j]->intervals == blocks[j - 1]->intervals + blocks[j - 1]->count) j++;
-        RGL_CUDA(cudaMemcpyAsync(c->iv.as<rgl_interval>() + off[i], blocks[i]->intervals,
-                                 (off[j] - off[i]) * sizeof(rgl_interval), cudaMemcpyHostToDevice, st));
-        i = j;
+// Page-locked staging per context, for inputs and outputs of the host entry points.
+constexpr uint64_t kHostIoBytes = 512ull << 10;
+// A copy from pageable memory costs the stream about 4 us whatever its size; staging costs the host
+// about 80 us per MB.  Blocks of less than this on average are staged.
+constexpr uint64_t kStagePerCopy = 48ull << 10;
+
+// The run's input on the device: the blocks' host intervals at offsets off in the context's interval
+// buffer, and after them the block tables (offsets, shards, and the sort's segment-order layout where it
+// has one).  Short blocks are gathered into the staging buffer, tables included, and sent in one copy;
+// longer ones are copied from where they lie, one copy per run of blocks that lie back to back in host
+// memory (a file read into one buffer), and the tables in one.  (24 short blocks and their tables took
+// 26 copies, 100 of the 200 us of a 1,000-interval call.)
+int upload_blocks(rgl_context* c, const std::vector<const rgl_query_shard*>& blocks, const std::vector<uint64_t>& off,
+                  const std::vector<uint32_t>& ids, PipeIn* in, cudaStream_t st) {
+    const size_t nb = blocks.size(), nb1 = nb + 1;
+    if (!nb) return RGL_OK;
+    const bool layout = in->block_local && !in->ls.dst.empty();
+    const uint64_t iv_bytes = off[nb] * sizeof(rgl_interval);
+    const uint64_t at = (iv_bytes + 15) & ~15ull;  // the tables: off, soff, dst (8 bytes each), shards, idx
+    const uint64_t tab_bytes = nb1 * (layout ? 32 : 12);
+    size_t copies = 1;
+    for (size_t i = 1; i < nb; i++)
+        if (blocks[i]->intervals != blocks[i - 1]->intervals + blocks[i - 1]->count) copies++;
+    RGL_TRY(c->iv.ensure(at + tab_bytes));
+    unsigned char* dev = c->iv.as<unsigned char>();
+    const bool stage = at + tab_bytes <= kHostIoBytes && iv_bytes <= copies * kStagePerCopy;
+    std::vector<unsigned char> big;
+    unsigned char* tab = c->h_io + (stage ? at : 0);
+    if (!stage && tab_bytes > kHostIoBytes) {
+        big.resize(tab_bytes);
+        tab = big.data();
+    }
+    std::memcpy(tab, off.data(), nb1 * 8);
+    if (layout) {
+        std::memcpy(tab + nb1 * 8, in->ls.soff.data(), nb1 * 8);
+        std::memcpy(tab + nb1 * 16, in->ls.dst.data(), nb1 * 8);
+        std::memcpy(tab + nb1 * 28, in->ls.idx.data(), nb1 * 4);
+    }
+    std::memcpy(tab + nb1 * (layout ? 24 : 8), ids.data(), nb * 4);
+    if (stage) {
+        for (size_t i = 0; i < nb; i++)
+            std::memcpy(c->h_io + off[i] * sizeof(rgl_interval), blocks[i]->intervals,
+                        blocks[i]->count * sizeof(rgl_interval));
+        RGL_CUDA(cudaMemcpyAsync(dev, c->h_io, at + tab_bytes, cudaMemcpyHostToDevice, st));
+    } else {
+        for (size_t i = 0; i < nb;) {
+            size_t j = i + 1;
+            while (j < nb && blocks[j]->intervals == blocks[j - 1]->intervals + blocks[j - 1]->count) j++;
+            RGL_CUDA(cudaMemcpyAsync(dev + off[i] * sizeof(rgl_interval), blocks[i]->intervals,
+                                     (off[j] - off[i]) * sizeof(rgl_interval), cudaMemcpyHostToDevice, st));
+            i = j;
+        }
+        RGL_CUDA(cudaMemcpyAsync(dev + at, tab, tab_bytes, cudaMemcpyHostToDevice, st));
+        if (!big.empty()) RGL_CUDA(cudaStreamSynchronize(st));
+    }
+    in->iv = reinterpret_cast<const rgl_interval*>(dev);
+    in->blk_off = reinterpret_cast<const uint64_t*>(dev + at);
+    in->blk_shard = reinterpret_cast<const uint32_t*>(dev + at + nb1 * (layout ? 24 : 8));
+    if (layout) {
+        in->sort_off = in->blk_off + nb1;
+        in->sort_dst = in->blk_off + 2 * nb1;
+        in->sort_idx = reinterpret_cast<const uint32_t*>(dev + at + nb1 * 28);
     }
     return RGL_OK;
 }
@@ -2754,8 +2807,13 @@ int rgl_context_create(rgl_index* index, void* stream, rgl_context** out) {
     }
     for (int i = 0; i < 4 && s == RGL_OK; i++)
         if (cudaEventCreate(&c->ev[i]) != cudaSuccess) s = fail(RGL_ERR_DEVICE, "cudaEventCreate");
-    if (s == RGL_OK && cudaMallocHost(&c->h_small, 256) != cudaSuccess) s = fail(RGL_ERR_OOM, "pinned");
-    if (s == RGL_OK && cudaMallocHost(&c->h_acc, 64) != cudaSuccess) s = fail(RGL_ERR_OOM, "pinned");
+    // one page-locked allocation: the counter mirrors (256 bytes each), then the staging buffer
+    if (s == RGL_OK && cudaMallocHost(&c->h_small, 512 + kHostIoBytes) != cudaSuccess) s = fail(RGL_ERR_OOM, "pinned");
+    if (s == RGL_OK) {
+        unsigned char* base = reinterpret_cast<unsigned char*>(c->h_small);
+        c->h_acc = reinterpret_cast<unsigned long long*>(base + 256);
+        c->h_io = base + 512;
+    }
     if (s == RGL_OK) s = c->small.ensure(256);
     if (s != RGL_OK) {
         rgl_context_destroy(c);
@@ -2792,7 +2850,6 @@ int rgl_context_destroy(rgl_context* c) {
         if (e) cudaEventDestroy(e);
     for (auto& e : c->tev) cudaEventDestroy(e);
     if (c->h_small) cudaFreeHost(c->h_small);
-    if (c->h_acc) cudaFreeHost(c->h_acc);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
     if (c->side) cudaStreamDestroy(c->side);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
@@ -2868,21 +2925,30 @@ int rgl_query_counts(rgl_context* c, const rgl_query_batch* b, const rgl_query_o
     const uint64_t cells = (uint64_t)rows * c->idx->num_sources;
     RGL_TRY(ensure_workspace(c, n, rows, (uint32_t)blocks.size()));
     cudaStream_t st = c->stream;
-    RGL_TRY(copy_blocks(c, blocks, off, st));
-    if (!blocks.empty()) {
-        RGL_CUDA(cudaMemcpyAsync(c->blk_off.p, off.data(), off.size() * 8, cudaMemcpyHostToDevice, st));
-        RGL_CUDA(cudaMemcpyAsync(c->blk_shard.p, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, st));
-    }
-    PipeIn in{c->iv.as<rgl_interval>(), n, rows, 0, (uint32_t)blocks.size(), c->blk_off.as<uint64_t>(),
-              c->blk_shard.as<uint32_t>(), nullptr};
+    PipeIn in{nullptr, n, rows, 0, (uint32_t)blocks.size(), nullptr, nullptr, nullptr};
     in.block_local = blocks_local((uint32_t)blocks.size(), off.data(), ids.data(), nullptr, rows, 0, &in.ls);
-    RGL_TRY(run_pipeline(c, in, opts, c->out_counts.as<uint32_t>(),
-                         overlap_bp ? c->out_bp.as<unsigned long long>() : nullptr, stats));
-    if (cells) {
-        RGL_CUDA(cudaMemcpyAsync(counts, c->out_counts.p, cells * 4, cudaMemcpyDeviceToHost, st));
-        if (overlap_bp) RGL_CUDA(cudaMemcpyAsync(overlap_bp, c->out_bp.p, cells * 8, cudaMemcpyDeviceToHost, st));
+    // the outputs lie together on the device (overlaps, then counts), so that one copy brings both
+    unsigned long long* d_bp = c->out_bp.as<unsigned long long>();
+    uint32_t* d_counts = reinterpret_cast<uint32_t*>(d_bp + (overlap_bp ? cells : 0));
+    const uint64_t out_bytes = cells * (overlap_bp ? 12 : 4);
+    int s = upload_blocks(c, blocks, off, ids, &in, st);
+    if (s == RGL_OK) s = run_pipeline(c, in, opts, d_counts, overlap_bp ? d_bp : nullptr, stats);
+    if (s != RGL_OK) {
+        cudaStreamSynchronize(st);  // the staging buffer may be in use
+        return s;
+    }
+    const bool stage = cells && out_bytes <= kHostIoBytes;
+    if (stage) {
+            RGL_CUDA(cudaMemcpyAsync(c->h_io, c->out_bp.p, out_bytes, cudaMemcpyDeviceToHost, st));
+    } else if (cells) {
+        RGL_CUDA(cudaMemcpyAsync(counts, d_counts, cells * 4, cudaMemcpyDeviceToHost, st));
+        if (overlap_bp) RGL_CUDA(cudaMemcpyAsync(overlap_bp, d_bp, cells * 8, cudaMemcpyDeviceToHost, st));
     }
     RGL_CUDA(cudaStreamSynchronize(st));
+    if (stage) {
+        if (overlap_bp) std::memcpy(overlap_bp, c->h_io, cells * 8);
+        std::memcpy(counts, c->h_io + (overlap_bp ? cells * 8 : 0), cells * 4);
+    }
     return finish(c, pick_launch(opts), stats);
 }
 
@@ -3171,8 +3237,12 @@ int rgl_batch_autotune(rgl_context* c, const rgl_batch* b, uint64_t sub_batch, r
     return finish(c, L, nullptr);
 }
 
-int rgl_query_pairs(rgl_context* c, const rgl_query_batch* b, uint64_t capacity, rgl_pair* pairs,
-                    uint64_t* out_count) {
+}  // extern "C"
+
+namespace {
+// The pairs of a batch: place(count, &pairs) says where they go (null: nowhere), once their number is known.
+template <typename Place>
+int query_pairs(rgl_context* c, const rgl_query_batch* b, uint64_t* out_count, Place place) {
     clear_error();
     if (!c || !b || !out_count) return fail(RGL_ERR_INVALID_ARGUMENT, "null argument");
     RGL_CUDA(cudaSetDevice(c->idx->device));
@@ -3189,29 +3259,30 @@ int rgl_query_pairs(rgl_context* c, const rgl_query_batch* b, uint64_t capacity,
     off[blocks.size()] = n;
     RGL_TRY(ensure_workspace(c, n, 0, (uint32_t)blocks.size()));
     cudaStream_t st = c->stream;
-    RGL_TRY(copy_blocks(c, blocks, off, st));
-    if (!blocks.empty()) {
-        RGL_CUDA(cudaMemcpyAsync(c->blk_off.p, off.data(), off.size() * 8, cudaMemcpyHostToDevice, st));
-        RGL_CUDA(cudaMemcpyAsync(c->blk_shard.p, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, st));
-    }
     // every candidate run becomes a pair run: a range is swept pair by pair when its candidates are
     // at most pair_ratio x its union, which no range exceeds at this ratio
     rgl_query_opts q{};
     q.pair_ratio = 0xFFFFFFFFu;
-    PipeIn in{c->iv.as<rgl_interval>(), n, b->num_rows, 0, (uint32_t)blocks.size(), c->blk_off.as<uint64_t>(),
-              c->blk_shard.as<uint32_t>(), nullptr};
+    PipeIn in{nullptr, n, b->num_rows, 0, (uint32_t)blocks.size(), nullptr, nullptr, nullptr};
     in.block_local = blocks_local((uint32_t)blocks.size(), off.data(), ids.data(), nullptr, b->num_rows, 0, &in.ls);
     PipeMode m;
     m.zero_out = false;
     m.no_sweep = true;
-    RGL_TRY(run_pipeline(c, in, &q, nullptr, nullptr, nullptr, m));
+    int s = upload_blocks(c, blocks, off, ids, &in, st);
+    if (s == RGL_OK) s = run_pipeline(c, in, &q, nullptr, nullptr, nullptr, m);
+    if (s == RGL_OK)  // the pair work space total (small[12..13]) with the error word
+        RGL_CUDA(cudaMemcpyAsync(c->h_small, c->small.p, 64, cudaMemcpyDeviceToHost, st));
     RGL_CUDA(cudaStreamSynchronize(st));
+    RGL_TRY(s);
     RGL_TRY(finish(c, pick_launch(&q), nullptr));
     if (!n || !c->idx->num_slots) return RGL_OK;
-    uint64_t positions = 0;  // the pair work space total, small[12..13]
-    RGL_CUDA(cudaMemcpy(&positions, c->small.as<uint32_t>() + 12, 8, cudaMemcpyDeviceToHost));
+    uint64_t positions = 0;
+    std::memcpy(&positions, c->h_small + 12, 8);
     const uint32_t* Lp = c->small.as<uint32_t>() + 8;
-    const uint32_t chunk = 2048;
+    // items for every warp of the grid below where there are that many positions (2,048 each: 133 warps
+    // walked the 272 thousand candidates of 1e5 queries, 118 us a pass)
+    const uint64_t even = (positions / ((uint64_t)c->num_sms * 64) + 31) & ~31ull;
+    const uint32_t chunk = (uint32_t)std::min<uint64_t>(2048, std::max<uint64_t>(64, even));
     const uint64_t items = (positions + chunk - 1) / chunk;
     if (!items) return RGL_OK;
     RGL_TRY(c->item_hits.ensure((items + 1) * 8));
@@ -3222,8 +3293,8 @@ int rgl_query_pairs(rgl_context* c, const rgl_query_batch* b, uint64_t capacity,
     const unsigned grid = (unsigned)std::min<uint64_t>((items * 32 + 255) / 256, (uint64_t)c->num_sms * 16);
     RGL_CUDA(cudaMemsetAsync(c->item_hits.as<uint64_t>() + items, 0, 8, st));
     k_pair_list<false><<<grid, 256, 0, st>>>(c->ppos.as<uint64_t>(), Lp, c->psegs.as<PairSeg>(),
-                                             c->prow.as<uint32_t>(), b->num_rows, c->idx->d_pos, c->idx->d_sid, items, chunk, c->item_hits.as<uint64_t>(), nullptr,
-                                             nullptr);
+                                             c->prow.as<uint32_t>(), b->num_rows, c->idx->d_pos, c->idx->d_sid, items,
+                                             chunk, c->item_hits.as<uint64_t>(), nullptr, nullptr);
     tb = c->cub_tmp.cap;
     RGL_CUDA(cub::DeviceScan::ExclusiveSum(c->cub_tmp.p, tb, c->item_hits.as<uint64_t>(), c->item_base.as<uint64_t>(),
                                            (int)(items + 1), st));
@@ -3231,8 +3302,10 @@ int rgl_query_pairs(rgl_context* c, const rgl_query_batch* b, uint64_t capacity,
     RGL_CUDA(cudaMemcpyAsync(&hits, c->item_base.as<uint64_t>() + items, 8, cudaMemcpyDeviceToHost, st));
     RGL_CUDA(cudaStreamSynchronize(st));
     *out_count = hits;
-    if (!pairs || !hits) return RGL_OK;
-    if (capacity < hits) return fail(RGL_ERR_INVALID_ARGUMENT, "pair capacity too small (needs " + std::to_string(hits) + ")");
+    if (!hits) return RGL_OK;
+    rgl_pair* pairs = nullptr;
+    RGL_TRY(place(hits, &pairs));
+    if (!pairs) return RGL_OK;
     RGL_TRY(c->pairs.ensure(hits * sizeof(rgl_pair)));
     k_pair_list<true><<<grid, 256, 0, st>>>(c->ppos.as<uint64_t>(), Lp, c->psegs.as<PairSeg>(),
                                             c->prow.as<uint32_t>(), b->num_rows, c->idx->d_pos, c->idx->d_sid, items, chunk, nullptr, c->item_base.as<uint64_t>(),
@@ -3241,6 +3314,31 @@ int rgl_query_pairs(rgl_context* c, const rgl_query_batch* b, uint64_t capacity,
     RGL_CUDA(cudaMemcpyAsync(pairs, c->pairs.p, hits * sizeof(rgl_pair), cudaMemcpyDeviceToHost, st));
     RGL_CUDA(cudaStreamSynchronize(st));
     return RGL_OK;
+}
+}  // namespace
+
+extern "C" {
+
+int rgl_query_pairs(rgl_context* c, const rgl_query_batch* b, uint64_t capacity, rgl_pair* pairs,
+                    uint64_t* out_count) {
+    return query_pairs(c, b, out_count, [&](uint64_t hits, rgl_pair** to) {
+        if (pairs && capacity < hits)
+            return fail(RGL_ERR_INVALID_ARGUMENT, "pair capacity too small (needs " + std::to_string(hits) + ")");
+        *to = pairs;
+        return (int)RGL_OK;
+    });
+}
+
+int rgl_query_pairs_alloc(rgl_context* c, const rgl_query_batch* b, rgl_pair* (*alloc)(void*, uint64_t), void* user,
+                          uint64_t* out_count) {
+    if (!alloc) {
+        clear_error();
+        return fail(RGL_ERR_INVALID_ARGUMENT, "null argument");
+    }
+    return query_pairs(c, b, out_count, [&](uint64_t hits, rgl_pair** to) {
+        *to = alloc(user, hits);
+        return *to ? (int)RGL_OK : fail(RGL_ERR_OOM, "no room for " + std::to_string(hits) + " pairs");
+    });
 }
 
 int rgl_context_check(rgl_context* c) {
