@@ -83,7 +83,7 @@ struct DevBuf {
 
 // Scratch of the batched stats stage (query length groups of a batch); one per concurrent caller.
 struct StatsScratch {
-    DevBuf key_a, key_b, len_a, len_b, ukey, agg, runs, groups, goff, tmp;
+    DevBuf key_a, key_b, len_a, len_b, ukey, agg, runs, groups, goff, rcoff, part, tmp;
     DevBuf plan;  // block-local form: the sort's plan and order flags, run-head counts per tile
 };
 
@@ -176,6 +176,9 @@ int batch_pvalues_enqueue(rgl_context* ctx, rgl_moments* m, StatsScratch* sc, co
 // Builds the moment store's shared device tables once (thread-safe).
 int moments_prepare(rgl_moments* m);
 void stats_scratch_release(StatsScratch* sc);
+// Device bytes of StatsScratch::part for rows x D cells over C chromosomes.
+uint64_t pv_scratch_bytes(uint32_t rows, uint32_t D, uint32_t C);
+uint32_t moments_chroms(const rgl_moments* m);
 uint32_t context_last_launches(rgl_context* c);
 
 }  // namespace rgl

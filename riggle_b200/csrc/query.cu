@@ -144,21 +144,12 @@ __global__ void k_expand_keys(uint32_t n, const rgl_interval* __restrict__ iv, c
         pdl_wait();
         pdl_release();
     }
-    // block b with blk_off[b] <= i < blk_off[b+1]: one search per thread block, for its first
-    // element, then a short walk (256 consecutive elements span few blocks)
-    __shared__ uint32_t s_b0;
-    const uint32_t i0 = blockIdx.x * blockDim.x, i = i0 + threadIdx.x;
-    if (threadIdx.x == 0) {
-        uint32_t lo = 0, hi = nblk;
-        while (hi - lo > 1) {
-            const uint32_t m = (lo + hi) >> 1;
-            if (blk_off[m] <= i0) lo = m; else hi = m;
-        }
-        s_b0 = lo;
-    }
-    __syncthreads();
+    // block b with blk_off[b] <= i < blk_off[b+1]: one search per warp, for its first element, then a short
+    // walk (32 consecutive elements span few blocks)
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, w0 = i & ~31u;
+    const uint32_t b0 = w0 < n ? find_block(blk_off, nblk, w0) : 0u;
     if (i >= n) return;
-    uint32_t lo = s_b0;
+    uint32_t lo = b0;
     while (lo + 1 < nblk && blk_off[lo + 1] <= i) lo++;
     const uint32_t* w = reinterpret_cast<const uint32_t*>(iv) + 3ull * i;
     // the block-local sort: block b's keys at sdst[b] + their place in the block (segment-order

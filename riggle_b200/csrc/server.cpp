@@ -81,6 +81,7 @@ struct rgl_server {
     double worker_bytes = 0;
     uint64_t promised = 0;  // device bytes admitted batches will still allocate
     bool with_stats = false;
+    uint32_t chroms = 0;  // of the moment store
     std::vector<uint32_t> shard_chrom;
     // stats
     uint64_t memory_limited = 0, refused = 0, grown_bytes = 0;
@@ -199,8 +200,10 @@ int batch_growth(rgl_server* S, Worker* W, uint64_t n, uint32_t R, uint32_t nblk
         // the stats stage's scratch: keys, lengths, runs and groups per interval (StatsScratch)
         b += grow(W->sc.key_a, n * 8 + 8) + grow(W->sc.key_b, n * 8 + 8) + grow(W->sc.len_a, n * 4 + 4) +
              grow(W->sc.len_b, n * 4 + 4) + grow(W->sc.ukey, n * 8 + 8) + grow(W->sc.agg, n * 32 + 32) +
-             grow(W->sc.groups, n * 40 + 40) + grow(W->sc.plan, stats_plan_bytes(n, nblk)) +
-             grow(W->sc.goff, stats_goff_bytes(S, R, nblk)) + grow(W->sc.runs, 64);
+             grow(W->sc.groups, n * 48 + 48) + grow(W->sc.plan, stats_plan_bytes(n, nblk)) +
+             grow(W->sc.goff, stats_goff_bytes(S, R, nblk)) + grow(W->sc.runs, 64) +
+             grow(W->sc.rcoff, ((uint64_t)R * S->chroms + 1) * 4) +
+             grow(W->sc.part, pv_scratch_bytes(R, S->D, S->chroms));
     }
     *bytes = b;
     return RGL_OK;
@@ -224,10 +227,12 @@ int size_worker(rgl_server* S, Worker* W, uint64_t n, uint32_t R, uint32_t nblk)
         RGL_TRY(W->sc.len_b.ensure(nn * 4 + 4));
         RGL_TRY(W->sc.ukey.ensure(nn * 8 + 8));
         RGL_TRY(W->sc.agg.ensure(nn * 32 + 32));
-        RGL_TRY(W->sc.groups.ensure(nn * 40 + 40));
+        RGL_TRY(W->sc.groups.ensure(nn * 48 + 48));
         RGL_TRY(W->sc.plan.ensure(stats_plan_bytes(nn, nblk)));
         RGL_TRY(W->sc.goff.ensure(stats_goff_bytes(S, R, nblk)));
         RGL_TRY(W->sc.runs.ensure(64));
+        RGL_TRY(W->sc.rcoff.ensure(((uint64_t)R * S->chroms + 1) * 4));
+        RGL_TRY(W->sc.part.ensure(pv_scratch_bytes(R, S->D, S->chroms)));
     }
     return RGL_OK;
 }
@@ -431,6 +436,7 @@ int rgl_server_create(rgl_index* index, const rgl_server_opts* opts, rgl_server*
         if (!S->with_bp) return fail(RGL_ERR_INVALID_ARGUMENT, "the stats stage needs the overlap (no RGL_QF_NO_OVERLAP)");
         if (S->o.num_shard_chrom && !S->o.shard_chrom) return fail(RGL_ERR_INVALID_ARGUMENT, "null shard_chrom");
         S->with_stats = true;
+        S->chroms = moments_chroms(S->o.moments);
         S->shard_chrom.assign(S->o.shard_chrom, S->o.shard_chrom + S->o.num_shard_chrom);
         RGL_TRY(moments_prepare(S->o.moments));
     }

@@ -7,10 +7,10 @@
 // [source][chromosome][slot]; slot = compact_index(L) and the tables hold the reference's L grid in
 // store order, so a lookup is one gather.  Query groups are flattened per query row: every group
 // carries its chromosome, its slot (computed on the host with the same f64 ln as the reference,
-// never on the device) and its FP64 sums.  One warp evaluates one (query row, source) pair:
-// lanes stride over the row's groups, accumulate mu, sigma^2 and mu_raw in FP64, reduce, and lane
-// 0 dispatches NB / Poisson, evaluates the LLR and the A&S 7.1.26 tail exactly as the reference
-// writes it (src/fourier/stats.rs:65-126).
+// never on the device) and its FP64 sums.  mu, sigma^2 and mu_raw of a (query row, source) cell are
+// accumulated in FP64 over the row's groups, and one thread per cell dispatches NB / Poisson,
+// evaluates the LLR and the A&S 7.1.26 tail exactly as the reference writes it
+// (src/fourier/stats.rs:65-126).
 #include <cub/cub.cuh>
 #include <thrust/iterator/transform_iterator.h>
 
@@ -54,9 +54,10 @@ std::vector<uint64_t> moment_grid(uint64_t n) {
     return ls;
 }
 
-struct QGroupDev {
+struct __align__(16) QGroupDev {
+    double ss, ss2, cr;  // cr = count / l_int
     uint32_t chrom, slot;
-    double ss, ss2, l_int, count;
+    double l_int, count;
 };
 
 __device__ __forceinline__ double erfc_as(double x) {
@@ -75,88 +76,254 @@ __device__ __forceinline__ double ln_half_erfc_as(double x) {
     return log(0.5 * p) + (-x * x);
 }
 
-__global__ void k_pvalues(uint32_t rows, uint32_t D, uint32_t C, const uint32_t* __restrict__ counts,
-                          const unsigned long long* __restrict__ bp, double bin_size,
-                          const uint64_t* __restrict__ g_off, const QGroupDev* __restrict__ groups,
-                          const float2* __restrict__ mv, const uint64_t* __restrict__ chrom_off, uint64_t stride,
-                          const uint32_t* __restrict__ tab_len, double* __restrict__ p_out,
-                          double* __restrict__ llr_out, double* __restrict__ logp_out, uint8_t* __restrict__ flags) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; w < (uint64_t)rows * D; w += nw) {
-        const uint32_t q = (uint32_t)(w / D), d = (uint32_t)(w % D);
-        const uint32_t cnt = counts[w];
-        double p = 1.0, llr = 0.0, lp = 0.0;
-        uint8_t f = 0;
-        if (cnt) {  // zero-count pairs are not emitted (src/tasks/query/pvalues.rs:28-35)
-            double mu = 0.0, var = 0.0, raw = 0.0;
-            uint32_t any = 0;
-            const float2* src = mv + (uint64_t)d * stride;
-            for (uint64_t g = g_off[q] + lane; g < g_off[q + 1]; g += 32) {
-                const QGroupDev G = groups[g];
-                if (G.slot < tab_len[(uint64_t)d * C + G.chrom]) {
-                    const float2 m = src[chrom_off[G.chrom] + G.slot];
-                    const double mean = (double)m.x, v = (double)m.y;
-                    mu += mean * G.ss;
-                    var += v * G.ss2;
-                    raw += mean / G.l_int * G.count;
-                    any = 1;
-                }
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                mu += __shfl_xor_sync(0xffffffffu, mu, o);
-                var += __shfl_xor_sync(0xffffffffu, var, o);
-                raw += __shfl_xor_sync(0xffffffffu, raw, o);
-                any |= __shfl_xor_sync(0xffffffffu, any, o);
-            }
-            if (any) {
-                f = 1;
-                const double observed = (double)bp[w] / bin_size;
-                bool ok = false;
-                if (var > mu) {
-                    // nb_llr (src/fourier/stats.rs:101-113)
-                    if (mu > 0.0 && var > mu) {
-                        const double r = mu * mu / (var - mu);
-                        const double pp = mu / var;
-                        const double p_o = r / (r + observed);
-                        if (0.0 < pp && pp < 1.0 && 0.0 < p_o && p_o < 1.0) {
-                            const double theta = log((1.0 - p_o) / (1.0 - pp));
-                            llr = observed * theta + r * log(p_o / pp);
-                            ok = true;
-                        }
-                    }
-                } else {
-                    // Poisson on count units (src/fourier/stats.rs:65-74, 93-98)
-                    const double eff = raw > 0.0 ? mu / raw : 1.0;
-                    const double oc = observed / eff;
-                    if (raw > 0.0 && oc > 0.0) {
-                        llr = oc * log(oc / raw) - (oc - raw);
-                        ok = true;
-                    }
-                }
-                if (ok) f |= 2;
-                if (ok && llr > 0.0) {
-                    const double x = sqrt(llr);
-                    const double tail = erfc_as(x) * 0.5;
-                    const double ln_tail = ln_half_erfc_as(x);
-                    if (observed >= mu) {
-                        p = tail;
-                        lp = ln_tail;
-                    } else {
-                        p = 1.0 - tail;
-                        lp = log1p(-exp(ln_tail));
-                    }
-                }
-                if (!ok) llr = 0.0;
+// The NB / Poisson likelihood ratio and its tail for one cell with groups.
+__device__ __forceinline__ void pvalue_of(double mu, double var, double raw, double observed, double& p, double& llr,
+                                          double& lp, uint8_t& f) {
+    f = 1;
+    bool ok = false;
+    if (var > mu) {
+        // nb_llr (src/fourier/stats.rs:101-113)
+        if (mu > 0.0 && var > mu) {
+            const double r = mu * mu / (var - mu);
+            const double pp = mu / var;
+            const double p_o = r / (r + observed);
+            if (0.0 < pp && pp < 1.0 && 0.0 < p_o && p_o < 1.0) {
+                const double theta = log((1.0 - p_o) / (1.0 - pp));
+                llr = observed * theta + r * log(p_o / pp);
+                ok = true;
             }
         }
-        if (lane == 0) {
-            p_out[w] = p;
-            llr_out[w] = llr;
-            if (logp_out) logp_out[w] = lp;
-            flags[w] = f;
+    } else {
+        // Poisson on count units (src/fourier/stats.rs:65-74, 93-98)
+        const double eff = raw > 0.0 ? mu / raw : 1.0;
+        const double oc = observed / eff;
+        if (raw > 0.0 && oc > 0.0) {
+            llr = oc * log(oc / raw) - (oc - raw);
+            ok = true;
         }
     }
+    if (ok) f |= 2;
+    if (ok && llr > 0.0) {
+        const double x = sqrt(llr);
+        const double tail = erfc_as(x) * 0.5;
+        const double ln_tail = ln_half_erfc_as(x);
+        if (observed >= mu) {
+            p = tail;
+            lp = ln_tail;
+        } else {
+            p = 1.0 - tail;
+            lp = log1p(-exp(ln_tail));
+        }
+    }
+    if (!ok) llr = 0.0;
+}
+
+__device__ __forceinline__ void pvalue_cell(uint32_t count, uint32_t any, double mu, double var, double raw,
+                                            unsigned long long bp, double bin_size, uint64_t w,
+                                            double* __restrict__ p_out, double* __restrict__ llr_out,
+                                            double* __restrict__ logp_out, uint8_t* __restrict__ flags) {
+    double p = 1.0, llr = 0.0, lp = 0.0;
+    uint8_t f = 0;
+    // zero-count pairs are not emitted (src/tasks/query/pvalues.rs:28-35)
+    if (count && any) pvalue_of(mu, var, raw, (double)bp / bin_size, p, llr, lp, f);
+    p_out[w] = p;
+    llr_out[w] = llr;
+    if (logp_out) logp_out[w] = lp;
+    flags[w] = f;
+}
+
+// The sums over the groups.  A block takes 16 sources, WARPS x ROWS query rows (a warp takes ROWS of them
+// one after the other) and all chromosomes or (parts = C) one.  Per chromosome the sources' table entries
+// are staged in shared memory, slot by slot with the sources side by side (zero past a table's end); each
+// half-warp walks every second group of a row on that chromosome, a group read once for its 16 lanes, each
+// with its own source's entry and its own three sums, so that nothing is reduced over lanes but the two
+// halves.  Bound by the conversion of the entries to FP64 and the group reads from L1.  A warp per cell,
+// lanes over the groups, read 8 bytes of table per group and cell from L2 and divided there: 372 us for 128
+// files x 500 sources (8e7 group evaluations); this and k_pv_cells take 223.
+// A cell's sums do not depend on the rows around it: the order (chromosomes; within one, the chunks of
+// kPvSlots slots and the two halves) is the same for every shape of the launch, so that a request alone and
+// in a batch gets the same bits.
+constexpr int kPvSources = 16, kPvSlots = 256, kPvPitch = kPvSources + 1;
+struct PvCell {
+    double mu, var, raw;
+};
+template <int ROWS, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) k_pvalues(
+    uint32_t rows, uint32_t D, uint32_t C, uint32_t parts, const uint32_t* __restrict__ counts,
+    const unsigned long long* __restrict__ bp, double bin_size, const uint32_t* __restrict__ rc_off,
+    const QGroupDev* __restrict__ groups, const float2* __restrict__ mv, const uint64_t* __restrict__ chrom_off,
+    uint64_t stride, const uint32_t* __restrict__ tab_len, double* __restrict__ p_out, double* __restrict__ llr_out,
+    double* __restrict__ logp_out, uint8_t* __restrict__ flags, PvCell* __restrict__ part,
+    uint8_t* __restrict__ part_any) {
+    __shared__ float2 tab[kPvSlots * kPvPitch];
+    __shared__ uint32_t s_slots;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, src = lane & 15u, half = lane >> 4;
+    constexpr uint32_t per_tile = ROWS * WARPS;  // rows of a block
+    const uint32_t row_tiles = (rows + per_tile - 1) / per_tile;
+    const uint32_t pt = blockIdx.x % parts, rest = blockIdx.x / parts;
+    const uint32_t q0 = (rest % row_tiles) * per_tile, d0 = (rest / row_tiles) * kPvSources;
+    const uint32_t d = d0 + src;
+    PvCell acc[ROWS];
+    uint32_t any = 0;  // bit r: row r has a group in source d's tables
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) acc[r] = PvCell{0.0, 0.0, 0.0};
+    for (uint32_t c = parts > 1 ? pt : 0u; c < (parts > 1 ? pt + 1 : C); c++) {
+        const uint32_t n_slots = (uint32_t)((c + 1 < C ? chrom_off[c + 1] : stride) - chrom_off[c]);
+        // the slots that any row of the tile needs (a row's groups ascend by slot)
+        if (threadIdx.x == 0) s_slots = 0;
+        __syncthreads();
+        for (uint32_t r = threadIdx.x; r < per_tile && q0 + r < rows; r += WARPS * 32) {
+            const uint64_t rc = (uint64_t)(q0 + r) * C + c;
+            const uint32_t a = rc_off[rc], b = rc_off[rc + 1];
+            if (b > a && n_slots) atomicMax(&s_slots, min(groups[b - 1].slot, n_slots - 1) + 1);
+        }
+        __syncthreads();
+        const uint32_t slots = s_slots;
+        uint32_t at[ROWS], end[ROWS];
+        PvCell sum[ROWS];  // of this chromosome, this half
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) {
+            const uint32_t q = q0 + warp * ROWS + r;
+            const uint64_t rc = (uint64_t)q * C + c;
+            at[r] = q < rows ? rc_off[rc] + half : 0u;
+            end[r] = q < rows ? rc_off[rc + 1] : 0u;
+            sum[r] = PvCell{0.0, 0.0, 0.0};
+        }
+        const uint32_t len = d < D ? tab_len[(uint64_t)d * C + c] : 0u;
+        for (uint32_t s0 = 0; s0 < slots; s0 += kPvSlots) {
+            const uint32_t m = min((uint32_t)kPvSlots, slots - s0);
+            for (uint32_t w = warp; w < kPvSources; w += WARPS) {  // a warp stages source d0 + w
+                const uint32_t dw = d0 + w;
+                const uint32_t lw = dw < D ? tab_len[(uint64_t)dw * C + c] : 0u;
+                const float2* t = mv + (uint64_t)dw * stride + chrom_off[c] + s0;
+                for (uint32_t k = lane; k < m; k += 32)
+                    tab[k * kPvPitch + w] = s0 + k < lw ? __ldg(t + k) : make_float2(0.f, 0.f);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < ROWS; r++) {
+                constexpr int U = ROWS == 1 ? 4 : 2;  // groups in flight
+                double mu = 0.0, var = 0.0, raw = 0.0;
+                uint32_t hit = 0;
+                for (bool go = true; go;) {
+                    double2 a[U];
+                    uint4 b[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const uint32_t g = at[r] + 2 * u;
+                        b[u].w = 0xFFFFFFFFu;
+                        if (g < end[r]) {
+                            const QGroupDev* G = groups + g;
+                            a[u] = __ldg(reinterpret_cast<const double2*>(G));      // ss, ss2
+                            b[u] = __ldg(reinterpret_cast<const uint4*>(G) + 1);  // cr, chrom, slot
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        go = go && b[u].w - s0 < m;  // (slot >= s0: the groups ascend)
+                        if (!go) break;
+                        const float2 v = tab[(b[u].w - s0) * kPvPitch + src];
+                        const double mean = (double)v.x;
+                        mu += mean * a[u].x;
+                        var += (double)v.y * a[u].y;
+                        raw += mean * __hiloint2double((int)b[u].y, (int)b[u].x);
+                        hit |= b[u].w < len ? 1u : 0u;
+                        at[r] += 2;
+                    }
+                }
+                sum[r].mu += mu;
+                sum[r].var += var;
+                sum[r].raw += raw;
+                any |= hit << r;
+            }
+            __syncthreads();  // the entries may be replaced
+        }
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) {  // the halves together, then onto the chromosomes before
+            acc[r].mu += sum[r].mu + __shfl_xor_sync(0xffffffffu, sum[r].mu, 16);
+            acc[r].var += sum[r].var + __shfl_xor_sync(0xffffffffu, sum[r].var, 16);
+            acc[r].raw += sum[r].raw + __shfl_xor_sync(0xffffffffu, sum[r].raw, 16);
+        }
+    }
+    any |= __shfl_xor_sync(0xffffffffu, any, 16);
+    if (half || d >= D) return;
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+        const uint32_t q = q0 + warp * ROWS + r;
+        if (q >= rows) break;
+        const uint64_t w = (uint64_t)q * D + d;
+        if (parts > 1) {
+            const uint64_t x = (uint64_t)pt * rows * D + w;
+            part[x] = acc[r];
+            part_any[x] = any >> r & 1u;
+            continue;
+        }
+        pvalue_cell(counts[w], any >> r & 1u, acc[r].mu, acc[r].var, acc[r].raw, bp[w], bin_size, w, p_out, llr_out,
+                    logp_out, flags);
+    }
+}
+
+// One cell per thread: the parts of the chromosomes added up in order, then the p-value.
+__global__ void __launch_bounds__(128) k_pv_cells(uint64_t cells, uint32_t parts, const PvCell* __restrict__ part,
+                                                  const uint8_t* __restrict__ part_any,
+                                                  const uint32_t* __restrict__ counts,
+                                                  const unsigned long long* __restrict__ bp, double bin_size,
+                                                  double* __restrict__ p_out, double* __restrict__ llr_out,
+                                                  double* __restrict__ logp_out, uint8_t* __restrict__ flags) {
+    const uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (w >= cells) return;
+    PvCell s{0.0, 0.0, 0.0};
+    uint32_t any = 0;
+    for (uint32_t k = 0; k < parts; k++) {
+        const PvCell v = part[k * cells + w];
+        s.mu += v.mu;
+        s.var += v.var;
+        s.raw += v.raw;
+        any |= part_any[k * cells + w];
+    }
+    pvalue_cell(counts[w], any, s.mu, s.var, s.raw, bp[w], bin_size, w, p_out, llr_out, logp_out, flags);
+}
+
+// Shape of a launch: 32 rows a block (two a warp), or four where there are fewer than 16; a block per
+// chromosome where that leaves fewer than four for each of 148 SMs.
+struct PvShape {
+    bool many;
+    uint32_t parts;
+    uint64_t blocks;
+};
+PvShape pv_shape(uint32_t rows, uint32_t D, uint32_t C) {
+    PvShape s{rows >= 16, 1, 0};
+    const uint32_t per_tile = s.many ? 32 : 4;
+    const uint64_t tiles = (uint64_t)((rows + per_tile - 1) / per_tile) * ((D + kPvSources - 1) / kPvSources);
+    if (tiles < 148 * 4) s.parts = C;
+    s.blocks = tiles * s.parts;
+    return s;
+}
+uint64_t pv_scratch_bytes(uint32_t rows, uint32_t D, uint32_t C) {
+    const PvShape s = pv_shape(rows, D, C);
+    return s.parts > 1 ? s.parts * (uint64_t)rows * D * (sizeof(PvCell) + 1) + 64 : 0;
+}
+// scratch: pv_scratch_bytes of device memory.
+int launch_pvalues(uint32_t rows, uint32_t D, uint32_t C, const uint32_t* counts, const unsigned long long* bp,
+                   double bin_size, const uint32_t* rc_off, const QGroupDev* groups, const float2* mv,
+                   const uint64_t* chrom_off, uint64_t stride, const uint32_t* tab_len, double* p, double* llr,
+                   double* logp, uint8_t* flags, void* scratch, cudaStream_t st) {
+    const PvShape s = pv_shape(rows, D, C);
+    const uint64_t cells = (uint64_t)rows * D;
+    if (s.blocks >= (1ull << 31)) return fail(RGL_ERR_INVALID_ARGUMENT, "too many cells for one call");
+    PvCell* part = static_cast<PvCell*>(scratch);
+    uint8_t* any = reinterpret_cast<uint8_t*>(part + (s.parts > 1 ? s.parts * cells : 0));
+    auto run = [&](auto kernel, int threads) {
+        kernel<<<(unsigned)s.blocks, threads, 0, st>>>(rows, D, C, s.parts, counts, bp, bin_size, rc_off, groups, mv,
+                                                      chrom_off, stride, tab_len, p, llr, logp, flags, part, any);
+    };
+    if (s.many) run(k_pvalues<2, 16>, 512);
+    else run(k_pvalues<1, 4>, 128);
+    if (s.parts > 1)
+        k_pv_cells<<<(unsigned)((cells + 127) / 128), 128, 0, st>>>(cells, s.parts, part, any, counts, bp, bin_size, p,
+                                                                   llr, logp, flags);
+    RGL_CUDA(cudaGetLastError());
+    return RGL_OK;
 }
 
 // ---- query length groups of a whole device-resident batch ------------------------------------
@@ -189,28 +356,20 @@ struct LenToAgg {
 constexpr uint64_t kNoGroup = ~0ull;
 constexpr uint32_t kNoLen = 0xFFFFFFFFu;  // block-local keys: the low word of an interval in no group
 // the request server sizes each worker's StatsScratch with these record sizes
-static_assert(sizeof(LenAgg) == 32 && sizeof(QGroupDev) == 40, "stats scratch record sizes changed");
+static_assert(sizeof(LenAgg) == 32 && sizeof(QGroupDev) == 48, "stats scratch record sizes changed");
 
 __global__ void k_group_keys(uint64_t n, const rgl_interval* __restrict__ iv, const uint64_t* __restrict__ blk_off,
                              const uint32_t* __restrict__ blk_shard, const uint32_t* __restrict__ blk_row, uint32_t nblk,
                              const uint32_t* __restrict__ shard_chrom, uint32_t nshards, uint32_t C,
                              const uint64_t* __restrict__ n_bins, double bin, int local, uint64_t* __restrict__ key,
                              uint32_t* __restrict__ len_out) {
-    // last block with blk_off[b] <= j: one search per thread block, for its first element, then a
-    // short walk (256 consecutive intervals span few blocks)
-    __shared__ uint32_t s_b0;
+    // last block with blk_off[b] <= j: one search per warp, for its first element, then a short walk (32
+    // consecutive intervals span few blocks)
     const uint64_t j0 = blockIdx.x * (uint64_t)blockDim.x, j = j0 + threadIdx.x;
-    if (threadIdx.x == 0) {
-        uint32_t lo = 0, hi = nblk;
-        while (hi - lo > 1) {
-            const uint32_t m = (lo + hi) >> 1;
-            if (blk_off[m] <= j0) lo = m; else hi = m;
-        }
-        s_b0 = lo;
-    }
-    __syncthreads();
+    const uint64_t w0 = j0 + (threadIdx.x & ~31u);
+    const uint32_t b0 = w0 < n ? find_block(blk_off, nblk, w0) : 0u;
     if (j >= n) return;
-    uint32_t lo = s_b0;
+    uint32_t lo = b0;
     while (lo + 1 < nblk && blk_off[lo + 1] <= j) lo++;
     const rgl_interval v = iv[j];
     const uint32_t sh = blk_shard[lo];
@@ -240,15 +399,6 @@ __global__ void k_group_keys(uint64_t n, const rgl_interval* __restrict__ iv, co
 // the device-wide form.
 constexpr int kRunThreads = 256;
 
-__device__ inline uint32_t tile_block(const uint32_t* __restrict__ pre, uint32_t nblk, uint32_t x) {
-    uint32_t lo = 0, hi = nblk;  // pre[lo] <= x < pre[lo + 1]
-    while (hi - lo > 1) {
-        const uint32_t m = (lo + hi) >> 1;
-        if (__ldg(pre + m) <= x) lo = m; else hi = m;
-    }
-    return lo;
-}
-
 // Whether sorted element g (block [bbeg, bend)) starts a run / ends a run of a usable key.
 __device__ inline bool run_head(const uint64_t* __restrict__ key, uint64_t bbeg, uint64_t g) {
     const uint64_t k = key[g];
@@ -266,7 +416,7 @@ __global__ void __launch_bounds__(kRunThreads) k_run_count(uint32_t nblk, const 
                                                            uint32_t* __restrict__ tile_heads) {
     const uint32_t t = blockIdx.x;
     if (t >= __ldg(tile_pre + nblk)) return;
-    const uint32_t b = tile_block(tile_pre, nblk, t);
+    const uint32_t b = find_block(tile_pre, nblk, t);
     const uint64_t bbeg = blk_off[b], bend = blk_off[b + 1];
     const uint64_t base = bbeg + (uint64_t)(t - tile_pre[b]) * kBlockSortCap;
     const uint32_t cnt = (uint32_t)min((uint64_t)kBlockSortCap, bend - base);
@@ -313,7 +463,7 @@ __global__ void __launch_bounds__(kRunThreads) k_run_emit(uint32_t nblk, const u
     __shared__ typename Scan::TempStorage tmp;
     const uint32_t t = blockIdx.x;
     if (t >= __ldg(tile_pre + nblk)) return;
-    const uint32_t b = tile_block(tile_pre, nblk, t);
+    const uint32_t b = find_block(tile_pre, nblk, t);
     const uint64_t bbeg = blk_off[b], bend = blk_off[b + 1];
     const uint64_t base = bbeg + (uint64_t)(t - tile_pre[b]) * kBlockSortCap;
     const uint32_t cnt = (uint32_t)min((uint64_t)kBlockSortCap, bend - base);
@@ -370,7 +520,8 @@ __global__ void __launch_bounds__(kRunThreads) k_run_agg(const uint32_t* __restr
 __global__ void k_group_finish(const uint64_t* __restrict__ ukey, const LenAgg* __restrict__ agg,
                                const uint32_t* __restrict__ num_runs, uint32_t rows, uint32_t C, double bin,
                                const uint32_t* __restrict__ slot_tab, uint64_t slot_tab_len,
-                               QGroupDev* __restrict__ groups, uint64_t* __restrict__ g_off) {
+                               QGroupDev* __restrict__ groups, uint64_t* __restrict__ g_off,
+                               uint32_t* __restrict__ rc_off) {
     const uint32_t runs = *num_runs;
     // a trailing run of unusable intervals (key kNoGroup) sorts last and is dropped
     const uint32_t ng = (runs && ukey[runs - 1] == kNoGroup) ? runs - 1 : runs;
@@ -379,6 +530,8 @@ __global__ void k_group_finish(const uint64_t* __restrict__ ukey, const LenAgg* 
     if (g == ng) {  // rows after the last group's row
         const uint32_t r0 = ng ? (uint32_t)((ukey[ng - 1] >> 32) / C) + 1 : 0;
         for (uint32_t r = r0; r <= rows; r++) g_off[r] = ng;
+        const uint32_t rc0 = ng ? (uint32_t)(ukey[ng - 1] >> 32) + 1 : 0;
+        for (uint64_t r = rc0; r <= (uint64_t)rows * C; r++) rc_off[r] = ng;
         return;
     }
     const uint64_t k = ukey[g];
@@ -387,8 +540,11 @@ __global__ void k_group_finish(const uint64_t* __restrict__ ukey, const LenAgg* 
     const LenAgg a = agg[g];
     const double den = bin * (double)li;
     const double s2 = (double)a.s2hi * 18446744073709551616.0 + (double)a.s2lo;
-    groups[g] = QGroupDev{chrom, li < slot_tab_len ? slot_tab[li] : 0xFFFFFFFFu, (double)a.s1 / den,
-                          s2 / (den * den), (double)li, (double)a.cnt};
+    groups[g] = QGroupDev{(double)a.s1 / den, s2 / (den * den), (double)a.cnt / (double)li,
+                          chrom, li < slot_tab_len ? slot_tab[li] : 0xFFFFFFFFu, (double)li, (double)a.cnt};
+    const uint32_t rc_prev = g ? (uint32_t)(ukey[g - 1] >> 32) : 0xFFFFFFFFu;
+    if (rc_prev != rc)  // (row, chromosome) pairs (rc_prev, rc] start at this group
+        for (uint32_t r = (rc_prev == 0xFFFFFFFFu ? 0 : rc_prev + 1); r <= rc; r++) rc_off[r] = (uint32_t)g;
     const uint32_t prev = g ? (uint32_t)((ukey[g - 1] >> 32) / C) : 0xFFFFFFFFu;
     if (prev != row)  // rows (prev, row] start at this group
         for (uint32_t r = (prev == 0xFFFFFFFFu ? 0 : prev + 1); r <= row; r++) g_off[r] = g;
@@ -585,11 +741,11 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
     const uint64_t cells = (uint64_t)rows * D;
     if (!cells) return RGL_OK;
     // flatten the groups: validity on the host (l_int < n_bins of the chromosome, as the store's
-    // lookup requires, src/io/momentstore.rs:66-79); slot by compact_index
-    std::vector<uint64_t> goff(rows + 1, 0);
+    // lookup requires, src/io/momentstore.rs:66-79); slot by compact_index; (row, chromosome) by (row, chromosome) with the slots ascending, as k_pvalues walks them
+    std::vector<uint32_t> rcoff((uint64_t)rows * C + 1, 0);
     std::vector<QGroupDev> gs;
     for (uint32_t q = 0; q < rows; q++) {
-        goff[q] = gs.size();
+        const size_t first = gs.size();
         for (uint64_t g = b->row_group_offsets[q]; g < b->row_group_offsets[q + 1]; g++) {
             const uint32_t c = b->group_chrom[g];
             if (c >= C) return fail(RGL_ERR_INVALID_ARGUMENT, "group chromosome out of range");
@@ -597,15 +753,25 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
             if (l == 0 || l >= m->n_bins[c]) continue;
             const uint64_t slot = compact_index(l);
             if (slot >= m->n_slots[c]) continue;
-            gs.push_back(QGroupDev{c, (uint32_t)slot, b->group_sum_scale[g], b->group_sum_scale2[g], (double)l,
-                                   (double)b->group_count[g]});
+            const double cnt = (double)b->group_count[g];
+            gs.push_back(QGroupDev{b->group_sum_scale[g], b->group_sum_scale2[g], cnt / (double)l, c, (uint32_t)slot,
+                                   (double)l, cnt});
+        }
+        if (gs.size() >= (1ull << 32)) return fail(RGL_ERR_INVALID_ARGUMENT, "at most 2^32 - 1 groups per call");
+        std::stable_sort(gs.begin() + first, gs.end(), [](const QGroupDev& x, const QGroupDev& y) {
+            return x.chrom != y.chrom ? x.chrom < y.chrom : x.slot < y.slot;
+        });
+        size_t at = first;
+        for (uint32_t c = 0; c < C; c++) {
+            while (at < gs.size() && gs[at].chrom == c) at++;
+            rcoff[(uint64_t)q * C + c + 1] = (uint32_t)at;
         }
     }
-    goff[rows] = gs.size();
     RGL_CUDA(cudaSetDevice(m->device));
-    DevBuf d_goff, d_g, d_coff, d_cnt, d_bp, d_p, d_llr, d_lp, d_f;
+    DevBuf d_goff, d_g, d_coff, d_cnt, d_bp, d_p, d_llr, d_lp, d_f, d_part;
     int s = RGL_OK;
-    if (s == RGL_OK) s = d_goff.ensure((rows + 1) * 8ull);
+    if (s == RGL_OK) s = d_goff.ensure(rcoff.size() * 4);
+    if (s == RGL_OK) s = d_part.ensure(pv_scratch_bytes(rows, D, C));
     if (s == RGL_OK) s = d_g.ensure(std::max<size_t>(1, gs.size()) * sizeof(QGroupDev));
     if (s == RGL_OK) s = d_coff.ensure(C * 8ull);
     if (s == RGL_OK) s = d_cnt.ensure(cells * 4);
@@ -618,21 +784,16 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
         if (s == RGL_OK && n && cudaMemcpy(dst, src, n, cudaMemcpyHostToDevice) != cudaSuccess)
             s = fail(RGL_ERR_DEVICE, "p-value upload");
     };
-    cp(d_goff.p, goff.data(), goff.size() * 8);
+    cp(d_goff.p, rcoff.data(), rcoff.size() * 4);
     cp(d_g.p, gs.data(), gs.size() * sizeof(QGroupDev));
     cp(d_coff.p, m->chrom_off.data(), C * 8);
     cp(d_cnt.p, counts, cells * 4);
     cp(d_bp.p, overlap_bp, cells * 8);
-    if (s == RGL_OK) {
-        int nsm = 148;
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device);
-        const uint64_t warps = std::min<uint64_t>(cells, (uint64_t)nsm * 64);
-        k_pvalues<<<(unsigned)((warps * 32 + 255) / 256), 256>>>(
-            rows, D, C, d_cnt.as<uint32_t>(), d_bp.as<unsigned long long>(), (double)bin_size, d_goff.as<uint64_t>(),
-            d_g.as<QGroupDev>(), m->d_mv, d_coff.as<uint64_t>(), m->stride, m->d_len, d_p.as<double>(),
-            d_llr.as<double>(), d_lp.as<double>(), d_f.as<uint8_t>());
-        if (cudaGetLastError() != cudaSuccess) s = fail(RGL_ERR_DEVICE, "k_pvalues launch");
-    }
+    if (s == RGL_OK)
+        s = launch_pvalues(rows, D, C, d_cnt.as<uint32_t>(), d_bp.as<unsigned long long>(), (double)bin_size,
+                           d_goff.as<uint32_t>(), d_g.as<QGroupDev>(), m->d_mv, d_coff.as<uint64_t>(), m->stride,
+                           m->d_len, d_p.as<double>(), d_llr.as<double>(), d_lp.as<double>(), d_f.as<uint8_t>(),
+                           d_part.p, 0);
     auto back = [&](void* dst, const void* src, size_t n) {
         if (s == RGL_OK && dst && cudaMemcpy(dst, src, n, cudaMemcpyDeviceToHost) != cudaSuccess)
             s = fail(RGL_ERR_DEVICE, "p-value download");
@@ -641,7 +802,8 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
     back(llr, d_llr.p, cells * 8);
     back(log_p, d_lp.p, cells * 8);
     back(flags, d_f.p, cells);
-    for (DevBuf* x : {&d_goff, &d_g, &d_coff, &d_cnt, &d_bp, &d_p, &d_llr, &d_lp, &d_f}) x->release();
+    for (DevBuf* x : {&d_goff, &d_g, &d_coff, &d_cnt, &d_bp, &d_p, &d_llr, &d_lp, &d_f, &d_part})
+        x->release();
     return s;
 }
 
@@ -649,9 +811,11 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
 
 namespace rgl {
 
+uint32_t moments_chroms(const rgl_moments* m) { return m->num_chroms; }
+
 void stats_scratch_release(StatsScratch* sc) {
     for (DevBuf* b : {&sc->key_a, &sc->key_b, &sc->len_a, &sc->len_b, &sc->ukey, &sc->agg, &sc->runs, &sc->groups,
-                      &sc->goff, &sc->tmp, &sc->plan})
+                      &sc->goff, &sc->rcoff, &sc->part, &sc->tmp, &sc->plan})
         b->release();
 }
 
@@ -751,6 +915,7 @@ static int enqueue_batch_groups(rgl_context* ctx, rgl_moments* m, StatsScratch* 
     RGL_TRY(sc->groups.ensure(nn * sizeof(QGroupDev)));
     RGL_TRY(sc->goff.ensure((rows + 1ull) * 8 + (nblk + 1ull) * 8 + tabs.size() * 4 + 64));
     RGL_TRY(sc->runs.ensure(64));
+    RGL_TRY(sc->rcoff.ensure(((uint64_t)rows * C + 1) * 4));
     if (local) RGL_TRY(sc->plan.ensure((3ull * nblk + 2 * tiles + 8) * 4));
     uint64_t* d_goff = sc->goff.as<uint64_t>();
     uint64_t* d_boff = d_goff + rows + 1;
@@ -822,7 +987,7 @@ static int enqueue_batch_groups(rgl_context* ctx, rgl_moments* m, StatsScratch* 
     }
     k_group_finish<<<(unsigned)((nn + 256) / 256), 256, 0, st>>>(
         sc->ukey.as<uint64_t>(), sc->agg.as<LenAgg>(), sc->runs.as<uint32_t>(), rows, C, (double)bin_size,
-        m->slot_tab.as<uint32_t>(), lmax, sc->groups.as<QGroupDev>(), d_goff);
+        m->slot_tab.as<uint32_t>(), lmax, sc->groups.as<QGroupDev>(), d_goff, sc->rcoff.as<uint32_t>());
     RGL_CUDA(cudaGetLastError());
     *goff_out = d_goff;
     return RGL_OK;
@@ -846,15 +1011,11 @@ int batch_pvalues_enqueue(rgl_context* ctx, rgl_moments* m, StatsScratch* sc, co
     }
     const uint32_t rows = b->num_rows, D = m->num_sources, C = m->num_chroms;
     cudaStream_t st = context_stream(ctx);
-    // the p-value kernel drops groups whose slot lies past the source's table (slot >= tab_len)
-    int nsm = 148;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device);
-    const uint64_t cells = (uint64_t)rows * D;
-    const uint64_t warps = std::min<uint64_t>(cells, (uint64_t)nsm * 64);
-    k_pvalues<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>(
-        rows, D, C, d_counts, reinterpret_cast<const unsigned long long*>(d_overlap_bp), (double)bin_size, d_goff,
-        sc->groups.as<QGroupDev>(), m->d_mv, m->coff.as<uint64_t>(), m->stride, m->d_len, d_p, d_llr, d_log_p, d_flags);
-    RGL_CUDA(cudaGetLastError());
+    // groups whose slot lies past the source's table (slot >= tab_len) are dropped there
+    RGL_TRY(sc->part.ensure(pv_scratch_bytes(rows, D, C)));
+    RGL_TRY(launch_pvalues(rows, D, C, d_counts, reinterpret_cast<const unsigned long long*>(d_overlap_bp),
+                           (double)bin_size, sc->rcoff.as<uint32_t>(), sc->groups.as<QGroupDev>(), m->d_mv,
+                           m->coff.as<uint64_t>(), m->stride, m->d_len, d_p, d_llr, d_log_p, d_flags, sc->part.p, st));
     if (out_groups) {
         uint64_t ng = 0;
         RGL_CUDA(cudaMemcpyAsync(&ng, d_goff + rows, 8, cudaMemcpyDeviceToHost, st));
