@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(kBsThreads) k_tile_sort(uint32_t nblk, const u
     const uint64_t rest = bbeg + bcnt - base;
     const uint32_t cnt = (uint32_t)(rest < kBlockSortCap ? rest : kBlockSortCap);
     if (unsorted[blk] == 0u) return;  // an ordered block is copied by k_tile_copy
+    if (unsorted[blk] == kSkipBlock) return;
     const uint32_t passes = sort_passes(bcnt);
     if (threadIdx.x == 0 && tile == tile_pre[blk] && passes) atomicMax(maxp, passes);
     uint64_t* ko = (passes & 1u) ? kin : kout;
@@ -229,7 +230,7 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_pass(uint32_t q, uint32
     const uint32_t chunk = blockIdx.x;
     if (chunk >= __ldg(chunk_pre + nblk)) return;
     const uint32_t blk = find_block(chunk_pre, nblk, chunk);
-    if (unsorted[blk] == 0u) return;
+    if (unsorted[blk] == 0u || unsorted[blk] == kSkipBlock) return;
     const uint64_t bbeg = blk_off[blk];
     const uint32_t cnt = (uint32_t)(blk_off[blk + 1] - bbeg);
     const uint32_t p = sort_passes(cnt);

@@ -64,6 +64,9 @@ __device__ __forceinline__ uint32_t find_block(const T* __restrict__ pre, uint32
 }
 #endif
 
+// In unsorted[b]: nothing of block b is needed; its output is left as it is.
+constexpr uint32_t kSkipBlock = 2u;
+
 // Enqueues the block sort on `st`: the plan (tile and merge-chunk prefix counts, when `plan`), the
 // tiles, then `passes` merge passes.  off: nblk + 1 block offsets; unsorted[b] != 0 marks block b
 // as not in order; tiles / chunks / passes: the host's counts for these blocks (sort_tiles,

@@ -323,17 +323,18 @@ __device__ __forceinline__ T block_exclusive(T v) {
     __syncthreads();  // part may be reused by the next call
     return T::add(before, ex);
 }
-// Every tile of group blockIdx.x: sums[tile] becomes the sum of all tiles before it.
+// Every tile of group blockIdx.x: sums[tile] becomes the sum of all tiles before it; *total: the whole.
 template <class T>
 __global__ void __launch_bounds__(kTileThreads) k_group_scan(T* __restrict__ sums, uint32_t nt,
                                                              const uint32_t* __restrict__ count, uint32_t tile,
-                                                             const T* __restrict__ groups) {
+                                                             const T* __restrict__ groups, T* __restrict__ total) {
     static_assert(kGroup == kTileThreads, "one tile a thread");
     if (count) nt = (uint32_t)(((uint64_t)*count + tile - 1) / tile);
     const uint32_t k = blockIdx.x * kGroup + threadIdx.x;
     const T before = block_total(groups, blockIdx.x);
-    const T ex = block_exclusive(k < nt ? sums[k] : T::zero());
+    const T own = k < nt ? sums[k] : T::zero(), ex = block_exclusive(own);
     if (k < nt) sums[k] = T::add(before, ex);
+    if (total && k + 1 == nt) *total = T::add(T::add(before, ex), own);
 }
 
 // ---- 3. the sorted queries ------------------------------------------------------------------------------
@@ -543,6 +544,14 @@ __global__ void k_seg_tabsize(uint32_t n, const uint32_t* __restrict__ segnum, c
     tabs[sgi] = SegTab{beg, end, shift, nbins, 8 * beg + 2 * sgi, 0};
 }
 
+// The blocks (in the sort's layout) whose segment has no range swept by ranks: their ends stay unsorted.
+__global__ void k_skip_ends(uint32_t nblk, const uint64_t* __restrict__ off, const uint32_t* __restrict__ segnum,
+                            const unsigned long long* __restrict__ need, uint32_t* __restrict__ unsorted) {
+    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= nblk || off[b] == off[b + 1]) return;
+    if (!need[segnum[off[b]] - 1]) unsorted[b] = kSkipBlock;
+}
+
 // Rank tables from the sorted arrays: entry b of a segment holds the position of its first element of bin
 // >= b, so element j fills the entries from its predecessor's bin (exclusive) through its own with j, and
 // the last one the rest with the segment's end.  A lane fills up to kTabShort entries itself, longer
@@ -618,13 +627,16 @@ __device__ __forceinline__ void add_u64(unsigned long long* c, unsigned long lon
 //     E >= end             does not (its run ends at or before the partition point of E);
 //     back < E < end       starts one when no start lies in [back, E), i.e. when the run's first element
 //                          (live: it exists) starts at or after E.
-// Pass 1 (k_lohi) searches, stores [lo, hi) and a flag bit per entry and sums live entries, ranges and
-// candidates per tile of kTileThreads queries of one slot; pass 2 (k_emit) writes the live runs and the
-// ranges at their places.  Pass 1 is bound by its random reads (bucket table and starts): one query a
-// thread, so that the blocks running at once lie close together and the rows of a chromosome find its
-// starts in L2 (eight queries a thread: 0.75 -> 2.0 ms for 48 files against 2e8 intervals).  Before, the
-// flags, a compaction, a segmented running maximum and three scans over the entries took eleven launches
-// (3.9 of the 11 ms of 3.1e7 intervals against 3.2e6).
+// Pass 1 (k_lohi) searches, and stores the live entries of each tile (kTileThreads queries of one slot)
+// side by side: first element, length, place in the tile and whether they start a range; it sums live
+// entries, ranges and candidates per tile.  Pass 2 (k_emit) writes the live runs and the ranges at their
+// places.  Pass 1 is bound by its random reads (bucket table and starts) and, where those hit L2, by issue:
+// one query a thread, so that the blocks running at once lie close together and the rows of a chromosome
+// find its starts in L2 (eight queries a thread: 0.75 -> 2.0 ms for 48 files against 2e8 intervals).
+// Before, the flags, a compaction, a segmented running maximum and three scans over the entries took eleven
+// launches (3.9 of the 11 ms of 3.1e7 intervals against 3.2e6); with every entry's [lo, hi) stored and read
+// again, dead or live, k_emit took 2.1 of 8.9 ms there, now 1.2 of 6.4.
+constexpr uint32_t kStartsRange = 1u << 15;  // in an entry's `place`, beside its number in the tile
 __device__ __forceinline__ bool large_counts(uint32_t cnt) { return __any_sync(0xffffffffu, cnt >> 27); }
 
 // Sum of the lanes' counts, in 32 bits unless a count is so large that it may not fit.
@@ -641,7 +653,7 @@ __global__ void __launch_bounds__(kTileThreads) k_lohi(
     uint32_t n, uint32_t nslots, const uint32_t* __restrict__ starts, const uint32_t* __restrict__ qend,
     const uint32_t* __restrict__ emax, const uint32_t* __restrict__ shard, const int32_t* __restrict__ slot,
     const LayerDev* __restrict__ layers, const uint2* __restrict__ pos, const uint32_t* __restrict__ btab,
-    uint32_t* __restrict__ lo_out, uint32_t* __restrict__ hi_out, uint32_t* __restrict__ flags,
+    uint32_t* __restrict__ lo_out, uint32_t* __restrict__ cnt_out, uint16_t* __restrict__ place,
     LSum* __restrict__ sums) {
     if constexpr (PDL) {
         pdl_wait();
@@ -664,17 +676,19 @@ __global__ void __launch_bounds__(kTileThreads) k_lohi(
             if (hi < lo) hi = lo;
             if (hi > lo) start = back >= E || (E < en && __ldg(&p[lo].x) >= E);
         }
-        const uint64_t t = (uint64_t)K * n + i;
-        lo_out[t] = lo;
-        hi_out[t] = hi;
     }
     const uint32_t fl = __ballot_sync(0xffffffffu, start), live = __ballot_sync(0xffffffffu, hi > lo);
     const uint64_t cand = warp_count(hi - lo);
-    if (lane == 0) {
-        flags[tile * (kTileThreads / 32) + warp] = fl;
-        part[warp] = LSum{(uint32_t)__popc(live), (uint32_t)__popc(fl), cand};
-    }
+    if (lane == 0) part[warp] = LSum{(uint32_t)__popc(live), (uint32_t)__popc(fl), cand};
     __syncthreads();
+    uint32_t before = 0;
+    for (uint32_t w = 0; w < warp; w++) before += part[w].live;
+    if (hi > lo) {
+        const uint64_t at = (uint64_t)tile * kTileThreads + before + __popc(live & ((1u << lane) - 1u));
+        lo_out[at] = lo;
+        cnt_out[at] = hi - lo;
+        place[at] = (uint16_t)(threadIdx.x | (start ? kStartsRange : 0u));
+    }
     if (threadIdx.x == 0) {
         LSum s = part[0];
 #pragma unroll
@@ -723,83 +737,74 @@ __device__ __forceinline__ uint64_t warp_inclusive(uint32_t cnt, uint32_t lane) 
 // (shard * rows + row; the pair list).
 enum : int { RUN_PLAIN = 0, RUN_ROW = 1, RUN_SHARD_ROW = 2 };
 
-// A block takes ITEMS of k_lohi's tiles of its slot (tiles of them: per_slot).
-template <int ITEMS, bool PDL>
+// A warp takes one of k_lohi's tiles (per_slot of them a slot), 32 live entries at a time.
+template <bool PDL>
 __global__ void __launch_bounds__(kTileThreads) k_emit(
-    uint32_t n, uint32_t nslots, uint32_t rows, uint32_t per_slot, int tag, const uint32_t* __restrict__ starts,
-    const uint32_t* __restrict__ qend, const uint32_t* __restrict__ emax, const uint32_t* __restrict__ shard,
-    const uint32_t* __restrict__ row, const int32_t* __restrict__ slot, const LayerDev* __restrict__ layers,
-    const uint2* __restrict__ pos, const uint32_t* __restrict__ btab, const uint32_t* __restrict__ lo_in,
-    const uint32_t* __restrict__ hi_in, const uint32_t* __restrict__ flags, const LSum* __restrict__ sums, int scanned,
-    PairSeg* __restrict__ psegs, uint32_t* __restrict__ prow,
+    uint32_t n, uint32_t nslots, uint32_t rows, uint32_t per_slot, uint32_t tiles, int tag,
+    const uint32_t* __restrict__ starts, const uint32_t* __restrict__ qend, const uint32_t* __restrict__ emax,
+    const uint32_t* __restrict__ shard, const uint32_t* __restrict__ row, const int32_t* __restrict__ slot,
+    const LayerDev* __restrict__ layers, const uint2* __restrict__ pos, const uint32_t* __restrict__ btab,
+    const uint32_t* __restrict__ lo_in, const uint32_t* __restrict__ cnt_in, const uint16_t* __restrict__ place,
+    const LSum* __restrict__ sums, int scanned, PairSeg* __restrict__ psegs, uint32_t* __restrict__ prow,
     uint64_t* __restrict__ pc, uint32_t* __restrict__ cr, uint32_t* __restrict__ uhi, uint2* __restrict__ rt,
-    uint32_t* __restrict__ Lp, uint32_t* __restrict__ Rp) {
+    uint32_t* __restrict__ rlo, uint32_t* __restrict__ Lp, uint32_t* __restrict__ Rp) {
     if constexpr (PDL) {
         pdl_wait();
         pdl_release();
     }
-    constexpr uint32_t kWarps = kTileThreads / 32, kChunks = kWarps * ITEMS;  // chunks of 32 entries, in order
-    static_assert(kChunks <= 32, "one chunk a lane");
-    __shared__ LSum chunk[kChunks];
-    const uint32_t K = blockIdx.y, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t tile0 = K * per_slot + blockIdx.x * ITEMS;
-    uint32_t lo[ITEMS], cnt[ITEMS], fl[ITEMS], sh[ITEMS], qs[ITEMS], qe[ITEMS], E[ITEMS];
-#pragma unroll
-    for (int k = 0; k < ITEMS; k++) {
-        const uint32_t x = blockIdx.x * ITEMS + k, i = x * kTileThreads + threadIdx.x;
-        const uint64_t t = (uint64_t)K * n + i;
-        const bool in = x < per_slot && i < n;
-        lo[k] = in ? lo_in[t] : 0u;
-        cnt[k] = (in ? hi_in[t] : 0u) - lo[k];
-        fl[k] = x < per_slot ? flags[(tile0 + k) * kWarps + warp] : 0u;
-        const bool live = cnt[k] != 0;
-        sh[k] = live ? shard[i] : 0u;
-        qs[k] = live ? starts[i] : 0u;
-        qe[k] = live ? qend[i] : 0u;
-        E[k] = live ? emax[i] : 0u;
+    constexpr uint32_t kWarps = kTileThreads / 32;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, tile0 = blockIdx.x * kWarps, tile = tile0 + warp;
+    LSum at, all;  // before the tile, and through it
+    if (scanned) {  // sums[tiles] is the whole
+        at = tile < tiles ? sums[tile] : LSum::zero();
+        all = tile < tiles ? sums[tile + 1] : at;
+    } else {
+        at = block_total(sums, tile0);
+        for (uint32_t w = 0; w < warp && tile0 + w < tiles; w++) at = LSum::add(at, sums[tile0 + w]);
+        all = tile < tiles ? LSum::add(at, sums[tile]) : at;
     }
-#pragma unroll
-    for (int k = 0; k < ITEMS; k++) {
-        const uint64_t total = warp_count(cnt[k]);
-        const uint32_t live = __popc(__ballot_sync(0xffffffffu, cnt[k] != 0));
-        if (lane == 0) chunk[k * kWarps + warp] = LSum{live, (uint32_t)__popc(fl[k]), total};
+    if (tile >= tiles) return;
+    const uint32_t K = tile / per_slot, i0 = (tile - K * per_slot) * kTileThreads;
+    const uint64_t base = (uint64_t)tile * kTileThreads;
+    const uint32_t live = all.live - at.live;
+    if (tile + 1 == tiles && lane == 0) {
+        *Lp = all.live;
+        *Rp = all.ranges;
+        pc[all.live] = all.cand;
     }
-    const LSum before = tile_prefix(sums, scanned, tile0);
-    __syncthreads();
-    // the chunks' prefixes, by every warp for itself: lane h holds chunk h's
-    const LSum inc_chunk = LSum::add(before, warp_scan(lane < kChunks ? chunk[lane] : LSum::zero(), lane));
-    LSum ex_chunk = shfl_up_words(inc_chunk, 1);
-    if (lane == 0) ex_chunk = before;
-    if (K + 1 == gridDim.y && blockIdx.x + 1 == gridDim.x && threadIdx.x == 31) {
-        *Lp = inc_chunk.live;
-        *Rp = inc_chunk.ranges;
-        pc[inc_chunk.live] = inc_chunk.cand;
-    }
-#pragma unroll
-    for (int k = 0; k < ITEMS; k++) {
-        const uint32_t live = __ballot_sync(0xffffffffu, cnt[k] != 0);
-        const LSum at = shfl_words(ex_chunk, k * kWarps + warp);
-        if (!live) continue;
-        const uint64_t inc = warp_inclusive(cnt[k], lane);
-        if (!cnt[k]) continue;
-        const uint32_t i = (blockIdx.x * ITEMS + k) * kTileThreads + threadIdx.x;
-        const uint32_t c = at.live + __popc(live & ((1u << lane) - 1u));
-        const int32_t li = slot[(uint64_t)sh[k] * nslots + K];
-        psegs[c] = PairSeg{layers[li].off + lo[k], qs[k], qe[k]};
-        if (tag) prow[c] = (rows > 1 ? row[i] : 0u) + (tag == RUN_SHARD_ROW ? sh[k] * rows : 0u);
-        pc[c] = at.cand + inc - cnt[k];
-        cr[c] = at.ranges + __popc(fl[k] & ((2u << lane) - 1u)) - 1;  // the range it starts or continues
-        if (fl[k] >> lane & 1u) rt[at.ranges + __popc(fl[k] & ((1u << lane) - 1u))] = make_uint2(c, K * n + i);
-        // its range's last run unless the next live entry of the chunk goes on with the range
-        const uint32_t later = live & ~((2u << lane) - 1u);
-        if (!later || (fl[k] & later & (0u - later))) {
-            uint32_t end = lo[k] + cnt[k];
-            if (E[k] > qe[k]) {  // an earlier query reaches further
-                const LayerDev Ld = layers[li];
-                end = pp_layer(pos + Ld.off, btab + Ld.boff, Ld, E[k]);
+    for (uint32_t j0 = 0; j0 < live; j0 += 32) {
+        const uint32_t j = j0 + lane;
+        const bool in = j < live;
+        const uint32_t lo = in ? lo_in[base + j] : 0u, cnt = in ? cnt_in[base + j] : 0u;
+        const uint32_t pl = in ? place[base + j] : 0u;
+        const uint32_t i = i0 + (pl & (kStartsRange - 1));
+        const uint32_t sh = in ? shard[i] : 0u, qs = in ? starts[i] : 0u, qe = in ? qend[i] : 0u, E = in ? emax[i] : 0u;
+        const uint32_t fl = __ballot_sync(0xffffffffu, pl & kStartsRange);
+        const uint64_t inc = warp_inclusive(cnt, lane);
+        if (in) {
+            const uint32_t c = at.live + j;
+            const int32_t li = slot[(uint64_t)sh * nslots + K];
+            psegs[c] = PairSeg{layers[li].off + lo, qs, qe};
+            if (tag) prow[c] = (rows > 1 ? row[i] : 0u) + (tag == RUN_SHARD_ROW ? sh * rows : 0u);
+            pc[c] = at.cand + inc - cnt;
+            const uint32_t r = at.ranges + __popc(fl & ((2u << lane) - 1u)) - 1;  // the range it starts or continues
+            cr[c] = r;
+            if (pl & kStartsRange) {
+                rt[r] = make_uint2(c, K * n + i);
+                rlo[r] = lo;
             }
-            uhi[c] = end;
+            // its range's last run unless the next live entry of the 32 goes on with the range
+            if (lane == 31 || j + 1 == live || (fl >> (lane + 1) & 1u)) {
+                uint32_t end = lo + cnt;
+                if (E > qe) {  // an earlier query reaches further
+                    const LayerDev Ld = layers[li];
+                    end = pp_layer(pos + Ld.off, btab + Ld.boff, Ld, E);
+                }
+                uhi[c] = end;
+            }
         }
+        at.ranges += __popc(fl);
+        at.cand += __shfl_sync(0xffffffffu, inc, 31);
     }
 }
 
@@ -810,11 +815,19 @@ __global__ void __launch_bounds__(kTileThreads) k_emit(
 // metric), those swept by ranks per segment into seg_need.
 constexpr uint32_t kRItems = 4, kRTile = kTileThreads * kRItems;
 
+// Whether a range of `runs` runs, `cand` candidates and a union of `len` is swept by ranks.  A position of
+// the rank sweep costs about pair_ratio candidates of the pair sweep; and a range swept by ranks needs its
+// segment's ends sorted and summed and a rank table: about run_cost candidates a query.
+__device__ __forceinline__ bool by_ranks(uint64_t cand, uint32_t len, uint32_t runs, uint32_t pair_ratio,
+                                         uint32_t run_cost) {
+    return cand > (uint64_t)pair_ratio * len + (uint64_t)run_cost * runs;
+}
+
 template <bool PDL>
 __global__ void __launch_bounds__(kTileThreads) k_range_reduce(
     const uint32_t* __restrict__ Lp, const uint32_t* __restrict__ Rp, uint32_t n, const uint2* __restrict__ rt,
-    const uint64_t* __restrict__ pc, const uint32_t* __restrict__ uhi, const uint32_t* __restrict__ lo,
-    const uint32_t* __restrict__ segnum, uint32_t pair_ratio, uint32_t* __restrict__ ulen,
+    const uint64_t* __restrict__ pc, const uint32_t* __restrict__ uhi, const uint32_t* __restrict__ rlo,
+    const uint32_t* __restrict__ segnum, uint32_t pair_ratio, uint32_t run_cost, uint32_t* __restrict__ ulen,
     unsigned long long* __restrict__ seg_need, unsigned long long* __restrict__ union_total,
     RSum* __restrict__ sums) {
     if constexpr (PDL) {
@@ -839,10 +852,10 @@ __global__ void __launch_bounds__(kTileThreads) k_range_reduce(
             const uint64_t r = tile * kRTile + k * kTileThreads + threadIdx.x;
             if (r >= R) continue;
             const uint64_t cand = pc[c1[k]] - pc[f[k].x];
-            const uint32_t len = uhi[c1[k] - 1] - lo[f[k].y];
+            const uint32_t len = uhi[c1[k] - 1] - rlo[r];
             ulen[r] = len;
             uni += len;
-            if (cand <= (uint64_t)pair_ratio * len) s.pair += cand;
+            if (!by_ranks(cand, len, c1[k] - f[k].x, pair_ratio, run_cost)) s.pair += cand;
             else {
                 s.rank += len;
                 s.nrank++;
@@ -878,8 +891,8 @@ template <bool PDL>
 __global__ void __launch_bounds__(kTileThreads) k_range_apply(
     const uint32_t* __restrict__ Lp, const uint32_t* __restrict__ Rp, uint32_t n, uint32_t nslots, uint32_t rows,
     const uint2* __restrict__ rt, const uint64_t* __restrict__ pc, const uint32_t* __restrict__ ulen,
-    const uint32_t* __restrict__ lo, const uint32_t* __restrict__ shard, const uint32_t* __restrict__ row,
-    const uint32_t* __restrict__ segnum, const int32_t* __restrict__ slot, uint32_t pair_ratio,
+    const uint32_t* __restrict__ rlo, const uint32_t* __restrict__ shard, const uint32_t* __restrict__ row,
+    const uint32_t* __restrict__ segnum, const int32_t* __restrict__ slot, uint32_t pair_ratio, uint32_t run_cost,
     const RSum* __restrict__ sums, int scanned, RangeDesc* __restrict__ ranges,
     uint64_t* __restrict__ rpos, uint64_t* __restrict__ rpair, uint64_t* __restrict__ ppos,
     uint32_t* __restrict__ rank_count, unsigned long long* __restrict__ totals) {
@@ -899,23 +912,24 @@ __global__ void __launch_bounds__(kTileThreads) k_range_apply(
     }
     for (uint64_t tile = blockIdx.x; tile * kRTile < R; tile += gridDim.x) {
         uint64_t first[kRItems], cand[kRItems];
-        uint32_t len[kRItems], ent[kRItems];
+        uint32_t len[kRItems], ent[kRItems], runs[kRItems];
 #pragma unroll
         for (uint32_t k = 0; k < kRItems; k++) {
             const uint64_t r = tile * kRTile + k * kTileThreads + threadIdx.x;
             const uint2 f = r < R ? rt[r] : make_uint2(0, 0);
             const uint32_t c1 = r < R ? (r + 1 < R ? rt[r + 1].x : L) : 0u;
             ent[k] = f.y;
+            runs[k] = c1 - f.x;
             first[k] = pc[f.x];
             cand[k] = pc[c1] - first[k];
             len[k] = r < R ? ulen[r] : 0u;
         }
-        uint32_t rank = 0;  // bit k: range k of this thread is swept by ranks
+        uint32_t rank = 0;  // bit k: range k of this thread is swept by ranks (see by_ranks)
 #pragma unroll
         for (uint32_t k = 0; k < kRItems; k++) {
             const uint64_t r = tile * kRTile + k * kTileThreads + threadIdx.x;
             if (r >= R) cand[k] = 0;
-            else if (cand[k] > (uint64_t)pair_ratio * len[k]) rank |= 1u << k;
+            else if (by_ranks(cand[k], len[k], runs[k], pair_ratio, run_cost)) rank |= 1u << k;
             RSum s = RSum::zero();
             if (__any_sync(0xffffffffu, rank >> k & 1u)) {
                 s = rank >> k & 1u ? RSum{len[k], 0ull, 1ull} : RSum{0ull, cand[k], 0ull};
@@ -955,7 +969,7 @@ __global__ void __launch_bounds__(kTileThreads) k_range_apply(
                 const uint64_t q = inc.nrank - 1;
                 rpair[r] = kRankRange | inc.pair;
                 rpos[q] = inc.rank - len[k];
-                ranges[q] = RangeDesc{lo[ent[k]], (uint32_t)slot[(uint64_t)shard[i] * nslots + K],
+                ranges[q] = RangeDesc{rlo[r], (uint32_t)slot[(uint64_t)shard[i] * nslots + K],
                                       rows > 1 ? row[i] : 0u, segnum[i] - 1};
             } else {
                 rpair[r] = first[k] - (inc.pair - cand[k]);
@@ -1732,9 +1746,9 @@ struct rgl_context {
     int num_sms = 148;
     DevBuf iv, blk_off, blk_shard, key_a, key_b, val_a, val_b, ekey_a, ekey_b;
     DevBuf starts, ends, shard, row, segnum, seg_begin, ps, pe, emax;
-    DevBuf lo, hi, flags, ranges, rpos, cub_tmp, small, out_counts, out_bp, item_r0;
+    DevBuf lo, cnt, place, ranges, rpos, cub_tmp, small, out_counts, out_bp, item_r0;
     DevBuf segtab, tab2;
-    DevBuf pc, cr, uhi, rt, ulen, rpair, ppos, psegs, prow, item_t0, seg_need;
+    DevBuf pc, cr, uhi, rt, rlo, ulen, rpair, ppos, psegs, prow, item_t0, seg_need;
     DevBuf sums, esums;  // tile summaries, of the main and of the side stream
     DevBuf cub_tmp2;  // the side stream's own scratch
     DevBuf sortplan;  // block-local sort: order flags, tile and merge-chunk prefix counts, two pass words
@@ -1783,6 +1797,11 @@ constexpr uint64_t kItemCap = 1ull << 22;
 // Default work-item size of runs with several output rows.
 constexpr uint32_t kMultiRowChunk = 8192;
 
+// What a query of a range swept by ranks costs besides, in candidates of the pair sweep (see by_ranks).
+// 256 files against 3.2e6 intervals: hardly a range is worth it (7.6 -> 6.4 ms); 48 files against 2e8: 16
+// moved ranges to the pair sweep that were faster by ranks (k_pairs + k_sweep 6.2 -> 6.4 ms), 4 does not.
+constexpr uint32_t kRankRunCost = 4;
+
 // Runs up to this many query intervals chain their kernels with programmatic dependent launch.
 constexpr uint64_t kPdlMaxIntervals = 1ull << 21;
 
@@ -1830,9 +1849,11 @@ int size_workspace(rgl_context* c, uint64_t n, uint32_t rows, uint32_t nblk, uin
     RGL_TRY(z.ensure_in(c->seg_need, n * 8 + 8));
     RGL_TRY(z.ensure_in(c->ps, n * 8 + 16));
     RGL_TRY(z.ensure_in(c->pe, n * 8 + 16));
-    RGL_TRY(z.ensure_in(c->lo, tot * 4 + 4));
-    RGL_TRY(z.ensure_in(c->hi, tot * 4 + 4));
-    RGL_TRY(z.ensure_in(c->flags, tot / 8 + ns * 32 + 64));
+    const uint64_t tiled = tot + ns * kTileThreads;  // entries of whole tiles
+    RGL_TRY(z.ensure_in(c->lo, tiled * 4));
+    RGL_TRY(z.ensure_in(c->cnt, tiled * 4));
+    RGL_TRY(z.ensure_in(c->place, tiled * 2));
+    RGL_TRY(z.ensure_in(c->rlo, tot * 4 + 4));
     RGL_TRY(z.ensure_in(c->ranges, (tot / 2 + 2) * sizeof(RangeDesc)));  // a range swept by ranks has two runs or more
     RGL_TRY(z.ensure_in(c->rpos, (tot / 2 + 2) * 8));
     RGL_TRY(z.ensure_in(c->small, 256));
@@ -1876,8 +1897,8 @@ int size_workspace(rgl_context* c, uint64_t n, uint32_t rows, uint32_t nblk, uin
     c->ws_ready = true;
     uint64_t sig = 1469598103934665603ull;
     for (DevBuf* b : {&c->iv, &c->key_a, &c->key_b, &c->val_a, &c->val_b, &c->ekey_a, &c->ekey_b, &c->starts,
-                      &c->ends, &c->shard, &c->row, &c->segnum, &c->seg_begin, &c->ps, &c->pe, &c->emax, &c->lo, &c->hi,
-                      &c->flags, &c->ranges, &c->rpos, &c->cub_tmp, &c->small, &c->item_r0, &c->item_t0, &c->segtab,
+                      &c->ends, &c->shard, &c->row, &c->segnum, &c->seg_begin, &c->ps, &c->pe, &c->emax, &c->lo, &c->cnt,
+                      &c->place, &c->rlo, &c->ranges, &c->rpos, &c->cub_tmp, &c->small, &c->item_r0, &c->item_t0, &c->segtab,
                       &c->tab2, &c->pc, &c->cr, &c->uhi, &c->rt, &c->ulen, &c->rpair, &c->sums, &c->esums, &c->ppos,
                       &c->psegs, &c->prow, &c->seg_need, &c->acc, &c->cub_tmp2, &c->sortplan})
         sig = (sig ^ (uint64_t)(uintptr_t)b->p ^ ((uint64_t)b->cap << 17)) * 1099511628211ull;
@@ -1965,9 +1986,10 @@ int finish(rgl_context* c, const Launch& L, rgl_query_stats* stats) {
 
 // Tile summaries into exclusive prefixes (nt tiles, or those of *count elements), by groups of kGroup.
 template <class T>
-void scan_groups(T* sums, uint32_t nt, const uint32_t* count, uint32_t tile, T* groups, uint32_t ng, cudaStream_t st) {
+void scan_groups(T* sums, uint32_t nt, const uint32_t* count, uint32_t tile, T* groups, uint32_t ng, cudaStream_t st,
+                 T* total = nullptr) {
     k_group_sums<T><<<ng, kTileThreads, 0, st>>>(sums, nt, count, tile, groups);
-    k_group_scan<T><<<ng, kTileThreads, 0, st>>>(sums, nt, count, tile, groups);
+    k_group_scan<T><<<ng, kTileThreads, 0, st>>>(sums, nt, count, tile, groups, total);
 }
 
 // `to` waits for everything enqueued on `from` so far.
@@ -2111,6 +2133,8 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     const bool with_bp = d_bp != nullptr && !(opts && (opts->flags & RGL_QF_NO_OVERLAP));
     const bool ev = mode.events && stats;
     const bool pdl = in.n <= kPdlMaxIntervals;
+    // a caller's pair ratio is taken alone
+    const uint32_t run_cost = (opts && opts->pair_ratio) ? 0u : kRankRunCost;
 
     uint32_t* d_small = c->small.as<uint32_t>();  // [0] error bits, [1] queue, [2..] scratch
     ClearList clear{};
@@ -2200,10 +2224,17 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
                                        nullptr, nullptr, nullptr, st, true, pdl);
     RGL_TRY(stream_after(sd, st, c->ev_fork));
     size_t tb = c->cub_tmp2.cap;
-    if (in.block_local) {
+    // the end keys: on the side stream at once; or, in large runs whose blocks are segments, once it is
+    // known which of them a rank sweep needs (the sort, sums and tables of 3.1e7 ends were 1.6 of 8.9 ms
+    // of a batch against a small database that hardly any range sweeps by ranks)
+    const bool late_ends = in.block_local && !in.ls.wide && !pdl;
+    auto sort_ends = [&] {
         launches += block_sort_enqueue(in.nblk, soff, in.ls.tiles, in.ls.chunks, passes, d_tile_pre, d_chunk_pre,
                                        d_unsorted + in.nblk, c->ekey_a.as<uint64_t>(), nullptr,
                                        c->ekey_b.as<uint64_t>(), nullptr, d_maxp + 1, sd, false, pdl, in.ls.wide);
+    };
+    if (in.block_local) {
+        if (!late_ends) sort_ends();
         launches += block_sort_enqueue(in.nblk, soff, in.ls.tiles, in.ls.chunks, passes, d_tile_pre, d_chunk_pre,
                                        d_unsorted, c->key_a.as<uint64_t>(), c->val_a.as<uint32_t>(),
                                        c->key_b.as<uint64_t>(), c->val_b.as<uint32_t>(), d_maxp, st, false, pdl,
@@ -2226,11 +2257,15 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     const uint32_t qg = qt > kMaxLook ? (qt + kGroup - 1) / kGroup : 0u;  // groups of tiles, if any
     ESum* eg = qg ? c->esums.as<ESum>() + qt : nullptr;
     QSum* qgs = qg ? c->sums.as<QSum>() + qt : nullptr;
-    (void)launch_chain(pdl, k_e_reduce<true>, k_e_reduce<false>, qt, kTileThreads, 0, sd, n,
-                       c->ekey_b.as<uint64_t>(), c->esums.as<ESum>());
-    if (qg) scan_groups(c->esums.as<ESum>(), qt, nullptr, 0, eg, qg, sd);
-    (void)launch_chain(pdl, k_e_apply<true>, k_e_apply<false>, qt, kTileThreads, 0, sd, n, c->ekey_b.as<uint64_t>(),
-                       c->esums.as<ESum>(), (int)(qg != 0), c->ends.as<uint32_t>(), c->pe.as<uint64_t>());
+    auto sum_ends = [&] {
+        (void)launch_chain(pdl, k_e_reduce<true>, k_e_reduce<false>, qt, kTileThreads, 0, sd, n,
+                           c->ekey_b.as<uint64_t>(), c->esums.as<ESum>());
+        if (qg) scan_groups(c->esums.as<ESum>(), qt, nullptr, 0, eg, qg, sd);
+        (void)launch_chain(pdl, k_e_apply<true>, k_e_apply<false>, qt, kTileThreads, 0, sd, n, c->ekey_b.as<uint64_t>(),
+                           c->esums.as<ESum>(), (int)(qg != 0), c->ends.as<uint32_t>(), c->pe.as<uint64_t>());
+        launches += qg ? 4 : 2;
+    };
+    if (!late_ends) sum_ends();
     (void)launch_chain(pdl, k_q_reduce<true>, k_q_reduce<false>, qt, kTileThreads, 0, st, n,
                        c->key_b.as<uint64_t>(), c->val_b.as<uint32_t>(), c->sums.as<QSum>());
     if (qg) scan_groups(c->sums.as<QSum>(), qt, nullptr, 0, qgs, qg, st);
@@ -2238,42 +2273,48 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
                        c->key_b.as<uint64_t>(), c->val_b.as<uint32_t>(), c->sums.as<QSum>(), (int)(qg != 0),
                        c->starts.as<uint32_t>(), c->shard.as<uint32_t>(), c->row.as<uint32_t>(), c->segnum.as<uint32_t>(), c->seg_begin.as<uint32_t>(),
                        c->ps.as<uint64_t>(), c->emax.as<uint32_t>());
-    launches += qg ? 8 : 4;
+    launches += qg ? 4 : 2;
     uint32_t* Lp = d_small + 8;   // live runs L
     uint32_t* Rp = d_small + 9;   // ranges R
     uint32_t* RRp = d_small + 14;  // ranges swept by ranks
-    // partition points, live runs and ranges.  k_emit takes four tiles a block, one where that would leave
-    // fewer blocks than the SMs hold at once (8 each)
+    // partition points, live runs and ranges
     const dim3 lgrid(grid_for(n, kTileThreads), ns);
     const uint32_t lt = lgrid.x * ns, lg = lt > kMaxLook ? (lt + kGroup - 1) / kGroup : 0u;
     LSum* lsums = c->sums.as<LSum>();
-    LSum* lgs = lg ? lsums + lt : nullptr;
+    LSum* lgs = lg ? lsums + lt + 1 : nullptr;  // (the whole at lsums[lt])
     (void)launch_chain(pdl, k_lohi<true>, k_lohi<false>, lgrid, kTileThreads, 0, st, n, ns, c->starts.as<uint32_t>(),
                        c->val_b.as<uint32_t>(), c->emax.as<uint32_t>(), c->shard.as<uint32_t>(), idx->d_slot,
-                       idx->d_layers, idx->d_pos, idx->d_btab, c->lo.as<uint32_t>(), c->hi.as<uint32_t>(),
-                       c->flags.as<uint32_t>(), lsums);
-    if (lg) scan_groups(lsums, lt, nullptr, 0, lgs, lg, st);
-    const bool wide = lt >= (uint32_t)c->num_sms * 32;
+                       idx->d_layers, idx->d_pos, idx->d_btab, c->lo.as<uint32_t>(), c->cnt.as<uint32_t>(),
+                       c->place.as<uint16_t>(), lsums);
+    if (lg) scan_groups(lsums, lt, nullptr, 0, lgs, lg, st, lsums + lt);
     const int tag = mode.no_sweep ? RUN_SHARD_ROW : rows > 1 ? RUN_ROW : RUN_PLAIN;
-    (void)launch_chain(pdl, wide ? k_emit<4, true> : k_emit<1, true>, wide ? k_emit<4, false> : k_emit<1, false>,
-                       dim3(wide ? (lgrid.x + 3) / 4 : lgrid.x, ns), kTileThreads, 0, st, n, ns, rows, lgrid.x, tag,
-                       c->starts.as<uint32_t>(), c->val_b.as<uint32_t>(), c->emax.as<uint32_t>(),
-                       c->shard.as<uint32_t>(), c->row.as<uint32_t>(), idx->d_slot, idx->d_layers, idx->d_pos,
-                       idx->d_btab, c->lo.as<uint32_t>(), c->hi.as<uint32_t>(), c->flags.as<uint32_t>(), lsums, (int)(lg != 0),
-                       c->psegs.as<PairSeg>(), c->prow.as<uint32_t>(), c->pc.as<uint64_t>(), c->cr.as<uint32_t>(),
-                       c->uhi.as<uint32_t>(), c->rt.as<uint2>(), Lp, Rp);
+    (void)launch_chain(pdl, k_emit<true>, k_emit<false>, grid_for(lt, kTileThreads / 32), kTileThreads, 0, st, n, ns,
+                       rows, lgrid.x, lt, tag, c->starts.as<uint32_t>(), c->val_b.as<uint32_t>(),
+                       c->emax.as<uint32_t>(), c->shard.as<uint32_t>(), c->row.as<uint32_t>(), idx->d_slot,
+                       idx->d_layers, idx->d_pos, idx->d_btab, c->lo.as<uint32_t>(), c->cnt.as<uint32_t>(),
+                       c->place.as<uint16_t>(), lsums, (int)(lg != 0), c->psegs.as<PairSeg>(),
+                       c->prow.as<uint32_t>(), c->pc.as<uint64_t>(), c->cr.as<uint32_t>(), c->uhi.as<uint32_t>(),
+                       c->rt.as<uint2>(), c->rlo.as<uint32_t>(), Lp, Rp);
     // the ranges' unions, methods and places; R is a device count, at most tot
     const unsigned rgrid = (unsigned)std::min<uint64_t>(tot / kRTile + 1, (uint64_t)c->num_sms * 16);
     RSum* rsums = c->sums.as<RSum>();
     const uint32_t rtl = (uint32_t)(tot / kRTile + 1), rg = rtl > kMaxLook ? (rtl + kGroup - 1) / kGroup : 0u;
     RSum* rgs = rg ? rsums + rtl : nullptr;
     (void)launch_chain(pdl, k_range_reduce<true>, k_range_reduce<false>, rgrid, kTileThreads, 0, st, Lp, Rp, n,
-                       c->rt.as<uint2>(), c->pc.as<uint64_t>(), c->uhi.as<uint32_t>(), c->lo.as<uint32_t>(),
-                       c->segnum.as<uint32_t>(), L.pair_ratio, c->ulen.as<uint32_t>(),
+                       c->rt.as<uint2>(), c->pc.as<uint64_t>(), c->uhi.as<uint32_t>(), c->rlo.as<uint32_t>(),
+                       c->segnum.as<uint32_t>(), L.pair_ratio, run_cost, c->ulen.as<uint32_t>(),
                        c->seg_need.as<unsigned long long>(), reinterpret_cast<unsigned long long*>(d_small + 4), rsums);
     launches += lg ? 5 : 3;
     // side stream: rank tables of the query segments that have a rank-difference range
     RGL_TRY(stream_after(sd, st, c->ev_fork));
+    if (late_ends) {
+        k_skip_ends<<<grid_for(in.nblk, 256), 256, 0, sd>>>(in.nblk, soff, c->segnum.as<uint32_t>(),
+                                                            c->seg_need.as<unsigned long long>(),
+                                                            d_unsorted + in.nblk);
+        launches++;
+        sort_ends();
+        sum_ends();
+    }
     k_seg_tabsize<<<grid_for(max_segs, 256), 256, 0, sd>>>(n, c->segnum.as<uint32_t>(), c->seg_begin.as<uint32_t>(),
                                                            c->seg_need.as<unsigned long long>(),
                                                            c->ends.as<uint32_t>(), c->segtab.as<SegTab>());
@@ -2284,8 +2325,9 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     // main stream: the two work spaces
     if (rg) scan_groups(rsums, 0, Rp, kRTile, rgs, rg, st);
     (void)launch_chain(pdl, k_range_apply<true>, k_range_apply<false>, rgrid, kTileThreads, 0, st, Lp, Rp, n, ns, rows,
-                       c->rt.as<uint2>(), c->pc.as<uint64_t>(), c->ulen.as<uint32_t>(), c->lo.as<uint32_t>(),
-                       c->shard.as<uint32_t>(), c->row.as<uint32_t>(), c->segnum.as<uint32_t>(), idx->d_slot, L.pair_ratio, rsums, (int)(rg != 0),
+                       c->rt.as<uint2>(), c->pc.as<uint64_t>(), c->ulen.as<uint32_t>(), c->rlo.as<uint32_t>(),
+                       c->shard.as<uint32_t>(), c->row.as<uint32_t>(), c->segnum.as<uint32_t>(), idx->d_slot, L.pair_ratio, run_cost, rsums,
+                       (int)(rg != 0),
                        c->ranges.as<RangeDesc>(), c->rpos.as<uint64_t>(), c->rpair.as<uint64_t>(),
                        c->ppos.as<uint64_t>(), RRp, reinterpret_cast<unsigned long long*>(d_small + 10));
     const unsigned gc = (unsigned)std::min<uint64_t>(grid_for(tot, 256), (uint64_t)c->num_sms * 32);
@@ -2822,7 +2864,7 @@ int rgl_context_destroy(rgl_context* c) {
     if (c->side) cudaStreamSynchronize(c->side);
     DevBuf* bufs[] = {&c->iv, &c->blk_off, &c->blk_shard, &c->key_a, &c->key_b, &c->val_a, &c->val_b,
                       &c->ekey_a, &c->ekey_b, &c->starts, &c->ends, &c->shard, &c->row, &c->segnum, &c->seg_begin, &c->ps,
-                      &c->pe, &c->emax, &c->lo, &c->hi, &c->flags, &c->ranges, &c->rpos, &c->cub_tmp, &c->small,
+                      &c->pe, &c->emax, &c->lo, &c->cnt, &c->place, &c->rlo, &c->ranges, &c->rpos, &c->cub_tmp, &c->small,
                       &c->out_counts, &c->out_bp, &c->item_r0, &c->segtab, &c->tab2, &c->pc, &c->cr, &c->uhi, &c->rt,
                       &c->ulen, &c->rpair, &c->sums, &c->esums, &c->ppos, &c->psegs, &c->prow, &c->item_t0, &c->seg_need,
                       &c->item_hits, &c->item_base, &c->pairs, &c->bt_off, &c->bt_shard, &c->acc, &c->gc.t_off,

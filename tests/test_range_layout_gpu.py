@@ -65,3 +65,28 @@ def test_runs_of_more_than_2_to_27_candidates():
     by_pair, bp2, st = ctx.query_counts({0: q}, 1, pair_ratio=1_000_000)
     assert (by_rank == by_pair).all() and (bp == bp2).all()
     assert st["pair_candidates"] > 30 * sum(sizes[:2]) // 2
+
+
+@pytest.mark.parametrize("order", ["by start", "shuffled"])
+def test_ends_sorted_only_where_a_rank_sweep_needs_them(order):
+    # a run beyond 2^21 queries: shard 0 has ranges that are swept by ranks, shard 1 has none, shard 2 few queries
+    rng = np.random.default_rng(8)
+    m = 30_000
+    wide = rng.integers(0, 2_000_000, m)
+    narrow = rng.integers(0, 200_000_000, m)
+    db = [(0, np.stack([wide, wide + rng.integers(40_000, 100_000, m), rng.integers(0, 5, m)], 1).astype(np.uint32)),
+          (1, np.stack([narrow, narrow + rng.integers(1, 500, m), rng.integers(0, 5, m)], 1).astype(np.uint32)),
+          (2, np.stack([wide, wide + rng.integers(1, 100_000, m), rng.integers(0, 5, m)], 1).astype(np.uint32))]
+    layers = rg.bucket_layers(db)
+    q = {}
+    for sh, n, span in ((0, 3_000, 2_000_000), (1, 2_150_000, 200_000_000), (2, 40, 2_000_000)):
+        s = rng.integers(0, span, n)
+        s = np.sort(s) if order == "by start" else s
+        q[sh] = np.stack([s, s + rng.integers(1, 900, n), np.zeros(n)], 1).astype(np.uint32)
+    oc, _, obp, _ = O.query_database(layers, q, 1, 5, threads=8)
+    idx = rg.Index.from_layers(layers, 5, ["a", "b", "c"])
+    ctx = rg.Context(idx)
+    for ratio in (0, 1, 1_000_000):
+        c, bp, st = ctx.query_counts(q, 1, pair_ratio=ratio)
+        assert (c == oc).all() and (bp == obp).all()
+        assert (st["rank_positions"] > 0) == (ratio < 2)
