@@ -144,6 +144,15 @@ int index_finalize(rgl_index* idx) {
                             cudaMemcpyHostToDevice));
     if (!idx->slot.empty())
         RGL_CUDA(cudaMemcpy(idx->d_slot, idx->slot.data(), idx->slot.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    std::vector<LayerQuery> lq(ns, LayerQuery{0, 0, 0, 0, 0, 0});
+    for (size_t k = 0; k < idx->slot.size(); k++)
+        if (idx->slot[k] >= 0) {
+            const LayerDev& l = idx->layers[idx->slot[k]];
+            lq[k] = LayerQuery{l.off, l.boff, (uint32_t)l.n, l.max_size, l.bshift, l.nb};
+        }
+    RGL_CUDA(cudaMalloc(&idx->d_lq, ns * sizeof(LayerQuery)));
+    RGL_CUDA(cudaMemcpy(idx->d_lq, lq.data(), ns * sizeof(LayerQuery), cudaMemcpyHostToDevice));
+    idx->device_bytes += ns * sizeof(LayerQuery);
     return RGL_OK;
 }
 
@@ -163,6 +172,8 @@ void index_free(rgl_index* idx) {
     if (idx->d_btab) cudaFree(idx->d_btab);
     idx->d_btab = nullptr;
     if (idx->d_slot) cudaFree(idx->d_slot);
+    if (idx->d_lq) cudaFree(idx->d_lq);
+    idx->d_lq = nullptr;
     idx->d_pos = nullptr;
     idx->d_sid = nullptr;
     idx->d_layers = nullptr;

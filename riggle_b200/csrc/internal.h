@@ -67,6 +67,11 @@ struct LayerDev {
     uint64_t boff;
     uint32_t bshift, nb;
 };
+// What the partition search reads of a layer, by [shard * num_slots + K] (nb = 0: no such layer).
+struct __attribute__((aligned(16))) LayerQuery {
+    uint64_t off, boff;
+    uint32_t n, max_size, bshift, nb;
+};
 enum : uint32_t { LF_UNSORTED = 1u, LF_BAD_SID = 2u, LF_EMPTY_IV = 4u, LF_OVERSIZE = 8u };
 
 // A device allocation that grows on demand (never shrinks).
@@ -104,6 +109,7 @@ struct rgl_index {
     rgl::LayerDev* d_layers = nullptr;
     uint32_t* d_btab = nullptr;         // bucket tables of all layers
     int32_t* d_slot = nullptr;
+    rgl::LayerQuery* d_lq = nullptr;
     uint64_t device_bytes = 0;
     // one reference for the handle returned to the caller plus one per live context; the device
     // memory is released when the last reference goes (rgl_index_close may precede the contexts)

@@ -49,11 +49,18 @@ struct RangeDesc {
     uint32_t seg;        // query segment number
 };
 
-// One query's candidate run for the pair sweep: DB elements from `base` (of the index arrays) on.
+// One query's candidate run for the pair sweep: DB elements from `base` (of the index arrays) on; in the
+// several-row sweep the query's row lies above the element (2^36 elements of 12 bytes are 824 GB).
 struct __align__(16) PairSeg {
     uint64_t base;
     uint32_t qs, qe;
 };
+constexpr int kRunRowShift = 36;
+constexpr uint32_t kMaxPackedRows = 1u << (64 - kRunRowShift);
+template <int MULTI>
+__device__ __forceinline__ uint64_t run_base(uint64_t b) {
+    return MULTI ? b & ((1ull << kRunRowShift) - 1) : b;
+}
 
 // Rank table of one query segment: bin b (width 2^shift bp) holds, at tab2[off + b], the numbers
 // of the segment's sorted starts and ends below b << shift, as absolute positions in the sorted
@@ -90,10 +97,10 @@ __device__ __forceinline__ uint32_t ub_u32(const uint32_t* __restrict__ a, uint3
 // run in lockstep (both bucket reads issued together, then one probe of each bisection per round),
 // so their chains of dependent random reads overlap instead of following one another.
 __device__ __forceinline__ void pp_layer2(const uint2* __restrict__ pos, const uint32_t* __restrict__ btab,
-                                          const LayerDev& L, uint32_t x0, uint32_t x1, uint32_t& r0, uint32_t& r1) {
+                                          const LayerQuery& L, uint32_t x0, uint32_t x1, uint32_t& r0, uint32_t& r1) {
     const uint32_t last = L.nb - 1;
     const uint32_t b0 = x0 >> L.bshift, b1 = x1 >> L.bshift;
-    uint32_t lo0 = (uint32_t)L.n, hi0 = (uint32_t)L.n, lo1 = (uint32_t)L.n, hi1 = (uint32_t)L.n;
+    uint32_t lo0 = L.n, hi0 = L.n, lo1 = L.n, hi1 = L.n;
     if (b0 < last) {
         lo0 = __ldg(btab + b0);
         hi0 = __ldg(btab + b0 + 1);
@@ -651,9 +658,9 @@ __device__ __forceinline__ uint64_t warp_count(uint32_t cnt) {
 template <bool PDL>
 __global__ void __launch_bounds__(kTileThreads) k_lohi(
     uint32_t n, uint32_t nslots, const uint32_t* __restrict__ starts, const uint32_t* __restrict__ qend,
-    const uint32_t* __restrict__ emax, const uint32_t* __restrict__ shard, const int32_t* __restrict__ slot,
-    const LayerDev* __restrict__ layers, const uint2* __restrict__ pos, const uint32_t* __restrict__ btab,
-    uint32_t* __restrict__ lo_out, uint32_t* __restrict__ cnt_out, uint16_t* __restrict__ place,
+    const uint32_t* __restrict__ emax, const uint32_t* __restrict__ shard, const LayerQuery* __restrict__ layers,
+    const uint2* __restrict__ pos, const uint32_t* __restrict__ btab, uint32_t* __restrict__ lo_out,
+    uint32_t* __restrict__ cnt_out, uint16_t* __restrict__ place,
     LSum* __restrict__ sums) {
     if constexpr (PDL) {
         pdl_wait();
@@ -666,9 +673,8 @@ __global__ void __launch_bounds__(kTileThreads) k_lohi(
     uint32_t lo = 0, hi = 0;
     bool start = false;
     if (i < n) {
-        const int32_t li = slot[(uint64_t)shard[i] * nslots + K];
-        if (li >= 0) {
-            const LayerDev L = layers[li];
+        const LayerQuery L = layers[(uint64_t)shard[i] * nslots + K];
+        if (L.nb) {
             const uint2* p = pos + L.off;
             const uint32_t st = starts[i], en = qend[i], E = emax[i];
             const uint32_t back = st >= L.max_size ? st - L.max_size : 0u;  // saturating_sub, src/sweep/query.rs:98
@@ -702,9 +708,9 @@ __global__ void __launch_bounds__(kTileThreads) k_lohi(
 // Range r: rt[r] = (its first live run, that run's entry K n + i).  The last block writes the totals: L, R
 // and pc[L].
 __device__ __forceinline__ uint32_t pp_layer(const uint2* __restrict__ pos, const uint32_t* __restrict__ btab,
-                                             const LayerDev& L, uint32_t x) {
+                                             const LayerQuery& L, uint32_t x) {
     const uint32_t b = x >> L.bshift;
-    if (b >= L.nb - 1) return (uint32_t)L.n;
+    if (b >= L.nb - 1) return L.n;
     uint32_t lo = __ldg(btab + b), hi = __ldg(btab + b + 1);
     while (lo < hi) {
         const uint32_t m = lo + ((hi - lo) >> 1);
@@ -733,18 +739,19 @@ __device__ __forceinline__ uint64_t warp_inclusive(uint32_t cnt, uint32_t lane) 
     return inc;
 }
 
-// What the runs carry beside their queries: nothing, the row (several-row sweeps), or shard and row
-// (shard * rows + row; the pair list).
-enum : int { RUN_PLAIN = 0, RUN_ROW = 1, RUN_SHARD_ROW = 2 };
+// What the runs carry beside their queries: nothing; the row, in the top bits of `base` (the several-row
+// pair sweep, which reads it with the rest) or on its own (several rows tallied straight into the outputs);
+// or shard and row (shard * rows + row; the pair list).
+enum : int { RUN_PLAIN = 0, RUN_ROW = 1, RUN_SHARD_ROW = 2, RUN_PACKED = 3 };
 
 // A warp takes one of k_lohi's tiles (per_slot of them a slot), 32 live entries at a time.
 template <bool PDL>
 __global__ void __launch_bounds__(kTileThreads) k_emit(
     uint32_t n, uint32_t nslots, uint32_t rows, uint32_t per_slot, uint32_t tiles, int tag,
     const uint32_t* __restrict__ starts, const uint32_t* __restrict__ qend, const uint32_t* __restrict__ emax,
-    const uint32_t* __restrict__ shard, const uint32_t* __restrict__ row, const int32_t* __restrict__ slot,
-    const LayerDev* __restrict__ layers, const uint2* __restrict__ pos, const uint32_t* __restrict__ btab,
-    const uint32_t* __restrict__ lo_in, const uint32_t* __restrict__ cnt_in, const uint16_t* __restrict__ place,
+    const uint32_t* __restrict__ shard, const uint32_t* __restrict__ row, const LayerQuery* __restrict__ layers,
+    const uint2* __restrict__ pos, const uint32_t* __restrict__ btab, const uint32_t* __restrict__ lo_in,
+    const uint32_t* __restrict__ cnt_in, const uint16_t* __restrict__ place,
     const LSum* __restrict__ sums, int scanned, PairSeg* __restrict__ psegs, uint32_t* __restrict__ prow,
     uint64_t* __restrict__ pc, uint32_t* __restrict__ cr, uint32_t* __restrict__ uhi, uint2* __restrict__ rt,
     uint32_t* __restrict__ rlo, uint32_t* __restrict__ Lp, uint32_t* __restrict__ Rp) {
@@ -783,9 +790,10 @@ __global__ void __launch_bounds__(kTileThreads) k_emit(
         const uint64_t inc = warp_inclusive(cnt, lane);
         if (in) {
             const uint32_t c = at.live + j;
-            const int32_t li = slot[(uint64_t)sh * nslots + K];
-            psegs[c] = PairSeg{layers[li].off + lo, qs, qe};
-            if (tag) prow[c] = (rows > 1 ? row[i] : 0u) + (tag == RUN_SHARD_ROW ? sh * rows : 0u);
+            const LayerQuery* L = layers + ((uint64_t)sh * nslots + K);
+            const uint64_t first = L->off + lo;
+            psegs[c] = PairSeg{tag == RUN_PACKED ? first | (uint64_t)row[i] << kRunRowShift : first, qs, qe};
+            if (tag == RUN_ROW || tag == RUN_SHARD_ROW) prow[c] = (rows > 1 ? row[i] : 0u) + (tag == RUN_SHARD_ROW ? sh * rows : 0u);
             pc[c] = at.cand + inc - cnt;
             const uint32_t r = at.ranges + __popc(fl & ((2u << lane) - 1u)) - 1;  // the range it starts or continues
             cr[c] = r;
@@ -797,8 +805,8 @@ __global__ void __launch_bounds__(kTileThreads) k_emit(
             if (lane == 31 || j + 1 == live || (fl >> (lane + 1) & 1u)) {
                 uint32_t end = lo + cnt;
                 if (E > qe) {  // an earlier query reaches further
-                    const LayerDev Ld = layers[li];
-                    end = pp_layer(pos + Ld.off, btab + Ld.boff, Ld, E);
+                    const LayerQuery Lq = *L;
+                    end = pp_layer(pos + Lq.off, btab + Lq.boff, Lq, E);
                 }
                 uhi[c] = end;
             }
@@ -1020,7 +1028,7 @@ struct SweepParams {
     const uint32_t* item_r0; // first range of each work item (items < item_cap)
     const uint64_t* ppos;    // pair work space: exclusive scan of candidate runs, L + 1 entries
     const PairSeg* psegs;
-    const uint32_t* prow;    // rows of the runs (several-row sweeps)
+    const uint32_t* prow;    // rows of the runs (several rows, no histogram)
     const uint32_t* item_t0; // first run of each pair work item
     const SegTab* segtabs;   // per query segment
     const uint2* tab2;       // rank tables, bin b = (#starts, #ends) below b << shift
@@ -1222,7 +1230,7 @@ __device__ __forceinline__ uint32_t cta_item_row(const SweepParams& P, uint32_t 
         while (lo < hi) { uint64_t m = (lo + hi + 1) >> 1; if (__ldg(off + m) <= p) lo = m; else hi = m - 1; }
         r = (uint32_t)lo;
     }
-    return RANK ? P.ranges[r].qrow : __ldg(P.prow + r);
+    return RANK ? P.ranges[r].qrow : (uint32_t)(__ldg(&P.psegs[r].base) >> kRunRowShift);
 }
 
 // The outer loop of the several-row sweeps.  Blocks pull block items (kCtaItems warp items) from the
@@ -1482,11 +1490,12 @@ __device__ __noinline__ void pairs_step_dense(const uint64_t* __restrict__ ppos,
             if (o <= span) {
                 const uint32_t run = t + cntr[o];
                 const uint4 w = __ldg(reinterpret_cast<const uint4*>(psegs + run));
-                const uint64_t di = (((uint64_t)w.y << 32) | w.x) + (pb + o - __ldg(ppos + run));
+                const uint64_t di = run_base<MULTI>(((uint64_t)w.y << 32) | w.x) + (pb + o - __ldg(ppos + run));
                 q[j] = make_uint2(w.z, w.w);
                 d[j] = __ldg(pos + di);
                 sid[j] = __ldg(sidv + di);
-                if ((!SMEM || MULTI) && prow) row[j] = __ldg(prow + run);
+                if (MULTI) row[j] = w.y >> (kRunRowShift - 32);
+                else if (!SMEM && prow) row[j] = __ldg(prow + run);
             }
         }
 #pragma unroll
@@ -1528,8 +1537,12 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t chunk,
     }
     uint64_t rlo = __ldg(P.ppos + t), rhi = __ldg(P.ppos + t + 1);
     PairSeg ps = P.psegs[t];
-    const bool rowed = (!SMEM || MULTI) && P.rows > 1;
-    uint32_t prow = rowed ? __ldg(P.prow + t) : 0u;
+    // the row of run t: packed in its base (MULTI), or beside it where the tally goes straight to several rows
+    const bool rowed = !SMEM && P.rows > 1;
+    auto row_of = [&](uint32_t run, uint64_t b) -> uint32_t {
+        return MULTI ? (uint32_t)(b >> kRunRowShift) : rowed ? __ldg(P.prow + run) : 0u;
+    };
+    uint32_t prow = row_of(t, ps.base);
     for (uint64_t pb = p0; pb < p1; pb += 32 * kPairUnroll) {
         const uint64_t pend = min(pb + 32 * kPairUnroll, p1) - 1;
         const uint32_t span = (uint32_t)(pend - pb);
@@ -1538,9 +1551,9 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t chunk,
             rlo = __ldg(P.ppos + t);
             rhi = __ldg(P.ppos + t + 1);
             ps = P.psegs[t];
-            if (rowed) prow = __ldg(P.prow + t);
+            prow = row_of(t, ps.base);
         }
-        const uint64_t base0 = ps.base - rlo + pb;  // element of offset 0 when it lies in run t
+        const uint64_t base0 = run_base<MULTI>(ps.base) - rlo + pb;  // element of offset 0 when it lies in run t
         if (pend < rhi) {
             uint2 d[kPairUnroll];
             uint32_t sid[kPairUnroll];
@@ -1586,7 +1599,7 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t chunk,
             const uint32_t o = lane + 32 * j;
             const uint32_t rb = __shfl_sync(0xffffffffu, rel, k[j] ? k[j] - 1 : 0);
             if (o <= span) {
-                const uint64_t di = k[j] ? __ldg(&P.psegs[t + k[j]].base) + (o - rb) : base0 + o;
+                const uint64_t di = k[j] ? run_base<MULTI>(__ldg(&P.psegs[t + k[j]].base)) + (o - rb) : base0 + o;
                 d[j] = __ldg(P.pos + di);
                 sid[j] = __ldg(P.sid + di);
             } else {
@@ -1597,8 +1610,11 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t chunk,
 #pragma unroll
         for (uint32_t j = 0; j < kPairUnroll; j++) {
             const PairSeg* q = P.psegs + t + k[j];
-            pair_tally<WITH_BP, SMEM, MULTI>(P.counts, P.bp, P.D, __ldg(&q->qs), __ldg(&q->qe), rowed ? __ldg(P.prow + t + k[j]) : 0u,
-                                             d[j], sid[j], s_cnt, s_bp, cta_row);
+            const uint2 qse = __ldg(reinterpret_cast<const uint2*>(&q->qs));
+            const uint32_t qrow = MULTI ? __ldg(reinterpret_cast<const uint32_t*>(q) + 1) >> (kRunRowShift - 32)
+                                        : rowed ? __ldg(P.prow + t + k[j]) : 0u;
+            pair_tally<WITH_BP, SMEM, MULTI>(P.counts, P.bp, P.D, qse.x, qse.y, qrow, d[j], sid[j], s_cnt, s_bp,
+                                             cta_row);
         }
         // the run of the next step's first position pend + 1, from the boundaries in hand (at
         // least one boundary, ppos[t + 1] <= pend, lies at or below it)
@@ -1608,7 +1624,7 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t chunk,
             rlo = __ldg(P.ppos + t);
             rhi = __ldg(P.ppos + t + 1);
             ps = P.psegs[t];
-            if (rowed) prow = __ldg(P.prow + t);
+            prow = row_of(t, ps.base);
         }
     }
 }
@@ -2176,6 +2192,12 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
         return fail(RGL_ERR_INVALID_ARGUMENT, "num_shards x regions x num_rows must be < 2^32");
     const uint32_t sps = (uint32_t)(nreg * rows);  // segments per shard
 
+    // tally: one row in a block-wide histogram for the whole kernel (1); several rows in a histogram
+    // of each block item's row (2); else (or with RGL_QF_GLOBAL_TALLY) atomics on the outputs (0)
+    size_t smem = (size_t)D * (with_bp ? 12 : 4);
+    const int tally = smem > 160 * 1024 ? 0 : rows == 1 ? 1
+                      : (opts && (opts->flags & RGL_QF_GLOBAL_TALLY)) || rows > kMaxPackedRows ? 0 : 2;
+
     if (ev) RGL_CUDA(cudaEventRecord(c->ev[0], st));
     // Two streams: `st` carries the chain from the sorted starts to the sweeps, `sd` the chains that
     // only the rank sweep needs (the end-key sort and unpack, the prefix sums of starts and ends,
@@ -2283,16 +2305,15 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     LSum* lsums = c->sums.as<LSum>();
     LSum* lgs = lg ? lsums + lt + 1 : nullptr;  // (the whole at lsums[lt])
     (void)launch_chain(pdl, k_lohi<true>, k_lohi<false>, lgrid, kTileThreads, 0, st, n, ns, c->starts.as<uint32_t>(),
-                       c->val_b.as<uint32_t>(), c->emax.as<uint32_t>(), c->shard.as<uint32_t>(), idx->d_slot,
-                       idx->d_layers, idx->d_pos, idx->d_btab, c->lo.as<uint32_t>(), c->cnt.as<uint32_t>(),
+                       c->val_b.as<uint32_t>(), c->emax.as<uint32_t>(), c->shard.as<uint32_t>(), idx->d_lq,
+                       idx->d_pos, idx->d_btab, c->lo.as<uint32_t>(), c->cnt.as<uint32_t>(),
                        c->place.as<uint16_t>(), lsums);
     if (lg) scan_groups(lsums, lt, nullptr, 0, lgs, lg, st, lsums + lt);
-    const int tag = mode.no_sweep ? RUN_SHARD_ROW : rows > 1 ? RUN_ROW : RUN_PLAIN;
+    const int tag = mode.no_sweep ? RUN_SHARD_ROW : tally == 2 ? RUN_PACKED : rows > 1 ? RUN_ROW : RUN_PLAIN;
     (void)launch_chain(pdl, k_emit<true>, k_emit<false>, grid_for(lt, kTileThreads / 32), kTileThreads, 0, st, n, ns,
                        rows, lgrid.x, lt, tag, c->starts.as<uint32_t>(), c->val_b.as<uint32_t>(),
-                       c->emax.as<uint32_t>(), c->shard.as<uint32_t>(), c->row.as<uint32_t>(), idx->d_slot,
-                       idx->d_layers, idx->d_pos, idx->d_btab, c->lo.as<uint32_t>(), c->cnt.as<uint32_t>(),
-                       c->place.as<uint16_t>(), lsums, (int)(lg != 0), c->psegs.as<PairSeg>(),
+                       c->emax.as<uint32_t>(), c->shard.as<uint32_t>(), c->row.as<uint32_t>(), idx->d_lq,
+                       idx->d_pos, idx->d_btab, c->lo.as<uint32_t>(), c->cnt.as<uint32_t>(), c->place.as<uint16_t>(), lsums, (int)(lg != 0), c->psegs.as<PairSeg>(),
                        c->prow.as<uint32_t>(), c->pc.as<uint64_t>(), c->cr.as<uint32_t>(), c->uhi.as<uint32_t>(),
                        c->rt.as<uint2>(), c->rlo.as<uint32_t>(), Lp, Rp);
     // the ranges' unions, methods and places; R is a device count, at most tot
@@ -2375,12 +2396,8 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     P.spread = L.spread;
     c->last_chunk = L.chunk;
     c->last_spread = L.spread;
-    size_t smem = (size_t)D * (with_bp ? 12 : 4);
-    // tally: one row in a block-wide histogram for the whole kernel (1); several rows in a histogram
-    // of each block item's row (2); else (or with RGL_QF_GLOBAL_TALLY) atomics on the outputs (0)
-    P.smem_tally = smem > 160 * 1024 ? 0 : rows == 1 ? 1 : (opts && (opts->flags & RGL_QF_GLOBAL_TALLY)) ? 0 : 2;
-
-    if (!P.smem_tally) smem = 0;
+    P.smem_tally = tally;
+    if (!tally) smem = 0;
     unsigned grid = (unsigned)(c->num_sms * L.ctas_per_sm);
     // the rank tables are joined before the sweeps; the two sweeps run one after the other on
     // `st` (each fills every SM with persistent blocks; run side by side they were slower)
