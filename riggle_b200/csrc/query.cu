@@ -1242,20 +1242,19 @@ __device__ __forceinline__ uint32_t cta_item_row(const SweepParams& P, uint32_t 
 template <bool RANK, typename ItemFn, typename FlushFn>
 __device__ __forceinline__ void multi_row_loop(const SweepParams& P, uint32_t chunk, uint64_t items, uint32_t rcap,
                                                ItemFn item_fn, FlushFn flush_fn) {
-    __shared__ uint32_t s_ctl[2];
+    __shared__ uint32_t s_ctl[2][2];  // (item, row) of this turn and of the next
     constexpr uint32_t kNone = 0xFFFFFFFFu;
     uint32_t cur = kNone;  // the row the histogram holds (block-uniform)
-    for (;;) {
-        if (threadIdx.x == 0) {
-            const uint32_t ci = atomicAdd(P.queue, 1u);
-            s_ctl[0] = ci;
-            if ((uint64_t)ci * kCtaItems < items) s_ctl[1] = cta_item_row<RANK>(P, chunk, ci, items, rcap);
-        }
-        __syncthreads();
-        const uint64_t ci = s_ctl[0];
-        const uint32_t row = s_ctl[1];
-        __syncthreads();  // every thread has read s_ctl
+    auto publish = [&](uint32_t turn, uint32_t ci) {
+        s_ctl[turn][0] = ci;
+        if ((uint64_t)ci * kCtaItems < items) s_ctl[turn][1] = cta_item_row<RANK>(P, chunk, ci, items, rcap);
+    };
+    if (threadIdx.x == 0) publish(0, atomicAdd(P.queue, 1u));
+    __syncthreads();
+    for (uint32_t turn = 0;; turn ^= 1) {
+        const uint64_t ci = s_ctl[turn][0];
         if (ci * kCtaItems >= items) break;
+        const uint32_t row = s_ctl[turn][1];
         if (row != cur) {
             if (cur != kNone) {
                 flush_fn(cur);
@@ -1263,8 +1262,11 @@ __device__ __forceinline__ void multi_row_loop(const SweepParams& P, uint32_t ch
             }
             cur = row;
         }
+        uint32_t next = 0;
+        if (threadIdx.x == 0) next = atomicAdd(P.queue, 1u);  // arrives while the item is walked
         const uint64_t item = ci * kCtaItems + (threadIdx.x >> 5);
         if (item < items) item_fn((uint32_t)item, cur);
+        if (threadIdx.x == 0) publish(turn ^ 1, next);  // read by all before this turn: one barrier ago
         __syncthreads();  // the item is done before the histogram may be flushed
     }
     if (cur != kNone) flush_fn(cur);
@@ -1436,12 +1438,11 @@ __device__ __forceinline__ void pair_tally(uint32_t* counts, unsigned long long*
 // own) and the counts summed along the step, which gives every position's run; its descriptor, element and
 // tally follow with all four positions of a lane in flight.  A stretch of more than kDenseGroups x 32
 // boundaries (empty runs of ranges swept by ranks) is searched position by position instead.
-// Kept out of line: inlined its registers would count against the whole kernel.
 // Files of 1e6 intervals against 3.2e6 have about two candidates a run: 52e9 candidates/s with a search per
 // position, 1.3e11 so.
 constexpr int kDenseGroups = 16;
 template <bool WITH_BP, bool SMEM, int MULTI>
-__device__ __noinline__ void pairs_step_dense(const uint64_t* __restrict__ ppos, const PairSeg* __restrict__ psegs,
+__device__ __forceinline__ void pairs_step_dense(const uint64_t* __restrict__ ppos, const PairSeg* __restrict__ psegs,
                                               const uint32_t* __restrict__ prow, const uint2* __restrict__ pos,
                                               const uint32_t* __restrict__ sidv, uint32_t* counts,
                                               unsigned long long* bp, uint32_t D, uint32_t t, uint32_t rcap,
@@ -1476,7 +1477,7 @@ __device__ __noinline__ void pairs_step_dense(const uint64_t* __restrict__ ppos,
         for (uint32_t o = lane; o <= span; o += 32) cntr[o] = range_advance(ppos, t, rcap, pb + o) - t;
     }
     __syncwarp();
-    constexpr uint32_t U = MULTI ? kPairUnroll : kPairUnroll / 2;  // the one-row sweep has 32 registers a thread
+    constexpr uint32_t U = kPairUnroll / 2;  // four at once need more registers than the sweep has
 #pragma unroll 1
     for (uint32_t o0 = lane; o0 <= span; o0 += 32 * U) {
         uint2 d[U], q[U];
@@ -1505,20 +1506,38 @@ __device__ __noinline__ void pairs_step_dense(const uint64_t* __restrict__ ppos,
     __syncwarp();  // cntr is reused by the next step
 }
 
+// The same as a call.  Inlined into the one-row sweep, which has 32 registers a thread, it spills; a call in
+// the several-row sweep (40) leaves 16 registers for all that lives across it, and that spilled 148 bytes a
+// thread into the loop: 48 files against 2e8 intervals 4,201 us so, 3,638 inlined.
+template <bool WITH_BP, bool SMEM>
+__device__ __noinline__ void pairs_step_dense_call(const uint64_t* __restrict__ ppos, const PairSeg* __restrict__ psegs,
+                                                   const uint32_t* __restrict__ prow, const uint2* __restrict__ pos,
+                                                   const uint32_t* __restrict__ sidv, uint32_t* counts,
+                                                   unsigned long long* bp, uint32_t D, uint32_t t, uint32_t rcap,
+                                                   uint64_t pb, uint32_t span, uint32_t lane, uint32_t* cntr,
+                                                   uint32_t* s_cnt, unsigned long long* s_bp) {
+    pairs_step_dense<WITH_BP, SMEM, 0>(ppos, psegs, prow, pos, sidv, counts, bp, D, t, rcap, pb, span, lane, cntr, s_cnt,
+                                       s_bp, 0u);
+}
+
 // The pair sweep: the reference's scan (src/sweep/query.rs:104-115) over the candidate runs of the
 // queries of pair ranges, every candidate read once by one lane (consecutive positions of a run are
 // consecutive DB elements, so the loads coalesce).  A candidate d of query q overlaps when
 // d.end > q.start (d.start < q.end and the look-back bound hold by construction of the run); it
 // adds 1 and min(ends) - max(starts).
 //
-// A warp takes work items of `chunk` positions from the queue and walks each in steps of the
-// 32 * kPairUnroll consecutive positions [pb, pend], lane l taking pb + l + 32 j.  The warp keeps
-// the run t of the step's first position (uniform), so the choice between the forms below never
-// splits the warp.  When the step lies in run t, every lane requests all its DB intervals and sids
-// before using any.  When it spans several runs (about a quarter of the steps at hundreds of
-// candidates per run), lane l holds the boundary ppos[t + 1 + l] of the following runs: a
-// position's run is t plus the number of boundaries at or below it, counted over the few
-// boundaries inside the step, and the run descriptors come from L1.
+// A warp takes work items of `chunk` positions from the queue and walks each in steps of 32 *
+// kPairUnroll consecutive positions, lane l taking l + 32 j, in 32-bit offsets from the item's first.
+// The warp keeps the run t of the step's first position (uniform), so the choice between the forms
+// below never splits the warp.  When the step lies in run t, every lane requests all its DB intervals
+// and sids before using any.  When it spans several runs (most steps, at the seventy candidates a run
+// of whole-genome files), lane l holds the boundary ppos[t + 1 + l] of the following runs: a position's
+// run is t plus the number of boundaries at or below it, counted over the few boundaries inside the
+// step, and the run descriptors come from L1.
+// Bound: L1 wavefronts (70% of its cycles: 12 bytes and two shared-memory atomics a candidate) and
+// issue (65%).  64-bit offsets, one register a count and three loads a descriptor spilled in the
+// several-row form: 1.04e9 candidates of 48 files against 2e8 intervals 4,201 us, 3,638 as it is; five
+// blocks an SM instead of six, to hold the rest of the registers, 3,826.
 // One work item of the pair sweep (positions [item * chunk, (item + 1) * chunk) of the concatenated
 // candidate runs), walked by one warp.
 template <bool WITH_BP, bool SMEM, int MULTI>
@@ -1526,7 +1545,7 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t chunk,
                                            uint64_t total, uint32_t* cntr, uint32_t* s_cnt,
                                            unsigned long long* s_bp, uint32_t cta_row) {
     const uint64_t p0 = (uint64_t)item * chunk;
-    const uint64_t p1 = min(p0 + chunk, total);
+    const uint32_t len = (uint32_t)min((uint64_t)chunk, total - p0);
     uint32_t t;
     if (item < P.item_cap) {
         t = __ldg(P.item_t0 + item);
@@ -1535,96 +1554,94 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t chunk,
         while (lo < hi) { uint64_t m = (lo + hi + 1) >> 1; if (__ldg(P.ppos + m) <= p0) lo = m; else hi = m - 1; }
         t = (uint32_t)lo;
     }
-    uint64_t rlo = __ldg(P.ppos + t), rhi = __ldg(P.ppos + t + 1);
-    PairSeg ps = P.psegs[t];
-    // the row of run t: packed in its base (MULTI), or beside it where the tally goes straight to several rows
+    // the row of a run: packed in its base (MULTI), or beside it where the tally goes straight to several rows
     const bool rowed = !SMEM && P.rows > 1;
-    auto row_of = [&](uint32_t run, uint64_t b) -> uint32_t {
-        return MULTI ? (uint32_t)(b >> kRunRowShift) : rowed ? __ldg(P.prow + run) : 0u;
+    // run t: its candidates are the elements base + (offset in the item), up to offset rhi
+    uint64_t base;
+    uint32_t rhi, qs, qe, prow;
+    auto load_run = [&]() {
+        const uint64_t lo = __ldg(P.ppos + t), hi = __ldg(P.ppos + t + 1);
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(P.psegs + t));
+        base = run_base<MULTI>(((uint64_t)w.y << 32) | w.x) - lo + p0;
+        rhi = (uint32_t)min(hi - p0, (uint64_t)0xffffffffu);
+        qs = w.z;
+        qe = w.w;
+        prow = MULTI ? w.y >> (kRunRowShift - 32) : rowed ? __ldg(P.prow + t) : 0u;
     };
-    uint32_t prow = row_of(t, ps.base);
-    for (uint64_t pb = p0; pb < p1; pb += 32 * kPairUnroll) {
-        const uint64_t pend = min(pb + 32 * kPairUnroll, p1) - 1;
-        const uint32_t span = (uint32_t)(pend - pb);
-        if (pb >= rhi) {
-            t = range_advance(P.ppos, t, rcap, pb);
-            rlo = __ldg(P.ppos + t);
-            rhi = __ldg(P.ppos + t + 1);
-            ps = P.psegs[t];
-            prow = row_of(t, ps.base);
+    load_run();
+    for (uint32_t ob = 0; ob < len; ob = len - ob > 32 * kPairUnroll ? ob + 32 * kPairUnroll : len) {
+        const uint32_t span = min(32 * kPairUnroll, len - ob) - 1;
+        if (ob >= rhi) {
+            t = range_advance(P.ppos, t, rcap, p0 + ob);
+            load_run();
         }
-        const uint64_t base0 = run_base<MULTI>(ps.base) - rlo + pb;  // element of offset 0 when it lies in run t
-        if (pend < rhi) {
+        if (ob + span < rhi) {
+            const uint2* pos = P.pos + (base + ob);
+            const uint32_t* sidv = P.sid + (base + ob);
             uint2 d[kPairUnroll];
             uint32_t sid[kPairUnroll];
 #pragma unroll
             for (uint32_t j = 0; j < kPairUnroll; j++) {
                 const uint32_t o = lane + 32 * j;
+                d[j] = make_uint2(0, 0);  // never a hit: d.y = 0 <= qs
+                sid[j] = 0;
                 if (o <= span) {
-                    d[j] = __ldg(P.pos + base0 + o);
-                    sid[j] = __ldg(P.sid + base0 + o);
-                } else {
-                    d[j] = make_uint2(0, 0);  // never a hit: d.y = 0 <= qs
-                    sid[j] = 0;
+                    d[j] = __ldg(pos + o);
+                    sid[j] = __ldg(sidv + o);
                 }
             }
 #pragma unroll
             for (uint32_t j = 0; j < kPairUnroll; j++)
-                pair_tally<WITH_BP, SMEM, MULTI>(P.counts, P.bp, P.D, ps.qs, ps.qe, prow, d[j], sid[j], s_cnt, s_bp, cta_row);
+                pair_tally<WITH_BP, SMEM, MULTI>(P.counts, P.bp, P.D, qs, qe, prow, d[j], sid[j], s_cnt, s_bp, cta_row);
             continue;
         }
-        // lane l: boundary ppos[t + 1 + l] as an offset from pb (> 0, since run t holds pb);
-        // offsets inside the step fit 32 bits
-        const uint64_t B = (uint64_t)t + 1 + lane <= rcap ? __ldg(P.ppos + t + 1 + lane) : ~0ull;
-        const uint32_t rel = B - pb < 0xffffffffull ? (uint32_t)(B - pb) : 0xffffffffu;
+        // lane l: boundary ppos[t + 1 + l] as an offset in the step (> 0, since run t holds its first
+        // position); offsets inside the step fit 32 bits
+        const uint64_t B = (uint64_t)t + 1 + lane <= rcap ? __ldg(P.ppos + t + 1 + lane) - (p0 + ob) : ~0ul;
+        const uint32_t rel = (uint32_t)min(B, (uint64_t)0xffffffffu);
         const uint32_t nb = __popc(__ballot_sync(0xffffffffu, rel <= span));
         if (nb > kFewBounds) {
-            pairs_step_dense<WITH_BP, SMEM, MULTI>(P.ppos, P.psegs, rowed ? P.prow : nullptr, P.pos, P.sid, P.counts,
-                                                   P.bp, P.D, t, rcap, pb, span, lane, cntr, s_cnt, s_bp, cta_row);
+            if constexpr (MULTI)
+                pairs_step_dense<WITH_BP, SMEM, MULTI>(P.ppos, P.psegs, nullptr, P.pos, P.sid, P.counts, P.bp, P.D, t,
+                                                       rcap, p0 + ob, span, lane, cntr, s_cnt, s_bp, cta_row);
+            else
+                pairs_step_dense_call<WITH_BP, SMEM>(P.ppos, P.psegs, rowed ? P.prow : nullptr, P.pos, P.sid, P.counts,
+                                                     P.bp, P.D, t, rcap, p0 + ob, span, lane, cntr, s_cnt, s_bp);
             continue;  // the next step starts past rhi: range_advance finds its run
         }
-        uint32_t k[kPairUnroll];  // position lane + 32 j lies in run t + k[j]
-#pragma unroll
-        for (uint32_t j = 0; j < kPairUnroll; j++) k[j] = 0;
-        for (uint32_t i = 0; i < nb; i++) {  // rel[0..nb) are the boundaries inside the step
-            const uint32_t bv = __shfl_sync(0xffffffffu, rel, i);
-#pragma unroll
-            for (uint32_t j = 0; j < kPairUnroll; j++) k[j] += bv <= lane + 32 * j ? 1u : 0u;
-        }
+        // byte j of kk: position lane + 32 j lies in run t + that; a boundary at offset v counts for the
+        // positions at or past it, which are those of j >= (v + 31 - lane) / 32
+        uint32_t kk = 0;
+        for (uint32_t i = 0; i < nb; i++)  // rel[0..nb) are the boundaries inside the step
+            kk += __funnelshift_lc(0u, 0x01010101u, ((__shfl_sync(0xffffffffu, rel, i) + 31 - lane) >> 2) & 0x38u);
         uint2 d[kPairUnroll];
         uint32_t sid[kPairUnroll];
 #pragma unroll
         for (uint32_t j = 0; j < kPairUnroll; j++) {
-            // run t + k (k > 0) starts at offset rel[k - 1]; t + k < rcap since ppos[rcap] = total > pend
-            const uint32_t o = lane + 32 * j;
-            const uint32_t rb = __shfl_sync(0xffffffffu, rel, k[j] ? k[j] - 1 : 0);
+            // run t + k (k > 0) starts at offset rel[k - 1]; t + k < rcap since ppos[rcap] = total > the step's last
+            const uint32_t k = (kk >> (8 * j)) & 0xffu, o = lane + 32 * j;
+            const uint32_t rb = __shfl_sync(0xffffffffu, rel, k - 1);
+            d[j] = make_uint2(0, 0);
+            sid[j] = 0;
             if (o <= span) {
-                const uint64_t di = k[j] ? run_base<MULTI>(__ldg(&P.psegs[t + k[j]].base)) + (o - rb) : base0 + o;
+                const uint64_t di = k ? run_base<MULTI>(__ldg(&P.psegs[t + k].base)) + (o - rb) : base + (ob + o);
                 d[j] = __ldg(P.pos + di);
                 sid[j] = __ldg(P.sid + di);
-            } else {
-                d[j] = make_uint2(0, 0);
-                sid[j] = 0;
             }
         }
 #pragma unroll
         for (uint32_t j = 0; j < kPairUnroll; j++) {
-            const PairSeg* q = P.psegs + t + k[j];
-            const uint2 qse = __ldg(reinterpret_cast<const uint2*>(&q->qs));
-            const uint32_t qrow = MULTI ? __ldg(reinterpret_cast<const uint32_t*>(q) + 1) >> (kRunRowShift - 32)
-                                        : rowed ? __ldg(P.prow + t + k[j]) : 0u;
-            pair_tally<WITH_BP, SMEM, MULTI>(P.counts, P.bp, P.D, qse.x, qse.y, qrow, d[j], sid[j], s_cnt, s_bp,
-                                             cta_row);
+            const uint32_t run = t + ((kk >> (8 * j)) & 0xffu);
+            const uint4 w = __ldg(reinterpret_cast<const uint4*>(P.psegs + run));
+            const uint32_t qrow = MULTI ? w.y >> (kRunRowShift - 32) : rowed ? __ldg(P.prow + run) : 0u;
+            pair_tally<WITH_BP, SMEM, MULTI>(P.counts, P.bp, P.D, w.z, w.w, qrow, d[j], sid[j], s_cnt, s_bp, cta_row);
         }
-        // the run of the next step's first position pend + 1, from the boundaries in hand (at
-        // least one boundary, ppos[t + 1] <= pend, lies at or below it)
+        // the run of the next step's first position, from the boundaries in hand (at least one, ppos[t + 1],
+        // lies at or below it)
         const uint32_t kn = __popc(__ballot_sync(0xffffffffu, rel <= span + 1));
-        if (pend + 1 < p1 && kn < 32) {
+        if (ob + span + 1 < len && kn < 32) {
             t += kn;
-            rlo = __ldg(P.ppos + t);
-            rhi = __ldg(P.ppos + t + 1);
-            ps = P.psegs[t];
-            prow = row_of(t, ps.base);
+            load_run();
         }
     }
 }
