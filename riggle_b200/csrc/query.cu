@@ -1536,8 +1536,8 @@ __device__ __noinline__ void pairs_step_dense_call(const uint64_t* __restrict__ 
 // step, and the run descriptors come from L1.
 // Bound: L1 wavefronts (70% of its cycles: 12 bytes and two shared-memory atomics a candidate) and
 // issue (65%).  64-bit offsets, one register a count and three loads a descriptor spilled in the
-// several-row form: 1.04e9 candidates of 48 files against 2e8 intervals 4,201 us, 3,638 as it is; five
-// blocks an SM instead of six, to hold the rest of the registers, 3,826.
+// several-row form: 1.04e9 candidates of 48 files against 2e8 intervals 4,201 us, 3,638 without; five,
+// six, seven, eight blocks an SM: 3,826, 3,638, 3,530, 3,545 (256 files against 3.2e6: 893, 823, 681, 685).
 // One work item of the pair sweep (positions [item * chunk, (item + 1) * chunk) of the concatenated
 // candidate runs), walked by one warp.
 template <bool WITH_BP, bool SMEM, int MULTI>
@@ -1647,7 +1647,7 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t chunk,
 }
 
 template <bool WITH_BP, bool SMEM, int MULTI>
-__global__ void __launch_bounds__(256, MULTI ? 6 : 8) k_pairs(const __grid_constant__ SweepParams P) {
+__global__ void __launch_bounds__(256, MULTI ? 7 : 8) k_pairs(const __grid_constant__ SweepParams P) {
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned long long* s_bp = reinterpret_cast<unsigned long long*>(smem);
     uint32_t* s_cnt = reinterpret_cast<uint32_t*>(smem + (WITH_BP ? (size_t)P.D * 8 : 0));
