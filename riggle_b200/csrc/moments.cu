@@ -803,15 +803,17 @@ __global__ void __launch_bounds__(kSigThreads) k_center(uint64_t n, const float*
 
 enum Term : int { T_A = 0, T_MA = 1, T_U2 = 2, T_V2 = 3, T_U = 4, kTerms = 5 };
 
-// Adds the five terms of element t (0 .. n) to s.  uN = U[n].
+// Adds four terms of element t (0 .. n) to s and the fifth, U[t], to su.  uN = U[n].
+// su is in double-double in both precisions, as are the prefix sums over the tiles: the window mean of a short
+// L is what is left of sums of U a few 1e6 times its size (in 48 bits that was wrong by 4e-10 of it at 2^21 bins; 713 -> 732 us at 2^21 bins in float-float).
 template <class P>
 __device__ __forceinline__ void add_terms(uint64_t t, uint64_t n, const typename P::S* __restrict__ A,
                                           const typename P::S* __restrict__ U, typename P::S uN,
-                                          typename P::T* s) {
+                                          typename P::T* s, DD& su) {
     using S = typename P::S;
     if (t > n) return;
     const S u = U[t];
-    s[T_U] = P::add_s(s[T_U], u);
+    su = P64::add_s(su, P::value(u, 0));
     if (t == 0) return;
     s[T_U2] = P::add_s(s[T_U2], P::mul(u, u));  // U[t]^2, t >= 1
     if (t >= n) return;
@@ -828,35 +830,41 @@ template <class P>
 __global__ void __launch_bounds__(kTermThreads) k_term_tiles(uint64_t n, uint64_t nt,
                                                              const typename P::S* __restrict__ A,
                                                              const typename P::S* __restrict__ U,
-                                                             typename P::T* __restrict__ tsum) {
+                                                             DD* __restrict__ tsum) {
     using T = typename P::T;
-    __shared__ T part[kTerms][kTermThreads / 32];
+    __shared__ T part[T_U][kTermThreads / 32];
+    __shared__ DD part_u[kTermThreads / 32];
     const typename P::S uN = U[n];
-    T s[kTerms];
+    T s[T_U];
+    DD su{0.0, 0.0};
 #pragma unroll
-    for (int q = 0; q < kTerms; q++) s[q] = P::zero();
+    for (int q = 0; q < T_U; q++) s[q] = P::zero();
 #pragma unroll
     for (int k = 0; k < kTermTile / kTermThreads; k++)
-        add_terms<P>(blockIdx.x * (uint64_t)kTermTile + k * kTermThreads + threadIdx.x, n, A, U, uN, s);
+        add_terms<P>(blockIdx.x * (uint64_t)kTermTile + k * kTermThreads + threadIdx.x, n, A, U, uN, s, su);
 #pragma unroll
-    for (int q = 0; q < kTerms; q++) {
+    for (int q = 0; q < T_U; q++) {
         const T v = warp_sum<P>(s[q]);
         if ((threadIdx.x & 31) == 0) part[q][threadIdx.x >> 5] = v;
     }
+    su = warp_sum<P64>(su);
+    if ((threadIdx.x & 31) == 0) part_u[threadIdx.x >> 5] = su;
     __syncthreads();
-    if (threadIdx.x < kTerms) {
+    if (threadIdx.x < T_U) {
         T v = part[threadIdx.x][0];
         for (int w = 1; w < kTermThreads / 32; w++) v = P::add(v, part[threadIdx.x][w]);
-        tsum[threadIdx.x * nt + blockIdx.x] = v;
+        tsum[threadIdx.x * nt + blockIdx.x] = P::sum_dd(v, 0);
+    } else if (threadIdx.x == T_U) {
+        DD v = part_u[0];
+        for (int w = 1; w < kTermThreads / 32; w++) v = dd_add(v, part_u[w]);
+        tsum[T_U * nt + blockIdx.x] = v;
     }
 }
 
 // Block q: term q's tile sums into exclusive prefix sums; total[q] = the whole.
-template <class P>
-__global__ void __launch_bounds__(1024) k_term_tops(uint64_t nt, typename P::T* __restrict__ tsum,
-                                                    typename P::T* __restrict__ total) {
-    typename P::T t;
-    scan_tiles<P>(nt, tsum + blockIdx.x * nt, &t);
+__global__ void __launch_bounds__(1024) k_term_tops(uint64_t nt, DD* __restrict__ tsum, DD* __restrict__ total) {
+    DD t;
+    scan_tiles<P64>(nt, tsum + blockIdx.x * nt, &t);
     if (threadIdx.x == 0) total[blockIdx.x] = t;
 }
 
@@ -903,31 +911,41 @@ __global__ void __launch_bounds__(256) k_direct_part(const uint64_t* __restrict_
 // final reduction and the variance subtraction in FP64.  parts > 0: grid points from `first` on take
 // their variance from k_direct_part's sums.
 constexpr int kPointThreads = 128;
+__device__ __forceinline__ DD scaled_dd(DD a, int sc) { return DD{ldexp(a.hi, sc), ldexp(a.lo, sc)}; }
 template <class P>
 __global__ void __launch_bounds__(kPointThreads) k_window_moments(
     const uint64_t* __restrict__ grid, uint64_t n, uint64_t nt, const typename P::S* __restrict__ A,
-    const typename P::S* __restrict__ U, const typename P::T* __restrict__ tpre,
-    const typename P::T* __restrict__ total, const MomentState* __restrict__ msp, uint32_t first, uint32_t parts,
+    const typename P::S* __restrict__ U, const DD* __restrict__ tpre,
+    const DD* __restrict__ total, const MomentState* __restrict__ msp, uint32_t first, uint32_t parts,
     const DD* __restrict__ direct, float2* __restrict__ out, double* __restrict__ mean_out,
     double* __restrict__ var_out) {
     using T = typename P::T;
-    __shared__ T part[kTerms + 1][kPointThreads / 32];
+    __shared__ T part[T_U][kPointThreads / 32];
+    __shared__ DD part_u[2][kPointThreads / 32];
     const uint32_t i = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t L = grid[i];
     // inclusive prefix up to t = L - 1 (the t = 0 terms of A and t A are zero); UU(N-L+1) = sum of U[0 .. N-L]
     const uint64_t at_l = L - 1, at_r = n - L;
     const uint64_t tl = at_l / kTermTile, tr = at_r / kTermTile;
     const typename P::S uN = U[n];
-    T s[kTerms + 1];
+    T s[T_U];
+    DD ul{0.0, 0.0}, ur{0.0, 0.0};
 #pragma unroll
-    for (int q = 0; q <= kTerms; q++) s[q] = P::zero();
-    for (uint64_t t = tl * kTermTile + threadIdx.x; t <= at_l; t += kPointThreads) add_terms<P>(t, n, A, U, uN, s);
+    for (int q = 0; q < T_U; q++) s[q] = P::zero();
+    for (uint64_t t = tl * kTermTile + threadIdx.x; t <= at_l; t += kPointThreads)
+        add_terms<P>(t, n, A, U, uN, s, ul);
     for (uint64_t t = tr * kTermTile + threadIdx.x; t <= at_r; t += kPointThreads)
-        s[kTerms] = P::add_s(s[kTerms], U[t]);
+        ur = P64::add_s(ur, P::value(U[t], 0));
 #pragma unroll
-    for (int q = 0; q <= kTerms; q++) {
+    for (int q = 0; q < T_U; q++) {
         const T v = warp_sum<P>(s[q]);
         if (lane == 0) part[q][warp] = v;
+    }
+    ul = warp_sum<P64>(ul);
+    ur = warp_sum<P64>(ur);
+    if (lane == 0) {
+        part_u[0][warp] = ul;
+        part_u[1][warp] = ur;
     }
     DD d1{0.0, 0.0}, d2{0.0, 0.0};
     const bool few = parts && i >= first;
@@ -948,15 +966,16 @@ __global__ void __launch_bounds__(kPointThreads) k_window_moments(
 #pragma unroll
     for (int q = 0; q <= kTerms; q++) {
         const int term = q < kTerms ? q : T_U;
-        T v = tpre[term * nt + (q < kTerms ? tl : tr)];
-        for (int w = 0; w < kPointThreads / 32; w++) v = P::add(v, part[q][w]);
-        p[q] = P::sum_dd(v, term == T_U ? e : 2 * e);
+        DD v = tpre[term * nt + (q < kTerms ? tl : tr)];
+        for (int w = 0; w < kPointThreads / 32; w++)
+            v = dd_add(v, term == T_U ? part_u[q - T_U][w] : P::sum_dd(part[q][w], 0));
+        p[q] = scaled_dd(v, term == T_U ? e : 2 * e);
     }
     const double nw = (double)(n - L + 1);
     const double gbar = ms.gsum.hi / (double)n + ms.gsum.lo / (double)n;
     const double a0 = P::value(A[0], 2 * e);
     // sum_j F_L(j) = (UU(N+1) - UU(L)) - UU(N-L+1)
-    const DD sf = dd_add(dd_add(P::sum_dd(total[T_U], e), dd_neg(p[T_U])), dd_neg(p[kTerms]));
+    const DD sf = dd_add(dd_add(scaled_dd(total[T_U], e), dd_neg(p[T_U])), dd_neg(p[kTerms]));
     const double fbar = (sf.hi + sf.lo) / nw;
     // sum_j F_L(j)^2 = L A[0] + 2 (L P0 - P1) - Q - V
     DD s2 = DD{(double)L * a0, fma((double)L, a0, -(double)L * a0)};
@@ -1145,7 +1164,7 @@ int moments_dev(MomentWs& w, uint64_t N, const std::vector<uint64_t>& grid, floa
     RGL_TRY(w.pw.ensure((H + 2) * sizeof(S)));
     RGL_TRY(w.U.ensure((N + 2) * sizeof(S)));
     RGL_TRY(w.A.ensure((N + 2) * sizeof(S)));
-    RGL_TRY(w.sums.ensure((2 * nt + kTerms * (mt + 1) + 4) * sizeof(T)));
+    RGL_TRY(w.sums.ensure(2 * nt * sizeof(T) + (kTerms * (mt + 1) + 4) * sizeof(DD)));
     RGL_TRY(w.state.ensure(sizeof(MomentState) + nt * 4 + 64));
     // windows with few positions: reduced directly, in parts of at least 2,048 windows
     const uint64_t few = std::max<uint64_t>(65536, N / 32);
@@ -1160,8 +1179,8 @@ int moments_dev(MomentWs& w, uint64_t N, const std::vector<uint64_t>& grid, floa
     float* tmax = reinterpret_cast<float*>(ms + 1);
     T* tsum = w.sums.as<T>();
     T* usum = kFF ? tsum + nt : tsum;
-    T* terms = tsum + 2 * nt;
-    T* totals = terms + kTerms * mt;
+    DD* terms = reinterpret_cast<DD*>(tsum + 2 * nt);
+    DD* totals = terms + kTerms * mt;
     S* U = w.U.as<S>();
     S* A = w.A.as<S>();
     k_g_tiles<P><<<(unsigned)nt, kSigThreads, 0, st>>>(N, g, tsum, tmax);
@@ -1181,7 +1200,7 @@ int moments_dev(MomentWs& w, uint64_t N, const std::vector<uint64_t>& grid, floa
     k_autocorr<P><<<blocks_for(H / 2 + 1), 256, 0, st>>>(H, N, Q, A);
     // K7
     k_term_tiles<P><<<(unsigned)mt, kTermThreads, 0, st>>>(N, mt, A, U, terms);
-    k_term_tops<P><<<kTerms, 1024, 0, st>>>(mt, terms, totals);
+    k_term_tops<<<kTerms, 1024, 0, st>>>(mt, terms, totals);
     if (parts)
         k_direct_part<S><<<dim3(parts, G - first), 256, 0, st>>>(d_grid, first, N, U, (most + parts - 1) / parts,
                                                                  w.direct.as<DD>());
