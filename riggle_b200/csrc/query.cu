@@ -176,7 +176,9 @@ __global__ void k_expand_keys(uint32_t n, const rgl_interval* __restrict__ iv, c
     if (s >= e) bad |= ERR_BAD_INTERVAL;
     if (q >= rows || (blk_row && row != blk_row[lo])) {
         bad |= ERR_BAD_ROW;
-        q = 0;
+        // The run is refused at its end, but goes through to there: its key stays in its block's segment, so that
+        // a block sorted on its own is one segment and there are no more segments than (shard, row) pairs.
+        q = blk_row ? blk_row[lo] - row_base : 0u;
         if (wide && unsorted) {  // its key goes by row 0 now: out of order
             const uint32_t k = sidx ? sidx[lo] : lo;
             unsorted[k] = unsorted[nblk + k] = 1u;
