@@ -434,6 +434,10 @@ typedef struct rgl_pvalue_batch {
 int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* batch, uint32_t bin_size, const uint32_t* counts,
                       const uint64_t* overlap_bp, double* p, double* llr, double* log_p, uint8_t* flags);
 
+/* Device bytes of scratch that the p-values of up to num_rows query rows take at most, which a request server
+ * with a moment store sets aside for each worker; never less for more rows. */
+uint64_t rgl_pvalue_scratch_bytes(uint32_t num_rows, uint32_t num_sources, uint32_t num_chroms);
+
 /* The stats stage of the batched form, all on the device: compute_analytic_pvalues
  * (src/tasks/query/pvalues.rs:22-77) for every (row, source) cell of a batch whose counts and overlap
  * are in device memory (the outputs of rgl_query_batch_device), with the query length groups

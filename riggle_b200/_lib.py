@@ -236,6 +236,7 @@ _SIGS = {
     "rgl_moments_build": (C.c_int, [_P, C.c_uint32, C.c_uint32, _P, C.c_uint64, C.c_uint32, _P, _P]),
     "rgl_moments_build_ex": (C.c_int, [_P, C.c_uint32, C.c_uint32, _P, C.c_uint64, C.c_uint32, C.c_uint32, _P, _P]),
     "rgl_query_pvalues": (C.c_int, [_P, C.POINTER(PValueBatch), C.c_uint32, _P, _P, _P, _P, _P, _P]),
+    "rgl_pvalue_scratch_bytes": (C.c_uint64, [C.c_uint32, C.c_uint32, C.c_uint32]),
     "rgl_batch_pvalues_device": (C.c_int, [_P, _P, C.POINTER(BatchDesc), _P, C.c_uint32, C.c_uint32, _P, _P, _P, _P,
                                            _P, _P, C.POINTER(C.c_uint64)]),
     "rgl_batch_query_groups": (C.c_int, [_P, _P, C.POINTER(BatchDesc), _P, C.c_uint32, C.c_uint32, _P, _P, _P, _P,

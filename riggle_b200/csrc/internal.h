@@ -182,8 +182,10 @@ int batch_pvalues_enqueue(rgl_context* ctx, rgl_moments* m, StatsScratch* sc, co
 // Builds the moment store's shared device tables once (thread-safe).
 int moments_prepare(rgl_moments* m);
 void stats_scratch_release(StatsScratch* sc);
-// Device bytes of StatsScratch::part for rows x D cells over C chromosomes.
+// Device bytes of StatsScratch::part for rows x D cells over C chromosomes, and for up to that many rows (never
+// fewer for more rows, where the former may be).
 uint64_t pv_scratch_bytes(uint32_t rows, uint32_t D, uint32_t C);
+uint64_t pv_scratch_bound(uint32_t rows, uint32_t D, uint32_t C);
 uint32_t moments_chroms(const rgl_moments* m);
 uint32_t context_last_launches(rgl_context* c);
 

@@ -203,7 +203,7 @@ int batch_growth(rgl_server* S, Worker* W, uint64_t n, uint32_t R, uint32_t nblk
              grow(W->sc.groups, n * 48 + 48) + grow(W->sc.plan, stats_plan_bytes(n, nblk)) +
              grow(W->sc.goff, stats_goff_bytes(S, R, nblk)) + grow(W->sc.runs, 64) +
              grow(W->sc.rcoff, ((uint64_t)R * S->chroms + 1) * 4) +
-             grow(W->sc.part, pv_scratch_bytes(R, S->D, S->chroms));
+             grow(W->sc.part, pv_scratch_bound(R, S->D, S->chroms));
     }
     *bytes = b;
     return RGL_OK;
@@ -232,7 +232,7 @@ int size_worker(rgl_server* S, Worker* W, uint64_t n, uint32_t R, uint32_t nblk)
         RGL_TRY(W->sc.goff.ensure(stats_goff_bytes(S, R, nblk)));
         RGL_TRY(W->sc.runs.ensure(64));
         RGL_TRY(W->sc.rcoff.ensure(((uint64_t)R * S->chroms + 1) * 4));
-        RGL_TRY(W->sc.part.ensure(pv_scratch_bytes(R, S->D, S->chroms)));
+        RGL_TRY(W->sc.part.ensure(pv_scratch_bound(R, S->D, S->chroms)));
     }
     return RGL_OK;
 }
@@ -287,6 +287,7 @@ bool formation_grows(rgl_server* S, Worker* W) {
 void worker_main(rgl_server* S, Worker* W) {
     cudaSetDevice(S->device);
     std::vector<Req*> batch, refused;
+    bool ask = false;  // the last formation took nothing: ask for the free memory whatever it would need
     for (;;) {
         uint64_t n = 0, promise = 0;
         uint32_t nblk = 0;
@@ -300,7 +301,7 @@ void worker_main(rgl_server* S, Worker* W) {
             for (;;) {
                 S->cv_work.wait(lk, [&] { return S->stop || !S->pending.empty(); });
                 if (S->pending.empty()) return;  // stop requested and the queue is drained
-                if (have_free || !formation_grows(S, W)) break;
+                if (have_free || !(ask || formation_grows(S, W))) break;
                 lk.unlock();
                 free_b = free_device_memory(S);
                 have_free = true;
@@ -335,6 +336,7 @@ void worker_main(rgl_server* S, Worker* W) {
                 nblk += qb;
                 S->pending.pop_front();
             }
+            ask = batch.empty();
             S->pending_n -= n;
             S->promised += promise;
             const double t = S->now();

@@ -286,6 +286,7 @@ __global__ void __launch_bounds__(128) k_pv_cells(uint64_t cells, uint32_t parts
 
 // Shape of a launch: 32 rows a block (two a warp), or four where there are fewer than 16; a block per
 // chromosome where that leaves fewer than four for each of 148 SMs.
+constexpr uint64_t kPvFill = 148 * 4;
 struct PvShape {
     bool many;
     uint32_t parts;
@@ -293,15 +294,24 @@ struct PvShape {
 };
 PvShape pv_shape(uint32_t rows, uint32_t D, uint32_t C) {
     PvShape s{rows >= 16, 1, 0};
-    const uint32_t per_tile = s.many ? 32 : 4;
-    const uint64_t tiles = (uint64_t)((rows + per_tile - 1) / per_tile) * ((D + kPvSources - 1) / kPvSources);
-    if (tiles < 148 * 4) s.parts = C;
+    const uint64_t per_tile = s.many ? 32 : 4;
+    const uint64_t tiles = ((rows + per_tile - 1) / per_tile) * (((uint64_t)D + kPvSources - 1) / kPvSources);
+    if (tiles < kPvFill) s.parts = C;
     s.blocks = tiles * s.parts;
     return s;
 }
+uint64_t pv_part_bytes(uint64_t rows, uint32_t D, uint32_t parts) {
+    return parts > 1 ? parts * rows * D * (sizeof(PvCell) + 1) + 64 : 0;
+}
 uint64_t pv_scratch_bytes(uint32_t rows, uint32_t D, uint32_t C) {
-    const PvShape s = pv_shape(rows, D, C);
-    return s.parts > 1 ? s.parts * (uint64_t)rows * D * (sizeof(PvCell) + 1) + 64 : 0;
+    return pv_part_bytes(rows, D, pv_shape(rows, D, C).parts);
+}
+// The scratch falls to nothing where the rows alone fill the chip, and comes back at 16 rows, where the tiles
+// grow: the bound is that of the largest row count up to `rows` whose launch is split.
+uint64_t pv_scratch_bound(uint32_t rows, uint32_t D, uint32_t C) {
+    const uint64_t tiles = (kPvFill - 1) / std::max<uint64_t>(1, ((uint64_t)D + kPvSources - 1) / kPvSources);
+    const uint64_t many = std::min<uint64_t>(rows, 32 * tiles), few = std::min<uint64_t>({rows, 15, 4 * tiles});
+    return pv_part_bytes(many >= 16 ? many : few, D, C);
 }
 // scratch: pv_scratch_bytes of device memory.
 int launch_pvalues(uint32_t rows, uint32_t D, uint32_t C, const uint32_t* counts, const unsigned long long* bp,
@@ -730,6 +740,10 @@ int rgl_moments_get(const rgl_moments* m, uint32_t sid, uint32_t chrom, float* m
     RGL_CUDA(cudaMemcpy(mean_var, m->d_mv + (uint64_t)sid * m->stride + m->chrom_off[chrom], l * 8,
                         cudaMemcpyDeviceToHost));
     return RGL_OK;
+}
+
+uint64_t rgl_pvalue_scratch_bytes(uint32_t num_rows, uint32_t num_sources, uint32_t num_chroms) {
+    return pv_scratch_bound(num_rows, num_sources, num_chroms);
 }
 
 int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_size, const uint32_t* counts,

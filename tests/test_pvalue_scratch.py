@@ -1,0 +1,19 @@
+"""The scratch that the p-values of up to so many rows take: never less for more rows (the request server forms its
+batches by that).  Needs no GPU."""
+import pytest
+
+import riggle_b200 as rg
+
+
+@pytest.mark.parametrize("chroms", [1, 2, 24, 455])
+def test_scratch_never_falls(chroms):
+    f = rg.load().rgl_pvalue_scratch_bytes
+    for sources in list(range(1, 200, 7)) + [500, 1169, 1905, 3000, 5585, 6000, 9456, 9457, 40_000]:
+        sizes = [f(r, sources, chroms) for r in range(1, 1200)]
+        assert all(a <= b for a, b in zip(sizes, sizes[1:])), sources
+        # a launch of `r` rows is split where its tiles are fewer than 592, and then holds its cells' sums apart
+        for r in (1, 4, 15, 16, 17, 128, 256, 1199):
+            tiles = -(-r // (32 if r >= 16 else 4)) * -(-sources // 16)
+            if tiles < 592 and chroms > 1:
+                assert sizes[r - 1] >= 25 * r * sources * min(chroms, 24)
+    assert f(0, 100, chroms) <= 64
