@@ -133,7 +133,7 @@ __device__ __forceinline__ void pvalue_cell(uint32_t count, uint32_t any, double
 }
 
 // The sums over the groups.  A block takes 16 sources, WARPS x ROWS query rows (a warp takes ROWS of them
-// one after the other) and all chromosomes or (parts = C) one.  Per chromosome the sources' table entries
+// one after the other) and all chromosomes or (with `part`, one of `parts` blocks) chromosome c0 + its part.  Per chromosome the sources' table entries
 // are staged in shared memory, slot by slot with the sources side by side (zero past a table's end); each
 // half-warp walks every second group of a row on that chromosome, a group read once for its 16 lanes, each
 // with its own source's entry and its own three sums, so that nothing is reduced over lanes but the two
@@ -149,7 +149,7 @@ struct PvCell {
 };
 template <int ROWS, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) k_pvalues(
-    uint32_t rows, uint32_t D, uint32_t C, uint32_t parts, const uint32_t* __restrict__ counts,
+    uint32_t rows, uint32_t D, uint32_t C, uint32_t c0, uint32_t parts, const uint32_t* __restrict__ counts,
     const unsigned long long* __restrict__ bp, double bin_size, const uint32_t* __restrict__ rc_off,
     const QGroupDev* __restrict__ groups, const float2* __restrict__ mv, const uint64_t* __restrict__ chrom_off,
     uint64_t stride, const uint32_t* __restrict__ tab_len, double* __restrict__ p_out, double* __restrict__ llr_out,
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) k_pvalues(
     uint32_t any = 0;  // bit r: row r has a group in source d's tables
 #pragma unroll
     for (int r = 0; r < ROWS; r++) acc[r] = PvCell{0.0, 0.0, 0.0};
-    for (uint32_t c = parts > 1 ? pt : 0u; c < (parts > 1 ? pt + 1 : C); c++) {
+    for (uint32_t c = part ? c0 + pt : 0u, c1 = part ? c + 1 : C; c < c1; c++) {
         const uint32_t n_slots = (uint32_t)((c + 1 < C ? chrom_off[c + 1] : stride) - chrom_off[c]);
         // the slots that any row of the tile needs (a row's groups ascend by slot)
         if (threadIdx.x == 0) s_slots = 0;
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) k_pvalues(
         const uint32_t q = q0 + warp * ROWS + r;
         if (q >= rows) break;
         const uint64_t w = (uint64_t)q * D + d;
-        if (parts > 1) {
+        if (part) {
             const uint64_t x = (uint64_t)pt * rows * D + w;
             part[x] = acc[r];
             part_any[x] = any >> r & 1u;
@@ -263,17 +263,19 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) k_pvalues(
     }
 }
 
-// One cell per thread: the parts of the chromosomes added up in order, then the p-value.
-__global__ void __launch_bounds__(128) k_pv_cells(uint64_t cells, uint32_t parts, const PvCell* __restrict__ part,
-                                                  const uint8_t* __restrict__ part_any,
+// One cell per thread: the sums of `parts` chromosomes added up in order, onto those of the chromosomes before
+// them (not `first`: slot `keep` of the sums), then kept there, or (`last`) the p-value.
+__global__ void __launch_bounds__(128) k_pv_cells(uint64_t cells, uint32_t parts, uint32_t keep, int first, int last,
+                                                  PvCell* __restrict__ part, uint8_t* __restrict__ part_any,
                                                   const uint32_t* __restrict__ counts,
                                                   const unsigned long long* __restrict__ bp, double bin_size,
                                                   double* __restrict__ p_out, double* __restrict__ llr_out,
                                                   double* __restrict__ logp_out, uint8_t* __restrict__ flags) {
     const uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (w >= cells) return;
-    PvCell s{0.0, 0.0, 0.0};
-    uint32_t any = 0;
+    const uint64_t kept = keep * cells + w;
+    PvCell s = first ? PvCell{0.0, 0.0, 0.0} : part[kept];
+    uint32_t any = first ? 0u : part_any[kept];
     for (uint32_t k = 0; k < parts; k++) {
         const PvCell v = part[k * cells + w];
         s.mu += v.mu;
@@ -281,37 +283,50 @@ __global__ void __launch_bounds__(128) k_pv_cells(uint64_t cells, uint32_t parts
         s.raw += v.raw;
         any |= part_any[k * cells + w];
     }
+    if (!last) {
+        part[kept] = s;
+        part_any[kept] = (uint8_t)any;
+        return;
+    }
     pvalue_cell(counts[w], any, s.mu, s.var, s.raw, bp[w], bin_size, w, p_out, llr_out, logp_out, flags);
 }
 
 // Shape of a launch: 32 rows a block (two a warp), or four where there are fewer than 16; a block per
-// chromosome where that leaves fewer than four for each of 148 SMs.
-constexpr uint64_t kPvFill = 148 * 4;
+// chromosome where that leaves fewer than four for each of 148 SMs.  The blocks' sums are kept per chromosome for
+// at most kPvScratch bytes (24 chromosomes at the most cells that are split); of more chromosomes, `parts` at a time
+// with the sums so far in one more slot, in the same order.  (All of 3,000 chromosomes at once were 3 GB for 40,000
+// cells.)
+constexpr uint64_t kPvFill = 148 * 4, kPvScratch = 192ull << 20, kPvCellBytes = sizeof(PvCell) + 1;
 struct PvShape {
-    bool many;
-    uint32_t parts;
-    uint64_t blocks;
+    bool many, split;
+    uint32_t parts;        // chromosomes at a time
+    uint64_t tiles, slots; // of 16 sources x rows; sums kept per cell
 };
 PvShape pv_shape(uint32_t rows, uint32_t D, uint32_t C) {
-    PvShape s{rows >= 16, 1, 0};
+    PvShape s{rows >= 16, false, 1, 0, 0};
     const uint64_t per_tile = s.many ? 32 : 4;
-    const uint64_t tiles = ((rows + per_tile - 1) / per_tile) * (((uint64_t)D + kPvSources - 1) / kPvSources);
-    if (tiles < kPvFill) s.parts = C;
-    s.blocks = tiles * s.parts;
+    s.tiles = ((rows + per_tile - 1) / per_tile) * (((uint64_t)D + kPvSources - 1) / kPvSources);
+    if (C > 1 && s.tiles < kPvFill) {
+        const uint64_t room = kPvScratch / std::max<uint64_t>(1, (uint64_t)rows * D * kPvCellBytes);
+        s.split = true;
+        s.slots = std::min<uint64_t>({C, room, 65536});  // (the grid's size fits 31 bits)
+        s.parts = (uint32_t)(s.slots == C ? C : s.slots - 1);
+    }
     return s;
 }
-uint64_t pv_part_bytes(uint64_t rows, uint32_t D, uint32_t parts) {
-    return parts > 1 ? parts * rows * D * (sizeof(PvCell) + 1) + 64 : 0;
-}
+static_assert((kPvFill - 1) * 32 * kPvSources * kPvCellBytes * 2 <= kPvScratch, "room for a chromosome and the sums so far");
 uint64_t pv_scratch_bytes(uint32_t rows, uint32_t D, uint32_t C) {
-    return pv_part_bytes(rows, D, pv_shape(rows, D, C).parts);
+    const PvShape s = pv_shape(rows, D, C);
+    return s.split ? s.slots * rows * D * kPvCellBytes + 64 : 0;
 }
 // The scratch falls to nothing where the rows alone fill the chip, and comes back at 16 rows, where the tiles
 // grow: the bound is that of the largest row count up to `rows` whose launch is split.
 uint64_t pv_scratch_bound(uint32_t rows, uint32_t D, uint32_t C) {
+    if (C < 2) return 0;
     const uint64_t tiles = (kPvFill - 1) / std::max<uint64_t>(1, ((uint64_t)D + kPvSources - 1) / kPvSources);
     const uint64_t many = std::min<uint64_t>(rows, 32 * tiles), few = std::min<uint64_t>({rows, 15, 4 * tiles});
-    return pv_part_bytes(many >= 16 ? many : few, D, C);
+    const uint64_t cells = (many >= 16 ? many : few) * D;
+    return std::min(C * cells * kPvCellBytes, kPvScratch) + 64;
 }
 // scratch: pv_scratch_bytes of device memory.
 int launch_pvalues(uint32_t rows, uint32_t D, uint32_t C, const uint32_t* counts, const unsigned long long* bp,
@@ -320,18 +335,23 @@ int launch_pvalues(uint32_t rows, uint32_t D, uint32_t C, const uint32_t* counts
                    double* logp, uint8_t* flags, void* scratch, cudaStream_t st) {
     const PvShape s = pv_shape(rows, D, C);
     const uint64_t cells = (uint64_t)rows * D;
-    if (s.blocks >= (1ull << 31)) return fail(RGL_ERR_INVALID_ARGUMENT, "too many cells for one call");
-    PvCell* part = static_cast<PvCell*>(scratch);
-    uint8_t* any = reinterpret_cast<uint8_t*>(part + (s.parts > 1 ? s.parts * cells : 0));
-    auto run = [&](auto kernel, int threads) {
-        kernel<<<(unsigned)s.blocks, threads, 0, st>>>(rows, D, C, s.parts, counts, bp, bin_size, rc_off, groups, mv,
-                                                      chrom_off, stride, tab_len, p, llr, logp, flags, part, any);
-    };
-    if (s.many) run(k_pvalues<2, 16>, 512);
-    else run(k_pvalues<1, 4>, 128);
-    if (s.parts > 1)
-        k_pv_cells<<<(unsigned)((cells + 127) / 128), 128, 0, st>>>(cells, s.parts, part, any, counts, bp, bin_size, p,
-                                                                   llr, logp, flags);
+    if (s.tiles * s.parts >= (1ull << 31)) return fail(RGL_ERR_INVALID_ARGUMENT, "too many cells for one call");
+    PvCell* part = s.split ? static_cast<PvCell*>(scratch) : nullptr;
+    uint8_t* any = reinterpret_cast<uint8_t*>(part + s.slots * cells);
+    for (uint32_t c0 = 0; c0 < (s.split ? C : 1u);) {
+        const uint32_t parts = s.split ? std::min(s.parts, C - c0) : 1u;
+        auto run = [&](auto kernel, int threads) {
+            kernel<<<(unsigned)(s.tiles * parts), threads, 0, st>>>(rows, D, C, c0, parts, counts, bp, bin_size, rc_off,
+                                                                   groups, mv, chrom_off, stride, tab_len, p, llr, logp,
+                                                                   flags, part, any);
+        };
+        if (s.many) run(k_pvalues<2, 16>, 512);
+        else run(k_pvalues<1, 4>, 128);
+        if (s.split)
+            k_pv_cells<<<(unsigned)((cells + 127) / 128), 128, 0, st>>>(cells, parts, s.parts, c0 == 0, c0 + parts == C, part,
+                                                                       any, counts, bp, bin_size, p, llr, logp, flags);
+        c0 += parts;
+    }
     RGL_CUDA(cudaGetLastError());
     return RGL_OK;
 }

@@ -17,3 +17,8 @@ def test_scratch_never_falls(chroms):
             if tiles < 592 and chroms > 1:
                 assert sizes[r - 1] >= 25 * r * sources * min(chroms, 24)
     assert f(0, 100, chroms) <= 64
+
+
+def test_scratch_is_bounded():
+    f = rg.load().rgl_pvalue_scratch_bytes
+    assert max(f(r, s, 1_000_000) for r in (1, 15, 128, 5000) for s in (1, 500, 20_000)) <= 200 << 20
