@@ -200,7 +200,7 @@ int batch_growth(rgl_server* S, Worker* W, uint64_t n, uint32_t R, uint32_t nblk
         // the stats stage's scratch: keys, lengths, runs and groups per interval (StatsScratch)
         b += grow(W->sc.key_a, n * 8 + 8) + grow(W->sc.key_b, n * 8 + 8) + grow(W->sc.len_a, n * 4 + 4) +
              grow(W->sc.len_b, n * 4 + 4) + grow(W->sc.ukey, n * 8 + 8) + grow(W->sc.agg, n * 32 + 32) +
-             grow(W->sc.groups, n * 48 + 48) + grow(W->sc.plan, stats_plan_bytes(n, nblk)) +
+             grow(W->sc.groups, n * 40 + 40) + grow(W->sc.plan, stats_plan_bytes(n, nblk)) +
              grow(W->sc.goff, stats_goff_bytes(S, R, nblk)) + grow(W->sc.runs, 64) +
              grow(W->sc.rcoff, ((uint64_t)R * S->chroms + 1) * 4) +
              grow(W->sc.part, pv_scratch_bound(R, S->D, S->chroms));
@@ -227,7 +227,7 @@ int size_worker(rgl_server* S, Worker* W, uint64_t n, uint32_t R, uint32_t nblk)
         RGL_TRY(W->sc.len_b.ensure(nn * 4 + 4));
         RGL_TRY(W->sc.ukey.ensure(nn * 8 + 8));
         RGL_TRY(W->sc.agg.ensure(nn * 32 + 32));
-        RGL_TRY(W->sc.groups.ensure(nn * 48 + 48));
+        RGL_TRY(W->sc.groups.ensure(nn * 40 + 40));
         RGL_TRY(W->sc.plan.ensure(stats_plan_bytes(nn, nblk)));
         RGL_TRY(W->sc.goff.ensure(stats_goff_bytes(S, R, nblk)));
         RGL_TRY(W->sc.runs.ensure(64));

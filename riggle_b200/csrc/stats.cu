@@ -57,7 +57,10 @@ std::vector<uint64_t> moment_grid(uint64_t n) {
 struct __align__(16) QGroupDev {
     double ss, ss2, cr;  // cr = count / l_int
     uint32_t chrom, slot;
-    double l_int, count;
+};
+// What only rgl_batch_query_groups reports of a group of the batched stage.
+struct QGroupLen {
+    uint32_t l_int, count;
 };
 
 __device__ __forceinline__ double erfc_as(double x) {
@@ -386,7 +389,7 @@ struct LenToAgg {
 constexpr uint64_t kNoGroup = ~0ull;
 constexpr uint32_t kNoLen = 0xFFFFFFFFu;  // block-local keys: the low word of an interval in no group
 // the request server sizes each worker's StatsScratch with these record sizes
-static_assert(sizeof(LenAgg) == 32 && sizeof(QGroupDev) == 48, "stats scratch record sizes changed");
+static_assert(sizeof(LenAgg) == 32 && sizeof(QGroupDev) == 32 && sizeof(QGroupLen) == 8, "stats scratch record sizes changed");
 
 __global__ void k_group_keys(uint64_t n, const rgl_interval* __restrict__ iv, const uint64_t* __restrict__ blk_off,
                              const uint32_t* __restrict__ blk_shard, const uint32_t* __restrict__ blk_row, uint32_t nblk,
@@ -550,7 +553,8 @@ __global__ void __launch_bounds__(kRunThreads) k_run_agg(const uint32_t* __restr
 __global__ void k_group_finish(const uint64_t* __restrict__ ukey, const LenAgg* __restrict__ agg,
                                const uint32_t* __restrict__ num_runs, uint32_t rows, uint32_t C, double bin,
                                const uint32_t* __restrict__ slot_tab, uint64_t slot_tab_len,
-                               QGroupDev* __restrict__ groups, uint64_t* __restrict__ g_off,
+                               QGroupDev* __restrict__ groups, QGroupLen* __restrict__ lens,
+                               uint64_t* __restrict__ g_off,
                                uint32_t* __restrict__ rc_off) {
     const uint32_t runs = *num_runs;
     // a trailing run of unusable intervals (key kNoGroup) sorts last and is dropped
@@ -571,7 +575,8 @@ __global__ void k_group_finish(const uint64_t* __restrict__ ukey, const LenAgg* 
     const double den = bin * (double)li;
     const double s2 = (double)a.s2hi * 18446744073709551616.0 + (double)a.s2lo;
     groups[g] = QGroupDev{(double)a.s1 / den, s2 / (den * den), (double)a.cnt / (double)li,
-                          chrom, li < slot_tab_len ? slot_tab[li] : 0xFFFFFFFFu, (double)li, (double)a.cnt};
+                          chrom, li < slot_tab_len ? slot_tab[li] : 0xFFFFFFFFu};
+    lens[g] = QGroupLen{(uint32_t)li, (uint32_t)a.cnt};
     const uint32_t rc_prev = g ? (uint32_t)(ukey[g - 1] >> 32) : 0xFFFFFFFFu;
     if (rc_prev != rc)  // (row, chromosome) pairs (rc_prev, rc] start at this group
         for (uint32_t r = (rc_prev == 0xFFFFFFFFu ? 0 : rc_prev + 1); r <= rc; r++) rc_off[r] = (uint32_t)g;
@@ -600,6 +605,8 @@ struct rgl_moments {
     bool tables_ready = false;
     std::mutex tab_mu;
     StatsScratch sc;
+    DevBuf host_part;  // rgl_query_pvalues' scratch, under host_mu
+    std::mutex host_mu;
 };
 
 namespace rgl {
@@ -718,7 +725,7 @@ int rgl_moments_destroy(rgl_moments* m) {
     clear_error();
     if (!m) return RGL_OK;
     cudaSetDevice(m->device);
-    for (DevBuf* b : {&m->slot_tab, &m->coff, &m->nb}) b->release();
+    for (DevBuf* b : {&m->slot_tab, &m->coff, &m->nb, &m->host_part}) b->release();
     stats_scratch_release(&m->sc);
     if (m->d_mv) cudaFree(m->d_mv);
     if (m->d_len) cudaFree(m->d_len);
@@ -775,11 +782,22 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
     const uint64_t cells = (uint64_t)rows * D;
     if (!cells) return RGL_OK;
     // flatten the groups: validity on the host (l_int < n_bins of the chromosome, as the store's
-    // lookup requires, src/io/momentstore.rs:66-79); slot by compact_index; (row, chromosome) by (row, chromosome) with the slots ascending, as k_pvalues walks them
+    // lookup requires, src/io/momentstore.rs:66-79); slot by compact_index; every row by (chromosome, slot) as
+    // k_pvalues walks them (rows that are in that order already, as the library builds them, are not sorted:
+    // 2.4 of 5 ms for 1.7e5 groups of 128 rows)
     std::vector<uint32_t> rcoff((uint64_t)rows * C + 1, 0);
     std::vector<QGroupDev> gs;
+    uint64_t most = 0;
+    for (uint32_t q = 0; q < rows; q++)
+        if (b->row_group_offsets[q + 1] > b->row_group_offsets[q])
+            most += b->row_group_offsets[q + 1] - b->row_group_offsets[q];
+    gs.reserve(most);
+    const auto before = [](const QGroupDev& x, const QGroupDev& y) {
+        return x.chrom != y.chrom ? x.chrom < y.chrom : x.slot < y.slot;
+    };
     for (uint32_t q = 0; q < rows; q++) {
         const size_t first = gs.size();
+        bool ordered = true;
         for (uint64_t g = b->row_group_offsets[q]; g < b->row_group_offsets[q + 1]; g++) {
             const uint32_t c = b->group_chrom[g];
             if (c >= C) return fail(RGL_ERR_INVALID_ARGUMENT, "group chromosome out of range");
@@ -788,13 +806,11 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
             const uint64_t slot = compact_index(l);
             if (slot >= m->n_slots[c]) continue;
             const double cnt = (double)b->group_count[g];
-            gs.push_back(QGroupDev{b->group_sum_scale[g], b->group_sum_scale2[g], cnt / (double)l, c, (uint32_t)slot,
-                                   (double)l, cnt});
+            gs.push_back(QGroupDev{b->group_sum_scale[g], b->group_sum_scale2[g], cnt / (double)l, c, (uint32_t)slot});
+            if (gs.size() > first + 1 && before(gs.back(), gs[gs.size() - 2])) ordered = false;
         }
         if (gs.size() >= (1ull << 32)) return fail(RGL_ERR_INVALID_ARGUMENT, "at most 2^32 - 1 groups per call");
-        std::stable_sort(gs.begin() + first, gs.end(), [](const QGroupDev& x, const QGroupDev& y) {
-            return x.chrom != y.chrom ? x.chrom < y.chrom : x.slot < y.slot;
-        });
+        if (!ordered) std::stable_sort(gs.begin() + first, gs.end(), before);
         size_t at = first;
         for (uint32_t c = 0; c < C; c++) {
             while (at < gs.size() && gs[at].chrom == c) at++;
@@ -802,10 +818,9 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
         }
     }
     RGL_CUDA(cudaSetDevice(m->device));
-    DevBuf d_goff, d_g, d_coff, d_cnt, d_bp, d_p, d_llr, d_lp, d_f, d_part;
+    DevBuf d_off, d_g, d_coff, d_cnt, d_bp, d_p, d_llr, d_lp, d_f;
     int s = RGL_OK;
-    if (s == RGL_OK) s = d_goff.ensure(rcoff.size() * 4);
-    if (s == RGL_OK) s = d_part.ensure(pv_scratch_bytes(rows, D, C));
+    if (s == RGL_OK) s = d_off.ensure(rcoff.size() * 4);
     if (s == RGL_OK) s = d_g.ensure(std::max<size_t>(1, gs.size()) * sizeof(QGroupDev));
     if (s == RGL_OK) s = d_coff.ensure(C * 8ull);
     if (s == RGL_OK) s = d_cnt.ensure(cells * 4);
@@ -818,16 +833,22 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
         if (s == RGL_OK && n && cudaMemcpy(dst, src, n, cudaMemcpyHostToDevice) != cudaSuccess)
             s = fail(RGL_ERR_DEVICE, "p-value upload");
     };
-    cp(d_goff.p, rcoff.data(), rcoff.size() * 4);
+    cp(d_off.p, rcoff.data(), rcoff.size() * 4);
     cp(d_g.p, gs.data(), gs.size() * sizeof(QGroupDev));
     cp(d_coff.p, m->chrom_off.data(), C * 8);
     cp(d_cnt.p, counts, cells * 4);
     cp(d_bp.p, overlap_bp, cells * 8);
-    if (s == RGL_OK)
-        s = launch_pvalues(rows, D, C, d_cnt.as<uint32_t>(), d_bp.as<unsigned long long>(), (double)bin_size,
-                           d_goff.as<uint32_t>(), d_g.as<QGroupDev>(), m->d_mv, d_coff.as<uint64_t>(), m->stride,
-                           m->d_len, d_p.as<double>(), d_llr.as<double>(), d_lp.as<double>(), d_f.as<uint8_t>(),
-                           d_part.p, 0);
+    if (s == RGL_OK) {
+        // the scratch stays with the store (an allocation and release of 1 MB or more take 600 us, more than the
+        // kernels); calls of several threads take turns to launch, and their kernels run in turn on the one stream
+        std::lock_guard<std::mutex> lk(m->host_mu);
+        s = m->host_part.ensure(pv_scratch_bytes(rows, D, C));
+        if (s == RGL_OK)
+            s = launch_pvalues(rows, D, C, d_cnt.as<uint32_t>(), d_bp.as<unsigned long long>(), (double)bin_size,
+                               d_off.as<uint32_t>(), d_g.as<QGroupDev>(), m->d_mv, d_coff.as<uint64_t>(), m->stride,
+                               m->d_len, d_p.as<double>(), d_llr.as<double>(), d_lp.as<double>(), d_f.as<uint8_t>(),
+                               m->host_part.p, 0);
+    }
     auto back = [&](void* dst, const void* src, size_t n) {
         if (s == RGL_OK && dst && cudaMemcpy(dst, src, n, cudaMemcpyDeviceToHost) != cudaSuccess)
             s = fail(RGL_ERR_DEVICE, "p-value download");
@@ -836,8 +857,7 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
     back(llr, d_llr.p, cells * 8);
     back(log_p, d_lp.p, cells * 8);
     back(flags, d_f.p, cells);
-    for (DevBuf* x : {&d_goff, &d_g, &d_coff, &d_cnt, &d_bp, &d_p, &d_llr, &d_lp, &d_f, &d_part})
-        x->release();
+    for (DevBuf* x : {&d_off, &d_g, &d_coff, &d_cnt, &d_bp, &d_p, &d_llr, &d_lp, &d_f}) x->release();
     return s;
 }
 
@@ -946,7 +966,7 @@ static int enqueue_batch_groups(rgl_context* ctx, rgl_moments* m, StatsScratch* 
     RGL_TRY(sc->len_b.ensure(nn * 4));
     RGL_TRY(sc->ukey.ensure(nn * 8));
     RGL_TRY(sc->agg.ensure(nn * sizeof(LenAgg)));
-    RGL_TRY(sc->groups.ensure(nn * sizeof(QGroupDev)));
+    RGL_TRY(sc->groups.ensure(nn * (sizeof(QGroupDev) + sizeof(QGroupLen))));  // one after the other
     RGL_TRY(sc->goff.ensure((rows + 1ull) * 8 + (nblk + 1ull) * 8 + tabs.size() * 4 + 64));
     RGL_TRY(sc->runs.ensure(64));
     RGL_TRY(sc->rcoff.ensure(((uint64_t)rows * C + 1) * 4));
@@ -1021,7 +1041,8 @@ static int enqueue_batch_groups(rgl_context* ctx, rgl_moments* m, StatsScratch* 
     }
     k_group_finish<<<(unsigned)((nn + 256) / 256), 256, 0, st>>>(
         sc->ukey.as<uint64_t>(), sc->agg.as<LenAgg>(), sc->runs.as<uint32_t>(), rows, C, (double)bin_size,
-        m->slot_tab.as<uint32_t>(), lmax, sc->groups.as<QGroupDev>(), d_goff, sc->rcoff.as<uint32_t>());
+        m->slot_tab.as<uint32_t>(), lmax, sc->groups.as<QGroupDev>(),
+        reinterpret_cast<QGroupLen*>(sc->groups.as<QGroupDev>() + nn), d_goff, sc->rcoff.as<uint32_t>());
     RGL_CUDA(cudaGetLastError());
     *goff_out = d_goff;
     return RGL_OK;
@@ -1098,13 +1119,19 @@ int rgl_batch_query_groups(rgl_context* ctx, rgl_moments* m, const rgl_batch* b,
     if (!group_chrom && !group_l_int && !group_sum_scale && !group_sum_scale2 && !group_count) return RGL_OK;
     if (ng > capacity) return fail(RGL_ERR_INVALID_ARGUMENT, "group capacity too small");
     std::vector<QGroupDev> g(ng);
-    if (ng) RGL_CUDA(cudaMemcpy(g.data(), m->sc.groups.p, ng * sizeof(QGroupDev), cudaMemcpyDeviceToHost));
+    std::vector<QGroupLen> len(ng);
+    if (ng) {
+        const uint64_t nn = b->block_offsets[b->num_blocks] - b->block_offsets[0];
+        const QGroupDev* d_g = m->sc.groups.as<QGroupDev>();
+        RGL_CUDA(cudaMemcpy(g.data(), d_g, ng * sizeof(QGroupDev), cudaMemcpyDeviceToHost));
+        RGL_CUDA(cudaMemcpy(len.data(), d_g + nn, ng * sizeof(QGroupLen), cudaMemcpyDeviceToHost));
+    }
     for (uint64_t k = 0; k < ng; k++) {
         if (group_chrom) group_chrom[k] = g[k].chrom;
-        if (group_l_int) group_l_int[k] = (uint64_t)g[k].l_int;
+        if (group_l_int) group_l_int[k] = len[k].l_int;
         if (group_sum_scale) group_sum_scale[k] = g[k].ss;
         if (group_sum_scale2) group_sum_scale2[k] = g[k].ss2;
-        if (group_count) group_count[k] = (uint64_t)g[k].count;
+        if (group_count) group_count[k] = len[k].count;
     }
     return RGL_OK;
 }
