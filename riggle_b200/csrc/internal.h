@@ -186,6 +186,8 @@ void stats_scratch_release(StatsScratch* sc);
 // fewer for more rows, where the former may be).
 uint64_t pv_scratch_bytes(uint32_t rows, uint32_t D, uint32_t C);
 uint64_t pv_scratch_bound(uint32_t rows, uint32_t D, uint32_t C);
+// Device bytes of StatsScratch::rcoff.
+uint64_t pv_offset_bytes(uint32_t rows, uint32_t C);
 uint32_t moments_chroms(const rgl_moments* m);
 uint32_t context_last_launches(rgl_context* c);
 

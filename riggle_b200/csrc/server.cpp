@@ -202,7 +202,7 @@ int batch_growth(rgl_server* S, Worker* W, uint64_t n, uint32_t R, uint32_t nblk
              grow(W->sc.len_b, n * 4 + 4) + grow(W->sc.ukey, n * 8 + 8) + grow(W->sc.agg, n * 32 + 32) +
              grow(W->sc.groups, n * 40 + 40) + grow(W->sc.plan, stats_plan_bytes(n, nblk)) +
              grow(W->sc.goff, stats_goff_bytes(S, R, nblk)) + grow(W->sc.runs, 64) +
-             grow(W->sc.rcoff, ((uint64_t)R * S->chroms + 1) * 4) +
+             grow(W->sc.rcoff, pv_offset_bytes(R, S->chroms)) +
              grow(W->sc.part, pv_scratch_bound(R, S->D, S->chroms));
     }
     *bytes = b;
@@ -231,7 +231,7 @@ int size_worker(rgl_server* S, Worker* W, uint64_t n, uint32_t R, uint32_t nblk)
         RGL_TRY(W->sc.plan.ensure(stats_plan_bytes(nn, nblk)));
         RGL_TRY(W->sc.goff.ensure(stats_goff_bytes(S, R, nblk)));
         RGL_TRY(W->sc.runs.ensure(64));
-        RGL_TRY(W->sc.rcoff.ensure(((uint64_t)R * S->chroms + 1) * 4));
+        RGL_TRY(W->sc.rcoff.ensure(pv_offset_bytes(R, S->chroms)));
         RGL_TRY(W->sc.part.ensure(pv_scratch_bound(R, S->D, S->chroms)));
     }
     return RGL_OK;

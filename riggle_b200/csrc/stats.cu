@@ -136,7 +136,7 @@ __device__ __forceinline__ void pvalue_cell(uint32_t count, uint32_t any, double
 }
 
 // The sums over the groups.  A block takes 16 sources, WARPS x ROWS query rows (a warp takes ROWS of them
-// one after the other) and all chromosomes or (with `part`, one of `parts` blocks) chromosome c0 + its part.  Per chromosome the sources' table entries
+// one after the other) and all chromosomes or (parts = C) one.  Per chromosome the sources' table entries
 // are staged in shared memory, slot by slot with the sources side by side (zero past a table's end); each
 // half-warp walks every second group of a row on that chromosome, a group read once for its 16 lanes, each
 // with its own source's entry and its own three sums, so that nothing is reduced over lanes but the two
@@ -152,7 +152,7 @@ struct PvCell {
 };
 template <int ROWS, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) k_pvalues(
-    uint32_t rows, uint32_t D, uint32_t C, uint32_t c0, uint32_t parts, const uint32_t* __restrict__ counts,
+    uint32_t rows, uint32_t D, uint32_t C, uint32_t parts, const uint32_t* __restrict__ counts,
     const unsigned long long* __restrict__ bp, double bin_size, const uint32_t* __restrict__ rc_off,
     const QGroupDev* __restrict__ groups, const float2* __restrict__ mv, const uint64_t* __restrict__ chrom_off,
     uint64_t stride, const uint32_t* __restrict__ tab_len, double* __restrict__ p_out, double* __restrict__ llr_out,
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) k_pvalues(
     uint32_t any = 0;  // bit r: row r has a group in source d's tables
 #pragma unroll
     for (int r = 0; r < ROWS; r++) acc[r] = PvCell{0.0, 0.0, 0.0};
-    for (uint32_t c = part ? c0 + pt : 0u, c1 = part ? c + 1 : C; c < c1; c++) {
+    for (uint32_t c = parts > 1 ? pt : 0u; c < (parts > 1 ? pt + 1 : C); c++) {
         const uint32_t n_slots = (uint32_t)((c + 1 < C ? chrom_off[c + 1] : stride) - chrom_off[c]);
         // the slots that any row of the tile needs (a row's groups ascend by slot)
         if (threadIdx.x == 0) s_slots = 0;
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) k_pvalues(
         const uint32_t q = q0 + warp * ROWS + r;
         if (q >= rows) break;
         const uint64_t w = (uint64_t)q * D + d;
-        if (part) {
+        if (parts > 1) {
             const uint64_t x = (uint64_t)pt * rows * D + w;
             part[x] = acc[r];
             part_any[x] = any >> r & 1u;
@@ -266,19 +266,61 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) k_pvalues(
     }
 }
 
-// One cell per thread: the sums of `parts` chromosomes added up in order, onto those of the chromosomes before
-// them (not `first`: slot `keep` of the sums), then kept there, or (`last`) the p-value.
-__global__ void __launch_bounds__(128) k_pv_cells(uint64_t cells, uint32_t parts, uint32_t keep, int first, int last,
-                                                  PvCell* __restrict__ part, uint8_t* __restrict__ part_any,
+// The sums over the groups, and the p-value, of stores of more than kPvChroms chromosomes: a warp per cell, lanes
+// over the row's groups, each read with the source's entry.  Takes time by the groups there are, where k_pvalues
+// takes it by chromosomes and table entries.  500 sources, the same groups in 24, 48, 64, 100, 455 chromosomes: 128
+// files 206, 283, 343, 474, 1,445 us by k_pvalues and 293, 314, 329, 370, 653 by this; one file 22, 31, 34, 45, 127
+// and 28, 30, 32, 37, 63; 455 chromosomes of which 24 have groups 738 and 221.  The line is drawn by the store, not by
+// the batch, whose rows would otherwise add up in another order alone than together.
+constexpr uint32_t kPvChroms = 64;
+__global__ void __launch_bounds__(256) k_pvalues_cells(
+    uint32_t rows, uint32_t D, uint32_t C, const uint32_t* __restrict__ counts,
+    const unsigned long long* __restrict__ bp, double bin_size, const uint64_t* __restrict__ g_off,
+    const QGroupDev* __restrict__ groups, const float2* __restrict__ mv, const uint64_t* __restrict__ chrom_off,
+    uint64_t stride, const uint32_t* __restrict__ tab_len, double* __restrict__ p_out, double* __restrict__ llr_out,
+    double* __restrict__ logp_out, uint8_t* __restrict__ flags) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5, cells = (uint64_t)rows * D;
+    for (uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; w < cells; w += nw) {
+        const uint32_t q = (uint32_t)(w / D), d = (uint32_t)(w % D);
+        PvCell s{0.0, 0.0, 0.0};
+        uint32_t any = 0;
+        const uint32_t count = counts[w];
+        const float2* src = mv + (uint64_t)d * stride;
+        for (uint64_t g = g_off[q] + lane; count && g < g_off[q + 1]; g += 32) {
+            const double2 a = __ldg(reinterpret_cast<const double2*>(groups + g));      // ss, ss2
+            const uint4 b = __ldg(reinterpret_cast<const uint4*>(groups + g) + 1);  // cr, chrom, slot
+            if (b.w >= __ldg(tab_len + (uint64_t)d * C + b.z)) continue;
+            const float2 v = __ldg(src + chrom_off[b.z] + b.w);
+            const double mean = (double)v.x;
+            s.mu += mean * a.x;
+            s.var += (double)v.y * a.y;
+            s.raw += mean * __hiloint2double((int)b.y, (int)b.x);
+            any = 1;
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            s.mu += __shfl_xor_sync(0xffffffffu, s.mu, o);
+            s.var += __shfl_xor_sync(0xffffffffu, s.var, o);
+            s.raw += __shfl_xor_sync(0xffffffffu, s.raw, o);
+        }
+        any = __any_sync(0xffffffffu, any);
+        if (lane == 0)
+            pvalue_cell(count, any, s.mu, s.var, s.raw, bp[w], bin_size, w, p_out, llr_out, logp_out, flags);
+    }
+}
+
+// One cell per thread: the parts of the chromosomes added up in order, then the p-value.
+__global__ void __launch_bounds__(128) k_pv_cells(uint64_t cells, uint32_t parts, const PvCell* __restrict__ part,
+                                                  const uint8_t* __restrict__ part_any,
                                                   const uint32_t* __restrict__ counts,
                                                   const unsigned long long* __restrict__ bp, double bin_size,
                                                   double* __restrict__ p_out, double* __restrict__ llr_out,
                                                   double* __restrict__ logp_out, uint8_t* __restrict__ flags) {
     const uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (w >= cells) return;
-    const uint64_t kept = keep * cells + w;
-    PvCell s = first ? PvCell{0.0, 0.0, 0.0} : part[kept];
-    uint32_t any = first ? 0u : part_any[kept];
+    PvCell s{0.0, 0.0, 0.0};
+    uint32_t any = 0;
     for (uint32_t k = 0; k < parts; k++) {
         const PvCell v = part[k * cells + w];
         s.mu += v.mu;
@@ -286,75 +328,66 @@ __global__ void __launch_bounds__(128) k_pv_cells(uint64_t cells, uint32_t parts
         s.raw += v.raw;
         any |= part_any[k * cells + w];
     }
-    if (!last) {
-        part[kept] = s;
-        part_any[kept] = (uint8_t)any;
-        return;
-    }
     pvalue_cell(counts[w], any, s.mu, s.var, s.raw, bp[w], bin_size, w, p_out, llr_out, logp_out, flags);
 }
 
-// Shape of a launch: 32 rows a block (two a warp), or four where there are fewer than 16; a block per
-// chromosome where that leaves fewer than four for each of 148 SMs.  The blocks' sums are kept per chromosome for
-// at most kPvScratch bytes (24 chromosomes at the most cells that are split); of more chromosomes, `parts` at a time
-// with the sums so far in one more slot, in the same order.  (All of 3,000 chromosomes at once were 3 GB for 40,000
-// cells.)
-constexpr uint64_t kPvFill = 148 * 4, kPvScratch = 192ull << 20, kPvCellBytes = sizeof(PvCell) + 1;
+// Shape of a launch of k_pvalues: 32 rows a block (two a warp), or four where there are fewer than 16; a block per
+// chromosome where that leaves fewer than four for each of 148 SMs.
+constexpr uint64_t kPvFill = 148 * 4;
 struct PvShape {
-    bool many, split;
-    uint32_t parts;        // chromosomes at a time
-    uint64_t tiles, slots; // of 16 sources x rows; sums kept per cell
+    bool many;
+    uint32_t parts;
+    uint64_t blocks;
 };
 PvShape pv_shape(uint32_t rows, uint32_t D, uint32_t C) {
-    PvShape s{rows >= 16, false, 1, 0, 0};
+    PvShape s{rows >= 16, 1, 0};
     const uint64_t per_tile = s.many ? 32 : 4;
-    s.tiles = ((rows + per_tile - 1) / per_tile) * (((uint64_t)D + kPvSources - 1) / kPvSources);
-    if (C > 1 && s.tiles < kPvFill) {
-        const uint64_t room = kPvScratch / std::max<uint64_t>(1, (uint64_t)rows * D * kPvCellBytes);
-        s.split = true;
-        s.slots = std::min<uint64_t>({C, room, 65536});  // (the grid's size fits 31 bits)
-        s.parts = (uint32_t)(s.slots == C ? C : s.slots - 1);
-    }
+    const uint64_t tiles = ((rows + per_tile - 1) / per_tile) * (((uint64_t)D + kPvSources - 1) / kPvSources);
+    if (tiles < kPvFill) s.parts = C;
+    s.blocks = tiles * s.parts;
     return s;
 }
-static_assert((kPvFill - 1) * 32 * kPvSources * kPvCellBytes * 2 <= kPvScratch, "room for a chromosome and the sums so far");
+uint64_t pv_part_bytes(uint64_t rows, uint32_t D, uint32_t parts) {
+    return parts > 1 ? parts * rows * D * (sizeof(PvCell) + 1) + 64 : 0;
+}
 uint64_t pv_scratch_bytes(uint32_t rows, uint32_t D, uint32_t C) {
-    const PvShape s = pv_shape(rows, D, C);
-    return s.split ? s.slots * rows * D * kPvCellBytes + 64 : 0;
+    return C > kPvChroms ? 0 : pv_part_bytes(rows, D, pv_shape(rows, D, C).parts);
 }
 // The scratch falls to nothing where the rows alone fill the chip, and comes back at 16 rows, where the tiles
 // grow: the bound is that of the largest row count up to `rows` whose launch is split.
 uint64_t pv_scratch_bound(uint32_t rows, uint32_t D, uint32_t C) {
-    if (C < 2) return 0;
+    if (C > kPvChroms) return 0;
     const uint64_t tiles = (kPvFill - 1) / std::max<uint64_t>(1, ((uint64_t)D + kPvSources - 1) / kPvSources);
     const uint64_t many = std::min<uint64_t>(rows, 32 * tiles), few = std::min<uint64_t>({rows, 15, 4 * tiles});
-    const uint64_t cells = (many >= 16 ? many : few) * D;
-    return std::min(C * cells * kPvCellBytes, kPvScratch) + 64;
+    return pv_part_bytes(many >= 16 ? many : few, D, C);
 }
-// scratch: pv_scratch_bytes of device memory.
+uint64_t pv_offset_bytes(uint32_t rows, uint32_t C) { return C > kPvChroms ? 0 : ((uint64_t)rows * C + 1) * 4; }
+// g_off: the rows' groups; rc_off: those of (row, chromosome), unless there are more than kPvChroms; scratch:
+// pv_scratch_bytes of device memory.
 int launch_pvalues(uint32_t rows, uint32_t D, uint32_t C, const uint32_t* counts, const unsigned long long* bp,
-                   double bin_size, const uint32_t* rc_off, const QGroupDev* groups, const float2* mv,
-                   const uint64_t* chrom_off, uint64_t stride, const uint32_t* tab_len, double* p, double* llr,
-                   double* logp, uint8_t* flags, void* scratch, cudaStream_t st) {
-    const PvShape s = pv_shape(rows, D, C);
+                   double bin_size, const uint64_t* g_off, const uint32_t* rc_off, const QGroupDev* groups,
+                   const float2* mv, const uint64_t* chrom_off, uint64_t stride, const uint32_t* tab_len, double* p,
+                   double* llr, double* logp, uint8_t* flags, void* scratch, cudaStream_t st) {
     const uint64_t cells = (uint64_t)rows * D;
-    if (s.tiles * s.parts >= (1ull << 31)) return fail(RGL_ERR_INVALID_ARGUMENT, "too many cells for one call");
-    PvCell* part = s.split ? static_cast<PvCell*>(scratch) : nullptr;
-    uint8_t* any = reinterpret_cast<uint8_t*>(part + s.slots * cells);
-    for (uint32_t c0 = 0; c0 < (s.split ? C : 1u);) {
-        const uint32_t parts = s.split ? std::min(s.parts, C - c0) : 1u;
-        auto run = [&](auto kernel, int threads) {
-            kernel<<<(unsigned)(s.tiles * parts), threads, 0, st>>>(rows, D, C, c0, parts, counts, bp, bin_size, rc_off,
-                                                                   groups, mv, chrom_off, stride, tab_len, p, llr, logp,
-                                                                   flags, part, any);
-        };
-        if (s.many) run(k_pvalues<2, 16>, 512);
-        else run(k_pvalues<1, 4>, 128);
-        if (s.split)
-            k_pv_cells<<<(unsigned)((cells + 127) / 128), 128, 0, st>>>(cells, parts, s.parts, c0 == 0, c0 + parts == C, part,
-                                                                       any, counts, bp, bin_size, p, llr, logp, flags);
-        c0 += parts;
+    if (C > kPvChroms) {
+        k_pvalues_cells<<<(unsigned)std::min<uint64_t>((cells + 7) / 8, 148 * 8), 256, 0, st>>>(
+            rows, D, C, counts, bp, bin_size, g_off, groups, mv, chrom_off, stride, tab_len, p, llr, logp, flags);
+        RGL_CUDA(cudaGetLastError());
+        return RGL_OK;
     }
+    const PvShape s = pv_shape(rows, D, C);
+    if (s.blocks >= (1ull << 31)) return fail(RGL_ERR_INVALID_ARGUMENT, "too many cells for one call");
+    PvCell* part = static_cast<PvCell*>(scratch);
+    uint8_t* any = reinterpret_cast<uint8_t*>(part + (s.parts > 1 ? s.parts * cells : 0));
+    auto run = [&](auto kernel, int threads) {
+        kernel<<<(unsigned)s.blocks, threads, 0, st>>>(rows, D, C, s.parts, counts, bp, bin_size, rc_off, groups, mv,
+                                                      chrom_off, stride, tab_len, p, llr, logp, flags, part, any);
+    };
+    if (s.many) run(k_pvalues<2, 16>, 512);
+    else run(k_pvalues<1, 4>, 128);
+    if (s.parts > 1)
+        k_pv_cells<<<(unsigned)((cells + 127) / 128), 128, 0, st>>>(cells, s.parts, part, any, counts, bp, bin_size, p,
+                                                                   llr, logp, flags);
     RGL_CUDA(cudaGetLastError());
     return RGL_OK;
 }
@@ -555,7 +588,7 @@ __global__ void k_group_finish(const uint64_t* __restrict__ ukey, const LenAgg* 
                                const uint32_t* __restrict__ slot_tab, uint64_t slot_tab_len,
                                QGroupDev* __restrict__ groups, QGroupLen* __restrict__ lens,
                                uint64_t* __restrict__ g_off,
-                               uint32_t* __restrict__ rc_off) {
+                               uint32_t* __restrict__ rc_off) {  // null: not needed (launch_pvalues)
     const uint32_t runs = *num_runs;
     // a trailing run of unusable intervals (key kNoGroup) sorts last and is dropped
     const uint32_t ng = (runs && ukey[runs - 1] == kNoGroup) ? runs - 1 : runs;
@@ -565,7 +598,7 @@ __global__ void k_group_finish(const uint64_t* __restrict__ ukey, const LenAgg* 
         const uint32_t r0 = ng ? (uint32_t)((ukey[ng - 1] >> 32) / C) + 1 : 0;
         for (uint32_t r = r0; r <= rows; r++) g_off[r] = ng;
         const uint32_t rc0 = ng ? (uint32_t)(ukey[ng - 1] >> 32) + 1 : 0;
-        for (uint64_t r = rc0; r <= (uint64_t)rows * C; r++) rc_off[r] = ng;
+        for (uint64_t r = rc0; rc_off && r <= (uint64_t)rows * C; r++) rc_off[r] = ng;
         return;
     }
     const uint64_t k = ukey[g];
@@ -578,7 +611,7 @@ __global__ void k_group_finish(const uint64_t* __restrict__ ukey, const LenAgg* 
                           chrom, li < slot_tab_len ? slot_tab[li] : 0xFFFFFFFFu};
     lens[g] = QGroupLen{(uint32_t)li, (uint32_t)a.cnt};
     const uint32_t rc_prev = g ? (uint32_t)(ukey[g - 1] >> 32) : 0xFFFFFFFFu;
-    if (rc_prev != rc)  // (row, chromosome) pairs (rc_prev, rc] start at this group
+    if (rc_off && rc_prev != rc)  // (row, chromosome) pairs (rc_prev, rc] start at this group
         for (uint32_t r = (rc_prev == 0xFFFFFFFFu ? 0 : rc_prev + 1); r <= rc; r++) rc_off[r] = (uint32_t)g;
     const uint32_t prev = g ? (uint32_t)((ukey[g - 1] >> 32) / C) : 0xFFFFFFFFu;
     if (prev != row)  // rows (prev, row] start at this group
@@ -782,10 +815,12 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
     const uint64_t cells = (uint64_t)rows * D;
     if (!cells) return RGL_OK;
     // flatten the groups: validity on the host (l_int < n_bins of the chromosome, as the store's
-    // lookup requires, src/io/momentstore.rs:66-79); slot by compact_index; every row by (chromosome, slot) as
-    // k_pvalues walks them (rows that are in that order already, as the library builds them, are not sorted:
+    // lookup requires, src/io/momentstore.rs:66-79); slot by compact_index; every row by (chromosome, slot) where
+    // k_pvalues walks them so (rows that are in that order already, as the library builds them, are not sorted:
     // 2.4 of 5 ms for 1.7e5 groups of 128 rows)
-    std::vector<uint32_t> rcoff((uint64_t)rows * C + 1, 0);
+    const bool walked = C <= kPvChroms;
+    std::vector<uint64_t> goff(rows + 1ull, 0);
+    std::vector<uint32_t> rcoff(pv_offset_bytes(rows, C) / 4, 0);
     std::vector<QGroupDev> gs;
     uint64_t most = 0;
     for (uint32_t q = 0; q < rows; q++)
@@ -810,6 +845,8 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
             if (gs.size() > first + 1 && before(gs.back(), gs[gs.size() - 2])) ordered = false;
         }
         if (gs.size() >= (1ull << 32)) return fail(RGL_ERR_INVALID_ARGUMENT, "at most 2^32 - 1 groups per call");
+        goff[q + 1] = gs.size();
+        if (!walked) continue;
         if (!ordered) std::stable_sort(gs.begin() + first, gs.end(), before);
         size_t at = first;
         for (uint32_t c = 0; c < C; c++) {
@@ -820,7 +857,9 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
     RGL_CUDA(cudaSetDevice(m->device));
     DevBuf d_off, d_g, d_coff, d_cnt, d_bp, d_p, d_llr, d_lp, d_f;
     int s = RGL_OK;
-    if (s == RGL_OK) s = d_off.ensure(rcoff.size() * 4);
+    const void* offs = walked ? static_cast<const void*>(rcoff.data()) : goff.data();
+    const size_t off_bytes = walked ? rcoff.size() * 4 : goff.size() * 8;
+    if (s == RGL_OK) s = d_off.ensure(off_bytes);
     if (s == RGL_OK) s = d_g.ensure(std::max<size_t>(1, gs.size()) * sizeof(QGroupDev));
     if (s == RGL_OK) s = d_coff.ensure(C * 8ull);
     if (s == RGL_OK) s = d_cnt.ensure(cells * 4);
@@ -833,7 +872,7 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
         if (s == RGL_OK && n && cudaMemcpy(dst, src, n, cudaMemcpyHostToDevice) != cudaSuccess)
             s = fail(RGL_ERR_DEVICE, "p-value upload");
     };
-    cp(d_off.p, rcoff.data(), rcoff.size() * 4);
+    cp(d_off.p, offs, off_bytes);
     cp(d_g.p, gs.data(), gs.size() * sizeof(QGroupDev));
     cp(d_coff.p, m->chrom_off.data(), C * 8);
     cp(d_cnt.p, counts, cells * 4);
@@ -845,7 +884,7 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
         s = m->host_part.ensure(pv_scratch_bytes(rows, D, C));
         if (s == RGL_OK)
             s = launch_pvalues(rows, D, C, d_cnt.as<uint32_t>(), d_bp.as<unsigned long long>(), (double)bin_size,
-                               d_off.as<uint32_t>(), d_g.as<QGroupDev>(), m->d_mv, d_coff.as<uint64_t>(), m->stride,
+                               d_off.as<uint64_t>(), d_off.as<uint32_t>(), d_g.as<QGroupDev>(), m->d_mv, d_coff.as<uint64_t>(), m->stride,
                                m->d_len, d_p.as<double>(), d_llr.as<double>(), d_lp.as<double>(), d_f.as<uint8_t>(),
                                m->host_part.p, 0);
     }
@@ -969,7 +1008,7 @@ static int enqueue_batch_groups(rgl_context* ctx, rgl_moments* m, StatsScratch* 
     RGL_TRY(sc->groups.ensure(nn * (sizeof(QGroupDev) + sizeof(QGroupLen))));  // one after the other
     RGL_TRY(sc->goff.ensure((rows + 1ull) * 8 + (nblk + 1ull) * 8 + tabs.size() * 4 + 64));
     RGL_TRY(sc->runs.ensure(64));
-    RGL_TRY(sc->rcoff.ensure(((uint64_t)rows * C + 1) * 4));
+    RGL_TRY(sc->rcoff.ensure(pv_offset_bytes(rows, C)));
     if (local) RGL_TRY(sc->plan.ensure((3ull * nblk + 2 * tiles + 8) * 4));
     uint64_t* d_goff = sc->goff.as<uint64_t>();
     uint64_t* d_boff = d_goff + rows + 1;
@@ -1042,7 +1081,8 @@ static int enqueue_batch_groups(rgl_context* ctx, rgl_moments* m, StatsScratch* 
     k_group_finish<<<(unsigned)((nn + 256) / 256), 256, 0, st>>>(
         sc->ukey.as<uint64_t>(), sc->agg.as<LenAgg>(), sc->runs.as<uint32_t>(), rows, C, (double)bin_size,
         m->slot_tab.as<uint32_t>(), lmax, sc->groups.as<QGroupDev>(),
-        reinterpret_cast<QGroupLen*>(sc->groups.as<QGroupDev>() + nn), d_goff, sc->rcoff.as<uint32_t>());
+        reinterpret_cast<QGroupLen*>(sc->groups.as<QGroupDev>() + nn), d_goff,
+        C > kPvChroms ? nullptr : sc->rcoff.as<uint32_t>());
     RGL_CUDA(cudaGetLastError());
     *goff_out = d_goff;
     return RGL_OK;
@@ -1069,7 +1109,7 @@ int batch_pvalues_enqueue(rgl_context* ctx, rgl_moments* m, StatsScratch* sc, co
     // groups whose slot lies past the source's table (slot >= tab_len) are dropped there
     RGL_TRY(sc->part.ensure(pv_scratch_bytes(rows, D, C)));
     RGL_TRY(launch_pvalues(rows, D, C, d_counts, reinterpret_cast<const unsigned long long*>(d_overlap_bp),
-                           (double)bin_size, sc->rcoff.as<uint32_t>(), sc->groups.as<QGroupDev>(), m->d_mv,
+                           (double)bin_size, d_goff, sc->rcoff.as<uint32_t>(), sc->groups.as<QGroupDev>(), m->d_mv,
                            m->coff.as<uint64_t>(), m->stride, m->d_len, d_p, d_llr, d_log_p, d_flags, sc->part.p, st));
     if (out_groups) {
         uint64_t ng = 0;
