@@ -273,6 +273,7 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) k_pvalues(
 // and 28, 30, 32, 37, 63; 455 chromosomes of which 24 have groups 738 and 221.  The line is drawn by the store, not by
 // the batch, whose rows would otherwise add up in another order alone than together.
 constexpr uint32_t kPvChroms = 64;
+bool pv_walks(uint32_t C) { return C <= kPvChroms; }
 __global__ void __launch_bounds__(256) k_pvalues_cells(
     uint32_t rows, uint32_t D, uint32_t C, const uint32_t* __restrict__ counts,
     const unsigned long long* __restrict__ bp, double bin_size, const uint64_t* __restrict__ g_off,
@@ -351,25 +352,26 @@ uint64_t pv_part_bytes(uint64_t rows, uint32_t D, uint32_t parts) {
     return parts > 1 ? parts * rows * D * (sizeof(PvCell) + 1) + 64 : 0;
 }
 uint64_t pv_scratch_bytes(uint32_t rows, uint32_t D, uint32_t C) {
-    return C > kPvChroms ? 0 : pv_part_bytes(rows, D, pv_shape(rows, D, C).parts);
+    return pv_walks(C) ? pv_part_bytes(rows, D, pv_shape(rows, D, C).parts) : 0;
 }
 // The scratch falls to nothing where the rows alone fill the chip, and comes back at 16 rows, where the tiles
 // grow: the bound is that of the largest row count up to `rows` whose launch is split.
 uint64_t pv_scratch_bound(uint32_t rows, uint32_t D, uint32_t C) {
-    if (C > kPvChroms) return 0;
+    if (!pv_walks(C)) return 0;
     const uint64_t tiles = (kPvFill - 1) / std::max<uint64_t>(1, ((uint64_t)D + kPvSources - 1) / kPvSources);
     const uint64_t many = std::min<uint64_t>(rows, 32 * tiles), few = std::min<uint64_t>({rows, 15, 4 * tiles});
     return pv_part_bytes(many >= 16 ? many : few, D, C);
 }
-uint64_t pv_offset_bytes(uint32_t rows, uint32_t C) { return C > kPvChroms ? 0 : ((uint64_t)rows * C + 1) * 4; }
-// g_off: the rows' groups; rc_off: those of (row, chromosome), unless there are more than kPvChroms; scratch:
-// pv_scratch_bytes of device memory.
-int launch_pvalues(uint32_t rows, uint32_t D, uint32_t C, const uint32_t* counts, const unsigned long long* bp,
+uint64_t pv_offset_bytes(uint32_t rows, uint32_t C) { return pv_walks(C) ? ((uint64_t)rows * C + 1) * 4 : 0; }
+// walk (pv_walks, and every group's sums finite: k_pvalues adds zero times a group that is past a source's table):
+// k_pvalues with rc_off, the groups of (row, chromosome), and pv_scratch_bytes of device memory as scratch; else
+// k_pvalues_cells with g_off, the rows' groups.
+int launch_pvalues(bool walk, uint32_t rows, uint32_t D, uint32_t C, const uint32_t* counts, const unsigned long long* bp,
                    double bin_size, const uint64_t* g_off, const uint32_t* rc_off, const QGroupDev* groups,
                    const float2* mv, const uint64_t* chrom_off, uint64_t stride, const uint32_t* tab_len, double* p,
                    double* llr, double* logp, uint8_t* flags, void* scratch, cudaStream_t st) {
     const uint64_t cells = (uint64_t)rows * D;
-    if (C > kPvChroms) {
+    if (!walk) {
         k_pvalues_cells<<<(unsigned)std::min<uint64_t>((cells + 7) / 8, 148 * 8), 256, 0, st>>>(
             rows, D, C, counts, bp, bin_size, g_off, groups, mv, chrom_off, stride, tab_len, p, llr, logp, flags);
         RGL_CUDA(cudaGetLastError());
@@ -818,7 +820,7 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
     // lookup requires, src/io/momentstore.rs:66-79); slot by compact_index; every row by (chromosome, slot) where
     // k_pvalues walks them so (rows that are in that order already, as the library builds them, are not sorted:
     // 2.4 of 5 ms for 1.7e5 groups of 128 rows)
-    const bool walked = C <= kPvChroms;
+    bool walk = pv_walks(C);
     std::vector<uint64_t> goff(rows + 1ull, 0);
     std::vector<uint32_t> rcoff(pv_offset_bytes(rows, C) / 4, 0);
     std::vector<QGroupDev> gs;
@@ -841,12 +843,13 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
             const uint64_t slot = compact_index(l);
             if (slot >= m->n_slots[c]) continue;
             const double cnt = (double)b->group_count[g];
+            if (!std::isfinite(b->group_sum_scale[g]) || !std::isfinite(b->group_sum_scale2[g])) walk = false;
             gs.push_back(QGroupDev{b->group_sum_scale[g], b->group_sum_scale2[g], cnt / (double)l, c, (uint32_t)slot});
             if (gs.size() > first + 1 && before(gs.back(), gs[gs.size() - 2])) ordered = false;
         }
         if (gs.size() >= (1ull << 32)) return fail(RGL_ERR_INVALID_ARGUMENT, "at most 2^32 - 1 groups per call");
         goff[q + 1] = gs.size();
-        if (!walked) continue;
+        if (!walk) continue;
         if (!ordered) std::stable_sort(gs.begin() + first, gs.end(), before);
         size_t at = first;
         for (uint32_t c = 0; c < C; c++) {
@@ -857,8 +860,8 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
     RGL_CUDA(cudaSetDevice(m->device));
     DevBuf d_off, d_g, d_coff, d_cnt, d_bp, d_p, d_llr, d_lp, d_f;
     int s = RGL_OK;
-    const void* offs = walked ? static_cast<const void*>(rcoff.data()) : goff.data();
-    const size_t off_bytes = walked ? rcoff.size() * 4 : goff.size() * 8;
+    const void* offs = walk ? static_cast<const void*>(rcoff.data()) : goff.data();
+    const size_t off_bytes = walk ? rcoff.size() * 4 : goff.size() * 8;
     if (s == RGL_OK) s = d_off.ensure(off_bytes);
     if (s == RGL_OK) s = d_g.ensure(std::max<size_t>(1, gs.size()) * sizeof(QGroupDev));
     if (s == RGL_OK) s = d_coff.ensure(C * 8ull);
@@ -881,9 +884,9 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
         // the scratch stays with the store (an allocation and release of 1 MB or more take 600 us, more than the
         // kernels); calls of several threads take turns to launch, and their kernels run in turn on the one stream
         std::lock_guard<std::mutex> lk(m->host_mu);
-        s = m->host_part.ensure(pv_scratch_bytes(rows, D, C));
+        if (walk) s = m->host_part.ensure(pv_scratch_bytes(rows, D, C));
         if (s == RGL_OK)
-            s = launch_pvalues(rows, D, C, d_cnt.as<uint32_t>(), d_bp.as<unsigned long long>(), (double)bin_size,
+            s = launch_pvalues(walk, rows, D, C, d_cnt.as<uint32_t>(), d_bp.as<unsigned long long>(), (double)bin_size,
                                d_off.as<uint64_t>(), d_off.as<uint32_t>(), d_g.as<QGroupDev>(), m->d_mv, d_coff.as<uint64_t>(), m->stride,
                                m->d_len, d_p.as<double>(), d_llr.as<double>(), d_lp.as<double>(), d_f.as<uint8_t>(),
                                m->host_part.p, 0);
@@ -1082,7 +1085,7 @@ static int enqueue_batch_groups(rgl_context* ctx, rgl_moments* m, StatsScratch* 
         sc->ukey.as<uint64_t>(), sc->agg.as<LenAgg>(), sc->runs.as<uint32_t>(), rows, C, (double)bin_size,
         m->slot_tab.as<uint32_t>(), lmax, sc->groups.as<QGroupDev>(),
         reinterpret_cast<QGroupLen*>(sc->groups.as<QGroupDev>() + nn), d_goff,
-        C > kPvChroms ? nullptr : sc->rcoff.as<uint32_t>());
+        pv_walks(C) ? sc->rcoff.as<uint32_t>() : nullptr);
     RGL_CUDA(cudaGetLastError());
     *goff_out = d_goff;
     return RGL_OK;
@@ -1108,7 +1111,7 @@ int batch_pvalues_enqueue(rgl_context* ctx, rgl_moments* m, StatsScratch* sc, co
     cudaStream_t st = context_stream(ctx);
     // groups whose slot lies past the source's table (slot >= tab_len) are dropped there
     RGL_TRY(sc->part.ensure(pv_scratch_bytes(rows, D, C)));
-    RGL_TRY(launch_pvalues(rows, D, C, d_counts, reinterpret_cast<const unsigned long long*>(d_overlap_bp),
+    RGL_TRY(launch_pvalues(pv_walks(C), rows, D, C, d_counts, reinterpret_cast<const unsigned long long*>(d_overlap_bp),
                            (double)bin_size, d_goff, sc->rcoff.as<uint32_t>(), sc->groups.as<QGroupDev>(), m->d_mv,
                            m->coff.as<uint64_t>(), m->stride, m->d_len, d_p, d_llr, d_log_p, d_flags, sc->part.p, st));
     if (out_groups) {
