@@ -2736,10 +2736,10 @@ void graph_drop(rgl_context* c) {
     c->gc.key.clear();
 }
 
-std::vector<uint64_t> batch_key(rgl_context* c, const rgl_batch* b, const rgl_batch_opts* o, const Launch& L,
-                                const void* d_counts, const void* d_bp) {
+std::vector<uint64_t> batch_key(rgl_context* c, const rgl_batch* b, const rgl_batch_opts* o, const rgl_query_opts& q,
+                                const Launch& L, const void* d_counts, const void* d_bp) {
     std::vector<uint64_t> k;
-    k.reserve(16 + 3ull * b->num_blocks);
+    k.reserve(17 + 3ull * b->num_blocks);
     k.push_back(b->num_rows);
     k.push_back(b->num_blocks);
     k.push_back((uint64_t)(uintptr_t)b->d_intervals);
@@ -2747,6 +2747,8 @@ std::vector<uint64_t> batch_key(rgl_context* c, const rgl_batch* b, const rgl_ba
     k.push_back((uint64_t)(uintptr_t)d_bp);
     k.push_back(((uint64_t)L.chunk << 32) | L.ctas_per_sm);
     k.push_back(((uint64_t)L.pair_ratio << 32) | (o ? o->query.flags : 0));
+    // as asked for: a default is more than the value it stands for (items sized by the run, a cost per run)
+    k.push_back(((uint64_t)q.chunk << 32) | q.pair_ratio);
     k.push_back(o ? o->sub_batch : 0);
     k.push_back(o ? o->region_bits : 0);
     k.push_back(c->ws_sig);
@@ -3039,7 +3041,7 @@ int rgl_query_batch_device(rgl_context* c, const rgl_batch* b, const rgl_batch_o
     std::vector<uint64_t> key;
     bool replay = false;
     if (graph) {
-        key = batch_key(c, b, o, L, d_counts, d_bp);
+        key = batch_key(c, b, o, q, L, d_counts, d_bp);
         replay = c->gc.exec && key == c->gc.key;
     }
     if (!replay) {
@@ -3063,7 +3065,7 @@ int rgl_query_batch_device(rgl_context* c, const rgl_batch* b, const rgl_batch_o
         RGL_CUDA(cudaMemcpy(c->gc.t_off.p, ot.data(), ot.size() * 8, cudaMemcpyHostToDevice));
         RGL_CUDA(cudaMemcpy(c->gc.t_shard.p, sr.data(), sr.size() * 4, cudaMemcpyHostToDevice));
         // the key is taken after the workspace is sized, so that a later reallocation invalidates it
-        key = batch_key(c, b, o, L, d_counts, d_bp);
+        key = batch_key(c, b, o, q, L, d_counts, d_bp);
         RGL_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         int s = enqueue_batch(c, b, P, c->gc.t_off.as<uint64_t>(), c->gc.t_shard.as<uint32_t>(), &q, d_counts, d_bp,
                               false, &launches, o);
