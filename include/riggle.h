@@ -328,13 +328,14 @@ int rgl_query_batch_host(rgl_context* ctx, const rgl_batch* batch, const rgl_int
 
 typedef struct rgl_tune_trial {
     uint32_t chunk, ctas_per_sm, pair_ratio;
-    float sweep_ms; /* best of two runs of the sweep kernels of the largest sub-batch */
+    float sweep_ms; /* best of three runs of the sweep kernels of the largest sub-batch */
 } rgl_tune_trial;
 
-/* Autotuner: times the sweep kernels of the batch's largest sub-batch for pair_ratio in {1,2,4,8}
- * at the default shape, then for work-item size {512..8192} x CTAs per SM {2,3,4,6,8}; stores the
- * fastest shape in the context (used by RGL_BF_TUNED) and returns it in *best.  trials (optional)
- * receives up to max_trials measurements. */
+/* Autotuner: times runs of the batch's largest sub-batch for pair_ratio in {1,2,4,8} at the default
+ * shape (4 being the default, tried as such), then for work-item size {512..8192} x CTAs per SM
+ * {2,3,4,6,8}; stores the shape of the fastest whole run in the context (used by RGL_BF_TUNED) and
+ * returns it in *best, with the values that defaults stand for.  trials (optional) receives up to
+ * max_trials measurements. */
 int rgl_batch_autotune(rgl_context* ctx, const rgl_batch* batch, uint64_t sub_batch, rgl_query_opts* best,
                        rgl_tune_trial* trials, uint32_t max_trials, uint32_t* num_trials);
 

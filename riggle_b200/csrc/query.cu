@@ -3216,8 +3216,12 @@ int rgl_query_batch_host(rgl_context* c, const rgl_batch* b, const rgl_interval*
     return finish(c, L, nullptr);
 }
 
-// Autotuner: times the sweep kernels of the batch's largest sub-batch over a grid of launch shapes
-// (pair_ratio first at the default shape, then work-item size x CTAs per SM) and keeps the fastest.
+// Autotuner: times the batch's largest sub-batch over a grid of launch shapes (pair_ratio first at the default
+// shape, then work-item size x CTAs per SM) and keeps the one whose whole run is the fastest.  Ratio 4 stands for the
+// default, which is tried as such (see by_ranks), as is the default size (item_size): what wins as a default is kept as 0.
+// The sweeps alone do not say which ratio is the fastest, since ranges swept by ranks have their ends sorted and
+// tabled before: by the fastest sweeps 64 files of up to 1e5 intervals against 3.2e6 took 667 us (ratio 1) and 48 of up
+// to 1e6 2,128 (ratio 2), by the fastest run 321 and 1,343, the default's.
 int rgl_batch_autotune(rgl_context* c, const rgl_batch* b, uint64_t sub_batch, rgl_query_opts* best,
                        rgl_tune_trial* trials, uint32_t max_trials, uint32_t* num_trials) {
     clear_error();
@@ -3244,22 +3248,27 @@ int rgl_batch_autotune(rgl_context* c, const rgl_batch* b, uint64_t sub_batch, r
     set_regions(in, batch_region_bits(nullptr, sb.rows));
     const bool was_timing = c->timing;
     *best = rgl_query_opts{};
+    rgl_query_opts keep{};
     uint32_t nt = 0;
-    auto trial = [&](rgl_query_opts q, float* out_ms) -> int {
-        float best_ms = 1e30f;
-        for (int rep = 0; rep < 2; rep++) {
+    auto trial = [&](rgl_query_opts q, float* run_ms) -> int {
+        float sweep_ms = 1e30f;
+        *run_ms = 1e30f;
+        for (int rep = 0; rep < 3; rep++) {
             c->timing = true;
             c->tev_used = 0;
+            RGL_CUDA(cudaEventRecord(c->ev[0], st));
             RGL_TRY(run_pipeline(c, in, &q, c->out_counts.as<uint32_t>(), c->out_bp.as<unsigned long long>(), nullptr));
+            RGL_CUDA(cudaEventRecord(c->ev[2], st));
             RGL_CUDA(cudaStreamSynchronize(st));
             float ms = 0;
             RGL_CUDA(cudaEventElapsedTime(&ms, c->tev[0], c->tev[1]));
             c->tev_used = 0;
-            best_ms = std::min(best_ms, ms);
+            sweep_ms = std::min(sweep_ms, ms);
+            RGL_CUDA(cudaEventElapsedTime(&ms, c->ev[0], c->ev[2]));
+            *run_ms = std::min(*run_ms, ms);
         }
-        *out_ms = best_ms;
         const Launch L = pick_launch(&q);
-        if (trials && nt < max_trials) trials[nt] = rgl_tune_trial{L.chunk, L.ctas_per_sm, L.pair_ratio, best_ms};
+        if (trials && nt < max_trials) trials[nt] = rgl_tune_trial{L.chunk, L.ctas_per_sm, L.pair_ratio, sweep_ms};
         nt++;
         return RGL_OK;
     };
@@ -3269,15 +3278,15 @@ int rgl_batch_autotune(rgl_context* c, const rgl_batch* b, uint64_t sub_batch, r
     float cur_ms = 1e30f;
     for (uint32_t pr : {1u, 2u, 4u, 8u}) {
         rgl_query_opts q = cur;
-        q.pair_ratio = pr;
+        q.pair_ratio = pr == pick_launch(nullptr).pair_ratio ? 0 : pr;
         float ms;
         if ((s = trial(q, &ms)) != RGL_OK) break;
         if (ms < cur_ms) {
             cur_ms = ms;
-            best->pair_ratio = pr;
+            keep = q;
         }
     }
-    cur.pair_ratio = best->pair_ratio;
+    cur = keep;
     for (uint32_t ch : {512u, 1024u, 2048u, 4096u, 8192u}) {
         if (s != RGL_OK) break;
         for (uint32_t ct : {2u, 3u, 4u, 6u, 8u}) {
@@ -3288,20 +3297,15 @@ int rgl_batch_autotune(rgl_context* c, const rgl_batch* b, uint64_t sub_batch, r
             if ((s = trial(q, &ms)) != RGL_OK) break;
             if (ms < cur_ms) {
                 cur_ms = ms;
-                best->chunk = ch;
-                best->ctas_per_sm = ct;
+                keep = q;
             }
         }
     }
     c->timing = was_timing;
     if (s != RGL_OK) return s;
-    const Launch L = pick_launch(best);
-    best->chunk = L.chunk;
-    best->ctas_per_sm = L.ctas_per_sm;
-    best->pair_ratio = L.pair_ratio;
-    best->block = 256;
-    best->flags = 0;
-    c->tuned = *best;
+    const Launch L = pick_launch(&keep);
+    *best = rgl_query_opts{L.chunk, L.ctas_per_sm, 256, 0, L.pair_ratio};  // what a tuned batch reports
+    c->tuned = keep;
     c->has_tuned = true;
     if (num_trials) *num_trials = nt;
     RGL_CUDA(cudaStreamSynchronize(st));

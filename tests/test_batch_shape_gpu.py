@@ -57,3 +57,17 @@ def test_graph_of_a_default_is_not_that_of_its_value(setup, given):
     for key in ("rank_positions", "pair_candidates", "ranges"):
         assert st[key] == plain[key]
     assert _run(ctx, batch, want, graph=True, **out, **given)["graph_replayed"] == 1
+
+
+def test_tuned_shape_is_one_that_was_tried(setup):
+    idx, batch, _, want = setup
+    ctx = rg.Context(idx)
+    by_ratio = {r: _run(ctx, batch, want, pair_ratio=0 if r == 4 else r) for r in (1, 2, 4, 8)}
+    given = _run(ctx, batch, want, pair_ratio=4)
+    assert given["rank_positions"] != by_ratio[4]["rank_positions"]  # the default is not the ratio alone
+    best, trials = ctx.autotune(batch)
+    assert len(trials) == 29
+    st = _run(ctx, batch, want, tuned=True)
+    assert (st["chunk"], st["ctas_per_sm"], st["pair_ratio"]) == (best["chunk"], best["ctas_per_sm"], best["pair_ratio"])
+    for key in ("rank_positions", "pair_candidates"):
+        assert st[key] == by_ratio[best["pair_ratio"]][key]
