@@ -216,7 +216,8 @@ class Context:
                 name = C.c_char_p(k.encode())
                 keep.append(name)
                 name, k = C.cast(name, C.c_void_p).value, 0
-            arr[i] = (name, int(k), 0, n, ivs.__array_interface__["data"][0] if n else 0)
+            # (any number is taken as 32 bits: one that names no shard of the index is passed over, -1 among them)
+            arr[i] = (name, int(k) & 0xFFFFFFFF, 0, n, ivs.__array_interface__["data"][0] if n else 0)
         keep.append(arr)
         return _lib.QueryBatch(int(num_rows), len(shards),
                                C.cast(arr.__array_interface__["data"][0], C.POINTER(_lib.QueryShard)))
