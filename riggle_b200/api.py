@@ -229,12 +229,20 @@ class Context:
         batch = self._batch(shards, num_rows, keep)
         n = C.c_uint64()
         out = [np.empty((0, 8), np.uint32)]
+        failed = []
 
         def place(_, count):  # called once, when the number of pairs is known
-            out[0] = np.empty((count, 8), np.uint32)
-            return out[0].ctypes.data
+            try:
+                out[0] = np.empty((count, 8), np.uint32)
+                return out[0].ctypes.data
+            except BaseException as e:  # no room, or an interrupt: raised once the library has returned
+                failed.append(e)
+                return None
 
-        check(load().rgl_query_pairs_alloc(self._h, C.byref(batch), _lib.PAIR_ALLOC_FN(place), None, C.byref(n)))
+        status = load().rgl_query_pairs_alloc(self._h, C.byref(batch), _lib.PAIR_ALLOC_FN(place), None, C.byref(n))
+        if failed:
+            raise failed[0]
+        check(status)
         return out[0]
 
     def query_batch_device(self, batch, d_counts, d_bp=None, graph=False, tuned=False, sub_batch=0, chunk=0,
