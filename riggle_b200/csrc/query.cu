@@ -1869,6 +1869,9 @@ int size_workspace(rgl_context* c, uint64_t n, uint32_t rows, uint32_t nblk, uin
     // offsets and destinations; shards, rows, ranks), sized here so that no run reallocates them
     RGL_TRY(z.ensure_in(c->bt_off, 3ull * (nblk + 1) * 8 + 8));
     RGL_TRY(z.ensure_in(c->bt_shard, 3ull * (nblk + 1) * 4 + 4));
+    // and of the single-call entry points, whose blocks of several rows are sorted block by block too
+    RGL_TRY(z.ensure_in(c->sort_tab, 2ull * (nblk + 1) * 8));
+    RGL_TRY(z.ensure_in(c->sort_rank, (nblk + 1) * 4ull));
     RGL_TRY(z.ensure_in(c->key_a, n * 8 + 8));
     RGL_TRY(z.ensure_in(c->key_b, n * 8 + 8));
     RGL_TRY(z.ensure_in(c->val_a, n * 4 + 4));
