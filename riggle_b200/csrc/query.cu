@@ -1508,9 +1508,9 @@ __device__ __forceinline__ void pairs_step_dense(const uint64_t* __restrict__ pp
     __syncwarp();  // cntr is reused by the next step
 }
 
-// The same as a call.  Inlined into the one-row sweep, which has 32 registers a thread, it spills; a call in
-// the several-row sweep (40) leaves 16 registers for all that lives across it, and that spilled 148 bytes a
-// thread into the loop: 48 files against 2e8 intervals 4,201 us so, 3,638 inlined.
+// The same as a call.  Inlined into the one-row sweep, which has 32 registers a thread, it spills into the loop; a
+// call in the several-row sweep leaves 16 registers for all that lives across it, and that spilled 148 bytes a thread
+// there: 48 files against 2e8 intervals 4,201 us so (six blocks an SM), 3,638 inlined.
 template <bool WITH_BP, bool SMEM>
 __device__ __noinline__ void pairs_step_dense_call(const uint64_t* __restrict__ ppos, const PairSeg* __restrict__ psegs,
                                                    const uint32_t* __restrict__ prow, const uint2* __restrict__ pos,
@@ -1537,9 +1537,9 @@ __device__ __noinline__ void pairs_step_dense_call(const uint64_t* __restrict__ 
 // run is t plus the number of boundaries at or below it, counted over the few boundaries inside the
 // step, and the run descriptors come from L1.
 // Bound: L1 wavefronts (70% of its cycles: 12 bytes and two shared-memory atomics a candidate) and
-// issue (65%).  64-bit offsets, one register a count and three loads a descriptor spilled in the
-// several-row form: 1.04e9 candidates of 48 files against 2e8 intervals 4,201 us, 3,638 without; five,
-// six, seven, eight blocks an SM: 3,826, 3,638, 3,530, 3,545 (256 files against 3.2e6: 893, 823, 681, 685).
+// issue (65%).  Blocks an SM, 1.04e9 candidates of 48 files against 2e8 intervals and 256 files against 3.2e6,
+// several-row form: five 3,826 and 893 us; six (40 registers, 16 bytes spilled) 3,638 and 823; eight (32 registers, 36
+// bytes spilled, as seven compiles too) 3,530 to 3,545 and 681 to 685.
 // One work item of the pair sweep (positions [item * chunk, (item + 1) * chunk) of the concatenated
 // candidate runs), walked by one warp.
 template <bool WITH_BP, bool SMEM, int MULTI>
@@ -1649,7 +1649,7 @@ __device__ __forceinline__ void pairs_item(const SweepParams& P, uint32_t chunk,
 }
 
 template <bool WITH_BP, bool SMEM, int MULTI>
-__global__ void __launch_bounds__(256, MULTI ? 7 : 8) k_pairs(const __grid_constant__ SweepParams P) {
+__global__ void __launch_bounds__(256, 8) k_pairs(const __grid_constant__ SweepParams P) {
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned long long* s_bp = reinterpret_cast<unsigned long long*>(smem);
     uint32_t* s_cnt = reinterpret_cast<uint32_t*>(smem + (WITH_BP ? (size_t)P.D * 8 : 0));
