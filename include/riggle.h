@@ -192,14 +192,18 @@ typedef struct rgl_query_batch {
     const rgl_query_shard* shards;
 } rgl_query_batch;
 
-/* Launch shape.  0 = default / autotuned. */
+/* Launch shape.  0 = default / autotuned.  A default is more than the value it stands for: see chunk and
+ * pair_ratio. */
 typedef struct rgl_query_opts {
-    uint32_t chunk;       /* positions per work item (default 1024) */
+    uint32_t chunk;       /* positions per work item (default: 1024, 8192 in runs over several rows, or fewer,
+                             down to 128, where that leaves less than four items a warp; a given size is
+                             taken as it is) */
     uint32_t ctas_per_sm; /* persistent CTAs per SM (default 8) */
     uint32_t block;       /* threads per CTA */
     uint32_t flags;       /* RGL_QF_* */
     uint32_t pair_ratio;  /* a candidate range is swept pair by pair when its candidates are at most
-                             pair_ratio x its union size, else by rank differences (default 4) */
+                             pair_ratio x its union size, else by rank differences (default: 4, and 4
+                             candidates more for every query run of the range; a given ratio alone) */
 } rgl_query_opts;
 
 #define RGL_QF_NO_OVERLAP 1u /* skip base-pair accumulation (counts only) */

@@ -308,8 +308,8 @@ uint32_t enqueue_t(uint32_t nblk, const uint64_t* off, uint64_t tiles, uint64_t 
     }
     if (!tiles) return launches;
     // (the sort of keys alone opens the side stream's chain, after an event wait: a plain launch)
-    (void)launch_chain(pdl && VALUES, k_tile_copy<VALUES, true>, k_tile_copy<VALUES, false>, (unsigned)tiles, kBsThreads, 0, st,
-                       nblk, off, tile_pre, unsorted, ka, va, kb, vb);
+    (void)launch_chain(pdl && VALUES, k_tile_copy<VALUES, true>, k_tile_copy<VALUES, false>, (unsigned)tiles,
+                       kBsThreads, 0, st, nblk, off, tile_pre, unsorted, ka, va, kb, vb);
     (void)launch_chain(pdl, k_tile_sort<VALUES, WIDE, true>, k_tile_sort<VALUES, WIDE, false>, (unsigned)tiles,
                        kBsThreads, block_sort_smem<VALUES, WIDE>(), st, nblk, off, tile_pre, unsorted, ka, va, kb, vb, maxp);
     launches += 2;

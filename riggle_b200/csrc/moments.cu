@@ -7,9 +7,11 @@
 //     sequential f32 carry chain (only chunks with a non-zero total change the carry, so the chain
 //     runs over the compacted non-zero totals).  The f32 rounding residues of g move large-window
 //     means by ~1e-4 relative, so any other summation order could not match the reference.
-// K5  centred signal u = g - mean(g) in f64 and its prefix sum U (double-double scan).
-// K6  autocorrelation A[m] = sum_k u[k] u[k+m] by a hand-written Stockham FFT (radix 16/8/4/2
-//     passes, FP64): FFT(u zero-padded to 2^ceil(log2 2N)), |X|^2, FFT again, real part / M.
+// K5  centred signal u = g - mean(g) and its prefix sum U (tile sums, one block over them, a scan in each
+//     tile; sums in double-double, or float-float).
+// K6  autocorrelation A[m] = sum_k u[k] u[k+m] by a hand-written Stockham FFT (passes of radix 16 to 256
+//     through shared memory): FFT(u zero-padded to M = 2^ceil(log2 2N)), |X|^2, FFT again, real part / M, each as a
+//     complex transform of M / 2 packed points.
 // K7  window moments for the L grid of the compact store:
 //       sum_j F_L(j)   = (UU(N+1) - UU(L)) - UU(N-L+1)                    (UU = prefix of U)
 //       sum_j F_L(j)^2 = L A[0] + 2 (L P0(L) - P1(L)) - Q(L-1) - V(L-1)
@@ -18,7 +20,9 @@
 //     linear convolution).  mean(L) = L mean(g) + sum F / n_w, var(L) = sum F^2 / n_w - (sum F /
 //     n_w)^2 in FP64, clamped at 0 as the reference does.  Every term is bounded by the centred
 //     signal, so the cancellation that the reference's d*-autocorrelation suffers (~1e10,
-//     docs/todo.md) does not arise; all prefix sums are double-double (compensated two-sum).
+//     docs/todo.md) does not arise.  The prefix sums are taken at the grid's points only, from sums over
+//     tiles: in double-double over the tiles and for U, in the tiles in double-double, or in float-float for
+//     the other terms of the compensated path.
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
 
@@ -240,9 +244,9 @@ __device__ __forceinline__ DD u_at<double>(const double* U, uint64_t i) { return
 // the available precision", Numer. Math. 18, 1971; Y. Hida, X. S. Li, D. H. Bailey, "Algorithms for
 // quad-double precision floating point arithmetic", ARITH 2001, for the add / mul sequences).  The
 // centred signal is scaled by a power of two per chromosome so that it is O(1) (no denormal lo
-// parts), the FFT, the power spectrum and the prefix sums run in float-float, and FP64 appears only
-// when the per-L results are combined (k_window_moments: the final reduction and the variance
-// subtraction).
+// parts), and the FFT, the power spectrum and the sums inside a tile run in float-float.  FP64 appears in
+// the twiddles (sincospi, split into two floats), in the sums over the tiles and of U (double-double), and
+// when the per-L results are combined (k_window_moments: the final reduction and the variance subtraction).
 struct __align__(8) FF {
     float hi, lo;
 };
@@ -805,7 +809,8 @@ enum Term : int { T_A = 0, T_MA = 1, T_U2 = 2, T_V2 = 3, T_U = 4, kTerms = 5 };
 
 // Adds four terms of element t (0 .. n) to s and the fifth, U[t], to su.  uN = U[n].
 // su is in double-double in both precisions, as are the prefix sums over the tiles: the window mean of a short
-// L is what is left of sums of U a few 1e6 times its size (in 48 bits that was wrong by 4e-10 of it at 2^21 bins; 713 -> 732 us at 2^21 bins in float-float).
+// L is what is left of sums of U a few 1e6 times its size (in 48 bits that was wrong by 4e-10 of it at 2^21
+// bins; 713 -> 732 us there in float-float).
 template <class P>
 __device__ __forceinline__ void add_terms(uint64_t t, uint64_t n, const typename P::S* __restrict__ A,
                                           const typename P::S* __restrict__ U, typename P::S uN,
@@ -1078,8 +1083,8 @@ int depth_signal_dev(MomentWs& w, const rgl_interval* h_iv, uint64_t n, uint64_t
         RGL_CUDA(cub::DeviceSelect::Flagged(w.tmp.p, tb, thrust::counting_iterator<uint32_t>(0), w.nz.as<uint8_t>(),
                                             w.idx.as<uint32_t>(), w.cnt.as<int>(), (int)full, st));
     }
-    k_carry_chain<<<1, kChainThreads, 0, st>>>(w.cnt.as<int>(), w.idx.as<uint32_t>(), w.totals.as<float>(), w.cum.as<float>(),
-                                   w.g.as<float>(), N, full);
+    k_carry_chain<<<1, kChainThreads, 0, st>>>(w.cnt.as<int>(), w.idx.as<uint32_t>(), w.totals.as<float>(),
+                                               w.cum.as<float>(), w.g.as<float>(), N, full);
     if (full)
         k_apply_carry<<<blocks_for(full), 256, 0, st>>>(full, w.cnt.as<int>(), w.idx.as<uint32_t>(), w.cum.as<float>(),
                                                         w.g.as<float>());

@@ -705,10 +705,7 @@ __global__ void __launch_bounds__(kTileThreads) k_lohi(
     }
 }
 
-// Live run c: its query's candidates psegs[c], the candidates before it pc[c], its range cr[c] and uhi[c],
-// the end of the union of its range's runs through it (written only where the run may be its range's last).
-// Range r: rt[r] = (its first live run, that run's entry K n + i).  The last block writes the totals: L, R
-// and pc[L].
+// The partition point of (start < x) alone (see pp_layer2).
 __device__ __forceinline__ uint32_t pp_layer(const uint2* __restrict__ pos, const uint32_t* __restrict__ btab,
                                              const LayerQuery& L, uint32_t x) {
     const uint32_t b = x >> L.bshift;
@@ -746,7 +743,10 @@ __device__ __forceinline__ uint64_t warp_inclusive(uint32_t cnt, uint32_t lane) 
 // or shard and row (shard * rows + row; the pair list).
 enum : int { RUN_PLAIN = 0, RUN_ROW = 1, RUN_SHARD_ROW = 2, RUN_PACKED = 3 };
 
-// A warp takes one of k_lohi's tiles (per_slot of them a slot), 32 live entries at a time.
+// Live run c: its query's candidates psegs[c], the candidates before it pc[c], its range cr[c] and uhi[c],
+// the end of the union of its range's runs through it (written only where the run may be its range's last).
+// Range r: rt[r] = (its first live run, that run's entry K n + i).  The last tile's warp writes the totals: L, R
+// and pc[L].  A warp takes one of k_lohi's tiles (per_slot of them a slot), 32 live entries at a time.
 template <bool PDL>
 __global__ void __launch_bounds__(kTileThreads) k_emit(
     uint32_t n, uint32_t nslots, uint32_t rows, uint32_t per_slot, uint32_t tiles, int tag,
@@ -795,7 +795,8 @@ __global__ void __launch_bounds__(kTileThreads) k_emit(
             const LayerQuery* L = layers + ((uint64_t)sh * nslots + K);
             const uint64_t first = L->off + lo;
             psegs[c] = PairSeg{tag == RUN_PACKED ? first | (uint64_t)row[i] << kRunRowShift : first, qs, qe};
-            if (tag == RUN_ROW || tag == RUN_SHARD_ROW) prow[c] = (rows > 1 ? row[i] : 0u) + (tag == RUN_SHARD_ROW ? sh * rows : 0u);
+            if (tag == RUN_ROW || tag == RUN_SHARD_ROW)
+                prow[c] = (rows > 1 ? row[i] : 0u) + (tag == RUN_SHARD_ROW ? sh * rows : 0u);
             pc[c] = at.cand + inc - cnt;
             const uint32_t r = at.ranges + __popc(fl & ((2u << lane) - 1u)) - 1;  // the range it starts or continues
             cr[c] = r;
@@ -2315,7 +2316,8 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     if (qg) scan_groups(c->sums.as<QSum>(), qt, nullptr, 0, qgs, qg, st);
     (void)launch_chain(pdl, k_q_apply<true>, k_q_apply<false>, qt, kTileThreads, 0, st, n, rows, sps,
                        c->key_b.as<uint64_t>(), c->val_b.as<uint32_t>(), c->sums.as<QSum>(), (int)(qg != 0),
-                       c->starts.as<uint32_t>(), c->shard.as<uint32_t>(), c->row.as<uint32_t>(), c->segnum.as<uint32_t>(), c->seg_begin.as<uint32_t>(),
+                       c->starts.as<uint32_t>(), c->shard.as<uint32_t>(), c->row.as<uint32_t>(),
+                       c->segnum.as<uint32_t>(), c->seg_begin.as<uint32_t>(),
                        c->ps.as<uint64_t>(), c->emax.as<uint32_t>());
     launches += qg ? 4 : 2;
     uint32_t* Lp = d_small + 8;   // live runs L
@@ -2335,7 +2337,8 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     (void)launch_chain(pdl, k_emit<true>, k_emit<false>, grid_for(lt, kTileThreads / 32), kTileThreads, 0, st, n, ns,
                        rows, lgrid.x, lt, tag, c->starts.as<uint32_t>(), c->val_b.as<uint32_t>(),
                        c->emax.as<uint32_t>(), c->shard.as<uint32_t>(), c->row.as<uint32_t>(), idx->d_lq,
-                       idx->d_pos, idx->d_btab, c->lo.as<uint32_t>(), c->cnt.as<uint32_t>(), c->place.as<uint16_t>(), lsums, (int)(lg != 0), c->psegs.as<PairSeg>(),
+                       idx->d_pos, idx->d_btab, c->lo.as<uint32_t>(), c->cnt.as<uint32_t>(), c->place.as<uint16_t>(),
+                       lsums, (int)(lg != 0), c->psegs.as<PairSeg>(),
                        c->prow.as<uint32_t>(), c->pc.as<uint64_t>(), c->cr.as<uint32_t>(), c->uhi.as<uint32_t>(),
                        c->rt.as<uint2>(), c->rlo.as<uint32_t>(), Lp, Rp);
     // the ranges' unions, methods and places; R is a device count, at most tot
@@ -2369,8 +2372,8 @@ int run_pipeline(rgl_context* c, const PipeIn& in, const rgl_query_opts* opts, u
     if (rg) scan_groups(rsums, 0, Rp, kRTile, rgs, rg, st);
     (void)launch_chain(pdl, k_range_apply<true>, k_range_apply<false>, rgrid, kTileThreads, 0, st, Lp, Rp, n, ns, rows,
                        c->rt.as<uint2>(), c->pc.as<uint64_t>(), c->ulen.as<uint32_t>(), c->rlo.as<uint32_t>(),
-                       c->shard.as<uint32_t>(), c->row.as<uint32_t>(), c->segnum.as<uint32_t>(), idx->d_slot, L.pair_ratio, run_cost, rsums,
-                       (int)(rg != 0),
+                       c->shard.as<uint32_t>(), c->row.as<uint32_t>(), c->segnum.as<uint32_t>(), idx->d_slot,
+                       L.pair_ratio, run_cost, rsums, (int)(rg != 0),
                        c->ranges.as<RangeDesc>(), c->rpos.as<uint64_t>(), c->rpair.as<uint64_t>(),
                        c->ppos.as<uint64_t>(), RRp, reinterpret_cast<unsigned long long*>(d_small + 10));
     const unsigned gc = (unsigned)std::min<uint64_t>(grid_for(tot, 256), (uint64_t)c->num_sms * 32);
@@ -2490,8 +2493,9 @@ int resolve_blocks(rgl_context* c, const rgl_query_batch* b, std::vector<uint32_
 
 // Page-locked staging per context, for inputs and outputs of the host entry points.
 constexpr uint64_t kHostIoBytes = 512ull << 10;
-// A copy from pageable memory costs the stream about 4 us whatever its size; staging costs the host
-// about 80 us per MB.  Blocks of less than this on average are staged.
+// Blocks of less than this on average are staged.  24 copies of pageable memory took 3.2, 3.3, 4.0, 5.3, 6.0, 8.9, 13.8 us
+// each at 0.5, 16, 32, 48, 64, 100, 200 KB; gathered into the buffer and sent as one, 20 us and 80 us per MB in all: 27, 46,
+// 70, 101, 141, 207, 390 us against 77, 79, 97, 126, 144, 214, 332.
 constexpr uint64_t kStagePerCopy = 48ull << 10;
 
 // The run's input on the device: the blocks' host intervals at offsets off in the context's interval
@@ -3013,7 +3017,7 @@ int rgl_query_counts(rgl_context* c, const rgl_query_batch* b, const rgl_query_o
     }
     const bool stage = cells && out_bytes <= kHostIoBytes;
     if (stage) {
-            RGL_CUDA(cudaMemcpyAsync(c->h_io, c->out_bp.p, out_bytes, cudaMemcpyDeviceToHost, st));
+        RGL_CUDA(cudaMemcpyAsync(c->h_io, c->out_bp.p, out_bytes, cudaMemcpyDeviceToHost, st));
     } else if (cells) {
         RGL_CUDA(cudaMemcpyAsync(counts, d_counts, cells * 4, cudaMemcpyDeviceToHost, st));
         if (overlap_bp) RGL_CUDA(cudaMemcpyAsync(overlap_bp, d_bp, cells * 8, cudaMemcpyDeviceToHost, st));
@@ -3386,8 +3390,8 @@ int query_pairs(rgl_context* c, const rgl_query_batch* b, uint64_t* out_count, P
     if (!pairs) return RGL_OK;
     RGL_TRY(c->pairs.ensure(hits * sizeof(rgl_pair)));
     k_pair_list<true><<<grid, 256, 0, st>>>(c->ppos.as<uint64_t>(), Lp, c->psegs.as<PairSeg>(),
-                                            c->prow.as<uint32_t>(), b->num_rows, c->idx->d_pos, c->idx->d_sid, items, chunk, nullptr, c->item_base.as<uint64_t>(),
-                                            c->pairs.as<rgl_pair>());
+                                            c->prow.as<uint32_t>(), b->num_rows, c->idx->d_pos, c->idx->d_sid, items,
+                                            chunk, nullptr, c->item_base.as<uint64_t>(), c->pairs.as<rgl_pair>());
     RGL_CUDA(cudaGetLastError());
     RGL_CUDA(cudaMemcpyAsync(pairs, c->pairs.p, hits * sizeof(rgl_pair), cudaMemcpyDeviceToHost, st));
     RGL_CUDA(cudaStreamSynchronize(st));

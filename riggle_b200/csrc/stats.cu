@@ -887,8 +887,8 @@ int rgl_query_pvalues(rgl_moments* m, const rgl_pvalue_batch* b, uint32_t bin_si
         if (walk) s = m->host_part.ensure(pv_scratch_bytes(rows, D, C));
         if (s == RGL_OK)
             s = launch_pvalues(walk, rows, D, C, d_cnt.as<uint32_t>(), d_bp.as<unsigned long long>(), (double)bin_size,
-                               d_off.as<uint64_t>(), d_off.as<uint32_t>(), d_g.as<QGroupDev>(), m->d_mv, d_coff.as<uint64_t>(), m->stride,
-                               m->d_len, d_p.as<double>(), d_llr.as<double>(), d_lp.as<double>(), d_f.as<uint8_t>(),
+                               d_off.as<uint64_t>(), d_off.as<uint32_t>(), d_g.as<QGroupDev>(), m->d_mv,
+                               d_coff.as<uint64_t>(), m->stride, m->d_len, d_p.as<double>(), d_llr.as<double>(), d_lp.as<double>(), d_f.as<uint8_t>(),
                                m->host_part.p, 0);
     }
     auto back = [&](void* dst, const void* src, size_t n) {
